@@ -26,7 +26,7 @@ HcclResult CheckConfig(const HcclMoeConfig &c, uint32_t nranks)
 
 uint32_t Capacity(const HcclMoeConfig &c) { return c.maxRecvRows ? c.maxRecvRows : 2 * c.maxTokens * c.topK; }
 
-MoeLayout MakeLayout(const HcclMoeConfig &c, uint32_t maxCtas)
+MoeLayout MakeLayout(const HcclMoeConfig &c)
 {
     MoeLayout L{};
     const uint64_t cap = Capacity(c), entries = (uint64_t)c.maxTokens * c.topK;
@@ -36,10 +36,7 @@ MoeLayout MakeLayout(const HcclMoeConfig &c, uint32_t maxCtas)
     L.recvSrc = off; off += Al(cap * 4);
     L.yBuf = off; off += Al(cap * c.hidden * 2);
     L.recvCounts = off; off += Al((uint64_t)kMaxExperts * 4);
-    L.pos = off; off += Al(entries * 4);
     L.slotMap = off; off += Al(entries * 8);
-    L.cntCta = off; off += Al((uint64_t)maxCtas * c.numExperts * 4);
-    L.baseSend = off; off += Al((uint64_t)kMaxExperts * 4);
     L.total = off;
     return L;
 }
@@ -51,6 +48,7 @@ struct MoeState {
     void *ws = nullptr;
     uint64_t wsOff = 0;
     uint32_t ctas = 0;
+    bool solo = false;
     uint32_t lastTokens = 0;
 };
 
@@ -71,12 +69,22 @@ MoeArgs MakeArgs(const HcclMoeConfig &cfg, const MoeLayout &L, uint64_t wsOff, u
     return a;
 }
 
-template <bool EMU> HcclResult LaunchMoe(bool dispatch, const DevComm *comms, const MoeArgs &a, const MoeArgs *emuArgs, uint32_t ctas, uint32_t ranksY, cudaStream_t s)
+// solo: a communicator of one rank needs no barrier among CTAs, so the kernel is launched without the cooperative constraint.
+template <bool EMU> HcclResult LaunchMoe(bool dispatch, const DevComm *comms, const MoeArgs &a, const MoeArgs *emuArgs, uint32_t ctas, uint32_t ranksY, cudaStream_t s,
+                                         bool solo = false)
 {
-    const void *fn = dispatch ? (const void *)MoeDispatchKernel<EMU> : (const void *)MoeCombineKernel<EMU>;
     MoeArgs av = a;
     void *params[] = {(void *)&comms, (void *)&av, (void *)&emuArgs};
-    cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(ctas, ranksY), dim3(kMoeThreads), params, 0, s);
+    cudaError_t e;
+    if (!EMU && solo) {
+        const void *fn = dispatch ? (const void *)MoeDispatchKernel<false, true>
+                                  : a.K <= 8 ? (const void *)MoeCombineKernel<false, true, 8> : (const void *)MoeCombineKernel<false, true, 16>;
+        e = cudaLaunchKernel(fn, dim3(ctas), dim3(kMoeThreads), params, 0, s);
+    } else {
+        const void *fn = dispatch ? (const void *)MoeDispatchKernel<EMU, false>
+                                  : a.K <= 8 ? (const void *)MoeCombineKernel<EMU, false, 8> : (const void *)MoeCombineKernel<EMU, false, 16>;
+        e = cudaLaunchCooperativeKernel(fn, dim3(ctas, ranksY), dim3(kMoeThreads), params, 0, s);
+    }
     if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u x %u)", cudaGetErrorString(e), ctas, ranksY); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -101,8 +109,11 @@ HcclResult HcclMoeCreate(HcclComm comm, const HcclMoeConfig *config, HcclMoeHand
     st->cfg = *config;
     // leave SMs for the expert GEMMs of the neighbouring streams; all CTAs must be co-resident (cooperative launch)
     st->ctas = (uint32_t)std::min(SmCountNow(), 64);
+    // one rank: the rows stay in this GPU's memory, 64 SMs do not keep HBM busy and no CTA waits for another
+    st->solo = c->nranks == 1;
+    if (st->solo) st->ctas = (uint32_t)SmCountNow() * 2;
     if (const char *e = getenv("HCCL_MOE_CTAS")) { int v = atoi(e); if (v > 0 && v <= SmCountNow()) st->ctas = (uint32_t)v; }
-    st->L = MakeLayout(*config, st->ctas);
+    st->L = MakeLayout(*config);
     HcclResult r = SymAlloc(c, st->L.total, &st->ws);
     if (r != HCCL_SUCCESS) { delete st; return r; }
     st->wsOff = SymOffsetOf(c, st->ws);
@@ -131,7 +142,7 @@ HcclResult HcclMoeDispatch(HcclMoeHandle handle, const void *x, const int32_t *t
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.x = x;
     a.topkIdx = topkIdx;
-    CHK_RET(LaunchMoe<false>(true, c->devCommPtr, a, nullptr, st->ctas, 1, stream));
+    CHK_RET(LaunchMoe<false>(true, c->devCommPtr, a, nullptr, st->ctas, 1, stream, st->solo));
     st->lastTokens = numTokens;
     c->counters.kernelsLaunched++;
     CountLaunch();
@@ -162,7 +173,7 @@ HcclResult HcclMoeCombine(HcclMoeHandle handle, const float *topkWeights, void *
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.weights = topkWeights;
     a.out = out;
-    CHK_RET(LaunchMoe<false>(false, c->devCommPtr, a, nullptr, st->ctas, 1, stream));
+    CHK_RET(LaunchMoe<false>(false, c->devCommPtr, a, nullptr, st->ctas, 1, stream, st->solo));
     c->counters.kernelsLaunched++;
     CountLaunch();
     c->counters.ops++;
@@ -176,7 +187,7 @@ HcclResult HcclEmuMoeRoundTrip(void *emu, const HcclMoeConfig *config, void **xs
     if (!w || !config || !xs || !idxs || !weights || !outs) return HCCL_E_PTR;
     uint32_t R = (uint32_t)w->nranks;
     CHK_RET(CheckConfig(*config, R));
-    MoeLayout L = MakeLayout(*config, ctasPerRank);
+    MoeLayout L = MakeLayout(*config);
     if (L.total > w->arenaBytes) { HCCL_ERROR("emu arena too small for MoE: need %llu bytes", (unsigned long long)L.total); return HCCL_E_MEMORY; }
     if (sizeof(MoeArgs) * R > 2048 * R) return HCCL_E_INTERNAL;
     std::vector<MoeArgs> args(R);

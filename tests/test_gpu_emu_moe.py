@@ -111,3 +111,42 @@ def test_mxfp8_dispatch_round_trip_matches_the_reference_quantiser(nranks, T, E,
                 # and the format itself stays within e4m3's half-ulp (2^-4) of the block maximum
                 blk = xs[r].float().view(T, H // 32, 32)
                 assert bool(((deq.view(T, H // 32, 32) - blk).abs().amax(2) <= blk.abs().amax(2) * 2.0 ** -4 + 1e-30).all())
+
+
+@pytest.mark.parametrize("T,E,K,H,mxfp8", [(1, 8, 1, 256, False), (3, 60, 6, 1280, False), (700, 256, 8, 512, True), (300, 320, 16, 1024, False), (257, 5, 3, 2304, True)])
+def test_one_rank_layout_and_combine(T, E, K, H, mxfp8):
+    """One rank (no barrier among CTAs): rows sorted by expert, then by token; few and many tokens per CTA, widths that are not whole
+    2 KB pieces, topK 16, the largest expert count."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(T + E)
+        x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+        x[0, :32] = 0
+        idx = torch.stack([torch.randperm(E, generator=g, device="cuda")[:K] if K <= E else torch.zeros(K, device="cuda") for _ in range(T)]).to(torch.int32).contiguous()
+        w = torch.rand(T, K, generator=g, device="cuda")
+        d = MoeDispatcher(comm, E, K, H, T, max_recv_rows=T * K, mxfp8=mxfp8)
+        rx, rs, counts, src = d.dispatch(x, idx)
+        y = torch.randn(T * K, H, generator=g, device="cuda").to(torch.bfloat16)
+        d.expert_out.copy_(y)
+        out = d.combine(w)
+        torch.cuda.synchronize()
+        order = torch.argsort(idx.flatten().long(), stable=True)
+        assert torch.equal(counts.long(), torch.bincount(idx.flatten().long(), minlength=E))
+        assert torch.equal(src.long(), order // K)
+        rows = x[order // K]
+        if mxfp8:
+            val = rx.float().view(T * K, H // 32, 32) * torch.exp2(rs.float() - 127)[..., None]
+            amax = rows.float().view(T * K, H // 32, 32).abs().amax(2, keepdim=True)
+            assert bool(((val - rows.float().view_as(val)).abs() <= amax * 2.0 ** -4).all())     # 3 mantissa bits, no saturation
+        else:
+            assert torch.equal(rx, rows)
+        slot = torch.empty_like(order)
+        slot[order] = torch.arange(T * K, device="cuda")
+        terms = w.double()[..., None] * y[slot.view(T, K)].double()
+        ref = terms.sum(1)
+        assert bool(((out.double() - ref).abs() <= terms.abs().sum(1) * K * 2.0 ** -23 + ref.abs() * 2.0 ** -8).all())
+        d.close()
+    finally:
+        comm.destroy()
