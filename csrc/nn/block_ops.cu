@@ -1,0 +1,449 @@
+// Element-wise parts of a decoder block (RMSNorm, rotary embedding of a packed QKV projection, SwiGLU, vocabulary-parallel cross
+// entropy), forward and backward, bf16 in and out with fp32 arithmetic. All are bound by memory: each reads its inputs once and
+// writes its outputs once, 16 bytes per thread and load, in place of chains of element-wise framework kernels that write every
+// intermediate (most of them in fp32) back to memory. HCCL has no counterpart; the decoder exists for the end-to-end benchmarks.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <math.h>
+#include <algorithm>
+#include "../common/launch_count.h"
+#include "../common/log.h"
+#include "hccl/hccl_nn.h"
+
+namespace hccl {
+namespace nn {
+
+namespace {
+
+constexpr int kThreads = 256;
+
+__device__ __forceinline__ void Unpack8(const uint4 &r, float (&f)[8])
+{
+    const __nv_bfloat162 *h = (const __nv_bfloat162 *)&r;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { const float2 p = __bfloat1622float2(h[j]); f[2 * j] = p.x; f[2 * j + 1] = p.y; }
+}
+__device__ __forceinline__ uint4 Pack8(const float (&f)[8])
+{
+    uint4 o;
+    __nv_bfloat162 t0 = __floats2bfloat162_rn(f[0], f[1]), t1 = __floats2bfloat162_rn(f[2], f[3]);
+    __nv_bfloat162 t2 = __floats2bfloat162_rn(f[4], f[5]), t3 = __floats2bfloat162_rn(f[6], f[7]);
+    o.x = *(uint32_t *)&t0; o.y = *(uint32_t *)&t1; o.z = *(uint32_t *)&t2; o.w = *(uint32_t *)&t3;
+    return o;
+}
+
+// Sum over the TPR threads that share a row: a warp (TPR = 32) or the whole block.
+template <int TPR> __device__ __forceinline__ float RowSum(float v, float *red)
+{
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (TPR == 32) return v;
+    __syncthreads();                                     // red may still be read from the previous sum
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < TPR / 32; ++w) s += red[w];
+    return s;
+}
+
+// y = x * rsqrt(mean(x^2) + eps) * w. A row is shared by TPR threads; the second pass over it hits L1 / L2.
+template <int TPR>
+__global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ y,
+                                                         float *__restrict__ rstd, uint32_t T, uint32_t H, float eps)
+{
+    __shared__ float red[kThreads / 32];
+    const uint32_t row = blockIdx.x * (kThreads / TPR) + threadIdx.x / TPR, lane = threadIdx.x % TPR;
+    if (row >= T) return;                                // whole warps (TPR = 32) or no thread at all (one row per block)
+    const uint4 *xr = (const uint4 *)(x + (size_t)row * H), *wr = (const uint4 *)w;
+    float s = 0.f;
+    for (uint32_t v = lane; v < H / 8; v += TPR) {
+        float f[8];
+        Unpack8(xr[v], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s += f[j] * f[j];
+    }
+    const float r = rsqrtf(RowSum<TPR>(s, red) / (float)H + eps);
+    if (lane == 0) rstd[row] = r;
+    uint4 *yr = (uint4 *)(y + (size_t)row * H);
+    for (uint32_t v = lane; v < H / 8; v += TPR) {
+        float f[8], g[8];
+        Unpack8(xr[v], f);
+        Unpack8(wr[v], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
+        yr[v] = Pack8(f);
+    }
+}
+
+// dx = r * (dy * w - xhat * mean(dy * w * xhat)), xhat = x * r; dw = sum over rows of dy * xhat. A thread owns NV vectors of columns of
+// every row its block walks over (with a stride of the grid): x, dy and w of a row are loaded once and stay in registers between the
+// row sum and the result, and so does the thread's part of dw, which goes to partial[block] at the end. A second kernel adds the
+// blocks in order: the same bits on every run. 2048 x 4096 on one B200: 27.5 us with dw in shared memory and a second load of the row.
+template <int TPR, int NV>
+__global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16 *__restrict__ dy, const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
+                                                            const float *__restrict__ rstd, __nv_bfloat16 *__restrict__ dx, float *__restrict__ partial, uint32_t T,
+                                                            uint32_t H)
+{
+    __shared__ float red[kThreads / 32];
+    constexpr uint32_t kRows = kThreads / TPR;
+    __shared__ float acc[TPR == 32 ? kRows * NV * 256 : 1];   // warps of a block that share the columns: their parts of dw
+    const uint32_t group = threadIdx.x / TPR, lane = threadIdx.x % TPR;
+    uint4 wv[NV];
+    float part[NV][8];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const uint32_t v = lane + i * TPR;
+        wv[i] = v < H / 8 ? ((const uint4 *)w)[v] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) part[i][j] = 0.f;
+    }
+    for (uint32_t row = blockIdx.x * kRows + group; row < T; row += gridDim.x * kRows) {
+        const uint4 *xr = (const uint4 *)(x + (size_t)row * H), *dr = (const uint4 *)(dy + (size_t)row * H);
+        uint4 xv[NV], dv[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const uint32_t v = lane + i * TPR;
+            xv[i] = v < H / 8 ? xr[v] : make_uint4(0, 0, 0, 0);
+            dv[i] = v < H / 8 ? dr[v] : make_uint4(0, 0, 0, 0);
+        }
+        const float r = rstd[row];
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            float f[8], g[8], d[8];
+            Unpack8(xv[i], f);
+            Unpack8(wv[i], g);
+            Unpack8(dv[i], d);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s += d[j] * g[j] * (f[j] * r);
+        }
+        const float m = RowSum<TPR>(s, red) / (float)H;
+        uint4 *o = (uint4 *)(dx + (size_t)row * H);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            float f[8], g[8], d[8];
+            Unpack8(xv[i], f);
+            Unpack8(wv[i], g);
+            Unpack8(dv[i], d);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float xh = f[j] * r;
+                f[j] = r * (d[j] * g[j] - xh * m);
+                part[i][j] += d[j] * xh;
+            }
+            if (lane + i * TPR < H / 8) o[lane + i * TPR] = Pack8(f);
+        }
+    }
+    float *out = partial + (size_t)blockIdx.x * H;
+    if (TPR == kThreads) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const uint32_t v = lane + i * TPR;
+            if (v >= H / 8) continue;
+            ((float4 *)out)[v * 2] = make_float4(part[i][0], part[i][1], part[i][2], part[i][3]);
+            ((float4 *)out)[v * 2 + 1] = make_float4(part[i][4], part[i][5], part[i][6], part[i][7]);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[((group * NV + i) * 8 + j) * 32 + lane] = part[i][j];
+        __syncthreads();
+        for (uint32_t c = threadIdx.x; c < H; c += kThreads) {
+            const uint32_t v = c / 8, at = ((v / 32) * 8 + c % 8) * 32 + v % 32;
+            float s = 0.f;
+            for (uint32_t g = 0; g < kRows; ++g) s += acc[g * NV * 256 + at];
+            out[c] = s;
+        }
+    }
+}
+
+// out[c] = sum over parts of partial[part][c]: 32 columns per block, 8 threads per column, added up in a fixed order.
+__global__ void __launch_bounds__(kThreads) SumPartsKernel(const float *__restrict__ partial, __nv_bfloat16 *__restrict__ out, uint32_t parts, uint32_t H)
+{
+    __shared__ float sm[8][32];
+    const uint32_t c = blockIdx.x * 32 + (threadIdx.x & 31), q = threadIdx.x >> 5;
+    float s = 0.f;
+    if (c < H)
+        for (uint32_t p = q; p < parts; p += 8) s += partial[(size_t)p * H + c];
+    sm[q][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (q == 0 && c < H) {
+        float t = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) t += sm[j][threadIdx.x];
+        out[c] = __float2bfloat16(t);
+    }
+}
+
+// Packed projection [T, (hq + 2 hk) * D] -> rotated q [T, hq, D], rotated k [T, hk, D], v [T, hk, D]; BWD runs the other way with the
+// transposed rotation. A thread takes 8 elements of the first half of a head and the 8 they are paired with in the second half.
+template <bool BWD>
+__global__ void __launch_bounds__(kThreads) RopeQkvKernel(__nv_bfloat16 *__restrict__ qkv, __nv_bfloat16 *__restrict__ q, __nv_bfloat16 *__restrict__ k,
+                                                         __nv_bfloat16 *__restrict__ v, const float *__restrict__ cosT, const float *__restrict__ sinT, uint32_t T,
+                                                         uint32_t seq, uint32_t hq, uint32_t hk, uint32_t D)
+{
+    const uint32_t half = D / 2, perHead = half / 8, heads = hq + 2 * hk, perTok = heads * perHead;
+    const uint64_t idx = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (idx >= (uint64_t)T * perTok) return;
+    const uint32_t t = (uint32_t)(idx / perTok), in = (uint32_t)(idx % perTok), h = in / perHead, j = (in % perHead) * 8;
+    __nv_bfloat16 *pk = qkv + ((size_t)t * heads + h) * D + j;
+    __nv_bfloat16 *un = (h < hq ? q + ((size_t)t * hq + h) * D : h < hq + hk ? k + ((size_t)t * hk + (h - hq)) * D : v + ((size_t)t * hk + (h - hq - hk)) * D) + j;
+    const __nv_bfloat16 *src = BWD ? un : pk;
+    __nv_bfloat16 *dst = BWD ? pk : un;
+    const uint4 r1 = *(const uint4 *)src, r2 = *(const uint4 *)(src + half);
+    if (h >= hq + hk) {
+        *(uint4 *)dst = r1;
+        *(uint4 *)(dst + half) = r2;
+        return;
+    }
+    float a[8], b[8], c[8], s[8];
+    Unpack8(r1, a);
+    Unpack8(r2, b);
+    const size_t at = (size_t)(t % seq) * half + j;
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const float4 cc = *(const float4 *)(cosT + at + 4 * x), ss = *(const float4 *)(sinT + at + 4 * x);
+        c[4 * x] = cc.x; c[4 * x + 1] = cc.y; c[4 * x + 2] = cc.z; c[4 * x + 3] = cc.w;
+        s[4 * x] = ss.x; s[4 * x + 1] = ss.y; s[4 * x + 2] = ss.z; s[4 * x + 3] = ss.w;
+    }
+    float o1[8], o2[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        const float sn = BWD ? -s[x] : s[x];
+        // products rounded before the sum, as the element-wise form does it
+        o1[x] = __fsub_rn(__fmul_rn(a[x], c[x]), __fmul_rn(b[x], sn));
+        o2[x] = __fadd_rn(__fmul_rn(b[x], c[x]), __fmul_rn(a[x], sn));
+    }
+    *(uint4 *)dst = Pack8(o1);
+    *(uint4 *)(dst + half) = Pack8(o2);
+}
+
+// gu = [T, 2F] (gate | up): h = silu(gate) * up. silu is rounded to bf16 before the product, as two separate operations round it: the
+// forward pass keeps the bits of the plain form.
+__global__ void __launch_bounds__(kThreads) SwiGluKernel(const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ h, uint64_t vecs, uint32_t F)
+{
+    const uint64_t idx = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (idx >= vecs) return;
+    const uint32_t per = F / 8;
+    const uint64_t t = idx / per, j = idx % per;
+    const uint4 *row = (const uint4 *)(gu + t * 2 * F);
+    float g[8], u[8];
+    Unpack8(row[j], g);
+    Unpack8(row[per + j], u);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) g[x] = __bfloat162float(__float2bfloat16(g[x] / (1.f + expf(-g[x])))) * u[x];
+    ((uint4 *)h)[idx] = Pack8(g);
+}
+
+__global__ void __launch_bounds__(kThreads) SwiGluBwdKernel(const __nv_bfloat16 *__restrict__ dh, const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ dgu,
+                                                           uint64_t vecs, uint32_t F)
+{
+    const uint64_t idx = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (idx >= vecs) return;
+    const uint32_t per = F / 8;
+    const uint64_t t = idx / per, j = idx % per;
+    const uint4 *row = (const uint4 *)(gu + t * 2 * F);
+    uint4 *out = (uint4 *)(dgu + t * 2 * F);
+    float g[8], u[8], d[8];
+    Unpack8(row[j], g);
+    Unpack8(row[per + j], u);
+    Unpack8(((const uint4 *)dh)[idx], d);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        const float sg = 1.f / (1.f + expf(-g[x])), si = g[x] * sg;
+        const float dg = d[x] * u[x] * sg * (1.f + g[x] * (1.f - sg));
+        u[x] = d[x] * si;
+        g[x] = dg;
+    }
+    out[j] = Pack8(g);
+    out[per + j] = Pack8(u);
+}
+
+// Cross entropy over vocabulary shards, one block per row. STEP 0: row maximum. STEP 1: sum of exp(l - max) and the target's
+// logit - max (0 on ranks that do not own it). STEP 2: gradient. The collectives over the shards run between the steps.
+template <int STEP, bool VEC>
+__global__ void __launch_bounds__(kThreads) XentKernel(const __nv_bfloat16 *__restrict__ logits, const int64_t *__restrict__ targets, int64_t vocabStart, float *__restrict__ mx,
+                                                      float *__restrict__ packed, const float *__restrict__ gOut, __nv_bfloat16 *__restrict__ grad, uint32_t T, uint32_t V)
+{
+    __shared__ float red[kThreads / 32];
+    const uint32_t t = blockIdx.x;
+    const __nv_bfloat16 *row = logits + (size_t)t * V;
+    if (STEP == 0) {
+        float m = -INFINITY;
+        bool nan = false;                                // a NaN logit makes the maximum NaN, as a plain maximum over the row does
+        auto take = [&](float f) { nan |= isnan(f); m = fmaxf(m, f); };
+        if (VEC) {
+            for (uint32_t v = threadIdx.x; v < V / 8; v += kThreads) {
+                float f[8];
+                Unpack8(((const uint4 *)row)[v], f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) take(f[j]);
+            }
+        } else {
+            for (uint32_t v = threadIdx.x; v < V; v += kThreads) take(__bfloat162float(row[v]));
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+        const int anyNan = __syncthreads_or(nan ? 1 : 0);
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kThreads / 32; ++w) m = fmaxf(m, red[w]);
+            mx[t] = anyNan ? NAN : m;
+        }
+        return;
+    }
+    const float m = mx[t];
+    const int64_t target = targets[t] - vocabStart;
+    if (STEP == 1) {
+        float s = 0.f;
+        if (VEC) {
+            for (uint32_t v = threadIdx.x; v < V / 8; v += kThreads) {
+                float f[8];
+                Unpack8(((const uint4 *)row)[v], f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) s += expf(f[j] - m);
+            }
+        } else {
+            for (uint32_t v = threadIdx.x; v < V; v += kThreads) s += expf(__bfloat162float(row[v]) - m);
+        }
+        s = RowSum<kThreads>(s, red);
+        if (threadIdx.x == 0) {
+            packed[t] = s;
+            packed[T + t] = target >= 0 && target < (int64_t)V ? __bfloat162float(row[target]) - m : 0.f;
+        }
+        return;
+    }
+    const float denom = packed[t], scale = gOut[0] / (float)T;
+    __nv_bfloat16 *out = grad + (size_t)t * V;
+    if (VEC) {
+        for (uint32_t v = threadIdx.x; v < V / 8; v += kThreads) {
+            float f[8];
+            Unpack8(((const uint4 *)row)[v], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = (expf(f[j] - m) / denom - ((int64_t)(v * 8 + j) == target ? 1.f : 0.f)) * scale;
+            ((uint4 *)out)[v] = Pack8(f);
+        }
+    } else {
+        for (uint32_t v = threadIdx.x; v < V; v += kThreads)
+            out[v] = __float2bfloat16((expf(__bfloat162float(row[v]) - m) / denom - ((int64_t)v == target ? 1.f : 0.f)) * scale);
+    }
+}
+
+bool Aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
+
+HcclResult Launched(const char *what)
+{
+    CountLaunch();
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { HCCL_ERROR("%s launch failed: %s", what, cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    return HCCL_SUCCESS;
+}
+
+int Sms()
+{
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+}
+
+constexpr uint64_t kWarpRowMax = 1024;     // rows up to this wide are handled by a warp, wider ones by a block
+constexpr uint64_t kNormMax = 12288;       // widest row: six vectors per thread of a block
+
+template <int TPR, int NV>
+void LaunchRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, float *partial, uint32_t T, uint32_t H, uint32_t parts, cudaStream_t s)
+{
+    RmsNormBwdKernel<TPR, NV><<<parts, kThreads, 0, s>>>((const __nv_bfloat16 *)dy, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, rstd, (__nv_bfloat16 *)dx, partial, T, H);
+}
+
+bool NormShapeOk(uint64_t T, uint64_t H) { return T > 0 && T <= 0x7fffffff && H > 0 && H % 8 == 0 && H <= kNormMax; }
+
+}  // namespace
+}  // namespace nn
+}  // namespace hccl
+
+using namespace hccl;
+using namespace hccl::nn;
+
+extern "C" {
+
+HcclResult HcclRmsNorm(const void *x, const void *w, void *y, float *rstd, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
+{
+    if (!x || !w || !y || !rstd) return HCCL_E_PTR;
+    if (!NormShapeOk(rows, hidden) || !Aligned16(x) || !Aligned16(w) || !Aligned16(y)) return HCCL_E_PARA;
+    const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden;
+    if (hidden <= kWarpRowMax)
+        RmsNormKernel<32><<<(T + 7) / 8, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, T, H, eps);
+    else RmsNormKernel<kThreads><<<T, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, T, H, eps);
+    return Launched("RMSNorm");
+}
+
+uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden)
+{
+    const uint64_t perBlock = hidden <= kWarpRowMax ? kThreads / 32 : 1;
+    return std::min<uint64_t>((rows + perBlock - 1) / perBlock, (uint64_t)Sms() * 3);
+}
+
+HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, void *dw, float *partial, uint64_t rows, uint64_t hidden,
+                          cudaStream_t stream)
+{
+    if (!dy || !x || !w || !rstd || !dx || !dw || !partial) return HCCL_E_PTR;
+    if (!NormShapeOk(rows, hidden) || !Aligned16(dy) || !Aligned16(x) || !Aligned16(w) || !Aligned16(dx)) return HCCL_E_PARA;
+    const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden, parts = (uint32_t)HcclRmsNormBwdParts(rows, hidden);
+    auto launch = [&](auto kern) { kern(dy, x, w, rstd, dx, partial, T, H, parts, stream); };
+    const uint32_t nv = (H / 8 + (hidden <= kWarpRowMax ? 31 : kThreads - 1)) / (hidden <= kWarpRowMax ? 32 : kThreads);
+    if (hidden <= kWarpRowMax) launch(nv == 1 ? LaunchRmsNormBwd<32, 1> : nv == 2 ? LaunchRmsNormBwd<32, 2> : LaunchRmsNormBwd<32, 4>);
+    else launch(nv == 1 ? LaunchRmsNormBwd<kThreads, 1> : nv == 2 ? LaunchRmsNormBwd<kThreads, 2> : nv <= 4 ? LaunchRmsNormBwd<kThreads, 4> : LaunchRmsNormBwd<kThreads, 6>);
+    CHK_RET(Launched("RMSNorm backward"));
+    SumPartsKernel<<<(H + 31) / 32, kThreads, 0, stream>>>(partial, (__nv_bfloat16 *)dw, parts, H);
+    return Launched("RMSNorm weight gradient");
+}
+
+HcclResult HcclRopeQkv(void *qkv, void *q, void *k, void *v, const float *cosT, const float *sinT, uint64_t tokens, uint64_t seq, uint32_t qHeads, uint32_t kvHeads,
+                       uint32_t headDim, int backward, cudaStream_t stream)
+{
+    if (!qkv || !q || !k || !v || !cosT || !sinT) return HCCL_E_PTR;
+    if (tokens == 0 || tokens > 0x7fffffff || seq == 0 || seq > tokens || qHeads == 0 || kvHeads == 0 || headDim == 0 || headDim % 16) return HCCL_E_PARA;
+    if (!Aligned16(qkv) || !Aligned16(q) || !Aligned16(k) || !Aligned16(v) || !Aligned16(cosT) || !Aligned16(sinT)) return HCCL_E_PARA;
+    const uint64_t items = tokens * (qHeads + 2 * kvHeads) * (headDim / 16), blocks = (items + kThreads - 1) / kThreads;
+    if (blocks > 0x7fffffff) return HCCL_E_PARA;
+    auto kern = backward ? RopeQkvKernel<true> : RopeQkvKernel<false>;
+    kern<<<(uint32_t)blocks, kThreads, 0, stream>>>((__nv_bfloat16 *)qkv, (__nv_bfloat16 *)q, (__nv_bfloat16 *)k, (__nv_bfloat16 *)v, cosT, sinT, (uint32_t)tokens, (uint32_t)seq,
+                                                   qHeads, kvHeads, headDim);
+    return Launched("rotary embedding");
+}
+
+HcclResult HcclSwiGlu(const void *gateUp, void *h, uint64_t rows, uint64_t ffn, cudaStream_t stream)
+{
+    if (!gateUp || !h) return HCCL_E_PTR;
+    const uint64_t vecs = rows * (ffn / 8), blocks = (vecs + kThreads - 1) / kThreads;
+    if (rows == 0 || ffn == 0 || ffn % 8 || ffn > 0x7fffffff || blocks > 0x7fffffff || !Aligned16(gateUp) || !Aligned16(h)) return HCCL_E_PARA;
+    SwiGluKernel<<<(uint32_t)blocks, kThreads, 0, stream>>>((const __nv_bfloat16 *)gateUp, (__nv_bfloat16 *)h, vecs, (uint32_t)ffn);
+    return Launched("SwiGLU");
+}
+
+HcclResult HcclSwiGluBwd(const void *dh, const void *gateUp, void *dGateUp, uint64_t rows, uint64_t ffn, cudaStream_t stream)
+{
+    if (!dh || !gateUp || !dGateUp) return HCCL_E_PTR;
+    const uint64_t vecs = rows * (ffn / 8), blocks = (vecs + kThreads - 1) / kThreads;
+    if (rows == 0 || ffn == 0 || ffn % 8 || ffn > 0x7fffffff || blocks > 0x7fffffff || !Aligned16(dh) || !Aligned16(gateUp) || !Aligned16(dGateUp)) return HCCL_E_PARA;
+    SwiGluBwdKernel<<<(uint32_t)blocks, kThreads, 0, stream>>>((const __nv_bfloat16 *)dh, (const __nv_bfloat16 *)gateUp, (__nv_bfloat16 *)dGateUp, vecs, (uint32_t)ffn);
+    return Launched("SwiGLU backward");
+}
+
+HcclResult HcclXent(int step, const void *logits, const int64_t *targets, int64_t vocabStart, float *rowMax, float *packed, const float *gradOut, void *grad, uint64_t rows,
+                    uint64_t vocab, cudaStream_t stream)
+{
+    if (!logits || !rowMax || (step > 0 && (!targets || !packed)) || (step == 2 && (!gradOut || !grad))) return HCCL_E_PTR;
+    if (step < 0 || step > 2 || rows == 0 || rows > 0x7fffffff || vocab == 0 || vocab > 0x7fffffff) return HCCL_E_PARA;
+    const bool vec = vocab % 8 == 0 && Aligned16(logits) && (step != 2 || Aligned16(grad));
+    auto kern = step == 0 ? (vec ? XentKernel<0, true> : XentKernel<0, false>) : step == 1 ? (vec ? XentKernel<1, true> : XentKernel<1, false>)
+                                                                                         : (vec ? XentKernel<2, true> : XentKernel<2, false>);
+    kern<<<(uint32_t)rows, kThreads, 0, stream>>>((const __nv_bfloat16 *)logits, targets, vocabStart, rowMax, packed, gradOut, (__nv_bfloat16 *)grad, (uint32_t)rows,
+                                                 (uint32_t)vocab);
+    return Launched("cross entropy");
+}
+
+}  // extern "C"

@@ -18,6 +18,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from ..ops import block as _block
 from ..parallel.tensor_parallel import ColumnParallelLinear, RowParallelLinear, TensorParallelMLP
 
 
@@ -63,9 +64,13 @@ class RMSNorm(nn.Module):
         self.weight.replicated_under_sequence_parallel = True
 
     def forward(self, x):
+        y = _block.rms_norm(x, self.weight, self.eps, self._plain)
+        return self._plain(x, self.weight) if y is None else y
+
+    def _plain(self, x, w):
         v = x.float()
         v = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)
-        return (v * self.weight.float()).to(x.dtype)
+        return (v * w.float()).to(x.dtype)
 
 
 def _rope_tables(seq: int, head_dim: int, theta: float, device):
@@ -106,13 +111,18 @@ class Attention(nn.Module):
 
     def forward(self, x_local, batch: int, seq: int, cos, sin):
         qkv = self.qkv(x_local)                                            # [B*S, (hl + 2 kvl) * hd]
-        q, k, v = qkv.split([self.h_local * self.hd, self.kv_local * self.hd, self.kv_local * self.hd], dim=-1)
-        q = _apply_rope(q.reshape(batch, seq, self.h_local, self.hd), cos, sin).transpose(1, 2)
-        k = _apply_rope(k.reshape(batch, seq, self.kv_local, self.hd), cos, sin).transpose(1, 2)
-        v = v.reshape(batch, seq, self.kv_local, self.hd).transpose(1, 2)
+        plain = lambda t: self._rotated(t, batch, seq, cos, sin)
+        out = _block.rope_qkv(qkv, cos, sin, batch, self.h_local, self.kv_local, self.hd, plain)
+        q, k, v = (t.transpose(1, 2) for t in (plain(qkv) if out is None else out))
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.h_local != self.kv_local)
         o = o.transpose(1, 2).reshape(batch * seq, self.h_local * self.hd)
         return self.out(o)                                                  # [B*S / tp, hidden]
+
+    def _rotated(self, qkv, batch, seq, cos, sin):
+        q, k, v = qkv.split([self.h_local * self.hd, self.kv_local * self.hd, self.kv_local * self.hd], dim=-1)
+        q = _apply_rope(q.reshape(batch, seq, self.h_local, self.hd), cos, sin)
+        k = _apply_rope(k.reshape(batch, seq, self.kv_local, self.hd), cos, sin)
+        return q, k, v.reshape(batch, seq, self.kv_local, self.hd)
 
 
 class Block(nn.Module):
@@ -135,27 +145,41 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits_local, targets, comm, vocab_start):
         from ..types import ReduceOp
-        lf = logits_local.float()
-        mx = lf.max(dim=-1).values.contiguous()
+        vloc = logits_local.shape[-1]
+        ctx.fused = _block.xent_usable(logits_local, targets)
+        if ctx.fused:
+            mx = _block.xent_row_max(logits_local)
+        else:
+            lf = logits_local.float()
+            mx = lf.max(dim=-1).values.contiguous()
         if comm.size > 1:
             comm.all_reduce(mx, op=ReduceOp.MAX)
             _sync(comm, mx)
-        ex = (lf - mx[:, None]).exp()
-        vloc = logits_local.shape[-1]
-        mine = (targets >= vocab_start) & (targets < vocab_start + vloc)
-        idx = (targets - vocab_start).clamp(0, vloc - 1)
-        tgt = torch.where(mine, lf.gather(1, idx[:, None])[:, 0] - mx, torch.zeros_like(mx))
-        packed = torch.stack([ex.sum(-1), tgt]).contiguous()
+        if ctx.fused:
+            packed = _block.xent_sums(logits_local, targets, vocab_start, mx)
+        else:
+            ex = (lf - mx[:, None]).exp()
+            mine = (targets >= vocab_start) & (targets < vocab_start + vloc)
+            idx = (targets - vocab_start).clamp(0, vloc - 1)
+            tgt = torch.where(mine, lf.gather(1, idx[:, None])[:, 0] - mx, torch.zeros_like(mx))
+            packed = torch.stack([ex.sum(-1), tgt]).contiguous()
         if comm.size > 1:
             comm.all_reduce(packed)
             _sync(comm, packed)
         denom, tgt = packed[0], packed[1]
         loss = (denom.log() - tgt).mean()
-        ctx.save_for_backward(ex / denom[:, None], mine, idx)
+        if ctx.fused:
+            ctx.vocab_start = vocab_start
+            ctx.save_for_backward(logits_local, targets, mx, packed)
+        else:
+            ctx.save_for_backward(ex / denom[:, None], mine, idx)
         return loss
 
     @staticmethod
     def backward(ctx, g):
+        if ctx.fused:
+            logits, targets, mx, packed = ctx.saved_tensors
+            return _block.xent_grad(logits, targets, ctx.vocab_start, mx, packed, g.float()), None, None, None
         p, mine, idx = ctx.saved_tensors
         grad = p.clone()
         grad[torch.arange(p.shape[0], device=p.device)[mine], idx[mine]] -= 1.0

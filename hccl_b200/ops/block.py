@@ -1,0 +1,190 @@
+"""Element-wise parts of a decoder block on one kernel each (include/hccl/hccl_nn.h): RMSNorm, rotary embedding of a packed
+QKV projection, SwiGLU, vocabulary-parallel cross entropy.
+
+Each function returns None where its kernel does not apply (another type or device, odd sizes, an active function transform,
+tracing or dispatch mode) and the caller keeps its plain PyTorch form; the same plain form computes the gradient of a
+gradient.
+"""
+from __future__ import annotations
+
+import ctypes
+from typing import Callable, Optional
+
+import torch
+
+from .._lib import check, lib
+
+
+def _decl():
+    l = lib()
+    if not getattr(l, "_nn_declared", False):
+        vp, u32, u64, i32, i64, f32 = ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int, ctypes.c_int64, ctypes.c_float
+        l.HcclRmsNorm.argtypes = [vp, vp, vp, vp, u64, u64, f32, vp]
+        l.HcclRmsNormBwdParts.argtypes = [u64, u64]
+        l.HcclRmsNormBwdParts.restype = u64
+        l.HcclRmsNormBwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, u64, u64, vp]
+        l.HcclRopeQkv.argtypes = [vp, vp, vp, vp, vp, vp, u64, u64, u32, u32, u32, i32, vp]
+        l.HcclSwiGlu.argtypes = [vp, vp, u64, u64, vp]
+        l.HcclSwiGluBwd.argtypes = [vp, vp, vp, u64, u64, vp]
+        l.HcclXent.argtypes = [i32, vp, vp, i64, vp, vp, vp, vp, u64, u64, vp]
+        for f in (l.HcclRmsNorm, l.HcclRmsNormBwd, l.HcclRopeQkv, l.HcclSwiGlu, l.HcclSwiGluBwd, l.HcclXent):
+            f.restype = ctypes.c_int
+        l._nn_declared = True
+    return l
+
+
+def _stream(t: torch.Tensor) -> int:
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
+
+
+def _usable(*ts: torch.Tensor) -> bool:
+    """Plain bf16 tensors on the current GPU, contiguous and 16-byte aligned, and nothing that has to see the single operations."""
+    if (torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() or torch.autograd.forward_ad._current_level >= 0
+            or torch.compiler.is_compiling() or torch.jit.is_tracing()):
+        return False
+    dev = ts[0].device
+    if dev.type != "cuda" or dev.index != torch.cuda.current_device():
+        return False
+    for t in ts:
+        if type(t) not in (torch.Tensor, torch.nn.Parameter) or t.dtype != torch.bfloat16 or t.device != dev or not t.is_contiguous() or t.numel() == 0 \
+                or t.data_ptr() % 16:
+            return False
+    return True
+
+
+def _second_order(plain: Callable, inputs, grads):
+    """Gradients of `plain(*inputs)` as a differentiable function of inputs and grads (backward with create_graph)."""
+    wanted = [t for t in inputs if t.requires_grad]
+    with torch.enable_grad():
+        got = iter(torch.autograd.grad(plain(*inputs), wanted, grads, create_graph=True))
+    return [next(got) if t.requires_grad else None for t in inputs]
+
+
+class _RmsNorm(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w, eps, plain):
+        h = x.shape[-1]
+        y = torch.empty_like(x)
+        rstd = torch.empty(x.numel() // h, dtype=torch.float32, device=x.device)
+        check(_decl().HcclRmsNorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), rstd.numel(), h, eps, _stream(x)), "HcclRmsNorm")
+        ctx.save_for_backward(x, w, rstd)
+        ctx.plain = plain
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w, rstd = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return (*_second_order(ctx.plain, (x, w), dy), None, None)
+        h, rows = x.shape[-1], rstd.numel()
+        dy = _aligned(dy)
+        dx, dw = torch.empty_like(x), torch.empty_like(w)
+        l = _decl()
+        partial = torch.empty(l.HcclRmsNormBwdParts(rows, h), h, dtype=torch.float32, device=x.device)
+        check(l.HcclRmsNormBwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), dw.data_ptr(), partial.data_ptr(), rows, h, _stream(x)),
+              "HcclRmsNormBwd")
+        return dx, dw, None, None
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
+def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> Optional[torch.Tensor]:
+    """x * rsqrt(mean(x^2) + eps) * w over the last dimension; `plain(x, w)` is the same in PyTorch."""
+    h = x.shape[-1] if x.dim() else 0
+    if h % 8 or h > 12288 or w.shape != (h,) or not _usable(x, w):
+        return None
+    return _RmsNorm.apply(x, w, eps, plain)
+
+
+class _RopeQkv(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, heads, kv_heads, head_dim, plain):
+        t, seq = qkv.shape[0], cos.shape[0]
+        q = torch.empty(t // seq, seq, heads, head_dim, dtype=qkv.dtype, device=qkv.device)
+        k = torch.empty(t // seq, seq, kv_heads, head_dim, dtype=qkv.dtype, device=qkv.device)
+        v = torch.empty_like(k)
+        check(_decl().HcclRopeQkv(qkv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), t, seq, heads, kv_heads, head_dim, 0,
+                                  _stream(qkv)), "HcclRopeQkv")
+        ctx.save_for_backward(qkv, cos, sin)
+        ctx.dims, ctx.plain = (heads, kv_heads, head_dim), plain
+        return q, k, v
+
+    @staticmethod
+    def backward(ctx, dq, dk, dv):
+        qkv, cos, sin = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return (*_second_order(ctx.plain, (qkv,), (dq, dk, dv)), None, None, None, None, None, None)
+        dq, dk, dv = _aligned(dq), _aligned(dk), _aligned(dv)
+        out = torch.empty_like(qkv)
+        check(_decl().HcclRopeQkv(out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cos.data_ptr(), sin.data_ptr(), qkv.shape[0], cos.shape[0], *ctx.dims, 1,
+                                  _stream(out)), "HcclRopeQkv")
+        return out, None, None, None, None, None, None
+
+
+def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable):
+    """Packed [batch * seq, (heads + 2 kv_heads) * head_dim] -> rotated q, k and v as [batch, seq, heads, head_dim]; cos / sin are fp32
+    [seq, head_dim / 2] constants. `plain(qkv)` is the same in PyTorch."""
+    seq = cos.shape[0]
+    if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or not _usable(qkv):
+        return None
+    for t in (cos, sin):
+        if type(t) is not torch.Tensor or t.dtype != torch.float32 or t.device != qkv.device or t.shape != (seq, head_dim // 2) or not t.is_contiguous() \
+                or t.requires_grad or t.data_ptr() % 16:
+            return None
+    return _RopeQkv.apply(qkv, cos, sin, heads, kv_heads, head_dim, plain)
+
+
+class _SwiGlu(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, gu, plain):
+        t, f = gu.shape[0], gu.shape[1] // 2
+        h = torch.empty(t, f, dtype=gu.dtype, device=gu.device)
+        check(_decl().HcclSwiGlu(gu.data_ptr(), h.data_ptr(), t, f, _stream(gu)), "HcclSwiGlu")
+        ctx.save_for_backward(gu)
+        ctx.plain = plain
+        return h
+
+    @staticmethod
+    def backward(ctx, dh):
+        gu, = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            return (*_second_order(ctx.plain, (gu,), dh), None)
+        dh = _aligned(dh)
+        out = torch.empty_like(gu)
+        check(_decl().HcclSwiGluBwd(dh.data_ptr(), gu.data_ptr(), out.data_ptr(), gu.shape[0], gu.shape[1] // 2, _stream(gu)), "HcclSwiGluBwd")
+        return out, None
+
+
+def swiglu(gu: torch.Tensor, plain: Callable) -> Optional[torch.Tensor]:
+    """silu(gate) * up for gu = [rows, gate | up]; `plain(gu)` is the same in PyTorch."""
+    if gu.dim() != 2 or gu.shape[1] % 16 or not _usable(gu):
+        return None
+    return _SwiGlu.apply(gu, plain)
+
+
+def xent_usable(logits: torch.Tensor, targets: torch.Tensor) -> bool:
+    return logits.dim() == 2 and _usable(logits) and targets.dtype == torch.int64 and targets.device == logits.device and targets.is_contiguous() \
+        and targets.shape == logits.shape[:1]
+
+
+def xent_row_max(logits: torch.Tensor) -> torch.Tensor:
+    mx = torch.empty(logits.shape[0], dtype=torch.float32, device=logits.device)
+    check(_decl().HcclXent(0, logits.data_ptr(), None, 0, mx.data_ptr(), None, None, None, *logits.shape, _stream(logits)), "HcclXent")
+    return mx
+
+
+def xent_sums(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, mx: torch.Tensor) -> torch.Tensor:
+    """[2, rows]: sum of exp(logit - max) over this shard, the target's logit - max (0 where another shard owns it)."""
+    packed = torch.empty(2, logits.shape[0], dtype=torch.float32, device=logits.device)
+    check(_decl().HcclXent(1, logits.data_ptr(), targets.data_ptr(), vocab_start, mx.data_ptr(), packed.data_ptr(), None, None, *logits.shape, _stream(logits)), "HcclXent")
+    return packed
+
+
+def xent_grad(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, mx: torch.Tensor, packed: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
+    out = torch.empty_like(logits)
+    check(_decl().HcclXent(2, logits.data_ptr(), targets.data_ptr(), vocab_start, mx.data_ptr(), packed.data_ptr(), g.data_ptr(), out.data_ptr(), *logits.shape,
+                           _stream(logits)), "HcclXent")
+    return out

@@ -18,6 +18,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
+from ..ops import block as _block
 from ..ops import gemm as _gemm
 from ..ops import mc2 as _mc2
 
@@ -251,5 +252,9 @@ class TensorParallelMLP(nn.Module):
 
     def forward(self, x_local):
         gu = self.gate_up(x_local)
+        h = _block.swiglu(gu, self._plain)
+        return self.down(self._plain(gu) if h is None else h)
+
+    def _plain(self, gu):
         g, u = gu[:, : self.ffn_local], gu[:, self.ffn_local:]
-        return self.down(torch.nn.functional.silu(g) * u)
+        return torch.nn.functional.silu(g) * u

@@ -1,0 +1,38 @@
+/* Element-wise parts of a decoder block on one GPU: bf16 in and out, fp32 arithmetic. Matrices are row-major and contiguous,
+ * pointers 16-byte aligned. The Python models call these between the fused matmul + collective operators. */
+#ifndef HCCL_NN_H_
+#define HCCL_NN_H_
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include "hccl_types.h"
+
+#ifdef __cplusplus
+extern "C" {
+#endif
+
+/* y[rows, hidden] = x * rsqrt(mean(x^2) + eps) * w; rstd[rows] receives the reciprocal norms for the backward pass.
+ * hidden: a multiple of 8, at most 12288. */
+HcclResult HcclRmsNorm(const void *x, const void *w, void *y, float *rstd, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
+/* Rows of the fp32 workspace `partial` [parts, hidden] that HcclRmsNormBwd needs. */
+uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden);
+HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, void *dw, float *partial, uint64_t rows, uint64_t hidden,
+                          cudaStream_t stream);
+/* qkv[tokens, (qHeads + 2 kvHeads) * headDim] -> q, k rotated (pairs are element j and j + headDim / 2) and v, each
+ * [tokens, heads, headDim]; cos / sin: fp32 [seq, headDim / 2], token t takes row t % seq. headDim: a multiple of 16.
+ * backward != 0: gradients of q, k, v -> gradient of qkv. */
+HcclResult HcclRopeQkv(void *qkv, void *q, void *k, void *v, const float *cosT, const float *sinT, uint64_t tokens, uint64_t seq, uint32_t qHeads, uint32_t kvHeads,
+                       uint32_t headDim, int backward, cudaStream_t stream);
+/* h[rows, ffn] = silu(gate) * up with gateUp[rows, 2 ffn] = [gate | up]. ffn: a multiple of 8. */
+HcclResult HcclSwiGlu(const void *gateUp, void *h, uint64_t rows, uint64_t ffn, cudaStream_t stream);
+HcclResult HcclSwiGluBwd(const void *dh, const void *gateUp, void *dGateUp, uint64_t rows, uint64_t ffn, cudaStream_t stream);
+/* Cross entropy over a vocabulary shard. step 0: rowMax[rows]. step 1: packed[0][rows] = sum exp(logit - rowMax), packed[1][rows] =
+ * target logit - rowMax, 0 where the target lies outside [vocabStart, vocabStart + vocab). step 2: grad = (exp(logit - rowMax) /
+ * packed[0] - onehot(target)) * gradOut[0] / rows. The maxima and sums over the shards are the caller's, between the steps. */
+HcclResult HcclXent(int step, const void *logits, const int64_t *targets, int64_t vocabStart, float *rowMax, float *packed, const float *gradOut, void *grad, uint64_t rows,
+                    uint64_t vocab, cudaStream_t stream);
+
+#ifdef __cplusplus
+}
+#endif
+#endif
