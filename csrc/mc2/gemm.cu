@@ -42,7 +42,7 @@ HcclResult EncodeTmap2D(CUtensorMap *out, const void *base, uint64_t rows, uint6
     cuuint64_t strides[1] = {pitchBytes};
     cuuint32_t box[2] = {boxCols, boxRows};
     cuuint32_t estr[2] = {1, 1};
-    CUtensorMapDataType dt = elemBytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+    CUtensorMapDataType dt = elemBytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : elemBytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
     CUresult r = enc(out, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { HCCL_ERROR("cuTensorMapEncodeTiled failed: %d", (int)r); return HCCL_E_DRV; }
@@ -62,6 +62,12 @@ HcclResult EncodeTmapSf(CUtensorMap *out, const void *scales, uint64_t atoms)
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { HCCL_ERROR("cuTensorMapEncodeTiled (scale atoms) failed: %d", (int)r); return HCCL_E_DRV; }
     return HCCL_SUCCESS;
+}
+
+HcclResult EncodeTmapC(CUtensorMap *out, void *c, uint64_t M, uint64_t N, bool fp32)
+{
+    const uint32_t elem = fp32 ? 4 : 2;
+    return EncodeTmap2D(out, c, M, N, N * elem, 128, 128 / elem, elem);
 }
 
 uint32_t *GemmErrorWord()
@@ -127,6 +133,7 @@ template <int BN> static HcclResult LaunchPlain(const void *a, const void *b, vo
     GemmParams p{};
     CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * 2, kBM, kBK, 2));
     CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * 2, BN, kBK, 2));
+    CHK_RET(EncodeTmapC(&p.tmapC, c, M, N, outFp32));
     p.C = c; p.M = M; p.N = N; p.K = K; p.ldc = N; p.outFp32 = outFp32; p.groupM = GroupMOverride(16); p.errorWord = GemmErrorWord(); p.waitSleepNs = GemmWaitSleepNs();
     using S = GemmSmem<BN>;
     static std::atomic<bool> attrSet{false};
@@ -146,12 +153,14 @@ template <int BN> static HcclResult LaunchPlain(const void *a, const void *b, vo
 }
 
 // 256 x 256 tiles on CTA pairs (cta_group::2). Needs an even grid; one cluster of two CTAs per tile.
-template <int BN> static HcclResult LaunchPlain2CtaT(const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
+template <int BN>
+static HcclResult LaunchPlain2CtaT(const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
 {
     GemmParams p{};
     using S = Gemm2CtaSmemT<BN>;
     CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * 2, kBM, kBK, 2));
     CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * 2, S::BN / 2, kBK, 2));
+    CHK_RET(EncodeTmapC(&p.tmapC, c, M, N, outFp32));
     p.C = c; p.M = M; p.N = N; p.K = K; p.ldc = N; p.outFp32 = outFp32; p.groupM = GroupMOverride(8); p.errorWord = GemmErrorWord(); p.waitHintNs = GemmWaitHintNs(); p.epiSleepNs = GemmEpiSleepNs();
     static std::atomic<bool> attrSet{false};
     auto kern = GemmKernel2Cta<PlainPolicy, BN>;

@@ -15,7 +15,8 @@
 //   TileCoord(p, ctx, t, mBlocks, nBlocks, &mb, &nb)   tile order
 //   WaitRowsReady(p, ctx, mb, abort)     producer-side gate before loading A rows
 //   SelectA(p, ctx, mb, &tmap, &row)     which tensor map / row coordinate serves this row block
-//   Store(p, ctx, row, col0, v[32])      epilogue sink (local C, a peer's reduce-scatter slot, ...)
+//   kTmaStore                            true: the result is local and leaves through p.tmapC (StoreTileTma); the other sinks are unused
+//   RowDst(p, ctx, row, col)             epilogue sink otherwise (local C, a peer's reduce-scatter slot, ...)
 //   EpilogueGate / Combine               per-tile gate and per-chunk transform of the accumulator (add received partials)
 //   TileDone(p, ctx, mb, nb, ew, lane)   after a tile's stores (signal the consumer rank)
 //   PostPhase(p, ctx, cta, ctas, abort)  work after the last tile (ordered reduction of the received partials)
@@ -26,6 +27,7 @@
 // kernels (reference: include/hccl_mc2.h:25-82, src/common/hccl_mc2.cc:141-165).
 #pragma once
 #include <cuda_bf16.h>
+#include "gemm_epilogue.cuh"
 #include "sm100_ptx.cuh"
 
 // Debug flavor: stores through peer pointers are range-checked when the including file brought the collective primitives in
@@ -48,6 +50,7 @@ struct GemmParams {
     CUtensorMap tmapA1;          // policy-specific second A map (other parity half)
     CUtensorMap tmapALocal;      // policy-specific third A map (the local shard)
     CUtensorMap tmapB;           // [N, K] bf16, box 64 x BN
+    CUtensorMap tmapC;           // kTmaStore policies: [M, N], box 128 rows x 128 bytes
     CUtensorMap tmapSfA, tmapSfB; // block-scaled CTA-pair kernel: scale atoms as [atoms][128 x u32] (box = one atom, no swizzle)
     CUtensorMap tmapSfA1, tmapSfALocal;   // policy-specific further scale maps of A (other parity half, the local shard)
     void *C;                     // output, row-major, leading dimension ldc (elements)
@@ -76,34 +79,11 @@ template <int BN> struct GemmSmem {
     static constexpr int kRing = kStages * (kABytes + kBBytes);
     static constexpr int kStageCols = BN < 128 ? BN : 128;                 // columns staged per epilogue pass
     static constexpr int kStagingOff = kRing;
-    static constexpr int kStagingBytes = kBM * kStageCols * 2;             // bf16 tile slice, XOR-swizzled 16-byte chunks
+    static constexpr int kStageBufs = 2;
+    static constexpr int kStagingBytes = 2 * kStageTileBytes;              // bf16 tile slice, XOR-swizzled 16-byte chunks, or two TMA store tiles
     static constexpr int kBarOff = kRing + kStagingBytes;
     static constexpr int kTotal = kBarOff + 256;
 };
-
-__device__ __forceinline__ void StoreRow32(void *C, uint32_t ldc, uint32_t N, bool fp32, uint32_t row, uint32_t col0, const uint32_t (&v)[32])
-{
-    if (fp32) {
-        float *c = (float *)C + (size_t)row * ldc + col0;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-            if (col0 + j < N) *(uint4 *)(c + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-    } else {
-        __nv_bfloat16 *c = (__nv_bfloat16 *)C + (size_t)row * ldc + col0;
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-            if (col0 + j < N) {
-                uint4 o;
-                __nv_bfloat162 t0 = __floats2bfloat162_rn(__uint_as_float(v[j]), __uint_as_float(v[j + 1]));
-                __nv_bfloat162 t1 = __floats2bfloat162_rn(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-                __nv_bfloat162 t2 = __floats2bfloat162_rn(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5]));
-                __nv_bfloat162 t3 = __floats2bfloat162_rn(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7]));
-                o.x = *(uint32_t *)&t0; o.y = *(uint32_t *)&t1; o.z = *(uint32_t *)&t2; o.w = *(uint32_t *)&t3;
-                *(uint4 *)(c + j) = o;
-            }
-        }
-    }
-}
 
 struct PlainPolicy {
     struct Ctx {};
@@ -142,18 +122,8 @@ struct PlainPolicy {
         *tm = &p.tmapSfA;
         *atomRow = (int32_t)(mb * (p.K / 128));
     }
-    // fp32 output goes straight from registers; bf16 output is staged through shared memory and written as whole
-    // 16-byte chunks of contiguous row segments
-    __device__ static bool UseDirect(const GemmParams &p) { return p.outFp32 != 0; }
-    __device__ static void Store(const GemmParams &p, const Ctx &, uint32_t row, uint32_t col0, const uint32_t (&v)[32])
-    {
-        if (row < p.M) StoreRow32(p.C, p.ldc, p.N, p.outFp32 != 0, row, col0, v);
-    }
-    // destination of 8 consecutive bf16 results at (row, col), or nullptr when outside the output
-    __device__ static __nv_bfloat16 *RowDst(const GemmParams &p, const Ctx &, uint32_t row, uint32_t col)
-    {
-        return (row < p.M && col < p.N) ? (__nv_bfloat16 *)p.C + (size_t)row * p.ldc + col : nullptr;
-    }
+    static constexpr bool kTmaStore = true;
+    __device__ static __nv_bfloat16 *RowDst(const GemmParams &, const Ctx &, uint32_t, uint32_t) { return nullptr; }
     // called by all 128 epilogue threads before a tile's accumulator is read / for every 32-column chunk read
     __device__ static bool EpilogueGate(const GemmParams &, Ctx &, uint32_t, volatile uint32_t *) { return true; }
     __device__ static void Combine(const GemmParams &, const Ctx &, uint32_t, uint32_t, uint32_t, uint32_t (&)[32]) {}
@@ -259,7 +229,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel(const __grid_const
         }
     } else if (warp >= 4) {
         const uint32_t ew = warp - 4;
-        uint32_t acc = 0, accPhase = 0;
+        uint32_t acc = 0, accPhase = 0, staged = 0;
         bool ok = true;
         for (uint32_t t = cta; t < numTiles && ok; t += ctas) {
             uint32_t mb, nb;
@@ -269,16 +239,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel(const __grid_const
             TcFenceAfter();
             const uint32_t rowInTile = ew * 32 + lane;
             const uint32_t row = mb * kBM + rowInTile;
-            if (Policy::UseDirect(p)) {
-#pragma unroll 1
-                for (uint32_t c = 0; c < BN / 32; ++c) {
-                    uint32_t v[32];
-                    TmemLd32x32(tmemBase + ((ew * 32) << 16) + acc * BN + c * 32, v);
-                    TmemLdWait();
-                    Policy::Store(p, ctx, row, nb * BN + c * 32, v);
-                }
-                TcFenceBefore();
-                MbarArrive(&tmemEmpty[acc]);
+            if constexpr (Policy::kTmaStore) {
+                StoreTileTma<BN, S::kStageBufs>(&p.tmapC, p.outFp32 != 0, p.N, tmemBase + ((ew * 32) << 16) + acc * BN, smem + S::kStagingOff, threadIdx.x - 128, mb * kBM,
+                                                nb * BN, staged, [](uint32_t (&)[32], uint32_t) {}, [&] { TcFenceBefore(); MbarArrive(&tmemEmpty[acc]); });
             } else {
                 constexpr uint32_t SC = S::kStageCols, CH = SC / 8;          // staged columns / 16-byte chunks per row
                 uint4 *stg = (uint4 *)(smem + S::kStagingOff);
@@ -321,6 +284,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel(const __grid_const
             acc ^= 1;
             if (acc == 0) accPhase ^= 1;
         }
+        if (Policy::kTmaStore && threadIdx.x == 128) TmaStoreWaitAll();
+        __syncwarp();
     }
     __syncthreads();
     if (warp == 2) { TcFenceAfter(); TmemDealloc(tmemBase, kTmemCols); }

@@ -84,9 +84,11 @@ template <int BN_> struct Gemm2CtaSmemT {
     static constexpr int kRing = kStages * (kABytes + kBBytes);
     static constexpr int kStageCols = BN % 64 == 0 ? 64 : 32;
     static constexpr int kStagingOff = kRing;
-    static constexpr int kStagingBytes = kBM * kStageCols * 2;
+    static constexpr int kStageBufs = 2;
+    static constexpr int kStagingBytes = kStageBufs * kStageTileBytes;
     static constexpr int kBarOff = kRing + kStagingBytes;
     static constexpr int kTotal = kBarOff + 256;
+    static_assert(kTotal + 1024 <= 232448, "shared memory per CTA");
 };
 using Gemm2CtaSmem = Gemm2CtaSmemT<256>;
 
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
         Policy::SpareWarps(p, ctx, warp - 2, blockIdx.x - commCtas, gridDim.x - commCtas, lane, abortWord);
     } else if (warp >= 4) {
         const uint32_t ew = warp - 4;
-        uint32_t acc = 0, accPhase = 0;
+        uint32_t acc = 0, accPhase = 0, staged = 0;
         bool ok = true;
         const uint32_t emptyLeader0 = cg2::MapToCta(SmemAddr(&tmemEmpty[0]), 0), emptyLeader1 = cg2::MapToCta(SmemAddr(&tmemEmpty[1]), 0);
         for (uint32_t t = pair; t < numTiles && ok; t += pairs) {
@@ -214,6 +216,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
             uint4 *stg = (uint4 *)(smem + S::kStagingOff);
             const uint32_t et = threadIdx.x - 128;
             if (valid && !Policy::EpilogueGate(p, ctx, mb, abortWord)) { ok = false; break; }
+            if constexpr (Policy::kTmaStore) {
+                auto release = [&] {                                         // accumulator fully read: hand it back to the leader's MMA thread
+                    TcFenceBefore();
+                    cg2::MbarArriveRemote(acc ? emptyLeader1 : emptyLeader0);
+                };
+                if (valid)
+                    StoreTileTma<BN, S::kStageBufs>(&p.tmapC, p.outFp32 != 0, p.N, tmemBase + ((ew * 32) << 16) + acc * BN, smem + S::kStagingOff, et, mb * kBM, nb * BN,
+                                                    staged, [](uint32_t (&)[32], uint32_t) {}, release);
+                else release();
+            } else {
 #pragma unroll 1
             for (uint32_t pass = 0; pass < BN / SC; ++pass) {
 #pragma unroll 1
@@ -221,29 +233,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
                     uint32_t v[32];
                     TmemLd32x32(tmemBase + ((ew * 32) << 16) + acc * BN + pass * SC + c * 32, v);
                     TmemLdWait();
-                    if (valid) {
-                        if (Policy::UseDirect(p)) {
-                            Policy::Store(p, ctx, row, nb * BN + pass * SC + c * 32, v);
-                            continue;
-                        }
-                        Policy::Combine(p, ctx, mb, row, nb * BN + pass * SC + c * 32, v);
-                    }
+                    if (valid) Policy::Combine(p, ctx, mb, row, nb * BN + pass * SC + c * 32, v);
 #pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q) {
-                        uint4 o;
-                        __nv_bfloat162 t0 = __floats2bfloat162_rn(__uint_as_float(v[q * 8 + 0]), __uint_as_float(v[q * 8 + 1]));
-                        __nv_bfloat162 t1 = __floats2bfloat162_rn(__uint_as_float(v[q * 8 + 2]), __uint_as_float(v[q * 8 + 3]));
-                        __nv_bfloat162 t2 = __floats2bfloat162_rn(__uint_as_float(v[q * 8 + 4]), __uint_as_float(v[q * 8 + 5]));
-                        __nv_bfloat162 t3 = __floats2bfloat162_rn(__uint_as_float(v[q * 8 + 6]), __uint_as_float(v[q * 8 + 7]));
-                        o.x = *(uint32_t *)&t0; o.y = *(uint32_t *)&t1; o.z = *(uint32_t *)&t2; o.w = *(uint32_t *)&t3;
-                        stg[rowInTile * CH + ((c * 4 + q) ^ (rowInTile & kSwz))] = o;
-                    }
+                    for (uint32_t q = 0; q < 4; ++q) stg[rowInTile * CH + ((c * 4 + q) ^ (rowInTile & kSwz))] = PackBf16x8(&v[q * 8]);
                 }
                 if (pass + 1 == BN / SC) {                               // accumulator fully read: hand it back to the leader's MMA thread
                     TcFenceBefore();
                     cg2::MbarArriveRemote(acc ? emptyLeader1 : emptyLeader0);
                 }
-                if (Policy::UseDirect(p)) continue;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (valid) {
 #pragma unroll 4
@@ -255,10 +252,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
+            }
             if (valid) Policy::TileDone(p, ctx, mb, nb, ew, lane);
             acc ^= 1;
             if (acc == 0) accPhase ^= 1;
         }
+        if (Policy::kTmaStore && threadIdx.x == 128) TmaStoreWaitAll();
+        __syncwarp();
     }
     // A CTA must not leave while its peer can still reach its shared memory, barriers or tensor memory.
     TcFenceBefore();

@@ -38,8 +38,9 @@ template <int BN> struct GemmMxSmem {
     static constexpr int kRing = kStages * (kABytes + kBBytes);
     static constexpr int kSfOff = kRing;
     static constexpr int kStageCols = 64;
-    static constexpr int kStagingOff = kSfOff + kStages * kSfBytes;
-    static constexpr int kStagingBytes = kBM * kStageCols * 2;
+    static constexpr int kStagingOff = (kSfOff + kStages * kSfBytes + 1023) / 1024 * 1024;
+    static constexpr int kStageBufs = 1;
+    static constexpr int kStagingBytes = kStageTileBytes;
     static constexpr int kBarOff = kStagingOff + kStagingBytes;
     static constexpr int kTotal = kBarOff + 256;
     // tensor memory columns
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx(const __grid_con
         }
     } else if (warp >= 4) {
         const uint32_t ew = warp - 4;
-        uint32_t acc = 0, accPhase = 0;
+        uint32_t acc = 0, accPhase = 0, staged = 0;
         bool ok = true;
         for (uint32_t t = cta; t < numTiles && ok; t += ctas) {
             uint32_t mb, nb;
@@ -179,16 +180,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx(const __grid_con
             TcFenceAfter();
             const uint32_t rowInTile = ew * 32 + lane;
             const uint32_t row = mb * kBM + rowInTile;
-            if (Policy::UseDirect(p)) {
-#pragma unroll 1
-                for (uint32_t c = 0; c < BN / 32; ++c) {
-                    uint32_t v[32];
-                    TmemLd32x32(tmemBase + ((ew * 32) << 16) + acc * BN + c * 32, v);
-                    TmemLdWait();
-                    Policy::Store(p, ctx, row, nb * BN + c * 32, v);
-                }
-                TcFenceBefore();
-                MbarArrive(&tmemEmpty[acc]);
+            if constexpr (Policy::kTmaStore) {
+                StoreTileTma<BN, S::kStageBufs>(&p.tmapC, p.outFp32 != 0, p.N, tmemBase + ((ew * 32) << 16) + acc * BN, smem + S::kStagingOff, threadIdx.x - 128, mb * kBM,
+                                                nb * BN, staged, [](uint32_t (&)[32], uint32_t) {}, [&] { TcFenceBefore(); MbarArrive(&tmemEmpty[acc]); });
             } else {
                 constexpr uint32_t SC = S::kStageCols, CH = SC / 8;
                 uint4 *stg = (uint4 *)(smem + S::kStagingOff);
@@ -230,6 +224,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx(const __grid_con
             Policy::TileDone(p, ctx, mb, nb, ew, lane);
             if (++acc == NACC) { acc = 0; accPhase ^= 1; }
         }
+        if (Policy::kTmaStore && threadIdx.x == 128) TmaStoreWaitAll();
+        __syncwarp();
     }
     __syncthreads();
     if (warp == 2) { TcFenceAfter(); TmemDealloc(tmemBase, kTmemCols); }

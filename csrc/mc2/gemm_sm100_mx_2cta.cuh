@@ -52,7 +52,9 @@ template <int BN_> struct GemmMx2CtaSmem {
     static constexpr int kSfOff = kRing;
     static constexpr int kStageCols = 64;
     static constexpr int kStagingOff = kSfOff + kStages * kSfBytes;
-    static constexpr int kStagingBytes = kBM * kStageCols * 2;
+    static constexpr int kStageBufs = BN <= 192 ? 2 : 1;
+    static constexpr int kStagingBytes = kStageBufs * kStageTileBytes;
+    static_assert(kStagingOff % 1024 == 0, "TMA store tiles");
     static constexpr int kBarOff = kStagingOff + kStagingBytes;
     static constexpr int kTotal = kBarOff + 256;
     static constexpr int kAccs = BN <= 192 ? 2 : 1;
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx2Cta(const __grid
         }
     } else if (warp >= 4) {
         const uint32_t ew = warp - 4;
-        uint32_t acc = 0, accPhase = 0;
+        uint32_t acc = 0, accPhase = 0, staged = 0;
         bool ok = true;
         const uint32_t emptyLeader0 = cg2::MapToCta(SmemAddr(&tmemEmpty[0]), 0), emptyLeader1 = cg2::MapToCta(SmemAddr(&tmemEmpty[1]), 0);
         for (uint32_t t = pair; t < numTiles && ok; t += pairs) {
@@ -205,6 +207,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx2Cta(const __grid
             uint4 *stg = (uint4 *)(smem + S::kStagingOff);
             const uint32_t et = threadIdx.x - 128;
             if (valid && !Policy::EpilogueGate(p, ctx, mb, abortWord)) { ok = false; break; }
+            if constexpr (Policy::kTmaStore) {
+                auto release = [&] {                                         // accumulator fully read: hand it back to the leader's MMA thread
+                    TcFenceBefore();
+                    cg2::MbarArriveRemote(acc ? emptyLeader1 : emptyLeader0);
+                };
+                if (valid)
+                    StoreTileTma<BN, S::kStageBufs>(&p.tmapC, p.outFp32 != 0, p.N, tmemBase + ((ew * 32) << 16) + acc * BN, smem + S::kStagingOff, et, mb * kBM, nb * BN,
+                                                    staged, [](uint32_t (&)[32], uint32_t) {}, release);
+                else release();
+            } else {
 #pragma unroll 1
             for (uint32_t pass = 0; pass < BN / SC; ++pass) {
 #pragma unroll 1
@@ -212,13 +224,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx2Cta(const __grid
                     uint32_t v[32];
                     TmemLd32x32(tmemBase + ((ew * 32) << 16) + acc * BN + pass * SC + c * 32, v);
                     TmemLdWait();
-                    if (valid) {
-                        if (Policy::UseDirect(p)) {
-                            Policy::Store(p, ctx, row, nb * BN + pass * SC + c * 32, v);
-                            continue;
-                        }
-                        Policy::Combine(p, ctx, mb, row, nb * BN + pass * SC + c * 32, v);
-                    }
+                    if (valid) Policy::Combine(p, ctx, mb, row, nb * BN + pass * SC + c * 32, v);
 #pragma unroll
                     for (uint32_t q = 0; q < 4; ++q) {
                         uint4 o;
@@ -234,7 +240,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx2Cta(const __grid
                     TcFenceBefore();
                     cg2::MbarArriveRemote(acc ? emptyLeader1 : emptyLeader0);
                 }
-                if (Policy::UseDirect(p)) continue;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (valid) {
 #pragma unroll 4
@@ -246,9 +251,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx2Cta(const __grid
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
+            }
             if (valid) Policy::TileDone(p, ctx, mb, nb, ew, lane);
             if (++acc == NACC) { acc = 0; accPhase ^= 1; }
         }
+        if (Policy::kTmaStore && threadIdx.x == 128) TmaStoreWaitAll();
+        __syncwarp();
     }
     // A CTA must not leave while its peer can still reach its shared memory, barriers or tensor memory.
     TcFenceBefore();

@@ -75,6 +75,7 @@ template <int BN> HcclResult LaunchPlainMx(const void *a, const void *sfa, const
     GemmParams p{};
     CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K, kBM, kMxBK, 1));
     CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K, BN, kMxBK, 1));
+    CHK_RET(EncodeTmapC(&p.tmapC, c, M, N, outFp32));
     p.C = c; p.M = M; p.N = N; p.K = K; p.ldc = N; p.outFp32 = outFp32; p.groupM = 16; p.errorWord = GemmErrorWord();
     p.sfA = (const uint8_t *)sfa; p.sfB = (const uint8_t *)sfb; p.sfAtomsB = (N + 127) / 128; p.elemBytes = 1;
     using S = GemmMxSmem<BN>;
@@ -104,6 +105,7 @@ template <int BN> HcclResult LaunchPlainMxPair(const void *a, const void *sfa, c
     CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K, BN / 2, kMxBK, 1));
     CHK_RET(EncodeTmapSf(&p.tmapSfA, sfa, (uint64_t)((M + 127) / 128) * (K / 128)));
     CHK_RET(EncodeTmapSf(&p.tmapSfB, sfb, (uint64_t)((N + 127) / 128) * (K / 128)));
+    CHK_RET(EncodeTmapC(&p.tmapC, c, M, N, outFp32));
     p.C = c; p.M = M; p.N = N; p.K = K; p.ldc = N; p.outFp32 = outFp32; p.groupM = 8; p.errorWord = GemmErrorWord();
     p.sfA = (const uint8_t *)sfa; p.sfB = (const uint8_t *)sfb; p.sfAtomsB = (N + 127) / 128; p.elemBytes = 1;
     static std::atomic<bool> attrSet{false};
