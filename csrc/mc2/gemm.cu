@@ -6,6 +6,7 @@
 #include "gemm_host.h"
 #include "gemm_sm100.cuh"
 #include "gemm_sm100_2cta.cuh"
+#include "gemm_splitk_launch.cuh"
 #include <cstdlib>
 #include "hccl/hccl_mc2.h"
 
@@ -224,11 +225,17 @@ HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint6
         HCCL_ERROR("HcclGemmBf16: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
         return HCCL_E_PARA;
     }
+    if (m <= 64) {
+        const SplitKChoice sk = ChooseSplitK(m, n, k, 0);
+        if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    }
     // narrow tiles when the problem has too few 128x256 tiles to fill the GPU
     uint64_t tiles256 = ((m + 127) / 128) * ((n + 255) / 256);
     if (Gemm2CtaEnabled(m, n, k) && tiles256 >= (uint64_t)SmCount()) return LaunchPlain2Cta(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (tiles256 >= (uint64_t)SmCount() || n % 256 == 0 && tiles256 * 2 > (uint64_t)SmCount()) return LaunchPlain<256>(a, b, c, m, n, k, outFp32 != 0, stream);
     uint64_t tiles128 = ((m + 127) / 128) * ((n + 127) / 128);
+    const SplitKChoice sk = ChooseSplitK(m, n, k, tiles128 >= (uint64_t)SmCount() / 2 ? tiles128 : ((m + 127) / 128) * ((n + 63) / 64));
+    if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (tiles128 >= (uint64_t)SmCount() / 2) return LaunchPlain<128>(a, b, c, m, n, k, outFp32 != 0, stream);
     return LaunchPlain<64>(a, b, c, m, n, k, outFp32 != 0, stream);
 }
@@ -240,6 +247,12 @@ HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m
         if (!a || !b || !c) return HCCL_E_PTR;
         if (m == 0 || n == 0 || k == 0 || (k % 8) || (n % 8) || m > 0x7fffffff || n > 0x7fffffff || k > 0x7fffffff) return HCCL_E_PARA;
         return LaunchPlain2Cta(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    }
+    // 1000 * S + BT: the split-K kernel with BT rows of A per tile and S CTAs along K
+    if (variant >= 1000) {
+        if (!a || !b || !c) return HCCL_E_PTR;
+        if (m == 0 || n == 0 || k == 0 || (k % 8) || (n % 8) || m > 0x7fffffff || n > 0x7fffffff || k > 0x7fffffff) return HCCL_E_PARA;
+        return LaunchSplitK<false>({(uint32_t)variant % 1000, (uint32_t)variant / 1000}, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
     return HcclGemmBf16(a, b, c, m, n, k, outFp32, stream);
 }

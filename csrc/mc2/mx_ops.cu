@@ -17,6 +17,7 @@
 #include "gemm_host.h"
 #include "gemm_sm100_mx.cuh"
 #include "gemm_sm100_mx_2cta.cuh"
+#include "gemm_splitk_launch.cuh"
 #include "hccl/hccl_mc2.h"
 
 namespace hccl {
@@ -171,6 +172,10 @@ HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const vo
                    (unsigned long long)k);
         return HCCL_E_PARA;
     }
+    if (!getenv("HCCL_MX_TILE_N")) {
+        const SplitKChoice sk = ChooseSplitK(m, n, k, ((m + 127) / 128) * ((n + 127) / 128));
+        if (sk.split) return LaunchSplitK<true>(sk, a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    }
     // CTA pairs when the product fills the GPU with pair tiles (HCCL_MX_PAIR=0 keeps the one-CTA kernels): 192-wide tiles with two
     // accumulators, or 256-wide ones when K is long enough to hide their exposed epilogue
     {
@@ -205,6 +210,9 @@ HcclResult HcclGemmMxfp8Variant(const void *a, const void *sfa, const void *b, c
     if (tileN == 2192) return LaunchPlainMxPair<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (tileN == 192) return LaunchPlainMx<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (tileN == 128) return LaunchPlainMx<128>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    // 100000 + 1000 * S + BT: the split-K kernel with BT rows of A per tile and S CTAs along K
+    if (tileN >= 100000)
+        return LaunchSplitK<true>({(uint32_t)tileN % 1000, (uint32_t)(tileN - 100000) / 1000}, a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     return HcclGemmMxfp8(a, sfa, b, sfb, c, m, n, k, outFp32, stream);
 }
 

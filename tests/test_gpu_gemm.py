@@ -52,3 +52,25 @@ def test_gemm_cta_pair_variant(shape, out_dtype):
     scale = ref.abs().max().item() + 1e-6
     tol = 2e-2 if out_dtype == torch.bfloat16 else 2e-3
     assert err / scale < tol, f"max err {err} vs scale {scale}"
+
+
+@pytest.mark.parametrize("shape,bt,split", [((1, 8, 8), 16, 1), ((4, 4096, 520), 16, 8), ((16, 136, 448), 16, 7), ((17, 264, 1032), 32, 5), ((33, 1000, 512), 64, 8),
+                                            ((128, 128, 4096), 128, 8), ((100, 72, 200), 128, 3), ((129, 520, 328), 64, 2), ((257, 384, 1024), 256, 4),
+                                            ((300, 256, 640), 128, 6), ((64, 8192, 64), 64, 1)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_split_k(shape, bt, split, out_dtype):
+    """Rows of A on the narrow side of the instruction, K shared by a cluster: remainders of every tile edge, one k-block per CTA, one row,
+    uneven K parts. The reference is a 64-bit product; 32-bit sums of K products err by less than K * 2^-24 of the absolute sum."""
+    from hccl_b200.ops import gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=out_dtype)                # a row past the end must stay
+    gemm.gemm_bf16(a, w, out[:M], variant=1000 * split + bt)
+    torch.cuda.synchronize()
+    gemm.check_error()
+    ref, mag = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out[:M].double() - ref).abs() <= bound + 1e-30).all())
+    assert bool((out[M] == 7.0).all())

@@ -129,3 +129,17 @@ def test_matmul_all_reduce_mxfp8(nranks, M, N, K):
             for r in range(nranks):
                 assert _rel(out[r], ref) < 1.5e-2
                 assert torch.equal(out[r], out[0])
+
+
+@pytest.mark.parametrize("m,n,k,bt,split", [(1, 8, 128, 16, 1), (16, 264, 1024, 16, 8), (20, 128, 896, 32, 7), (64, 1000, 512, 64, 2), (200, 264, 384, 64, 3),
+                                            (128, 8192, 256, 128, 2), (300, 136, 1024, 256, 4)])
+def test_block_scaled_split_k(m, n, k, bt, split):
+    """Split-K form: tiles of A that start inside a scale atom (32, 64 rows), two atoms (256), ragged rows and uneven K parts."""
+    from hccl_b200.ops import gemm as g, mxfp8 as mx
+    a, w = mx.quantize(_wild((m, k), 1 + m)), mx.quantize(_wild((n, k), 2 + n, 0.05))
+    da, dw = mx.dequantize(a).double(), mx.dequantize(w).double()
+    ref, mag = da @ dw.t(), da.abs() @ dw.abs().t()
+    out = mx.gemm(a, w, out_dtype=torch.float32, tile_n=100000 + 1000 * split + bt)
+    torch.cuda.synchronize()
+    g.check_error()
+    assert bool(((out.double() - ref).abs() <= mag * k * 2.0 ** -24 + 1e-30).all())
