@@ -129,16 +129,17 @@ int SmCount()
     return n[dev];
 }
 
-template <int BN> static HcclResult LaunchPlain(const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
+template <int BN, bool BMN = false> static HcclResult LaunchPlain(const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
 {
     GemmParams p{};
     CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * 2, kBM, kBK, 2));
-    CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * 2, BN, kBK, 2));
+    if (BMN) CHK_RET(EncodeTmap2D(&p.tmapB, b, K, N, (uint64_t)N * 2, kBK, 64, 2));
+    else CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * 2, BN, kBK, 2));
     CHK_RET(EncodeTmapC(&p.tmapC, c, M, N, outFp32));
     p.C = c; p.M = M; p.N = N; p.K = K; p.ldc = N; p.outFp32 = outFp32; p.groupM = GroupMOverride(16); p.errorWord = GemmErrorWord(); p.waitSleepNs = GemmWaitSleepNs();
     using S = GemmSmem<BN>;
     static std::atomic<bool> attrSet{false};
-    auto kern = GemmKernel<BN, PlainPolicy, false>;
+    auto kern = GemmKernel<BN, PlainPolicy, false, BMN>;
     size_t smem = S::kTotal + 1024;
     if (!attrSet) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return HCCL_E_RUNTIME;
@@ -154,17 +155,18 @@ template <int BN> static HcclResult LaunchPlain(const void *a, const void *b, vo
 }
 
 // 256 x 256 tiles on CTA pairs (cta_group::2). Needs an even grid; one cluster of two CTAs per tile.
-template <int BN>
+template <int BN, bool BMN = false>
 static HcclResult LaunchPlain2CtaT(const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
 {
     GemmParams p{};
     using S = Gemm2CtaSmemT<BN>;
     CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * 2, kBM, kBK, 2));
-    CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * 2, S::BN / 2, kBK, 2));
+    if (BMN) CHK_RET(EncodeTmap2D(&p.tmapB, b, K, N, (uint64_t)N * 2, kBK, 64, 2));
+    else CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * 2, S::BN / 2, kBK, 2));
     CHK_RET(EncodeTmapC(&p.tmapC, c, M, N, outFp32));
     p.C = c; p.M = M; p.N = N; p.K = K; p.ldc = N; p.outFp32 = outFp32; p.groupM = GroupMOverride(8); p.errorWord = GemmErrorWord(); p.waitHintNs = GemmWaitHintNs(); p.epiSleepNs = GemmEpiSleepNs();
     static std::atomic<bool> attrSet{false};
-    auto kern = GemmKernel2Cta<PlainPolicy, BN>;
+    auto kern = GemmKernel2Cta<PlainPolicy, BN, BMN>;
     size_t smem = S::kTotal + 1024;
     if (!attrSet) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return HCCL_E_RUNTIME;
@@ -255,6 +257,20 @@ HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m
         return LaunchSplitK<false>({(uint32_t)variant % 1000, (uint32_t)variant / 1000}, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
     return HcclGemmBf16(a, b, c, m, n, k, outFp32, stream);
+}
+
+// C[M,N] = A[M,K] * B[K,N], both row-major: the input gradient of a linear layer straight from its weight. Same rules as HcclGemmBf16.
+HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream)
+{
+    if (!a || !b || !c) return HCCL_E_PTR;
+    if (m == 0 || n == 0 || k == 0 || (k % 8) || (n % 8) || m > 0x7fffffff || n > 0x7fffffff || k > 0x7fffffff) {
+        HCCL_ERROR("HcclGemmBf16Nn: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
+        return HCCL_E_PARA;
+    }
+    const uint64_t sms = (uint64_t)SmCount(), tiles256 = ((m + 127) / 128) * ((n + 255) / 256), tiles128 = ((m + 127) / 128) * ((n + 127) / 128);
+    if (tiles256 >= sms) return LaunchPlain2CtaT<256, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    if (tiles128 >= sms / 2) return LaunchPlain<128, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    return LaunchPlain<64, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
 }
 
 HcclResult HcclGemmCheckError(void) { return GemmCheckError(); }

@@ -132,14 +132,17 @@ struct PlainPolicy {
     __device__ static void Exit(const GemmParams &, Ctx &) {}
 };
 
-template <int BN, class Policy, bool EMU>
+// BMN = true: B is given as [K, N] row-major (C = A * B), the operand of a backward pass through the same weight. Its tiles arrive
+// as boxes of 64 columns x 64 rows of K (128 bytes wide, 8 KB each) and the tensor core reads them MN-major, so no transposed copy
+// of B is ever made.
+template <int BN, class Policy, bool EMU, bool BMN = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel(const __grid_constant__ GemmParams pv, const GemmParams *emuParams)
 {
     const GemmParams &p = EMU ? emuParams[blockIdx.y] : pv;
     using S = GemmSmem<BN>;
     constexpr int STAGES = S::kStages;
     constexpr uint32_t kTmemCols = BN * 2 >= 32 ? BN * 2 : 32;       // two accumulators
-    constexpr uint32_t kIdesc = MakeInstrDesc(FMT_BF16, FMT_BF16, kBM, BN);
+    constexpr uint32_t kIdesc = MakeInstrDesc(FMT_BF16, FMT_BF16, kBM, BN) | (BMN ? kInstrBMajorMN : 0u);
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);   // swizzle atoms want 1024-byte alignment
 
@@ -195,7 +198,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel(const __grid_const
                     if (!ok) break;
                     MbarExpectTx(&full[stage], S::kABytes + S::kBBytes);
                     TmaLoad2D(sA + stage * S::kABytes, ta, &full[stage], (int32_t)(kb * kBK), rowA);
-                    TmaLoad2D(sB + stage * S::kBBytes, &p.tmapB, &full[stage], (int32_t)(kb * kBK), (int32_t)(nb * BN));
+                    if (BMN) {
+#pragma unroll
+                        for (int j = 0; j < BN / 64; ++j)
+                            TmaLoad2D(sB + stage * S::kBBytes + j * kMnBoxBytes, &p.tmapB, &full[stage], (int32_t)(nb * BN + j * 64), (int32_t)(kb * kBK));
+                    } else {
+                        TmaLoad2D(sB + stage * S::kBBytes, &p.tmapB, &full[stage], (int32_t)(kb * kBK), (int32_t)(nb * BN));
+                    }
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -214,10 +223,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel(const __grid_const
                     if (!ok) break;
                     TcFenceAfter();
                     uint64_t aDesc = MakeSmemDescSw128(SmemAddr(sA + stage * S::kABytes));
-                    uint64_t bDesc = MakeSmemDescSw128(SmemAddr(sB + stage * S::kBBytes));
+                    uint64_t bDesc = BMN ? MakeSmemDescMnSw128(SmemAddr(sB + stage * S::kBBytes)) : MakeSmemDescSw128(SmemAddr(sB + stage * S::kBBytes));
 #pragma unroll
                     for (uint32_t k = 0; k < kBK / 16; ++k)
-                        UmmaF16(dTmem, AdvanceDescK(aDesc, k * 32), AdvanceDescK(bDesc, k * 32), kIdesc, (kb | k) != 0 ? 1u : 0u);
+                        UmmaF16(dTmem, AdvanceDescK(aDesc, k * 32), AdvanceDescK(bDesc, k * (BMN ? 2048 : 32)), kIdesc, (kb | k) != 0 ? 1u : 0u);
                     UmmaCommit(&empty[stage]);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }

@@ -92,13 +92,15 @@ template <int BN_> struct Gemm2CtaSmemT {
 };
 using Gemm2CtaSmem = Gemm2CtaSmemT<256>;
 
-template <class Policy, int BN_ = 256>
+// BMN: B is [K, N] row-major, read MN-major (see GemmKernel); this CTA's half of the tile is BN / 128 boxes of 64 columns.
+template <class Policy, int BN_ = 256, bool BMN = false>
 __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_constant__ GemmParams p)
 {
     using S = Gemm2CtaSmemT<BN_>;
     constexpr int BN = S::BN, STAGES = S::kStages;
     constexpr uint32_t kTmemCols = 512;                                        // two 256-column accumulators
-    constexpr uint32_t kIdesc = MakeInstrDesc(FMT_BF16, FMT_BF16, 2 * kBM, BN);
+    constexpr uint32_t kIdesc = MakeInstrDesc(FMT_BF16, FMT_BF16, 2 * kBM, BN) | (BMN ? kInstrBMajorMN : 0u);
+    static_assert(!BMN || BN % 128 == 0, "each CTA's half of the tile is whole 64-column boxes");
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
 
@@ -162,7 +164,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
                     const uint32_t fullLeader = cg2::MapToCta(SmemAddr(&full[stage]), 0);
                     if (leader) MbarExpectTx(&full[stage], 2 * (S::kABytes + S::kBBytes));
                     cg2::TmaLoad2DPair(sA + stage * S::kABytes, ta, fullLeader, (int32_t)(kb * kBK), rowA);
-                    cg2::TmaLoad2DPair(sB + stage * S::kBBytes, &p.tmapB, fullLeader, (int32_t)(kb * kBK), (int32_t)(nb * BN + rankInPair * (BN / 2)));
+                    if (BMN) {
+#pragma unroll
+                        for (int j = 0; j < BN / 128; ++j)
+                            cg2::TmaLoad2DPair(sB + stage * S::kBBytes + j * kMnBoxBytes, &p.tmapB, fullLeader,
+                                               (int32_t)(nb * BN + rankInPair * (BN / 2) + j * 64), (int32_t)(kb * kBK));
+                    } else {
+                        cg2::TmaLoad2DPair(sB + stage * S::kBBytes, &p.tmapB, fullLeader, (int32_t)(kb * kBK), (int32_t)(nb * BN + rankInPair * (BN / 2)));
+                    }
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -181,10 +190,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
                     if (!ok) break;
                     TcFenceAfter();
                     uint64_t aDesc = MakeSmemDescSw128(SmemAddr(sA + stage * S::kABytes));
-                    uint64_t bDesc = MakeSmemDescSw128(SmemAddr(sB + stage * S::kBBytes));
+                    uint64_t bDesc = BMN ? MakeSmemDescMnSw128(SmemAddr(sB + stage * S::kBBytes)) : MakeSmemDescSw128(SmemAddr(sB + stage * S::kBBytes));
 #pragma unroll
                     for (uint32_t k = 0; k < kBK / 16; ++k)
-                        cg2::UmmaF16Pair(dTmem, AdvanceDescK(aDesc, k * 32), AdvanceDescK(bDesc, k * 32), kIdesc, (kb | k) != 0 ? 1u : 0u);
+                        cg2::UmmaF16Pair(dTmem, AdvanceDescK(aDesc, k * 32), AdvanceDescK(bDesc, k * (BMN ? 2048 : 32)), kIdesc, (kb | k) != 0 ? 1u : 0u);
                     cg2::UmmaCommitPair(&empty[stage]);
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }

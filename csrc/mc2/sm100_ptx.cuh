@@ -242,6 +242,21 @@ __device__ __forceinline__ uint64_t MakeSmemDescSw128(uint32_t smemAddr)
     d |= (uint64_t)2 << 61;                 // SWIZZLE_128B
     return d;
 }
+// MN-major operand tile: boxes of 64 MN elements (128 bytes, one swizzle row) x 64 rows of K, 8 KB each, side by side along MN.
+// Leading byte offset = from one box to the next, stride byte offset = from one group of 8 rows of K to the next; 16 rows of K
+// (one instruction) are 2048 bytes.
+constexpr uint32_t kMnBoxBytes = 64 * 128;
+constexpr uint32_t kInstrBMajorMN = 1u << 16;
+__device__ __forceinline__ uint64_t MakeSmemDescMnSw128(uint32_t smemAddr)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((smemAddr >> 4) & 0x3fffu);
+    d |= (uint64_t)(kMnBoxBytes >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;                 // descriptor version (Blackwell)
+    d |= (uint64_t)2 << 61;                 // SWIZZLE_128B
+    return d;
+}
 // Advance along K inside the swizzle atom by `bytes` (a multiple of 32): only the start-address field moves.
 __device__ __forceinline__ uint64_t AdvanceDescK(uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); }
 

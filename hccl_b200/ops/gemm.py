@@ -17,6 +17,8 @@ def _decl():
         l.HcclGemmBf16Variant.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_uint64, ctypes.c_uint64,
                                           ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
         l.HcclGemmBf16Variant.restype = ctypes.c_int
+        l.HcclGemmBf16Nn.argtypes = l.HcclGemmBf16.argtypes
+        l.HcclGemmBf16Nn.restype = ctypes.c_int
         l.HcclGemmCheckError.argtypes = []
         l.HcclGemmCheckError.restype = ctypes.c_int
         l._gemm_declared = True
@@ -38,6 +40,21 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
     s = torch.cuda.current_stream() if stream is None else stream
     check(_decl().HcclGemmBf16Variant(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, int(out.dtype == torch.float32), variant, s.cuda_stream),
           "HcclGemmBf16")
+    return out
+
+
+def gemm_bf16_nn(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, out_dtype: torch.dtype = torch.bfloat16, stream=None) -> torch.Tensor:
+    """a: [M, K] bf16, w: [K, N] bf16 (both row-major) -> a @ w in `out_dtype` (bf16 or fp32); no transposed copy of w is made."""
+    if not (a.is_cuda and w.is_cuda):
+        raise RuntimeError("gemm_bf16_nn needs CUDA tensors (the tcgen05 kernel has no CPU path)")
+    assert a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.is_contiguous() and w.is_contiguous()
+    M, K = a.shape
+    K2, N = w.shape
+    assert K == K2
+    if out is None:
+        out = torch.empty((M, N), dtype=out_dtype, device=a.device)
+    s = torch.cuda.current_stream() if stream is None else stream
+    check(_decl().HcclGemmBf16Nn(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, int(out.dtype == torch.float32), s.cuda_stream), "HcclGemmBf16Nn")
     return out
 
 

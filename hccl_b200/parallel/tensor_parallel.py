@@ -44,6 +44,11 @@ def _mm_nt(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     return a @ w.t()
 
 
+def _nn_ok(comm, dy: torch.Tensor, w: torch.Tensor) -> bool:
+    """The input gradient dy @ w needs no collective and the tcgen05 GEMM takes it: it reads w as stored, no transposed copy."""
+    return comm.size == 1 and _NATIVE_GEMM and getattr(comm, "fused", True) and _fused_ok(dy, w) and w.shape[0] % 8 == 0 and w.shape[1] % 8 == 0 and dy.numel() > 0
+
+
 _NATIVE_WGRAD = False
 
 
@@ -117,7 +122,10 @@ class _ColumnSeqParallel(torch.autograd.Function):
     def backward(ctx, dy):
         gathered, w = ctx.saved_tensors
         dy = dy.contiguous()
-        dx = matmul_reduce_scatter(ctx.comm, dy, w.t().contiguous())          # RS(dy @ W): the mirror of the forward
+        if _nn_ok(ctx.comm, dy, w):
+            dx = _gemm.gemm_bf16_nn(dy, w.contiguous())
+        else:
+            dx = matmul_reduce_scatter(ctx.comm, dy, w.t().contiguous())      # RS(dy @ W): the mirror of the forward
         dw = _wgrad(dy, gathered)                                               # dy^T @ AG(x)
         return dx, dw, None
 
@@ -134,7 +142,11 @@ class _RowSeqParallel(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy_local):
         x, w = ctx.saved_tensors
-        dx, dyg = all_gather_matmul(ctx.comm, dy_local.contiguous(), w.t().contiguous(), want_gathered=True)   # AG(dy) @ W
+        dyg = dy_local.contiguous()
+        if _nn_ok(ctx.comm, dyg, w):
+            dx = _gemm.gemm_bf16_nn(dyg, w.contiguous())
+        else:
+            dx, dyg = all_gather_matmul(ctx.comm, dyg, w.t().contiguous(), want_gathered=True)                 # AG(dy) @ W
         dw = _wgrad(dyg, x)                                                                                    # AG(dy)^T @ x
         return dx, dw, None
 
@@ -144,6 +156,7 @@ class _RowAllReduce(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w, comm):
+        ctx.comm = comm
         ctx.save_for_backward(x, w)
         return matmul_all_reduce(comm, x, w)
 
@@ -151,7 +164,8 @@ class _RowAllReduce(torch.autograd.Function):
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
         dy = dy.contiguous()
-        return _mm_nt(dy, w.t().contiguous()), _wgrad(dy, x), None
+        dx = _gemm.gemm_bf16_nn(dy, w.contiguous()) if _nn_ok(ctx.comm, dy, w) else _mm_nt(dy, w.t().contiguous())
+        return dx, _wgrad(dy, x), None
 
 
 class _ColumnReplicatedInput(torch.autograd.Function):
@@ -167,7 +181,7 @@ class _ColumnReplicatedInput(torch.autograd.Function):
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
         dy = dy.contiguous()
-        dx = matmul_all_reduce(ctx.comm, dy, w.t().contiguous())
+        dx = _gemm.gemm_bf16_nn(dy, w.contiguous()) if _nn_ok(ctx.comm, dy, w) else matmul_all_reduce(ctx.comm, dy, w.t().contiguous())
         return dx, _wgrad(dy, x), None
 
 

@@ -51,6 +51,8 @@ typedef struct HcclOpResCtxDef {
 HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream);
 /* variant 0 = automatic, 1 = one-CTA 128 x BN tiles, 2 = 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2) */
 HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, int variant, cudaStream_t stream);
+/* C[M,N] = A[M,K] * B[K,N], both row-major: the input gradient of a linear layer from its [K, N] weight as stored. */
+HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream);
 HcclResult HcclGemmCheckError(void);
 /* Kernels this library has launched in this process so far (all operators; benchmarks report the delta over a region). */
 uint64_t HcclGetKernelLaunchCount(void);

@@ -74,3 +74,20 @@ def test_gemm_split_k(shape, bt, split, out_dtype):
     bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
     assert bool(((out[:M].double() - ref).abs() <= bound + 1e-30).all())
     assert bool((out[M] == 7.0).all())
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 8), (128, 64, 64), (100, 72, 200), (1000, 264, 520), (384, 768, 1600), (2048, 4104, 1032), (4096, 2560, 264)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_nn(shape, out_dtype):
+    """B stored [K, N] and read MN-major: all three tile kernels, ragged edges in every dimension (bound as above)."""
+    from hccl_b200.ops import gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(K, N, generator=g, device="cuda").to(torch.bfloat16)
+    out = gemm.gemm_bf16_nn(a, w, out_dtype=out_dtype)
+    torch.cuda.synchronize()
+    gemm.check_error()
+    ref, mag = a.double() @ w.double(), a.double().abs() @ w.double().abs()
+    bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out.double() - ref).abs() <= bound + 1e-30).all())
