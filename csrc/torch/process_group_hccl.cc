@@ -237,8 +237,11 @@ c10::intrusive_ptr<c10d::Backend> createProcessGroupHCCL(const c10::intrusive_pt
 
 }  // namespace
 
+void BindFusedOps(py::module &m);   // fused_ops.cc
+
 PYBIND11_MODULE(hccl_b200_torch, m)
 {
-    m.doc() = "torch.distributed backend on the hccl_b200 C API";
+    m.doc() = "torch.distributed backend and matmul operators on the hccl_b200 C API";
+    BindFusedOps(m);
     m.def("create_process_group", &createProcessGroupHCCL, py::arg("store"), py::arg("rank"), py::arg("size"), py::arg("timeout"));
 }

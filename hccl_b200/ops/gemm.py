@@ -5,6 +5,7 @@ import ctypes
 
 import torch
 
+from .._ext import ops as _native
 from .._lib import check, lib
 
 
@@ -35,6 +36,12 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
     M, K = a.shape
     N, K2 = w.shape
     assert K == K2
+    n = _native()
+    if n is not None and (out is not None or out_dtype in (torch.bfloat16, torch.float32)):
+        rc, out = n.gemm(a, w, out, out_dtype == torch.float32, False, variant, None if stream is None else stream.cuda_stream)
+        if rc:
+            check(rc, "HcclGemmBf16")
+        return out
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
     s = torch.cuda.current_stream() if stream is None else stream
@@ -51,6 +58,12 @@ def gemm_bf16_nn(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = No
     M, K = a.shape
     K2, N = w.shape
     assert K == K2
+    n = _native()
+    if n is not None and (out is not None or out_dtype in (torch.bfloat16, torch.float32)):
+        rc, out = n.gemm(a, w, out, out_dtype == torch.float32, True, 0, None if stream is None else stream.cuda_stream)
+        if rc:
+            check(rc, "HcclGemmBf16Nn")
+        return out
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
     s = torch.cuda.current_stream() if stream is None else stream

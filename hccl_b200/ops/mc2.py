@@ -6,6 +6,7 @@ from typing import Optional
 
 import torch
 
+from .._ext import ops as _native
 from .._lib import check, lib
 from ..types import DataType
 
@@ -36,6 +37,12 @@ def _chk(*ts):
 def all_gather_matmul(comm, a_local: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None,
                       gathered: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """out[size*m, N] = all_gather(a_local[m, K]) @ w[N, K].T"""
+    n = _native()
+    if n is not None:
+        rc, out = n.fused(comm.handle, 0, comm.size, a_local, w, out, gathered, None if stream is None else stream.cuda_stream)
+        if rc:
+            check(rc, "HcclAllGatherMatmul")
+        return out
     _chk(a_local, w)
     m, k = a_local.shape
     n = w.shape[0]
@@ -48,6 +55,12 @@ def all_gather_matmul(comm, a_local: torch.Tensor, w: torch.Tensor, out: Optiona
 
 def matmul_reduce_scatter(comm, a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """out[M/size, N] = reduce_scatter_rows(a[M, Klocal] @ w[N, Klocal].T)"""
+    n = _native()
+    if n is not None:
+        rc, out = n.fused(comm.handle, 1, comm.size, a, w, out, None, None if stream is None else stream.cuda_stream)
+        if rc:
+            check(rc, "HcclMatmulReduceScatter")
+        return out
     _chk(a, w)
     m, k = a.shape
     n = w.shape[0]
@@ -60,6 +73,12 @@ def matmul_reduce_scatter(comm, a: torch.Tensor, w: torch.Tensor, out: Optional[
 
 def matmul_all_reduce(comm, a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """out[M, N] = all_reduce(a[M, Klocal] @ w[N, Klocal].T)"""
+    n = _native()
+    if n is not None:
+        rc, out = n.fused(comm.handle, 2, comm.size, a, w, out, None, None if stream is None else stream.cuda_stream)
+        if rc:
+            check(rc, "HcclMatmulAllReduce")
+        return out
     _chk(a, w)
     m, k = a.shape
     n = w.shape[0]

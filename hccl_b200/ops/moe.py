@@ -66,24 +66,29 @@ class MoeDispatcher:
         self.mxfp8 = mxfp8
         self.hidden = hidden
         self._tokens = 0
+        self._recv = None      # receive buffers as tensors, and the addresses they were made for
 
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, stream=None) -> Tuple[torch.Tensor, Optional[torch.Tensor], torch.Tensor, torch.Tensor]:
         assert x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and topk_idx.dtype == torch.int32 and topk_idx.is_contiguous()
-        s = (torch.cuda.current_stream() if stream is None else stream).cuda_stream
+        s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) if stream is None else stream.cuda_stream
         rx, rs, rc, rsrc = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
         check(_decl().HcclMoeDispatch(self._h, x.data_ptr(), topk_idx.data_ptr(), x.shape[0], ctypes.byref(rx), ctypes.byref(rs), ctypes.byref(rc),
                                       ctypes.byref(rsrc), s), "HcclMoeDispatch")
         self._tokens = x.shape[0]
-        dev = x.device
-        recv_x = _view(rx.value, (self.cap, self.hidden), torch.float8_e4m3fn if self.mxfp8 else torch.bfloat16, dev)
-        recv_scales = _view(rs.value, (self.cap, self.hidden // 32), torch.uint8, dev) if self.mxfp8 else None
-        return recv_x, recv_scales, _view(rc.value, (self.local_experts,), torch.int32, dev), _view(rsrc.value, (self.cap,), torch.int32, dev)
+        at = (rx.value, rs.value, rc.value, rsrc.value)
+        if self._recv is None or self._recv[0] != at:
+            dev = x.device
+            self._recv = (at, _view(rx.value, (self.cap, self.hidden), torch.float8_e4m3fn if self.mxfp8 else torch.bfloat16, dev),
+                          _view(rs.value, (self.cap, self.hidden // 32), torch.uint8, dev) if self.mxfp8 else None,
+                          _view(rc.value, (self.local_experts,), torch.int32, dev), _view(rsrc.value, (self.cap,), torch.int32, dev))
+        # new tensor objects over the same memory on every call, as the caller may do with them what it likes
+        return tuple(None if t is None else t.detach() for t in self._recv[1:])
 
     def combine(self, topk_weights: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
         assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
         if out is None:
             out = torch.empty((self._tokens, self.hidden), dtype=torch.bfloat16, device=topk_weights.device)
-        s = (torch.cuda.current_stream() if stream is None else stream).cuda_stream
+        s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) if stream is None else stream.cuda_stream
         check(_decl().HcclMoeCombine(self._h, topk_weights.data_ptr(), out.data_ptr(), self._tokens, s), "HcclMoeCombine")
         return out
 
