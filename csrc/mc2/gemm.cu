@@ -190,16 +190,6 @@ static HcclResult LaunchPlain2CtaT(const void *a, const void *b, void *c, uint32
     return HCCL_SUCCESS;
 }
 
-static HcclResult LaunchPlain2Cta(const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
-{
-    // 224-wide tiles when they waste fewer waves (e.g. N = 3584 = 16 x 224 on 74 CTA pairs)
-    const uint64_t rowPairs = (M + 2 * kBM - 1) / (2 * kBM), pairs = (uint64_t)SmCount() / 2;
-    auto cost = [&](uint32_t bn) { uint64_t tiles = rowPairs * ((N + bn - 1) / bn); return ((tiles + pairs - 1) / pairs) * bn; };
-    static const int level = [] { const char *e = getenv("HCCL_MC2_CTA_PAIR"); return e ? atoi(e) : 1; }();
-    if (level >= 2 && cost(224) < cost(256)) return LaunchPlain2CtaT<224>(a, b, c, M, N, K, outFp32, s);
-    return LaunchPlain2CtaT<256>(a, b, c, M, N, K, outFp32, s);
-}
-
 // HCCL_GEMM_2CTA: 0 never, otherwise (and unset) always. The CTA-pair kernel keeps the tensor pipe at 97 % of the active
 // cycles against 85-88 % for the one-CTA kernel and halves the B traffic per SM. Isolated it wins clearly (1635 against 1480
 // TFLOP/s on 8192 x 8192 x 4096); back to back under the board's power limit it runs at a lower clock (1140 against 1240 MHz)
@@ -209,6 +199,41 @@ bool Gemm2CtaEnabled(uint64_t, uint64_t, uint64_t)
 {
     static const int v = [] { const char *e = getenv("HCCL_GEMM_2CTA"); return e ? atoi(e) : -1; }();
     return v != 0;
+}
+
+// A CTA pair with tiles of that width (192, 224, otherwise 256).
+static HcclResult LaunchPlain2Cta(uint32_t bn, const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
+{
+    if (bn == 192) return LaunchPlain2CtaT<192>(a, b, c, M, N, K, outFp32, s);
+    if (bn == 224) return LaunchPlain2CtaT<224>(a, b, c, M, N, K, outFp32, s);
+    return LaunchPlain2CtaT<256>(a, b, c, M, N, K, outFp32, s);
+}
+
+// Which tile kernel: waves of tiles times what a wave of that kernel takes, relative to a wave of 256 x 256 pair tiles. The weights are
+// measured on one B200 at K = 4096 (time of 1 ... 3 waves): pair 224 wide 0.87, 192 wide 0.80 (160 and 128 wide, 0.67 and 0.64, never won
+// a shape by more than 2 %), one CTA 256 wide 1.05, 128 wide 0.75, 64 wide 0.62. What that decides, us with 256-wide pairs / chosen: 1000 x 6144 x 4096
+// 48.1 / 39.5 (192), 700 x 8192 x 2048 29.6 / 23.7 (192), 2048 x 14336 x 4096 180 / 158 (224), 2048 x 28672 x 4096 310 / 300 (224); and
+// 1500 x 3000 x 3000 takes 31.5 on pairs against 48 on one-CTA tiles, which a rule by the count of 128 x 256 tiles had picked.
+// Narrower pair tiles read more of A per result, so they have to win by 3 %.
+struct TileChoice { bool pair; uint32_t bn; };
+static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposedB)
+{
+    const uint64_t sms = (uint64_t)SmCount(), pairs = sms / 2, rows = (m + kBM - 1) / kBM, rowPairs = (rows + 1) / 2;
+    auto waves = [](uint64_t tiles, uint64_t slots) { return (tiles + slots - 1) / slots; };
+    TileChoice best{false, 64};
+    uint64_t cost = waves(rows * ((n + 63) / 64), sms) * 62;
+    auto offer = [&](bool pair, uint32_t bn, uint64_t tiles, uint64_t weight, uint64_t percent) {
+        const uint64_t c = waves(tiles, pair ? pairs : sms) * weight;
+        if (c * 100 <= cost * percent) { best = {pair, bn}; cost = c; }
+    };
+    offer(false, 128, rows * ((n + 127) / 128), 75, 100);
+    if (!transposedB) offer(false, 256, rows * ((n + 255) / 256), 105, 100);
+    if (!transposedB && !Gemm2CtaEnabled(m, n, k)) return best;
+    offer(true, 256, rowPairs * ((n + 255) / 256), 100, 100);
+    if (transposedB) return best;                // its tiles are whole 64-column boxes per CTA, and it has no 256-wide one-CTA form
+    offer(true, 224, rowPairs * ((n + 223) / 224), 87, 97);
+    offer(true, 192, rowPairs * ((n + 191) / 192), 80, 97);
+    return best;
 }
 
 }  // namespace mc2
@@ -231,26 +256,26 @@ HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint6
         const SplitKChoice sk = ChooseSplitK(m, n, k, 0);
         if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
-    // narrow tiles when the problem has too few 128x256 tiles to fill the GPU
-    uint64_t tiles256 = ((m + 127) / 128) * ((n + 255) / 256);
-    if (Gemm2CtaEnabled(m, n, k) && tiles256 >= (uint64_t)SmCount()) return LaunchPlain2Cta(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
-    if (tiles256 >= (uint64_t)SmCount() || n % 256 == 0 && tiles256 * 2 > (uint64_t)SmCount()) return LaunchPlain<256>(a, b, c, m, n, k, outFp32 != 0, stream);
-    uint64_t tiles128 = ((m + 127) / 128) * ((n + 127) / 128);
-    const SplitKChoice sk = ChooseSplitK(m, n, k, tiles128 >= (uint64_t)SmCount() / 2 ? tiles128 : ((m + 127) / 128) * ((n + 63) / 64));
-    if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
-    if (tiles128 >= (uint64_t)SmCount() / 2) return LaunchPlain<128>(a, b, c, m, n, k, outFp32 != 0, stream);
+    const TileChoice t = ChooseTile(m, n, k, false);
+    if (!t.pair && t.bn < 256) {
+        const SplitKChoice sk = ChooseSplitK(m, n, k, ((m + 127) / 128) * ((n + t.bn - 1) / t.bn));
+        if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    }
+    if (t.pair) return LaunchPlain2Cta(t.bn, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    if (t.bn == 256) return LaunchPlain<256>(a, b, c, m, n, k, outFp32 != 0, stream);
+    if (t.bn == 128) return LaunchPlain<128>(a, b, c, m, n, k, outFp32 != 0, stream);
     return LaunchPlain<64>(a, b, c, m, n, k, outFp32 != 0, stream);
 }
 
-// variant 0 = automatic choice, 1 = one-CTA tiles, 2 = 256 x 256 tiles on CTA pairs (cta_group::2)
+// variant 2 or 256 = 256 x 256 tiles on CTA pairs (cta_group::2), 192 / 224 = pair tiles of that width, 1000 * S + BT = the split-K
+// kernel with BT rows of A per tile and S CTAs along K; anything else = automatic choice
 HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, int variant, cudaStream_t stream)
 {
-    if (variant == 2) {
+    if (variant == 2 || variant == 192 || variant == 224 || variant == 256) {
         if (!a || !b || !c) return HCCL_E_PTR;
         if (m == 0 || n == 0 || k == 0 || (k % 8) || (n % 8) || m > 0x7fffffff || n > 0x7fffffff || k > 0x7fffffff) return HCCL_E_PARA;
-        return LaunchPlain2Cta(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+        return LaunchPlain2Cta((uint32_t)variant, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
-    // 1000 * S + BT: the split-K kernel with BT rows of A per tile and S CTAs along K
     if (variant >= 1000) {
         if (!a || !b || !c) return HCCL_E_PTR;
         if (m == 0 || n == 0 || k == 0 || (k % 8) || (n % 8) || m > 0x7fffffff || n > 0x7fffffff || k > 0x7fffffff) return HCCL_E_PARA;
@@ -267,9 +292,9 @@ HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uin
         HCCL_ERROR("HcclGemmBf16Nn: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    const uint64_t sms = (uint64_t)SmCount(), tiles256 = ((m + 127) / 128) * ((n + 255) / 256), tiles128 = ((m + 127) / 128) * ((n + 127) / 128);
-    if (tiles256 >= sms) return LaunchPlain2CtaT<256, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
-    if (tiles128 >= sms / 2) return LaunchPlain<128, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    const TileChoice t = ChooseTile(m, n, k, true);
+    if (t.pair) return LaunchPlain2CtaT<256, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    if (t.bn == 128) return LaunchPlain<128, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     return LaunchPlain<64, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
 }
 

@@ -176,16 +176,18 @@ HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const vo
         const SplitKChoice sk = ChooseSplitK(m, n, k, ((m + 127) / 128) * ((n + 127) / 128));
         if (sk.split) return LaunchSplitK<true>(sk, a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
-    // CTA pairs when the product fills the GPU with pair tiles (HCCL_MX_PAIR=0 keeps the one-CTA kernels): 192-wide tiles with two
-    // accumulators, or 256-wide ones when K is long enough to hide their exposed epilogue
+    // CTA pairs when the product about fills the GPU with pair tiles (HCCL_MX_PAIR=0 keeps the one-CTA kernels): 192-wide tiles with two
+    // accumulators or 256-wide ones with one, whose epilogue is exposed. Time of a wave of tiles, measured on one B200: 192 wide 11.2 us
+    // per 4096 of K, 256 wide 14 us per 4096 of K and 4.5 us. Us with 192- / 256-wide tiles: 2048 x 28672 x 4096 190 / 240, 1000 x 6144 x 4096
+    // 23.7 / 31.8, 600 x 6144 x 8192 56 / 44, 2048 x 4096 x 14336 110 / 104, 2048 x 4096 x 28672 230 / 205.
     {
         const char *e = getenv("HCCL_MX_PAIR");
-        const bool pair = !(e && e[0] == '0') && !getenv("HCCL_MX_TILE_N");
-        const uint64_t bn = k >= 16384 ? 256 : 192;
-        const uint64_t pairTiles = ((m + 255) / 256) * ((n + bn - 1) / bn);
-        if (pair && n >= 256 && pairTiles >= (uint64_t)SmCount() / 2)
-            return bn == 256 ? LaunchPlainMxPair<256>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream)
-                             : LaunchPlainMxPair<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+        const uint64_t pairs = (uint64_t)SmCount() / 2, rowPairs = (m + 255) / 256, t192 = rowPairs * ((n + 191) / 192), t256 = rowPairs * ((n + 255) / 256);
+        if (!(e && e[0] == '0') && !getenv("HCCL_MX_TILE_N") && n >= 256 && (t192 >= pairs || t256 * 8 >= pairs * 7)) {
+            const double k4 = (double)k / 4096, c192 = (double)((t192 + pairs - 1) / pairs) * 11.2 * k4, c256 = (double)((t256 + pairs - 1) / pairs) * (14.0 * k4 + 4.5);
+            return c256 < c192 ? LaunchPlainMxPair<256>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream)
+                               : LaunchPlainMxPair<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+        }
     }
     // HCCL_MX_TILE_N = 192 | 256 picks the wide tile of large products (as for the fused operators)
     if (const char *e = getenv("HCCL_MX_TILE_N")) {

@@ -91,3 +91,24 @@ def test_gemm_nn(shape, out_dtype):
     ref, mag = a.double() @ w.double(), a.double().abs() @ w.double().abs()
     bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
     assert bool(((out.double() - ref).abs() <= bound + 1e-30).all())
+
+
+@pytest.mark.parametrize("shape,variant", [((256, 192, 64), 192), ((1000, 200, 264), 192), ((300, 392, 128), 224), ((1000, 6144, 512), 0), ((2048, 14336, 256), 0),
+                                           ((1500, 3000, 520), 0)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_pair_tile_widths(shape, variant, out_dtype):
+    """Pair tiles of 192 and 224 columns (the last staging tile of a 224-wide one stores 32 columns twice), one tile and partial tiles, and
+    shapes for which the automatic choice picks them (bound as above)."""
+    from hccl_b200.ops import gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=out_dtype)
+    gemm.gemm_bf16(a, w, out[:M], variant=variant)
+    torch.cuda.synchronize()
+    gemm.check_error()
+    ref, mag = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out[:M].double() - ref).abs() <= bound + 1e-30).all())
+    assert bool((out[M] == 7.0).all())
