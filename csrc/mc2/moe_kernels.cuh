@@ -117,18 +117,25 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
     __syncthreads();
     {
         const uint32_t split = tLo * K;
-        uint32_t i = tid;
-        for (; (uint64_t)i + 7 * kMoeThreads < entries; i += 8 * kMoeThreads) {
-            uint32_t e[8];
+        auto add = [&](uint32_t i, uint32_t e) { if (e < E) atomicAdd(i < split ? &sBefore[e] : &sTotal[e], 1u); };
+        uint32_t done = 0;
+        if (((uintptr_t)A.topkIdx & 15u) == 0) {             // four entries per load, eight loads in flight
+            const uint4 *v = (const uint4 *)A.topkIdx;
+            const uint32_t vecs = entries / 4;
+            for (uint32_t i = tid; i < vecs; i += 8 * kMoeThreads) {
+                uint4 e[8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) e[j] = (uint32_t)A.topkIdx[i + j * kMoeThreads];
+                for (int j = 0; j < 8; ++j) if (i + j * kMoeThreads < vecs) e[j] = v[i + j * kMoeThreads];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) if (e[j] < E) atomicAdd(i + j * kMoeThreads < split ? &sBefore[e[j]] : &sTotal[e[j]], 1u);
+                for (int j = 0; j < 8; ++j)
+                    if (i + j * kMoeThreads < vecs) {
+                        const uint32_t at = (i + j * kMoeThreads) * 4;
+                        add(at, e[j].x); add(at + 1, e[j].y); add(at + 2, e[j].z); add(at + 3, e[j].w);
+                    }
+            }
+            done = vecs * 4;
         }
-        for (; i < entries; i += kMoeThreads) {
-            const uint32_t e = (uint32_t)A.topkIdx[i];
-            if (e < E) atomicAdd(i < split ? &sBefore[e] : &sTotal[e], 1u);
-        }
+        for (uint32_t i = done + tid; i < entries; i += kMoeThreads) add(i, (uint32_t)A.topkIdx[i]);
     }
     __syncthreads();
     for (uint32_t e = tid; e < E; e += kMoeThreads) sTotal[e] += sBefore[e];
