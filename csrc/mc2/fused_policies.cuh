@@ -172,6 +172,7 @@ struct AgmmPolicy {
         else { *tm = x.half ? &p.tmapSfA1 : &p.tmapSfA; *atomRow = (int32_t)(mb * (p.K / 128)); }
     }
     static constexpr bool kTmaStore = false;
+    static constexpr bool kDependentLaunch = false;
     __device__ static __nv_bfloat16 *RowDst(const GemmParams &p, const Ctx &, uint32_t row, uint32_t col)
     {
         return (row < p.M && col < p.N) ? (__nv_bfloat16 *)p.C + (size_t)row * p.ldc + col : nullptr;
@@ -262,6 +263,7 @@ struct MmrsPolicy {
         *atomRow = (int32_t)(mb * (p.K / 128));
     }
     static constexpr bool kTmaStore = false;
+    static constexpr bool kDependentLaunch = false;
     // Tiles of rows owned by a peer: the bf16 partial goes into slot[rank] of the owner's workspace. Tiles of the own
     // rows come last; by then the peers' partials have long arrived, so their epilogue adds them (rank order, fp32) to
     // the accumulator and writes the final result: no separate reduction pass, no round trip of the own partial.
@@ -373,6 +375,7 @@ struct MmarPolicy {
     }
     __device__ static const uint8_t *SelectSfA(const GemmParams &p, const Ctx &, uint32_t mb) { return p.sfA + (uint64_t)mb * (p.K / 128) * 512; }
     static constexpr bool kTmaStore = false;
+    static constexpr bool kDependentLaunch = false;
     __device__ static __nv_bfloat16 *RowDst(const GemmParams &p, const Ctx &x, uint32_t row, uint32_t col)
     {
         if (row >= p.M || col >= p.N) return nullptr;

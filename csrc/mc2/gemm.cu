@@ -147,10 +147,19 @@ template <int BN, bool BMN = false> static HcclResult LaunchPlain(const void *a,
     }
     uint32_t tiles = ((M + kBM - 1) / kBM) * ((N + BN - 1) / BN);
     uint32_t grid = std::min<uint32_t>(tiles, (uint32_t)SmCount());
-    kern<<<grid, kGemmThreads, smem, s>>>(p, nullptr);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p, (const GemmParams *)nullptr);
     CountLaunch();
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) { HCCL_ERROR("GEMM launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    if (e != cudaSuccess) { HCCL_ERROR("GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
 

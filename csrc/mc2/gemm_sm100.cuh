@@ -16,6 +16,7 @@
 //   WaitRowsReady(p, ctx, mb, abort)     producer-side gate before loading A rows
 //   SelectA(p, ctx, mb, &tmap, &row)     which tensor map / row coordinate serves this row block
 //   kTmaStore                            true: the result is local and leaves through p.tmapC (StoreTileTma); the other sinks are unused
+//   kDependentLaunch                     true: nothing before the tile loops touches global memory, the launch may overlap the kernel before
 //   RowDst(p, ctx, row, col)             epilogue sink otherwise (local C, a peer's reduce-scatter slot, ...)
 //   EpilogueGate / Combine               per-tile gate and per-chunk transform of the accumulator (add received partials)
 //   TileDone(p, ctx, mb, nb, ew, lane)   after a tile's stores (signal the consumer rank)
@@ -123,6 +124,7 @@ struct PlainPolicy {
         *atomRow = (int32_t)(mb * (p.K / 128));
     }
     static constexpr bool kTmaStore = true;
+    static constexpr bool kDependentLaunch = true;
     __device__ static __nv_bfloat16 *RowDst(const GemmParams &, const Ctx &, uint32_t, uint32_t) { return nullptr; }
     // called by all 128 epilogue threads before a tile's accumulator is read / for every 32-column chunk read
     __device__ static bool EpilogueGate(const GemmParams &, Ctx &, uint32_t, volatile uint32_t *) { return true; }
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel(const __grid_const
     __syncthreads();
     TcFenceAfter();
     const uint32_t tmemBase = *tmemPtr;
+    if (Policy::kDependentLaunch) { LetDependentsStart(); DependencyWait(); }
 
     if (warp == 0) {
         if (ElectOne()) {

@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
     __syncthreads();
     TcFenceAfter();
     const uint32_t tmemBase = *tmemPtr;
+    LetDependentsStart();
+    DependencyWait();                        // up to here nothing touched global memory but the kernel's own parameters
 
     if (warp == 0) {
         if (ElectOne()) {

@@ -54,11 +54,13 @@ HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const vo
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = split > 1 ? 1 : 0;
+    cfg.numAttrs = split > 1 ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
     CountLaunch();
     if (e != cudaSuccess) { HCCL_ERROR("split-K GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return HCCL_E_RUNTIME; }

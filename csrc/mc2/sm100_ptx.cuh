@@ -32,6 +32,12 @@ __device__ __forceinline__ bool ElectOne()
     return pred != 0;
 }
 
+// Programmatic dependent launch. A kernel launched with the attribute may start while the kernel before it in the stream drains:
+// DependencyWait() returns once that one has completed and its writes are visible, so everything before it must stay off global
+// memory. LetDependentsStart() allows the next kernel (if it carries the attribute) to take the slots that become free.
+__device__ __forceinline__ void DependencyWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void LetDependentsStart() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void MbarInit(uint64_t *bar, uint32_t count)
 {
