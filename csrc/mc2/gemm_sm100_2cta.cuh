@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
     cg2::ClusterSync();                     // both CTAs' barriers are initialised before anything remote touches them
     TcFenceAfter();
     const uint32_t tmemBase = *tmemPtr;
+    if (Policy::kDependentLaunch) { LetDependentsStart(); DependencyWait(); }
 
     if (warp == 0) {
         if (ElectOne()) {

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx2Cta(const __grid
     cg2::ClusterSync();
     TcFenceAfter();
     const uint32_t tmemBase = *tmemPtr;
+    if (Policy::kDependentLaunch) { LetDependentsStart(); DependencyWait(); }
 
     if (warp == 0) {
         if (ElectOne()) {

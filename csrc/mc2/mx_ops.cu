@@ -29,6 +29,7 @@ namespace {
 __global__ void QuantizeMxfp8Kernel(const __nv_bfloat16 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales, uint32_t rows,
                                     uint32_t rowsPadded, uint32_t K)
 {
+    LetDependentsStart();                        // the product that reads this sets up meanwhile
     const uint32_t kBlocks = K / 32;
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (uint64_t)rowsPadded * kBlocks) return;
@@ -123,11 +124,13 @@ template <int BN> HcclResult LaunchPlainMxPair(const void *a, const void *sfa, c
     cfg.blockDim = dim3(kGemmThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, p);
     CountLaunch();
     if (e != cudaSuccess) { HCCL_ERROR("block-scaled CTA-pair GEMM launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return HCCL_E_RUNTIME; }
