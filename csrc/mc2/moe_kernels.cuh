@@ -87,8 +87,8 @@ __device__ __forceinline__ void MoeItems(const MoeArgs &A, uint32_t cta, uint32_
 //      __match_any_sync within a warp and a running count over the warps: the layout is a function of the routing alone.
 //   4. a warp reads a 2 KB piece of a token row ONCE, quantises it once (block-scaled form: four lanes share a 1 x 32 block,
 //      so loads and stores stay coalesced) and writes it to all topK destinations.
-// One B200, one rank, 256 experts, top-8, hidden 7168, 4096 tokens, bf16: dispatch + combine took 530 us, now 210 (dispatch 113,
-// combine 94; reading and writing the rows alone 81 each); 100 tokens, block-scaled: 126 us, now 68 (what is left is host time).
+// One B200, one rank, 256 experts, top-8, hidden 7168, 4096 tokens, bf16: dispatch + combine took 530 us, now 206 (dispatch 111, combine
+// 92; reading and writing the rows alone 81 each); 100 tokens, block-scaled: 126 us, now 18, of which the host takes most.
 template <bool EMU, bool SOLO>
 __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *comms, const __grid_constant__ MoeArgs av, const MoeArgs *emuArgs)
 {

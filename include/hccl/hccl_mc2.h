@@ -49,7 +49,8 @@ typedef struct HcclOpResCtxDef {
 /* ---- Part 2: fused operators (bf16 here, block-scaled fp8 in part 3; weights are [N, K] row-major, i.e. K contiguous) ---------------------------- */
 /* C[M,N] = A[M,K] * B[N,K]^T on one GPU (the building block; also the N = 1 degenerate case of the fused ops). */
 HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream);
-/* variant 0 = automatic, 1 = one-CTA 128 x BN tiles, 2 = 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2) */
+/* variant 2 = 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2), 192 / 224 / 256 = pair tiles of that width, 1000 * S + BT = split-K with
+ * BT (16 ... 256) rows of A per tile and S (1 ... 8) CTAs along K; anything else = automatic */
 HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, int variant, cudaStream_t stream);
 /* C[M,N] = A[M,K] * B[K,N], both row-major: the input gradient of a linear layer from its [K, N] weight as stored. */
 HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream);
@@ -79,7 +80,7 @@ HcclResult HcclQuantizeMxfp8(const void *in, void *payload, void *scales, uint64
 /* C[m,n] = A[m,k] * B[n,k]^T on one GPU, both operands block-scaled, bf16 (or fp32) result. */
 HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
                          cudaStream_t stream);
-/* tileN 128 or 256 forces the tile width (0 = automatic). */
+/* tileN 128, 192 or 256 forces the tile width, 2192 / 2256 CTA pairs of that width, 100000 + 1000 * S + BT split-K (0 = automatic). */
 HcclResult HcclGemmMxfp8Variant(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
                                 int tileN, cudaStream_t stream);
 /* The three fused operators on block-scaled operands (bf16 results; shapes as for the bf16 forms, k a multiple of 128).
