@@ -175,7 +175,8 @@ HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const vo
                    (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    if (!getenv("HCCL_MX_TILE_N")) {
+    const char *tileEnv = getenv("HCCL_MX_TILE_N");
+    if (!tileEnv) {
         const SplitKChoice sk = ChooseSplitK(m, n, k, ((m + 127) / 128) * ((n + 127) / 128));
         if (sk.split) return LaunchSplitK<true>(sk, a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
@@ -186,15 +187,15 @@ HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const vo
     {
         const char *e = getenv("HCCL_MX_PAIR");
         const uint64_t pairs = (uint64_t)SmCount() / 2, rowPairs = (m + 255) / 256, t192 = rowPairs * ((n + 191) / 192), t256 = rowPairs * ((n + 255) / 256);
-        if (!(e && e[0] == '0') && !getenv("HCCL_MX_TILE_N") && n >= 256 && (t192 >= pairs || t256 * 8 >= pairs * 7)) {
+        if (!(e && e[0] == '0') && !tileEnv && n >= 256 && (t192 >= pairs || t256 * 8 >= pairs * 7)) {
             const double k4 = (double)k / 4096, c192 = (double)((t192 + pairs - 1) / pairs) * 11.2 * k4, c256 = (double)((t256 + pairs - 1) / pairs) * (14.0 * k4 + 4.5);
             return c256 < c192 ? LaunchPlainMxPair<256>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream)
                                : LaunchPlainMxPair<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
         }
     }
     // HCCL_MX_TILE_N = 192 | 256 picks the wide tile of large products (as for the fused operators)
-    if (const char *e = getenv("HCCL_MX_TILE_N")) {
-        const int v = atoi(e);
+    if (tileEnv) {
+        const int v = atoi(tileEnv);
         const uint64_t tiles = ((m + 127) / 128) * ((n + (uint64_t)(v > 0 ? v : 256) - 1) / (uint64_t)(v > 0 ? v : 256));
         if (v == 192 && tiles >= (uint64_t)SmCount()) return LaunchPlainMx<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
