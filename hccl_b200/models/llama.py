@@ -138,6 +138,11 @@ class Block(nn.Module):
         return x_local + self.mlp(self.mlp_norm(x_local))
 
 
+def _owned(targets, vocab_start, vloc):
+    """Which targets this shard owns, and the column of each (any column where it does not)."""
+    return (targets >= vocab_start) & (targets < vocab_start + vloc), (targets - vocab_start).clamp(0, vloc - 1)
+
+
 class _VocabParallelCrossEntropy(torch.autograd.Function):
     """Mean cross entropy over logits sharded along the vocabulary: max and sum-exp are all-reduced, the target logit is
     contributed by the rank that owns it."""
@@ -159,8 +164,7 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
             packed = _block.xent_sums(logits_local, targets, vocab_start, mx)
         else:
             ex = (lf - mx[:, None]).exp()
-            mine = (targets >= vocab_start) & (targets < vocab_start + vloc)
-            idx = (targets - vocab_start).clamp(0, vloc - 1)
+            mine, idx = _owned(targets, vocab_start, vloc)
             tgt = torch.where(mine, lf.gather(1, idx[:, None])[:, 0] - mx, torch.zeros_like(mx))
             packed = torch.stack([ex.sum(-1), tgt]).contiguous()
         if comm.size > 1:
@@ -179,8 +183,13 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
     def backward(ctx, g):
         if ctx.fused:
             logits, targets, mx, packed = ctx.saved_tensors
-            return _block.xent_grad(logits, targets, ctx.vocab_start, mx, packed, g.float()), None, None, None
-        p, mine, idx = ctx.saved_tensors
+            if _block.xent_grad_usable(logits, targets, g):
+                return _block.xent_grad(logits, targets, ctx.vocab_start, mx, packed, g), None, None, None
+            with torch.no_grad():                                           # what the plain form keeps
+                p = (logits.float() - mx[:, None]).exp() / packed[0][:, None]
+                mine, idx = _owned(targets, ctx.vocab_start, logits.shape[-1])
+        else:
+            p, mine, idx = ctx.saved_tensors
         grad = p.clone()
         grad[torch.arange(p.shape[0], device=p.device)[mine], idx[mine]] -= 1.0
         return (grad * (g / p.shape[0])).to(torch.bfloat16 if p.is_cuda else torch.float32), None, None, None

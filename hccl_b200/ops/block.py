@@ -37,16 +37,26 @@ def _stream(t: torch.Tensor) -> int:
     return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
+def _watched() -> bool:
+    """Whether something has to see the single operations: a function transform, dispatch mode, forward-mode level, compiler or tracer."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() > 0 or torch.autograd.forward_ad._current_level >= 0
+            or torch.compiler.is_compiling() or torch.jit.is_tracing())
+
+
+def _plain_tensor(t) -> bool:
+    """Not a subclass, and with memory of its own (a batched gradient has none)."""
+    return type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t)
+
+
 def _usable(*ts: torch.Tensor) -> bool:
     """Plain bf16 tensors on the current GPU, contiguous and 16-byte aligned, and nothing that has to see the single operations."""
-    if (torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() or torch.autograd.forward_ad._current_level >= 0
-            or torch.compiler.is_compiling() or torch.jit.is_tracing()):
+    if _watched():
         return False
     dev = ts[0].device
     if dev.type != "cuda" or dev.index != torch.cuda.current_device():
         return False
     for t in ts:
-        if type(t) not in (torch.Tensor, torch.nn.Parameter) or t.dtype != torch.bfloat16 or t.device != dev or not t.is_contiguous() or t.numel() == 0 \
+        if not _plain_tensor(t) or t.dtype != torch.bfloat16 or t.device != dev or not t.is_contiguous() or t.numel() == 0 \
                 or t.data_ptr() % 16:
             return False
     return True
@@ -166,8 +176,14 @@ def swiglu(gu: torch.Tensor, plain: Callable) -> Optional[torch.Tensor]:
 
 
 def xent_usable(logits: torch.Tensor, targets: torch.Tensor) -> bool:
-    return logits.dim() == 2 and _usable(logits) and targets.dtype == torch.int64 and targets.device == logits.device and targets.is_contiguous() \
+    return logits.dim() == 2 and _usable(logits) and _plain_tensor(targets) and targets.dtype == torch.int64 and targets.device == logits.device and targets.is_contiguous() \
         and targets.shape == logits.shape[:1]
+
+
+def xent_grad_usable(logits: torch.Tensor, targets: torch.Tensor, g: torch.Tensor) -> bool:
+    """Whether the gradient kernel may answer this backward pass: a gradient that is itself differentiated, batched or dual has to see
+    the operations."""
+    return not torch.is_grad_enabled() and xent_usable(logits, targets) and _plain_tensor(g) and g.device == logits.device
 
 
 def xent_row_max(logits: torch.Tensor) -> torch.Tensor:
@@ -184,7 +200,7 @@ def xent_sums(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, mx:
 
 
 def xent_grad(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, mx: torch.Tensor, packed: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
-    out = torch.empty_like(logits)
+    out, packed, g = torch.empty_like(logits), packed.contiguous(), g.float()
     check(_decl().HcclXent(2, logits.data_ptr(), targets.data_ptr(), vocab_start, mx.data_ptr(), packed.data_ptr(), g.data_ptr(), out.data_ptr(), *logits.shape,
                            _stream(logits)), "HcclXent")
     return out
