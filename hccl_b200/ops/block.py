@@ -62,12 +62,28 @@ def _usable(*ts: torch.Tensor) -> bool:
     return True
 
 
-def _second_order(plain: Callable, inputs, grads):
-    """Gradients of `plain(*inputs)` as a differentiable function of inputs and grads (backward with create_graph)."""
+def _plain_backward(plain: Callable, inputs, grads):
+    """Gradients of `plain(*inputs)` by the single operations, a differentiable function of inputs and grads under create_graph."""
+    again = torch.is_grad_enabled()
+    if not again:
+        inputs = [t.detach().requires_grad_(t.requires_grad) for t in inputs]
     wanted = [t for t in inputs if t.requires_grad]
     with torch.enable_grad():
-        got = iter(torch.autograd.grad(plain(*inputs), wanted, grads, create_graph=True))
+        got = iter(torch.autograd.grad(plain(*inputs), wanted, grads, create_graph=again))
     return [next(got) if t.requires_grad else None for t in inputs]
+
+
+def _direct(inputs, grads):
+    """The incoming gradients as the backward kernels read them, or None where the single operations have to run: a gradient that is
+    itself differentiated, batched or dual, an active mode, a saved tensor that came back as something else."""
+    if torch.is_grad_enabled() or not _usable(*inputs) or not all(_plain_tensor(g) and g.dtype == torch.bfloat16 and g.device == inputs[0].device for g in grads):
+        return None
+    return [_aligned(g) for g in grads]
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
 
 
 class _RmsNorm(torch.autograd.Function):
@@ -84,21 +100,17 @@ class _RmsNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd = ctx.saved_tensors
-        if torch.is_grad_enabled():
-            return (*_second_order(ctx.plain, (x, w), dy), None, None)
+        grads = _direct((x, w), (dy,))
+        if grads is None:
+            return (*_plain_backward(ctx.plain, (x, w), dy), None, None)
+        dy, = grads
         h, rows = x.shape[-1], rstd.numel()
-        dy = _aligned(dy)
         dx, dw = torch.empty_like(x), torch.empty_like(w)
         l = _decl()
         partial = torch.empty(l.HcclRmsNormBwdParts(rows, h), h, dtype=torch.float32, device=x.device)
         check(l.HcclRmsNormBwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), dw.data_ptr(), partial.data_ptr(), rows, h, _stream(x)),
               "HcclRmsNormBwd")
         return dx, dw, None, None
-
-
-def _aligned(t: torch.Tensor) -> torch.Tensor:
-    t = t.contiguous()
-    return t.clone() if t.data_ptr() % 16 else t
 
 
 def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> Optional[torch.Tensor]:
@@ -125,13 +137,19 @@ class _RopeQkv(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dq, dk, dv):
         qkv, cos, sin = ctx.saved_tensors
-        if torch.is_grad_enabled():
-            return (*_second_order(ctx.plain, (qkv,), (dq, dk, dv)), None, None, None, None, None, None)
-        dq, dk, dv = _aligned(dq), _aligned(dk), _aligned(dv)
+        grads = _direct((qkv,), (dq, dk, dv)) if _tables_ok(qkv, cos, sin) else None
+        if grads is None:
+            return (*_plain_backward(ctx.plain, (qkv,), (dq, dk, dv)), None, None, None, None, None, None)
+        dq, dk, dv = grads
         out = torch.empty_like(qkv)
         check(_decl().HcclRopeQkv(out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cos.data_ptr(), sin.data_ptr(), qkv.shape[0], cos.shape[0], *ctx.dims, 1,
                                   _stream(out)), "HcclRopeQkv")
         return out, None, None, None, None, None, None
+
+
+def _tables_ok(qkv, *tables) -> bool:
+    return all(type(t) is torch.Tensor and t.dtype == torch.float32 and t.device == qkv.device and t.is_contiguous() and not t.requires_grad and t.data_ptr() % 16 == 0
+               for t in tables)
 
 
 def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable):
@@ -140,10 +158,8 @@ def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int
     seq = cos.shape[0]
     if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or not _usable(qkv):
         return None
-    for t in (cos, sin):
-        if type(t) is not torch.Tensor or t.dtype != torch.float32 or t.device != qkv.device or t.shape != (seq, head_dim // 2) or not t.is_contiguous() \
-                or t.requires_grad or t.data_ptr() % 16:
-            return None
+    if not _tables_ok(qkv, cos, sin) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
+        return None
     return _RopeQkv.apply(qkv, cos, sin, heads, kv_heads, head_dim, plain)
 
 
@@ -160,9 +176,10 @@ class _SwiGlu(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dh):
         gu, = ctx.saved_tensors
-        if torch.is_grad_enabled():
-            return (*_second_order(ctx.plain, (gu,), dh), None)
-        dh = _aligned(dh)
+        grads = _direct((gu,), (dh,))
+        if grads is None:
+            return (*_plain_backward(ctx.plain, (gu,), dh), None)
+        dh, = grads
         out = torch.empty_like(gu)
         check(_decl().HcclSwiGluBwd(dh.data_ptr(), gu.data_ptr(), out.data_ptr(), gu.shape[0], gu.shape[1] // 2, _stream(gu)), "HcclSwiGluBwd")
         return out, None

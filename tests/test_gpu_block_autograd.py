@@ -45,3 +45,65 @@ def test_cross_entropy_gradient_depends_on_the_incoming_gradient():
     with fw.dual_level():
         gd, = torch.autograd.grad(loss, logits, fw.make_dual(torch.tensor(1.0, device="cuda"), torch.tensor(3.0, device="cuda")))
         _close(fw.unpack_dual(gd).tangent, 3 * ref, 3 * mag, logits.shape[1])
+
+
+def _op(name, seed=3):
+    """(fused function, plain function, inputs) of one part of a block."""
+    from hccl_b200.models.llama import Attention, RMSNorm, _rope_tables
+    from hccl_b200.ops import block
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(torch.bfloat16)
+    if name == "rms_norm":
+        norm = RMSNorm(64, 1e-5, torch.bfloat16, "cuda")
+        return lambda x, w: block.rms_norm(x, w, 1e-5, norm._plain), norm._plain, [draw(5, 64).requires_grad_(), draw(64).requires_grad_()]
+    if name == "rope":
+        att = Attention.__new__(Attention)
+        torch.nn.Module.__init__(att)
+        att.h_local, att.kv_local, att.hd = 4, 2, 16
+        cos, sin = _rope_tables(3, 16, 10000.0, "cuda")
+        plain = lambda t: att._rotated(t, 2, 3, cos, sin)
+        return lambda t: block.rope_qkv(t, cos, sin, 2, 4, 2, 16, plain), plain, [draw(6, 128).requires_grad_()]
+    plain = lambda t: torch.nn.functional.silu(t[:, :32]) * t[:, 32:]
+    return lambda t: block.swiglu(t, plain), plain, [draw(5, 64).requires_grad_()]
+
+
+def _outs(v):
+    return list(v) if isinstance(v, tuple) else [v]
+
+
+@pytest.mark.parametrize("name", ["rms_norm", "rope", "swiglu"])
+def test_backward_takes_what_the_single_operations_took(name):
+    """Batched and dual incoming gradients and a dispatch mode of the backward pass alone give what the plain operations give."""
+    import torch.autograd.forward_ad as fw
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    fused, plain, ins = _op(name)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    ups = [torch.randn(3, *o.shape, generator=g, device="cuda").to(torch.bfloat16) for o in _outs(plain(*ins))]
+    got, ref = (torch.autograd.grad(_outs(f(*ins)), ins, ups, is_grads_batched=True) for f in (fused, plain))
+    for a, b in zip(got, ref):
+        assert torch.equal(a, b)
+
+    def tangents(f):
+        out = _outs(f(*ins))
+        with fw.dual_level():
+            d = torch.autograd.grad(out, ins, [fw.make_dual(u[0], u[1]) for u in ups])
+            return [fw.unpack_dual(t).tangent for t in d]
+
+    if name != "swiglu":                                 # silu's backward has no forward-mode rule, in the plain form either
+        for a, b in zip(tangents(fused), tangents(plain)):
+            assert a is not None and torch.equal(a, b)
+
+    class Names(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.seen = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    out = _outs(fused(*ins))
+    with Names() as mode:
+        torch.autograd.grad(out, ins, [u[0] for u in ups])
+    assert any(s.startswith("aten.mul") for s in mode.seen)
