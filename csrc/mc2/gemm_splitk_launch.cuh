@@ -71,6 +71,10 @@ template <bool MX>
 HcclResult LaunchSplitK(SplitKChoice ch, const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32,
                         cudaStream_t s)
 {
+    if (((uintptr_t)c | (uintptr_t)sfa | (uintptr_t)sfb) & 15u) {           // four results per store, 16-byte bulk copies of the scales
+        HCCL_ERROR("split-K GEMM: result %p and block scales %p, %p must be 16-byte aligned", c, sfa, sfb);
+        return HCCL_E_PARA;
+    }
     const uint32_t kBlocks = (K + (MX ? kMxBK : kBK) - 1) / (MX ? kMxBK : kBK);
     // every CTA needs a k-block; the tensor-memory address of block scales is a multiple of two columns (64 rows), so smaller
     // block-scaled tiles have to start on a scale atom

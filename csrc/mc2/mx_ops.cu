@@ -75,6 +75,7 @@ template <int BN> HcclResult LaunchPlainMx(const void *a, const void *sfa, const
                                           cudaStream_t s)
 {
     GemmParams p{};
+    if (((uintptr_t)sfa | (uintptr_t)sfb) & 15u) { HCCL_ERROR("MXFP8 GEMM: block scales %p, %p must be 16-byte aligned", sfa, sfb); return HCCL_E_PARA; }   // bulk copies
     CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K, kBM, kMxBK, 1));
     CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K, BN, kMxBK, 1));
     CHK_RET(EncodeTmapC(&p.tmapC, c, M, N, outFp32));

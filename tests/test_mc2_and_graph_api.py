@@ -214,3 +214,21 @@ def test_graph_mode_variable_count_entry_points():
         assert np.array_equal(s.astype(np.float64), want_rs[lo:lo + int(counts[rank])])
         want = np.concatenate([a2a_in[src][int(M[src, :rank].sum()):int(M[src, :rank + 1].sum())] for src in range(n)])
         assert np.array_equal(o1, want) and np.array_equal(o2, want)
+
+
+def test_misaligned_results_and_scales_are_refused_before_any_launch():
+    """The kernel for few rows stores four results at a time and copies block scales in 16-byte pieces: an address that does not allow it
+    is a parameter error on the host. The pointers are never read here."""
+    l = lib()
+    l.HcclGemmBf16.argtypes = [vp, vp, vp, u64, u64, u64, ctypes.c_int, vp]
+    l.HcclGemmMxfp8.argtypes = [vp, vp, vp, vp, vp, u64, u64, u64, ctypes.c_int, vp]
+    l.HcclGemmMxfp8Variant.argtypes = [vp, vp, vp, vp, vp, u64, u64, u64, ctypes.c_int, ctypes.c_int, vp]
+    base = 1 << 20
+    para = int(Result.E_PARA)
+    for fp32 in (0, 1):
+        for off in (2, 4, 8):
+            assert l.HcclGemmBf16(base, base, base + off, 4, 4096, 4096, fp32, None) == para
+            assert l.HcclGemmMxfp8(base, base, base, base, base + off, 4, 4096, 4096, fp32, None) == para
+    for off in (1, 4, 8):
+        assert l.HcclGemmMxfp8(base, base + off, base, base, base, 4, 4096, 4096, 0, None) == para
+        assert l.HcclGemmMxfp8Variant(base, base, base, base + off, base, 4, 4096, 4096, 0, 128, None) == para
