@@ -63,6 +63,9 @@ __device__ __forceinline__ uint8_t ToE4m3(float v)
     return (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
 }
 
+// slotMap of an entry that has no row: its expert id lies outside [0, numExperts), or nothing was sent because a receive buffer is too small
+constexpr uint64_t kNoSlot = ~0ull;
+
 constexpr int kMoeWarps = kMoeThreads / 32;
 constexpr uint32_t kSegVecs = 128;                    // 16-byte vectors of a token row that one warp moves at a time (2 KB)
 
@@ -196,6 +199,9 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
         }
     }
 
+    if (overflow)
+        for (uint32_t i = tLo * K + tid; i < tHi * K; i += kMoeThreads) slotMap[i] = kNoSlot;
+
     // 4. scatter, in batches of whole tokens of at most kMoeThreads entries
     const uint32_t batch = kMoeThreads / K;
     const uint32_t rowVecs = A.H / 8, rowBytes = A.H * 2;
@@ -253,10 +259,16 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
             }
             for (uint32_t kk = 0; kk < K; ++kk) {
                 const uint32_t i = t * K + kk, ex = (uint32_t)A.topkIdx[i];
-                if (ex >= E) continue;
+                if (ex >= E) {
+                    if (seg == 0 && lane == 0) slotMap[i] = kNoSlot;
+                    continue;
+                }
                 const uint32_t d = ex / EL, row = sRow[(t - tb) * K + kk];
                 char *dws = c->heap[d] + A.wsOff;
-                if (!HCCL_RANGE_OK(dws + A.L.recvX + (uint64_t)row * (A.mxfp8 ? A.H : rowBytes), A.mxfp8 ? A.H : rowBytes)) continue;
+                if (!HCCL_RANGE_OK(dws + A.L.recvX + (uint64_t)row * (A.mxfp8 ? A.H : rowBytes), A.mxfp8 ? A.H : rowBytes)) {
+                    if (seg == 0 && lane == 0) slotMap[i] = kNoSlot;
+                    continue;
+                }
                 if (!A.mxfp8) {
                     uint4 *dst = (uint4 *)(dws + A.L.recvX + (uint64_t)row * rowBytes);
 #pragma unroll
@@ -312,7 +324,7 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
     }
 }
 
-// Combine: out[t] = sum over k, in order, of weight * expert row. Bound by reading topK rows per token. KMAX (8 or 16) keeps
+// Combine: out[t] = sum over k, in order, of weight * expert row, over the entries that have a row. Bound by reading topK rows per token. KMAX (8 or 16) keeps
 // the row addresses and weights of a token in registers; a warp takes 2 KB of the output row at a time, all KMAX source rows
 // of a vector in flight.
 template <bool EMU, bool SOLO, int KMAX>
@@ -345,8 +357,8 @@ __global__ void __launch_bounds__(kMoeThreads) MoeCombineKernel(const DevComm *c
         for (int j = 0; j < KMAX; ++j)
             if ((uint32_t)j < K) {
                 const uint64_t s = slotMap[t * K + j];
-                rows[j] = (const uint4 *)(c->heap[SOLO ? 0 : (uint32_t)(s >> 32)] + A.wsOff + A.L.yBuf + (uint64_t)(uint32_t)s * A.H * 2);
-                w[j] = A.weights[t * K + j];
+                rows[j] = s == kNoSlot ? nullptr : (const uint4 *)(c->heap[SOLO ? 0 : (uint32_t)(s >> 32)] + A.wsOff + A.L.yBuf + (uint64_t)(uint32_t)s * A.H * 2);
+                w[j] = s == kNoSlot ? 0.f : A.weights[t * K + j];
             }
         uint4 *dst = (uint4 *)((char *)A.out + (uint64_t)t * A.H * 2);
         const uint32_t vEnd = (seg + 1) * kSegVecs < rowVecs ? (seg + 1) * kSegVecs : rowVecs;
@@ -354,7 +366,7 @@ __global__ void __launch_bounds__(kMoeThreads) MoeCombineKernel(const DevComm *c
             float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             uint4 raw[KMAX];
 #pragma unroll
-            for (int j = 0; j < KMAX; ++j) if ((uint32_t)j < K) raw[j] = rows[j][v];
+            for (int j = 0; j < KMAX; ++j) if ((uint32_t)j < K) raw[j] = rows[j] ? rows[j][v] : make_uint4(0, 0, 0, 0);
 #pragma unroll
             for (int j = 0; j < KMAX; ++j) {
                 if ((uint32_t)j >= K) break;

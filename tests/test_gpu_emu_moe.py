@@ -150,3 +150,68 @@ def test_one_rank_layout_and_combine(T, E, K, H, mxfp8):
         d.close()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("T,E,K,H,mxfp8", [(5, 8, 2, 256, False), (40, 8, 4, 2304, True), (300, 16, 16, 512, False)])
+def test_one_rank_ids_outside_the_experts_add_nothing(T, E, K, H, mxfp8):
+    """Ids -1 and E are sent and counted nowhere; the combine leaves them out, also where an earlier call gave the entry a row and
+    whatever their weights hold."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(T)
+        x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+        idx = torch.randint(0, E, (T, K), generator=g, device="cuda").to(torch.int32)
+        w = torch.rand(T, K, generator=g, device="cuda")
+        d = MoeDispatcher(comm, E, K, H, T, max_recv_rows=T * K, mxfp8=mxfp8)
+        y = torch.randn(T * K, H, generator=g, device="cuda").to(torch.bfloat16)
+        for step in range(2):                                  # the second routing masks some entries of the first, one token wholly
+            if step:
+                idx[torch.rand(T, K, generator=g, device="cuda") < 0.3] = -1
+                idx[torch.rand(T, K, generator=g, device="cuda") < 0.1] = E
+                idx[T // 2] = -1
+            ok = (idx >= 0) & (idx < E)
+            w[~ok] = float("nan")
+            _, _, counts, src = d.dispatch(x, idx)
+            d.expert_out.copy_(y)
+            out = d.combine(w)
+            torch.cuda.synchronize()
+            flat = idx.flatten().long()
+            order = torch.argsort(torch.where(ok.flatten(), flat, E), stable=True)[: int(ok.sum())]
+            assert torch.equal(counts.long(), torch.bincount(flat[ok.flatten()], minlength=E))
+            assert torch.equal(src[: len(order)].long(), order // K)
+            slot = torch.zeros(T * K, dtype=torch.long, device="cuda")
+            slot[order] = torch.arange(len(order), device="cuda")
+            terms = torch.where(ok, w, 0.0).double()[..., None] * y[slot.view(T, K)].double()
+            ref = terms.sum(1)
+            assert bool(((out.double() - ref).abs() <= terms.abs().sum(1) * K * 2.0 ** -23 + ref.abs() * 2.0 ** -8).all())
+        assert bool((out[T // 2] == 0).all())
+        d.close()
+    finally:
+        comm.destroy()
+
+
+def test_one_rank_overflow_leaves_the_combine_no_rows():
+    """More rows than the receive buffer holds, on one rank: reported, nothing moved, and a combine that was already queued behind the
+    dispatch writes zeros."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    T, E, K, H = 64, 4, 2, 256
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        d = MoeDispatcher(comm, E, K, H, T, max_recv_rows=T * K - 1)
+        d.expert_out.fill_(3.0)
+        x, idx = torch.ones(T, H, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, K, dtype=torch.int32, device="cuda")
+        out, w = torch.ones(T, H, dtype=torch.bfloat16, device="cuda"), torch.ones(T, K, device="cuda")
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)                          # about 10 ms: the combine is queued before the dispatch has run
+        rx = d.dispatch(x, idx)[0]
+        d.combine(w, out)
+        torch.cuda.synchronize()
+        assert bool((out == 0).all())
+        with pytest.raises(Exception):
+            d.dispatch(x, idx)
+        assert rx.shape[0] == T * K - 1
+    finally:
+        comm.destroy()
