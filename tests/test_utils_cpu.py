@@ -116,3 +116,13 @@ def test_checker_command_line(tmp_path, capsys):
         assert "modelled time" in capsys.readouterr().out
     finally:
         lib().HcclSetLogLevel(2)
+
+
+def test_one_rank_moe_kernels_do_not_use_the_registered_communicator():
+    """The debug flavor's HCCL_RANGE_OK reads the communicator that MoeEnter registers. The one-rank form (SOLO) does not enter, so every use
+    it can reach has to be behind `SOLO ? ... :`, else the check would read the communicator of an earlier, perhaps destroyed, world."""
+    src = (ROOT / "csrc/mc2/moe_kernels.cuh").read_text()
+    solo = src[src.index("MoeDispatchKernel("):src.index("if (SOLO) return;")] + src[src.index("MoeCombineKernel("):]
+    for line in solo.splitlines():
+        if "HCCL_RANGE_OK" in line or "HCCL_CHECK_RANGE" in line or "BlockCopy(" in line:
+            assert "SOLO ?" in line, line
