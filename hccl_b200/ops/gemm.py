@@ -26,6 +26,14 @@ def _decl():
     return l
 
 
+def check_result(t: torch.Tensor, elems: int, dtypes, what: str = "out") -> None:
+    """`elems` results are written at the tensor's address: it has to be that large, dense and of a type the kernels write."""
+    if not t.is_contiguous() or t.numel() < elems or t.dtype not in dtypes:
+        raise ValueError(f"{what} must be a contiguous tensor of at least {elems} {' or '.join('fp32' if d is torch.float32 else 'bf16' for d in dtypes)} elements")
+    if not t.is_cuda:
+        raise ValueError(f"{what} must be a CUDA tensor")
+
+
 def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, out_dtype: torch.dtype = torch.bfloat16,
               stream=None, variant: int = 0) -> torch.Tensor:
     """a: [M, K] bf16, w: [N, K] bf16 (both row-major) -> [M, N] in `out_dtype` (bf16 or fp32).
@@ -45,6 +53,7 @@ def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None,
         return out
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
+    check_result(out, M * N, (torch.bfloat16, torch.float32))
     s = torch.cuda.current_stream() if stream is None else stream
     check(_decl().HcclGemmBf16Variant(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, int(out.dtype == torch.float32), variant, s.cuda_stream),
           "HcclGemmBf16")
@@ -67,6 +76,7 @@ def gemm_bf16_nn(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = No
         return out
     if out is None:
         out = torch.empty((M, N), dtype=out_dtype, device=a.device)
+    check_result(out, M * N, (torch.bfloat16, torch.float32))
     s = torch.cuda.current_stream() if stream is None else stream
     check(_decl().HcclGemmBf16Nn(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, int(out.dtype == torch.float32), s.cuda_stream), "HcclGemmBf16Nn")
     return out

@@ -9,6 +9,7 @@ import torch
 from .._ext import ops as _native
 from .._lib import check, lib
 from ..types import DataType
+from .gemm import check_result
 
 
 def _decl():
@@ -28,8 +29,14 @@ def _stream(stream):
     return (torch.cuda.current_stream() if stream is None else stream).cuda_stream
 
 
-def _chk(*ts):
-    for t in ts:
+def _chk(a, w, rows, out, gathered=None):
+    """The checks of the extension's `fused`: operands [m, k] and [n, k], results dense, bf16 and large enough."""
+    if a.dim() != 2 or w.dim() < 1 or w.numel() != w.shape[0] * a.shape[1]:
+        raise ValueError("fused ops take matrices [m, k] and [n, k]")
+    for t, elems, what in ((out, rows * w.shape[0], "out"), (gathered, rows * a.shape[1], "gathered")):
+        if t is not None:
+            check_result(t, elems, (torch.bfloat16,), what)
+    for t in (a, w):
         if not (t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous()):
             raise ValueError("fused ops take contiguous bf16 CUDA tensors")
 
@@ -43,7 +50,7 @@ def all_gather_matmul(comm, a_local: torch.Tensor, w: torch.Tensor, out: Optiona
         if rc:
             check(rc, "HcclAllGatherMatmul")
         return out
-    _chk(a_local, w)
+    _chk(a_local, w, a_local.shape[0] * comm.size, out, gathered)
     m, k = a_local.shape
     n = w.shape[0]
     if out is None:
@@ -61,7 +68,7 @@ def matmul_reduce_scatter(comm, a: torch.Tensor, w: torch.Tensor, out: Optional[
         if rc:
             check(rc, "HcclMatmulReduceScatter")
         return out
-    _chk(a, w)
+    _chk(a, w, a.shape[0] // comm.size, out)
     m, k = a.shape
     n = w.shape[0]
     if out is None:
@@ -79,7 +86,7 @@ def matmul_all_reduce(comm, a: torch.Tensor, w: torch.Tensor, out: Optional[torc
         if rc:
             check(rc, "HcclMatmulAllReduce")
         return out
-    _chk(a, w)
+    _chk(a, w, a.shape[0], out)
     m, k = a.shape
     n = w.shape[0]
     if out is None:

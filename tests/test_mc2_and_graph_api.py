@@ -9,6 +9,8 @@ entry addressed by group name and tag).
 import ctypes
 
 import numpy as np
+import pytest
+import torch
 
 from hccl_b200._lib import lib
 from hccl_b200.types import DataType, Result
@@ -232,3 +234,46 @@ def test_misaligned_results_and_scales_are_refused_before_any_launch():
     for off in (1, 4, 8):
         assert l.HcclGemmMxfp8(base, base + off, base, base, base, 4, 4096, 4096, 0, None) == para
         assert l.HcclGemmMxfp8Variant(base, base, base, base + off, base, 4, 4096, 4096, 0, 128, None) == para
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_fused_operators_check_shapes_and_results_on_the_host(native, monkeypatch):
+    """An operand or result that does not hold what the kernel reads or writes is an error before anything is launched, in the extension and
+    in the ctypes form (CPU tensors: a call that passed the checks of shape and type is refused for its device)."""
+    from types import SimpleNamespace
+
+    from hccl_b200.ops import gemm, mc2
+
+    if not native:
+        monkeypatch.setattr(mc2, "_native", lambda: None)
+    elif mc2._native() is None:
+        pytest.skip("the extension is not built")
+    comm = SimpleNamespace(handle=0, size=2)
+    e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt)
+    a, w = e(8, 16), e(24, 16)
+    calls = {"agmm": (mc2.all_gather_matmul, 16), "mmrs": (mc2.matmul_reduce_scatter, 4), "mmar": (mc2.matmul_all_reduce, 8)}
+    for fn, rows in calls.values():
+        for bad in (e(24, 8), e(24), e(24, 17)):
+            with pytest.raises(ValueError, match="matrices"):
+                fn(comm, a, bad)
+        with pytest.raises(ValueError, match="matrices"):
+            fn(comm, e(8, 2, 8), w)
+        for out in (e(rows, 23), e(rows * 24 - 1), e(rows, 24, dt=torch.float32), e(24, rows).t()):
+            with pytest.raises(ValueError, match="out must be a contiguous"):
+                fn(comm, a, w, out=out)
+        with pytest.raises(ValueError, match="out must be a CUDA"):
+            fn(comm, a, w, out=e(rows + 1, 24))
+        for good in (w, e(24, 4, 4)):
+            with pytest.raises(ValueError, match="contiguous bf16 CUDA"):
+                fn(comm, a, good)
+    for gathered in (e(15, 16), e(16, 16, dt=torch.float32)):
+        with pytest.raises(ValueError, match="gathered must be"):
+            mc2.all_gather_matmul(comm, a, w, gathered=gathered)
+    if native:
+        ext = mc2._native()
+        for out in (e(8, 23), e(8, 24, dt=torch.float16), e(24, 8).t()):
+            with pytest.raises(ValueError, match="out must be a contiguous"):
+                ext.gemm(a, w, out, False, False, 0, None)
+    else:
+        with pytest.raises(ValueError, match="bf16 or fp32"):
+            gemm.check_result(e(8, 23), 8 * 24, (torch.bfloat16, torch.float32))
