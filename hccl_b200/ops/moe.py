@@ -78,11 +78,12 @@ class MoeDispatcher:
         at = (rx.value, rs.value, rc.value, rsrc.value)
         if self._recv is None or self._recv[0] != at:
             dev = x.device
-            self._recv = (at, _view(rx.value, (self.cap, self.hidden), torch.float8_e4m3fn if self.mxfp8 else torch.bfloat16, dev),
-                          _view(rs.value, (self.cap, self.hidden // 32), torch.uint8, dev) if self.mxfp8 else None,
-                          _view(rc.value, (self.local_experts,), torch.int32, dev), _view(rsrc.value, (self.cap,), torch.int32, dev))
-        # new tensor objects over the same memory on every call, as the caller may do with them what it likes
-        return tuple(None if t is None else t.detach() for t in self._recv[1:])
+            with torch.inference_mode(False):        # kept beyond this call, which may be an inference pass
+                self._recv = (at, _view(rx.value, (self.cap, self.hidden), torch.float8_e4m3fn if self.mxfp8 else torch.bfloat16, dev),
+                              _view(rs.value, (self.cap, self.hidden // 32), torch.uint8, dev) if self.mxfp8 else None,
+                              _view(rc.value, (self.local_experts,), torch.int32, dev), _view(rsrc.value, (self.cap,), torch.int32, dev))
+        # new tensors over the same memory on every call (`data`: with a version count of their own), as the caller may do with them what it likes
+        return tuple(None if t is None else t.data for t in self._recv[1:])
 
     def combine(self, topk_weights: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
         assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()

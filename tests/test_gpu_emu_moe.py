@@ -215,3 +215,26 @@ def test_one_rank_overflow_leaves_the_combine_no_rows():
         assert rx.shape[0] == T * K - 1
     finally:
         comm.destroy()
+
+
+def test_receive_views_belong_to_their_call():
+    """A first dispatch under inference mode leaves later ones trainable, and writing one call's tensor does not mark another's as changed."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        d = MoeDispatcher(comm, 8, 2, 256, 16, max_recv_rows=32)
+        x = torch.randn(16, 256, device="cuda").to(torch.bfloat16)
+        idx = torch.randint(0, 8, (16, 2), device="cuda", dtype=torch.int32)
+        w = torch.randn(256, 64, device="cuda").to(torch.bfloat16).requires_grad_()
+        with torch.inference_mode():
+            d.dispatch(x, idx)
+        first = d.dispatch(x, idx)[0]
+        y = first @ w
+        second = d.dispatch(x, idx)[0]
+        second.mul_(1)
+        torch.autograd.backward(y, torch.ones_like(y))
+        assert torch.equal(w.grad, first.t() @ torch.ones_like(y))
+        d.close()
+    finally:
+        comm.destroy()
