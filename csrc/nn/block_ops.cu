@@ -48,10 +48,12 @@ template <int TPR> __device__ __forceinline__ float RowSum(float v, float *red)
     return s;
 }
 
-// y = x * rsqrt(mean(x^2) + eps) * w. A row is shared by TPR threads; the second pass over it hits L1 / L2.
-template <int TPR>
+// y = x * rsqrt(mean(x^2) + eps) * w. A row is shared by TPR threads; the second pass over it hits L1 / L2. KEEP: x and w are copied on
+// the way for a backward pass that may come after they were changed.
+template <int TPR, bool KEEP>
 __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ y,
-                                                         float *__restrict__ rstd, uint32_t T, uint32_t H, float eps)
+                                                         float *__restrict__ rstd, __nv_bfloat16 *__restrict__ xKept, __nv_bfloat16 *__restrict__ wKept, uint32_t T,
+                                                         uint32_t H, float eps)
 {
     __shared__ float red[kThreads / 32];
     const uint32_t row = blockIdx.x * (kThreads / TPR) + threadIdx.x / TPR, lane = threadIdx.x % TPR;
@@ -59,8 +61,10 @@ __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *_
     const uint4 *xr = (const uint4 *)(x + (size_t)row * H), *wr = (const uint4 *)w;
     float s = 0.f;
     for (uint32_t v = lane; v < H / 8; v += TPR) {
+        const uint4 raw = xr[v];
+        if (KEEP) ((uint4 *)(xKept + (size_t)row * H))[v] = raw;
         float f[8];
-        Unpack8(xr[v], f);
+        Unpack8(raw, f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += f[j] * f[j];
     }
@@ -68,9 +72,11 @@ __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *_
     if (lane == 0) rstd[row] = r;
     uint4 *yr = (uint4 *)(y + (size_t)row * H);
     for (uint32_t v = lane; v < H / 8; v += TPR) {
+        const uint4 wv = wr[v];
+        if (KEEP && row == 0) ((uint4 *)wKept)[v] = wv;
         float f[8], g[8];
         Unpack8(xr[v], f);
-        Unpack8(wr[v], g);
+        Unpack8(wv, g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
         yr[v] = Pack8(f);
@@ -362,6 +368,18 @@ void LaunchRmsNormBwd(const void *dy, const void *x, const void *w, const float 
 
 bool NormShapeOk(uint64_t T, uint64_t H) { return T > 0 && T <= 0x7fffffff && H > 0 && H % 8 == 0 && H <= kNormMax; }
 
+HcclResult LaunchRmsNorm(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
+{
+    if (!x || !w || !y || !rstd) return HCCL_E_PTR;
+    if (!NormShapeOk(rows, hidden) || !Aligned16(x) || !Aligned16(w) || !Aligned16(y) || !Aligned16(xKept) || !Aligned16(wKept)) return HCCL_E_PARA;
+    const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden;
+    const bool warp = hidden <= kWarpRowMax;
+    auto kern = warp ? (xKept ? RmsNormKernel<32, true> : RmsNormKernel<32, false>) : (xKept ? RmsNormKernel<kThreads, true> : RmsNormKernel<kThreads, false>);
+    kern<<<warp ? (T + 7) / 8 : T, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, (__nv_bfloat16 *)xKept,
+                                                         (__nv_bfloat16 *)wKept, T, H, eps);
+    return Launched("RMSNorm");
+}
+
 }  // namespace
 }  // namespace nn
 }  // namespace hccl
@@ -373,13 +391,13 @@ extern "C" {
 
 HcclResult HcclRmsNorm(const void *x, const void *w, void *y, float *rstd, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
 {
-    if (!x || !w || !y || !rstd) return HCCL_E_PTR;
-    if (!NormShapeOk(rows, hidden) || !Aligned16(x) || !Aligned16(w) || !Aligned16(y)) return HCCL_E_PARA;
-    const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden;
-    if (hidden <= kWarpRowMax)
-        RmsNormKernel<32><<<(T + 7) / 8, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, T, H, eps);
-    else RmsNormKernel<kThreads><<<T, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, T, H, eps);
-    return Launched("RMSNorm");
+    return LaunchRmsNorm(x, w, y, rstd, nullptr, nullptr, rows, hidden, eps, stream);
+}
+
+HcclResult HcclRmsNormKeep(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
+{
+    if (!xKept || !wKept) return HCCL_E_PTR;
+    return LaunchRmsNorm(x, w, y, rstd, xKept, wKept, rows, hidden, eps, stream);
 }
 
 uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden)

@@ -20,6 +20,7 @@ def _decl():
     if not getattr(l, "_nn_declared", False):
         vp, u32, u64, i32, i64, f32 = ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint64, ctypes.c_int, ctypes.c_int64, ctypes.c_float
         l.HcclRmsNorm.argtypes = [vp, vp, vp, vp, u64, u64, f32, vp]
+        l.HcclRmsNormKeep.argtypes = [vp, vp, vp, vp, vp, vp, u64, u64, f32, vp]
         l.HcclRmsNormBwdParts.argtypes = [u64, u64]
         l.HcclRmsNormBwdParts.restype = u64
         l.HcclRmsNormBwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, u64, u64, vp]
@@ -27,7 +28,7 @@ def _decl():
         l.HcclSwiGlu.argtypes = [vp, vp, u64, u64, vp]
         l.HcclSwiGluBwd.argtypes = [vp, vp, vp, u64, u64, vp]
         l.HcclXent.argtypes = [i32, vp, vp, i64, vp, vp, vp, vp, u64, u64, vp]
-        for f in (l.HcclRmsNorm, l.HcclRmsNormBwd, l.HcclRopeQkv, l.HcclSwiGlu, l.HcclSwiGluBwd, l.HcclXent):
+        for f in (l.HcclRmsNorm, l.HcclRmsNormKeep, l.HcclRmsNormBwd, l.HcclRopeQkv, l.HcclSwiGlu, l.HcclSwiGluBwd, l.HcclXent):
             f.restype = ctypes.c_int
         l._nn_declared = True
     return l
@@ -87,30 +88,38 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
 
 
 class _RmsNorm(torch.autograd.Function):
+    """-> (y, x, w). The backward pass reads copies of x and w that the kernel makes on its way, since the caller may change both before it
+    (x += f(norm(x)), an optimizer step). The copies are outputs, so that the gradient of a gradient finds its way to x and w."""
+
     @staticmethod
     def forward(ctx, x, w, eps, plain):
         h = x.shape[-1]
-        y = torch.empty_like(x)
+        y, xk, wk = torch.empty_like(x), torch.empty_like(x), torch.empty_like(w)
         rstd = torch.empty(x.numel() // h, dtype=torch.float32, device=x.device)
-        check(_decl().HcclRmsNorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), rstd.numel(), h, eps, _stream(x)), "HcclRmsNorm")
-        ctx.save_for_backward(x, w, rstd)
+        check(_decl().HcclRmsNormKeep(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), xk.data_ptr(), wk.data_ptr(), rstd.numel(), h, eps, _stream(x)),
+              "HcclRmsNormKeep")
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(xk, wk, rstd)
         ctx.plain = plain
-        return y
+        return y, xk, wk
 
     @staticmethod
-    def backward(ctx, dy):
+    def backward(ctx, dy, dxk, dwk):
         x, w, rstd = ctx.saved_tensors
+        if dy is None:
+            return dxk, dwk, None, None
         grads = _direct((x, w), (dy,))
         if grads is None:
-            return (*_plain_backward(ctx.plain, (x, w), dy), None, None)
-        dy, = grads
-        h, rows = x.shape[-1], rstd.numel()
-        dx, dw = torch.empty_like(x), torch.empty_like(w)
-        l = _decl()
-        partial = torch.empty(l.HcclRmsNormBwdParts(rows, h), h, dtype=torch.float32, device=x.device)
-        check(l.HcclRmsNormBwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), dw.data_ptr(), partial.data_ptr(), rows, h, _stream(x)),
-              "HcclRmsNormBwd")
-        return dx, dw, None, None
+            dx, dw = _plain_backward(ctx.plain, (x, w), dy)
+        else:
+            dy, = grads
+            h, rows = x.shape[-1], rstd.numel()
+            dx, dw = torch.empty_like(x), torch.empty_like(w)
+            l = _decl()
+            partial = torch.empty(l.HcclRmsNormBwdParts(rows, h), h, dtype=torch.float32, device=x.device)
+            check(l.HcclRmsNormBwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), dw.data_ptr(), partial.data_ptr(), rows, h, _stream(x)),
+                  "HcclRmsNormBwd")
+        return dx if dxk is None else dx + dxk, dw if dwk is None else dw + dwk, None, None
 
 
 def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> Optional[torch.Tensor]:
@@ -118,7 +127,11 @@ def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> O
     h = x.shape[-1] if x.dim() else 0
     if h % 8 or h > 12288 or w.shape != (h,) or not _usable(x, w):
         return None
-    return _RmsNorm.apply(x, w, eps, plain)
+    if torch.is_grad_enabled() and (x.requires_grad or w.requires_grad):
+        return _RmsNorm.apply(x, w, eps, plain)[0]
+    y, rstd = torch.empty_like(x), torch.empty(x.numel() // h, dtype=torch.float32, device=x.device)
+    check(_decl().HcclRmsNorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), rstd.numel(), h, eps, _stream(x)), "HcclRmsNorm")
+    return y
 
 
 class _RopeQkv(torch.autograd.Function):

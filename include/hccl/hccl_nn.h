@@ -14,6 +14,8 @@ extern "C" {
 /* y[rows, hidden] = x * rsqrt(mean(x^2) + eps) * w; rstd[rows] receives the reciprocal norms for the backward pass.
  * hidden: a multiple of 8, at most 12288. */
 HcclResult HcclRmsNorm(const void *x, const void *w, void *y, float *rstd, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
+/* The same, and copies of x and w: what the backward pass reads where x or w may be changed in between. */
+HcclResult HcclRmsNormKeep(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
 /* Rows of the fp32 workspace `partial` [parts, hidden] that HcclRmsNormBwd needs. */
 uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden);
 HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, void *dw, float *partial, uint64_t rows, uint64_t hidden,

@@ -107,3 +107,39 @@ def test_backward_takes_what_the_single_operations_took(name):
     with Names() as mode:
         torch.autograd.grad(out, ins, [u[0] for u in ups])
     assert any(s.startswith("aten.mul") for s in mode.seen)
+
+
+@pytest.mark.parametrize("rows,hidden", [(5, 64), (3, 2048)])
+def test_norm_input_and_weight_may_change_before_the_backward_pass(rows, hidden):
+    """x += ..., a changed weight and a changed result after the norm: first and second derivatives are those of the values it saw."""
+    from hccl_b200.models.llama import RMSNorm
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    norm = RMSNorm(hidden, 1e-5, torch.bfloat16, "cuda")
+    leaf = torch.randn(rows, hidden, generator=g, device="cuda").to(torch.bfloat16).requires_grad_()
+    dy = torch.randn(rows, hidden, generator=g, device="cuda").to(torch.bfloat16)
+    kept = norm.weight.detach().clone()
+
+    def grads(change):
+        with torch.no_grad():
+            norm.weight.copy_(kept)
+        x = leaf * 1
+        y = norm(x)
+        out = y * 1
+        if change:
+            with torch.no_grad():
+                y.zero_()
+                norm.weight.mul_(2)
+            x += 1
+        first = torch.autograd.grad(out, [x if not change else leaf, norm.weight], dy, create_graph=True)
+        return first, torch.autograd.grad(first[0].float().square().sum() + first[1].float().square().sum(), [leaf, norm.weight])
+
+    (a1, a2), (b1, b2) = grads(False), grads(True)
+    for a, b in zip(a1 + a2, b1 + b2):
+        assert torch.equal(a, b)
+    plain = norm._plain(leaf, kept.requires_grad_())
+    p1 = torch.autograd.grad(plain, [leaf, kept], dy, create_graph=True)
+    p2 = torch.autograd.grad(p1[0].float().square().sum() + p1[1].float().square().sum(), [leaf, kept])
+    for a, p in zip(a1 + a2, p1 + p2):                      # the same operations, rounded to bf16 in between at most three times more
+        assert (a.double() - p.double()).norm() <= 3 * 2.0 ** -8 * p.double().norm()
+    with torch.no_grad():
+        assert torch.equal(norm(leaf), norm._plain(leaf, norm.weight)) or (norm(leaf).double() - norm._plain(leaf, norm.weight).double()).norm() < 2.0 ** -8 * plain.norm()
