@@ -34,7 +34,7 @@ MoeLayout MakeLayout(const HcclMoeConfig &c)
     L.recvX = off; off += Al(cap * c.hidden * (c.mxfp8 ? 1 : 2));
     L.recvScales = off; off += Al(c.mxfp8 ? cap * (c.hidden / 32) : 0);
     L.recvSrc = off; off += Al(cap * 4);
-    L.yBuf = off; off += Al(cap * c.hidden * 2);
+    L.yBuf = off; off += Al((cap + 1) * c.hidden * 2);            // and a row of zeros
     L.recvCounts = off; off += Al((uint64_t)kMaxExperts * 4);
     L.slotMap = off; off += Al(entries * 8);
     L.total = off;

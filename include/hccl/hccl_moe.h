@@ -43,9 +43,9 @@ HcclResult HcclMoeDestroy(HcclMoeHandle handle);
  *   recvScales  [rows, hidden/32] e8m0 (mxfp8 only, else NULL)
  *   recvCounts  [numExperts / ranks] int32 rows per local expert
  *   recvSrc     [rows] int32 = (source rank << 24) | source token
- * An entry whose id lies outside [0, numExperts) (a masked choice) is sent nowhere, counted nowhere and adds nothing in the combine. Where
+ * An entry whose id lies outside [0, numExperts) (a masked choice) is sent nowhere, counted nowhere and answered by zeros in the combine. Where
  * some rank's rows exceed maxRecvRows nothing is sent, that rank's communicator reports an asynchronous error, and the combine of that routing
- * writes zeros. */
+ * sees zeros only. */
 HcclResult HcclMoeDispatch(HcclMoeHandle handle, const void *x, const int32_t *topkIdx, uint32_t numTokens, void **recvX, void **recvScales,
                            int32_t **recvCounts, int32_t **recvSrc, cudaStream_t stream);
 /* Symmetric buffer [maxRecvRows, hidden] bf16 the caller fills with expert outputs, row i answering recvX row i. */

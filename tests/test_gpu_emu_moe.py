@@ -154,8 +154,8 @@ def test_one_rank_layout_and_combine(T, E, K, H, mxfp8):
 
 @pytest.mark.parametrize("T,E,K,H,mxfp8", [(5, 8, 2, 256, False), (40, 8, 4, 2304, True), (300, 16, 16, 512, False)])
 def test_one_rank_ids_outside_the_experts_add_nothing(T, E, K, H, mxfp8):
-    """Ids -1 and E are sent and counted nowhere; the combine leaves them out, also where an earlier call gave the entry a row and
-    whatever their weights hold."""
+    """Ids -1 and E are sent and counted nowhere; the combine reads zeros for them, also where an earlier call gave the entry a
+    row and whatever the expert outputs hold."""
     from hccl_b200.comm import Communicator, get_root_info
     from hccl_b200.ops.moe import MoeDispatcher
     comm = Communicator.from_root_info(1, get_root_info(), 0)
@@ -165,15 +165,15 @@ def test_one_rank_ids_outside_the_experts_add_nothing(T, E, K, H, mxfp8):
         idx = torch.randint(0, E, (T, K), generator=g, device="cuda").to(torch.int32)
         w = torch.rand(T, K, generator=g, device="cuda")
         d = MoeDispatcher(comm, E, K, H, T, max_recv_rows=T * K, mxfp8=mxfp8)
-        y = torch.randn(T * K, H, generator=g, device="cuda").to(torch.bfloat16)
         for step in range(2):                                  # the second routing masks some entries of the first, one token wholly
             if step:
                 idx[torch.rand(T, K, generator=g, device="cuda") < 0.3] = -1
                 idx[torch.rand(T, K, generator=g, device="cuda") < 0.1] = E
                 idx[T // 2] = -1
             ok = (idx >= 0) & (idx < E)
-            w[~ok] = float("nan")
             _, _, counts, src = d.dispatch(x, idx)
+            y = torch.randn(T * K, H, generator=g, device="cuda").to(torch.bfloat16)
+            y[int(ok.sum()):] = float("nan")                   # no expert wrote these rows
             d.expert_out.copy_(y)
             out = d.combine(w)
             torch.cuda.synchronize()
@@ -183,7 +183,7 @@ def test_one_rank_ids_outside_the_experts_add_nothing(T, E, K, H, mxfp8):
             assert torch.equal(src[: len(order)].long(), order // K)
             slot = torch.zeros(T * K, dtype=torch.long, device="cuda")
             slot[order] = torch.arange(len(order), device="cuda")
-            terms = torch.where(ok, w, 0.0).double()[..., None] * y[slot.view(T, K)].double()
+            terms = torch.where(ok[..., None], w.double()[..., None] * y[slot.view(T, K)].double(), 0.0)
             ref = terms.sum(1)
             assert bool(((out.double() - ref).abs() <= terms.abs().sum(1) * K * 2.0 ** -23 + ref.abs() * 2.0 ** -8).all())
         assert bool((out[T // 2] == 0).all())
