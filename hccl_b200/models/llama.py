@@ -174,7 +174,8 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
         loss = (denom.log() - tgt).mean()
         if ctx.fused:
             ctx.vocab_start = vocab_start
-            ctx.save_for_backward(logits_local, targets, mx, packed)
+            if ctx.needs_input_grad[0]:                                     # copies: the caller may write its tensors before the backward pass
+                ctx.save_for_backward(logits_local.clone(), targets.clone(), mx, packed)
         else:
             ctx.save_for_backward(ex / denom[:, None], mine, idx)
         return loss

@@ -143,3 +143,15 @@ def test_norm_input_and_weight_may_change_before_the_backward_pass(rows, hidden)
         assert (a.double() - p.double()).norm() <= 3 * 2.0 ** -8 * p.double().norm()
     with torch.no_grad():
         assert torch.equal(norm(leaf), norm._plain(leaf, norm.weight)) or (norm(leaf).double() - norm._plain(leaf, norm.weight).double()).norm() < 2.0 ** -8 * plain.norm()
+
+
+def test_targets_and_logits_may_change_before_the_backward_pass():
+    """A token buffer refilled between two losses, logits scaled in place after the loss: the gradient is that of the values it saw."""
+    from hccl_b200.models.llama import _VocabParallelCrossEntropy as X
+    leaf, targets, ref, mag = _logits()
+    logits = leaf * 1
+    loss = X.apply(logits, targets, _OneRank, 0)
+    logits.mul_(3)
+    targets.zero_()
+    g, = torch.autograd.grad(loss, leaf)
+    _close(g, ref, mag, leaf.shape[1])
