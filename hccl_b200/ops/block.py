@@ -77,9 +77,10 @@ def _plain_backward(plain: Callable, inputs, grads):
 def _direct(inputs, grads):
     """The incoming gradients as the backward kernels read them, or None where the single operations have to run: a gradient that is
     itself differentiated, batched or dual, an active mode, a saved tensor that came back as something else."""
-    if torch.is_grad_enabled() or not _usable(*inputs) or not all(_plain_tensor(g) and g.dtype == torch.bfloat16 and g.device == inputs[0].device for g in grads):
+    if torch.is_grad_enabled() or not all(_plain_tensor(g) and g.dtype == torch.bfloat16 and g.device == grads[0].device for g in grads):
         return None
-    return [_aligned(g) for g in grads]
+    grads = [_aligned(g) for g in grads]
+    return grads if _usable(grads[0], *inputs) else None
 
 
 def _aligned(t: torch.Tensor) -> torch.Tensor:
@@ -143,25 +144,26 @@ class _RopeQkv(torch.autograd.Function):
         v = torch.empty_like(k)
         check(_decl().HcclRopeQkv(qkv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), t, seq, heads, kv_heads, head_dim, 0,
                                   _stream(qkv)), "HcclRopeQkv")
-        ctx.save_for_backward(qkv, cos, sin)
-        ctx.dims, ctx.plain = (heads, kv_heads, head_dim), plain
+        ctx.save_for_backward(cos, sin)                # the rotation is linear: its gradient does not depend on qkv
+        ctx.shape, ctx.dims, ctx.plain = qkv.shape, (heads, kv_heads, head_dim), plain
         return q, k, v
 
     @staticmethod
     def backward(ctx, dq, dk, dv):
-        qkv, cos, sin = ctx.saved_tensors
-        grads = _direct((qkv,), (dq, dk, dv)) if _tables_ok(qkv, cos, sin) else None
+        cos, sin = ctx.saved_tensors
+        grads = _direct((), (dq, dk, dv)) if _tables_ok(cos.device, cos, sin) else None
         if grads is None:
-            return (*_plain_backward(ctx.plain, (qkv,), (dq, dk, dv)), None, None, None, None, None, None)
+            at = torch.zeros(ctx.shape, dtype=torch.bfloat16, device=cos.device, requires_grad=True)
+            return (*_plain_backward(ctx.plain, (at,), (dq, dk, dv)), None, None, None, None, None, None)
         dq, dk, dv = grads
-        out = torch.empty_like(qkv)
-        check(_decl().HcclRopeQkv(out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cos.data_ptr(), sin.data_ptr(), qkv.shape[0], cos.shape[0], *ctx.dims, 1,
+        out = torch.empty(ctx.shape, dtype=dq.dtype, device=dq.device)
+        check(_decl().HcclRopeQkv(out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cos.data_ptr(), sin.data_ptr(), ctx.shape[0], cos.shape[0], *ctx.dims, 1,
                                   _stream(out)), "HcclRopeQkv")
         return out, None, None, None, None, None, None
 
 
-def _tables_ok(qkv, *tables) -> bool:
-    return all(type(t) is torch.Tensor and t.dtype == torch.float32 and t.device == qkv.device and t.is_contiguous() and not t.requires_grad and t.data_ptr() % 16 == 0
+def _tables_ok(device, *tables) -> bool:
+    return all(type(t) is torch.Tensor and t.dtype == torch.float32 and t.device == device and t.is_contiguous() and not t.requires_grad and t.data_ptr() % 16 == 0
                for t in tables)
 
 
@@ -171,7 +173,7 @@ def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int
     seq = cos.shape[0]
     if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or not _usable(qkv):
         return None
-    if not _tables_ok(qkv, cos, sin) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
+    if not _tables_ok(qkv.device, cos, sin) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
         return None
     return _RopeQkv.apply(qkv, cos, sin, heads, kv_heads, head_dim, plain)
 

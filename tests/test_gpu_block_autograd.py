@@ -155,3 +155,22 @@ def test_targets_and_logits_may_change_before_the_backward_pass():
     targets.zero_()
     g, = torch.autograd.grad(loss, leaf)
     _close(g, ref, mag, leaf.shape[1])
+
+
+def test_rotary_embedding_keeps_nothing_of_the_projection():
+    """The rotation is linear: the packed projection is neither kept for the backward pass nor missed when it has changed; the gradient of
+    a gradient (by the incoming gradient) is the plain form's."""
+    fused, plain, (leaf,) = _op("rope")
+    kept = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: kept.append(t.shape) or t, lambda t: t):
+        qkv = leaf * 1
+        out = fused(qkv)
+    assert leaf.shape not in kept
+    qkv.zero_()
+    ups = [torch.randn(o.shape, device="cuda").to(torch.bfloat16).requires_grad_() for o in out]
+    got, = torch.autograd.grad(out, leaf, ups, create_graph=True)
+    ref, = torch.autograd.grad(plain(leaf), leaf, ups, create_graph=True)
+    assert torch.equal(got, ref)
+    c = torch.randn(leaf.shape, device="cuda").to(torch.bfloat16)
+    for a, b in zip(torch.autograd.grad(got, ups, c), torch.autograd.grad(ref, ups, c)):
+        assert torch.equal(a, b)
