@@ -64,8 +64,11 @@ class RMSNorm(nn.Module):
         self.weight.replicated_under_sequence_parallel = True
 
     def forward(self, x):
-        y = _block.rms_norm(x, self.weight, self.eps, self._plain)
-        return self._plain(x, self.weight) if y is None else y
+        if not torch.jit.is_scripting():
+            y = _block.rms_norm(x, self.weight, self.eps, self._plain)
+            if y is not None:
+                return y
+        return self._plain(x, self.weight)
 
     def _plain(self, x, w):
         v = x.float()

@@ -81,3 +81,11 @@ def test_llama_loss_and_grads_match_single_rank(tp):
         assert torch.allclose(e, e1, atol=1e-5) and torch.allclose(n, n1, atol=1e-5)
         assert torch.allclose(o, o1[:, r * kl:(r + 1) * kl], atol=1e-5)
         assert torch.allclose(h, h1[r * vl:(r + 1) * vl], atol=1e-5)
+
+
+def test_rms_norm_can_be_scripted():
+    """TorchScript compiles the plain form of the norm."""
+    from hccl_b200.models.llama import RMSNorm
+    norm = RMSNorm(64, 1e-5, torch.bfloat16, "cpu")
+    x = torch.randn(3, 64, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    assert torch.equal(torch.jit.script(norm)(x), norm(x))
