@@ -51,7 +51,7 @@ def _plain_tensor(t) -> bool:
 
 def _usable(*ts: torch.Tensor) -> bool:
     """Plain bf16 tensors on the current GPU, contiguous and 16-byte aligned, and nothing that has to see the single operations."""
-    if _watched():
+    if _watched() or not _plain_tensor(ts[0]):
         return False
     dev = ts[0].device
     if dev.type != "cuda" or dev.index != torch.cuda.current_device():
@@ -125,8 +125,10 @@ class _RmsNorm(torch.autograd.Function):
 
 def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> Optional[torch.Tensor]:
     """x * rsqrt(mean(x^2) + eps) * w over the last dimension; `plain(x, w)` is the same in PyTorch."""
+    if not _usable(x, w):
+        return None
     h = x.shape[-1] if x.dim() else 0
-    if h % 8 or h > 12288 or w.shape != (h,) or not _usable(x, w):
+    if h % 8 or h > 12288 or w.shape != (h,):
         return None
     if torch.is_grad_enabled() and (x.requires_grad or w.requires_grad):
         return _RmsNorm.apply(x, w, eps, plain)[0]
@@ -170,10 +172,10 @@ def _tables_ok(device, *tables) -> bool:
 def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable):
     """Packed [batch * seq, (heads + 2 kv_heads) * head_dim] -> rotated q, k and v as [batch, seq, heads, head_dim]; cos / sin are fp32
     [seq, head_dim / 2] constants. `plain(qkv)` is the same in PyTorch."""
-    seq = cos.shape[0]
-    if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or not _usable(qkv):
+    if not _usable(qkv) or not _tables_ok(qkv.device, cos, sin):
         return None
-    if not _tables_ok(qkv.device, cos, sin) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
+    seq = cos.shape[0] if cos.dim() else 0
+    if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
         return None
     return _RopeQkv.apply(qkv, cos, sin, heads, kv_heads, head_dim, plain)
 
@@ -202,13 +204,13 @@ class _SwiGlu(torch.autograd.Function):
 
 def swiglu(gu: torch.Tensor, plain: Callable) -> Optional[torch.Tensor]:
     """silu(gate) * up for gu = [rows, gate | up]; `plain(gu)` is the same in PyTorch."""
-    if gu.dim() != 2 or gu.shape[1] % 16 or not _usable(gu):
+    if not _usable(gu) or gu.dim() != 2 or gu.shape[1] % 16:
         return None
     return _SwiGlu.apply(gu, plain)
 
 
 def xent_usable(logits: torch.Tensor, targets: torch.Tensor) -> bool:
-    return logits.dim() == 2 and _usable(logits) and _plain_tensor(targets) and targets.dtype == torch.int64 and targets.device == logits.device and targets.is_contiguous() \
+    return _usable(logits) and logits.dim() == 2 and _plain_tensor(targets) and targets.dtype == torch.int64 and targets.device == logits.device and targets.is_contiguous() \
         and targets.shape == logits.shape[:1]
 
 

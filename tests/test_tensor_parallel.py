@@ -83,6 +83,15 @@ def test_llama_loss_and_grads_match_single_rank(tp):
         assert torch.allclose(h, h1[r * vl:(r + 1) * vl], atol=1e-5)
 
 
+def test_rms_norm_can_be_traced_symbolically_and_compiled():
+    """Neither torch.fx's stand-ins for tensors nor the compiler's meet the choice between the forms."""
+    from hccl_b200.models.llama import RMSNorm
+    norm = RMSNorm(64, 1e-5, torch.bfloat16, "cpu")
+    x = torch.randn(3, 64, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    assert torch.equal(torch.fx.symbolic_trace(norm)(x), norm(x))
+    assert torch.equal(torch.compile(norm, backend="eager", fullgraph=True)(x), norm(x))
+
+
 def test_rms_norm_can_be_scripted():
     """TorchScript compiles the plain form of the norm."""
     from hccl_b200.models.llama import RMSNorm
