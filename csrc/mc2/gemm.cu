@@ -201,12 +201,12 @@ static HcclResult LaunchPlain2CtaT(const void *a, const void *b, void *c, uint32
     return HCCL_SUCCESS;
 }
 
-// HCCL_GEMM_2CTA: 0 never, otherwise (and unset) always. The CTA-pair kernel keeps the tensor pipe at 97 % of the active
+// HCCL_GEMM_2CTA: 0 keeps the automatic choice off the CTA pairs, otherwise (and unset) they are offered. The CTA-pair kernel keeps the tensor pipe at 97 % of the active
 // cycles against 85-88 % for the one-CTA kernel and halves the B traffic per SM. Isolated it wins clearly (1635 against 1480
 // TFLOP/s on 8192 x 8192 x 4096); back to back under the board's power limit it runs at a lower clock (1140 against 1240 MHz)
 // but still finishes sooner: 5.91-5.92 ms against 6.11-6.13 ms for the 8192 x 28672 x 8192 pair of the single-GPU step, two
 // interleaved runs each on one box (benchmarks/gemm_sustained.py), 5.53 ms for the library GEMM on the same box.
-bool Gemm2CtaEnabled(uint64_t, uint64_t, uint64_t)
+bool Gemm2CtaEnabled()
 {
     static const int v = [] { const char *e = getenv("HCCL_GEMM_2CTA"); return e ? atoi(e) : -1; }();
     return v != 0;
@@ -228,7 +228,7 @@ static HcclResult LaunchPlain2Cta(uint32_t bn, const void *a, const void *b, voi
 // 1500 x 3000 x 3000 takes 31.5 on pairs against 48 on one-CTA tiles, which a rule by the count of 128 x 256 tiles had picked.
 // Narrower pair tiles read more of A per result, so they have to win by 3 %.
 struct TileChoice { bool pair; uint32_t bn; };
-static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposedB)
+static TileChoice ChooseTile(uint64_t m, uint64_t n, bool transposedB)
 {
     const uint64_t sms = (uint64_t)SmCount(), pairs = sms / 2, rows = (m + kBM - 1) / kBM, rowPairs = (rows + 1) / 2;
     auto waves = [](uint64_t tiles, uint64_t slots) { return (tiles + slots - 1) / slots; };
@@ -241,7 +241,7 @@ static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposed
     offer(false, 128, rows * ((n + 127) / 128), 75, 100);
     // 256-wide one-CTA tiles only where N is made of them: with few rows the product is bound by reading B, which 112 CTAs do slower than 224
     if (!transposedB && n % 256 == 0) offer(false, 256, rows * ((n + 255) / 256), 142, 100);
-    if (!transposedB && !Gemm2CtaEnabled(m, n, k)) return best;
+    if (!Gemm2CtaEnabled()) return best;
     offer(true, 256, rowPairs * ((n + 255) / 256), 100, 100);
     if (transposedB) return best;                // its tiles are whole 64-column boxes per CTA, and it has no 256-wide one-CTA form
     offer(true, 224, rowPairs * ((n + 223) / 224), 87, 97);
@@ -269,7 +269,7 @@ HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint6
         const SplitKChoice sk = ChooseSplitK(m, n, k, 0);
         if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
-    const TileChoice t = ChooseTile(m, n, k, false);
+    const TileChoice t = ChooseTile(m, n, false);
     if (!t.pair && t.bn < 256) {
         const SplitKChoice sk = ChooseSplitK(m, n, k, ((m + 127) / 128) * ((n + t.bn - 1) / t.bn));
         if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
@@ -305,7 +305,7 @@ HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uin
         HCCL_ERROR("HcclGemmBf16Nn: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    const TileChoice t = ChooseTile(m, n, k, true);
+    const TileChoice t = ChooseTile(m, n, true);
     if (t.pair) return LaunchPlain2CtaT<256, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.bn == 128) return LaunchPlain<128, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     return LaunchPlain<64, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);

@@ -112,3 +112,30 @@ def test_gemm_pair_tile_widths(shape, variant, out_dtype):
     bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
     assert bool(((out[:M].double() - ref).abs() <= bound + 1e-30).all())
     assert bool((out[M] == 7.0).all())
+
+
+@pytest.mark.parametrize("pairs", ["", "0"])
+def test_pairs_can_be_switched_off(pairs):
+    """HCCL_GEMM_2CTA=0 keeps both operand layouts off the CTA-pair kernels (the variable is read once per process)."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    prog = """
+import torch
+from torch.profiler import ProfilerActivity, profile
+from hccl_b200.ops import gemm
+for fn, shape in ((gemm.gemm_bf16, (4096, 512)), (gemm.gemm_bf16_nn, (512, 4096))):
+    a, w = (torch.ones(s, device="cuda", dtype=torch.bfloat16) for s in ((8192, 512), shape))
+    fn(a, w)
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        out = fn(a, w)
+        torch.cuda.synchronize()
+    assert bool((out == 512).all())
+    print("KERNELS", [e.key for e in p.key_averages() if "Gemm" in e.key])
+"""
+    env = dict(os.environ, HCCL_GEMM_2CTA=pairs) if pairs else {k: v for k, v in os.environ.items() if k != "HCCL_GEMM_2CTA"}
+    res = subprocess.run([sys.executable, "-c", prog], cwd=Path(__file__).resolve().parents[1], env=env, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
+    lines = [l for l in res.stdout.splitlines() if l.startswith("KERNELS")]
+    assert len(lines) == 2 and all(("2Cta" in l) == (pairs != "0") and "GemmKernel" in l for l in lines), lines
