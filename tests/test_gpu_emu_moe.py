@@ -238,3 +238,26 @@ def test_receive_views_belong_to_their_call():
         d.close()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("T,E,K", [(1, 8, 1), (37, 16, 3), (700, 256, 8)])
+def test_one_rank_routing_table_that_is_not_16_byte_aligned(T, E, K):
+    """The histogram reads four entries at a time where it can, one at a time from an address that does not allow it."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(T)
+        x = torch.randn(T, 256, generator=g, device="cuda").to(torch.bfloat16)
+        idx = torch.empty(T * K + 1, dtype=torch.int32, device="cuda")[1:].view(T, K)
+        idx.copy_(torch.randint(0, E, (T, K), generator=g, device="cuda"))
+        assert idx.data_ptr() % 16
+        d = MoeDispatcher(comm, E, K, 256, T, max_recv_rows=T * K)
+        rx, _, counts, src = d.dispatch(x, idx)
+        torch.cuda.synchronize()
+        order = torch.argsort(idx.flatten().long(), stable=True)
+        assert torch.equal(counts.long(), torch.bincount(idx.flatten().long(), minlength=E))
+        assert torch.equal(src.long(), order // K) and torch.equal(rx, x[order // K])
+        d.close()
+    finally:
+        comm.destroy()

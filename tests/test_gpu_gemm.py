@@ -139,3 +139,71 @@ for fn, shape in ((gemm.gemm_bf16, (4096, 512)), (gemm.gemm_bf16_nn, (512, 4096)
     assert res.returncode == 0, res.stderr[-2000:]
     lines = [l for l in res.stdout.splitlines() if l.startswith("KERNELS")]
     assert len(lines) == 2 and all(("2Cta" in l) == (pairs != "0") and "GemmKernel" in l for l in lines), lines
+
+
+@pytest.mark.parametrize("m,variant", [(4, 0), (64, 0), (128, 0), (100, 2064), (1000, 0), (300, 2), (600, 192)])
+def test_chained_products_wait_for_one_another(m, variant):
+    """Products set up while the kernel before them drains. In a chain each reads the one before and writes the buffer that the one before
+    has read; the bits are those of the same chain with a synchronisation after every product, also from a captured graph."""
+    from hccl_b200.ops import gemm, mxfp8
+    H = 2048
+    g = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn(m, H, generator=g, device="cuda").to(torch.bfloat16)
+    ws = [(torch.randn(H, H, generator=g, device="cuda") * H ** -0.5).to(torch.bfloat16) for _ in range(3)]
+    wq = mxfp8.quantize(ws[2])
+    bufs = [torch.empty_like(x), torch.empty_like(x)]
+
+    def chain(sync):
+        bufs[0].copy_(x)
+        for step in range(12):
+            src, dst = bufs[step % 2], bufs[1 - step % 2]
+            if step % 4 == 3:
+                mxfp8.gemm(src, wq, out=dst)
+            elif step % 4 == 1:
+                gemm.gemm_bf16_nn(src, ws[1], out=dst)
+            else:
+                gemm.gemm_bf16(src, ws[0], out=dst, variant=variant)
+            if sync:
+                torch.cuda.synchronize()
+        return bufs[0].clone()
+
+    ref = chain(True)
+    assert torch.isfinite(ref.float()).all() and ref.float().abs().max() > 0.1
+    for _ in range(5):
+        assert torch.equal(chain(False), ref)
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        chain(False)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            out = chain(False)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+    gemm.check_error()
+
+
+@pytest.mark.parametrize("M", [16, 1000])
+def test_products_without_the_extension(M, monkeypatch):
+    """The ctypes form of the operators (another library chosen, or the extension not built) gives the same bits."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops import gemm, mc2
+    a, w = torch.randn(M, 2048, device="cuda").to(torch.bfloat16), torch.randn(520, 2048, device="cuda").to(torch.bfloat16)
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        def run():
+            gathered = torch.empty_like(a)
+            outs = [gemm.gemm_bf16(a, w), gemm.gemm_bf16(a, w, out_dtype=torch.float32), gemm.gemm_bf16_nn(a, w.t().contiguous()),
+                    mc2.all_gather_matmul(comm, a, w, gathered=gathered), mc2.matmul_reduce_scatter(comm, a, w), mc2.matmul_all_reduce(comm, a, w)]
+            torch.cuda.synchronize()
+            return outs + [gathered]
+
+        first = run()
+        for module in (gemm, mc2):
+            monkeypatch.setattr(module, "_native", lambda: None)
+        for x, y in zip(first, run()):
+            assert x.dtype == y.dtype and torch.equal(x, y)
+    finally:
+        comm.destroy()
