@@ -30,11 +30,10 @@ __device__ __forceinline__ uint4 PackBf16x8(const uint32_t *v)
 // Stores the 128 x BN accumulator tile at tensor-memory address `tmem` (this warp's lane quarter, first column) to rows row0 ... and
 // columns col0 ... of C. Called by the 128 epilogue threads (et = 0 ... 127, lane quarter = et / 32) together; thread 0 issues the
 // stores, waits for its staging tile to be free again, and has to TmaStoreWaitAll() before the CTA ends. `tiles` counts the staging
-// tiles used so far. add(v, c) may change the 32 columns from column c * 32 on; released() is called once by every thread when the
-// accumulator has been read.
-template <int BN, int BUFS, class Add, class Released>
+// tiles used so far. released() is called once by every thread when the accumulator has been read.
+template <int BN, int BUFS, class Released>
 __device__ __forceinline__ void StoreTileTma(const CUtensorMap *tmapC, bool fp32, uint32_t N, uint32_t tmem, uint8_t *staging, uint32_t et, uint32_t row0, uint32_t col0,
-                                             uint32_t &tiles, Add add, Released released)
+                                             uint32_t &tiles, Released released)
 {
     static_assert(BN % 32 == 0 && BN >= 64, "whole staging tiles");
     const uint32_t swz = et & 7;
@@ -52,8 +51,6 @@ __device__ __forceinline__ void StoreTileTma(const CUtensorMap *tmapC, bool fp32
         if (!fp32) TmemLd32x32(tmem + off + 32, *(uint32_t(*)[32])&v[32]);
         TmemLdWait();
         asm volatile("bar.sync 1, 128;" ::: "memory");       // the staging tile is free
-        add(*(uint32_t(*)[32])&v[0], off / 32);
-        if (!fp32) add(*(uint32_t(*)[32])&v[32], off / 32 + 1);
         if (fp32) {
 #pragma unroll
             for (uint32_t q = 0; q < 8; ++q) mine[q ^ swz] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);

@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernel2Cta(const __grid_c
                 };
                 if (valid)
                     StoreTileTma<BN, S::kStageBufs>(&p.tmapC, p.outFp32 != 0, p.N, tmemBase + ((ew * 32) << 16) + acc * BN, smem + S::kStagingOff, et, mb * kBM, nb * BN,
-                                                    staged, [](uint32_t (&)[32], uint32_t) {}, release);
+                                                    staged, release);
                 else release();
             } else {
 #pragma unroll 1

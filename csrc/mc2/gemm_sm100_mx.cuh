@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) GemmKernelMx(const __grid_con
             const uint32_t row = mb * kBM + rowInTile;
             if constexpr (Policy::kTmaStore) {
                 StoreTileTma<BN, S::kStageBufs>(&p.tmapC, p.outFp32 != 0, p.N, tmemBase + ((ew * 32) << 16) + acc * BN, smem + S::kStagingOff, threadIdx.x - 128, mb * kBM,
-                                                nb * BN, staged, [](uint32_t (&)[32], uint32_t) {}, [&] { TcFenceBefore(); MbarArrive(&tmemEmpty[acc]); });
+                                                nb * BN, staged, [&] { TcFenceBefore(); MbarArrive(&tmemEmpty[acc]); });
             } else {
                 constexpr uint32_t SC = S::kStageCols, CH = SC / 8;
                 uint4 *stg = (uint4 *)(smem + S::kStagingOff);
