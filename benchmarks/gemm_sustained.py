@@ -1,6 +1,6 @@
 """Back-to-back GEMM timing under the board's power cap, with the clocks sampled while it runs.
 
-    python benchmarks/gemm_sustained.py [--impl ours|cublas] [--variant 0|1|2] [--seconds 1.5] [--shapes MxNxK,MxNxK]
+    python benchmarks/gemm_sustained.py [--impl ours|cublas] [--variant 0|2|192|224] [--seconds 1.5] [--shapes MxNxK,MxNxK]
 
 A single GEMM timed in isolation finishes before the power controller reacts; a training or serving step does not. This
 runs the given shapes (default: the two GEMMs of the single-GPU headline step) in a loop for `--seconds`, times the loop with

@@ -162,7 +162,7 @@ def main():
     g = sub.add_parser("gemm")
     g.add_argument("--m", type=int, default=8192); g.add_argument("--n", type=int, default=8192); g.add_argument("--k", type=int, default=4096)
     g.add_argument("--iters", type=int, default=10); g.add_argument("--flush", action="store_true"); g.add_argument("--no-cublas", action="store_true")
-    g.add_argument("--variant", type=int, default=0, help="0 auto, 1 one-CTA tiles, 2 CTA-pair 256x256 tiles")
+    g.add_argument("--variant", type=int, default=0, help="0 auto, 2 or 256 CTA-pair 256x256 tiles, 192 / 224 pair tiles of that width, 1000 * S + BT split-K")
     x = sub.add_parser("mxgemm")
     x.add_argument("--m", type=int, default=8192); x.add_argument("--n", type=int, default=8192); x.add_argument("--k", type=int, default=4096)
     x.add_argument("--iters", type=int, default=10); x.add_argument("--flush", action="store_true"); x.add_argument("--no-cublas", action="store_true")

@@ -223,9 +223,10 @@ static HcclResult LaunchPlain2Cta(uint32_t bn, const void *a, const void *b, voi
 // Which tile kernel: waves of tiles times what a wave of that kernel takes, relative to a wave of 256 x 256 pair tiles. The weights are
 // measured on one B200 at K = 4096 (time of 1 ... 3 waves): pair 224 wide 0.87, 192 wide 0.80 (160 and 128 wide, 0.67 and 0.64, never won
 // a shape by more than 2 %), one CTA 256 wide 1.42 (3336 x 15080 x 2696: 321 us in 11 waves against 247 in 12 of
-// pairs), 128 wide 0.75, 64 wide 0.62. What that decides, us with 256-wide pairs / chosen: 1000 x 6144 x 4096
+// pairs), 128 wide 0.75, 64 wide 0.62. They serve every K: of 70 random products with K = 64 ... 2048 and 78 of 65 ... 256 rows none was slower
+// than by the rule that counted 128 x 256 tiles. What the weights decide, us with 256-wide pairs / chosen: 1000 x 6144 x 4096
 // 48.1 / 39.5 (192), 700 x 8192 x 2048 29.6 / 23.7 (192), 2048 x 14336 x 4096 180 / 158 (224), 2048 x 28672 x 4096 310 / 300 (224); and
-// 1500 x 3000 x 3000 takes 31.5 on pairs against 48 on one-CTA tiles, which a rule by the count of 128 x 256 tiles had picked.
+// 1500 x 3000 x 3000 takes 31.5 on pairs against 48 on one-CTA tiles, which the count had picked.
 // Narrower pair tiles read more of A per result, so they have to win by 3 %.
 struct TileChoice { bool pair; uint32_t bn; };
 static TileChoice ChooseTile(uint64_t m, uint64_t n, bool transposedB)
@@ -239,7 +240,9 @@ static TileChoice ChooseTile(uint64_t m, uint64_t n, bool transposedB)
         if (c * 100 <= cost * percent) { best = {pair, bn}; cost = c; }
     };
     offer(false, 128, rows * ((n + 127) / 128), 75, 100);
-    // 256-wide one-CTA tiles only where N is made of them: with few rows the product is bound by reading B, which 112 CTAs do slower than 224
+    // 256-wide one-CTA tiles where N is made of them, which takes one wave of up to 148 for two of 128-wide tiles: 128 x 28672 x 8192 81.5 us, 89.2
+    // on 128-wide tiles (N = 28664); 128 x 21504 x 4096 38.6 and 43.5; level at K <= 1024. Another N keeps the 128-wide ones, not measured against
+    // 256-wide tiles with a ragged last column
     if (!transposedB && n % 256 == 0) offer(false, 256, rows * ((n + 255) / 256), 142, 100);
     if (!Gemm2CtaEnabled()) return best;
     offer(true, 256, rowPairs * ((n + 255) / 256), 100, 100);

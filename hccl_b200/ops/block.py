@@ -2,8 +2,9 @@
 QKV projection, SwiGLU, vocabulary-parallel cross entropy.
 
 Each function returns None where its kernel does not apply (another type or device, odd sizes, an active function transform,
-tracing or dispatch mode) and the caller keeps its plain PyTorch form; the same plain form computes the gradient of a
-gradient.
+tracing or dispatch mode) and the caller keeps its plain PyTorch form. The same plain form computes the gradient of a gradient,
+and the gradient where the incoming one is batched or dual or something watches the backward pass. What the backward kernels read
+is not changed by a caller that writes its tensors in between.
 """
 from __future__ import annotations
 

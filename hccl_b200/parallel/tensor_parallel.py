@@ -53,8 +53,8 @@ _NATIVE_WGRAD = False
 
 
 def use_native_wgrad(flag: bool) -> None:
-    """True computes weight gradients on the tcgen05 GEMM (needs explicit transposes of both operands, because that kernel
-    takes K-major operands only); the default leaves this plain, collective-free GEMM with transposed operands to cuBLAS."""
+    """True computes weight gradients on the tcgen05 GEMM (needs explicit transposes of both operands: its A is K-major, and the form
+    that reads B MN-major is used for input gradients only); the default leaves this plain, collective-free GEMM with transposed operands to cuBLAS."""
     global _NATIVE_WGRAD
     _NATIVE_WGRAD = flag
 
