@@ -28,6 +28,17 @@ EncodeFn GetEncode()
     });
     return fn;
 }
+
+// The driver wants a current context, which a thread gets with its first runtime call that needs one. A product can be the first call of
+// its thread (autograd's worker, when the allocator has memory at hand): the runtime is then asked to make its context current.
+template <class... Args> CUresult Encode(EncodeFn enc, Args... args)
+{
+    const CUresult r = enc(args...);
+    if (r != CUDA_ERROR_INVALID_CONTEXT) return r;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return r;
+    return enc(args...);
+}
 }  // namespace
 
 HcclResult EncodeTmap2D(CUtensorMap *out, const void *base, uint64_t rows, uint64_t cols, uint64_t pitchBytes, uint32_t boxRows, uint32_t boxCols,
@@ -44,7 +55,7 @@ HcclResult EncodeTmap2D(CUtensorMap *out, const void *base, uint64_t rows, uint6
     cuuint32_t box[2] = {boxCols, boxRows};
     cuuint32_t estr[2] = {1, 1};
     CUtensorMapDataType dt = elemBytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : elemBytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-    CUresult r = enc(out, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    CUresult r = Encode(enc, out, dt, 2u, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { HCCL_ERROR("cuTensorMapEncodeTiled failed: %d", (int)r); return HCCL_E_DRV; }
     return HCCL_SUCCESS;
@@ -59,7 +70,7 @@ HcclResult EncodeTmapSf(CUtensorMap *out, const void *scales, uint64_t atoms)
     cuuint64_t strides[1] = {512};
     cuuint32_t box[2] = {128, 1};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(scales), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    CUresult r = Encode(enc, out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2u, const_cast<void *>(scales), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { HCCL_ERROR("cuTensorMapEncodeTiled (scale atoms) failed: %d", (int)r); return HCCL_E_DRV; }
     return HCCL_SUCCESS;

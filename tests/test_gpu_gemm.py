@@ -207,3 +207,33 @@ def test_products_without_the_extension(M, monkeypatch):
             assert x.dtype == y.dtype and torch.equal(x, y)
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("M", [16, 1000])
+def test_products_as_the_first_call_of_a_thread(M):
+    """A product may be the first CUDA call of its thread (autograd's worker thread starts its backward pass with one when the allocator
+    has memory at hand): there is no current context yet when the tensor maps are encoded."""
+    import threading
+
+    from hccl_b200.ops import gemm, mxfp8
+    a, w = torch.randn(M, 2048, device="cuda").to(torch.bfloat16), torch.randn(512, 2048, device="cuda").to(torch.bfloat16)
+    wt, qa, qw = w.t().contiguous(), mxfp8.quantize(a), mxfp8.quantize(w)
+    calls = [lambda o: gemm.gemm_bf16(a, w, out=o), lambda o: gemm.gemm_bf16_nn(a, wt, out=o), lambda o: gemm.gemm_bf16(a, w, out=o, variant=2),
+             lambda o: mxfp8.gemm(qa, qw, out=o), lambda o: mxfp8.gemm(qa, qw, out=o, tile_n=2192)]
+    for call in calls:
+        ref, out, failed = torch.empty(M, 512, device="cuda", dtype=torch.bfloat16), torch.zeros(M, 512, device="cuda", dtype=torch.bfloat16), []
+        call(ref)
+        torch.cuda.synchronize()
+
+        def run():
+            try:
+                call(out)
+            except Exception as e:
+                failed.append(e)
+
+        t = threading.Thread(target=run)
+        t.start()
+        t.join()
+        torch.cuda.synchronize()
+        assert not failed, failed
+        assert torch.equal(out, ref)
