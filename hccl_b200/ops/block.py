@@ -39,29 +39,32 @@ def _stream(t: torch.Tensor) -> int:
     return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
+# bound once: every forward and backward pass of a small model goes through the checks below
+_transforms, _modes, _forward_ad = torch._C._functorch.peek_interpreter_stack, torch._C._len_torch_dispatch_stack, torch.autograd.forward_ad
+_has_storage, _BF16 = torch._C._has_storage, torch.bfloat16
+
+
 def _watched() -> bool:
     """Whether something has to see the single operations: a function transform, dispatch mode, forward-mode level, compiler or tracer."""
-    return (torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack() > 0 or torch.autograd.forward_ad._current_level >= 0
-            or torch.compiler.is_compiling() or torch.jit.is_tracing())
+    return _transforms() is not None or _modes() > 0 or _forward_ad._current_level >= 0 or torch.compiler.is_compiling() or torch.jit.is_tracing()
 
 
 def _plain_tensor(t) -> bool:
     """Not a subclass, and with memory of its own (a batched gradient has none)."""
-    return type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t)
+    return (type(t) is torch.Tensor or type(t) is torch.nn.Parameter) and _has_storage(t)
+
+
+def _operand(t, device: int) -> bool:
+    """A plain bf16 tensor on that GPU, contiguous and 16-byte aligned."""
+    return _plain_tensor(t) and t.dtype is _BF16 and t.get_device() == device and t.is_contiguous() and t.data_ptr() % 16 == 0 and t.numel() > 0
 
 
 def _usable(*ts: torch.Tensor) -> bool:
-    """Plain bf16 tensors on the current GPU, contiguous and 16-byte aligned, and nothing that has to see the single operations."""
-    if _watched() or not _plain_tensor(ts[0]):
+    """Operands on the current GPU, and nothing that has to see the single operations."""
+    if _watched() or not _plain_tensor(ts[0]) or not ts[0].is_cuda:
         return False
-    dev = ts[0].device
-    if dev.type != "cuda" or dev.index != torch.cuda.current_device():
-        return False
-    for t in ts:
-        if not _plain_tensor(t) or t.dtype != torch.bfloat16 or t.device != dev or not t.is_contiguous() or t.numel() == 0 \
-                or t.data_ptr() % 16:
-            return False
-    return True
+    device = torch._C._cuda_getDevice()
+    return all([_operand(t, device) for t in ts])
 
 
 def _plain_backward(plain: Callable, inputs, grads):
@@ -78,10 +81,16 @@ def _plain_backward(plain: Callable, inputs, grads):
 def _direct(inputs, grads):
     """The incoming gradients as the backward kernels read them, or None where the single operations have to run: a gradient that is
     itself differentiated, batched or dual, an active mode, a saved tensor that came back as something else."""
-    if torch.is_grad_enabled() or not all(_plain_tensor(g) and g.dtype == torch.bfloat16 and g.device == grads[0].device for g in grads):
+    if torch.is_grad_enabled() or _watched():
         return None
-    grads = [_aligned(g) for g in grads]
-    return grads if _usable(grads[0], *inputs) else None
+    for g in grads:
+        if not _plain_tensor(g) or g.dtype is not _BF16 or not g.is_cuda:
+            return None
+    device = grads[0].get_device()
+    for t in inputs:
+        if not _operand(t, device):
+            return None
+    return [_aligned(g) for g in grads]
 
 
 def _aligned(t: torch.Tensor) -> torch.Tensor:
@@ -154,9 +163,9 @@ class _RopeQkv(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dq, dk, dv):
         cos, sin = ctx.saved_tensors
-        grads = _direct((), (dq, dk, dv)) if _tables_ok(cos.device, cos, sin) else None
-        if grads is None:
-            at = torch.zeros(ctx.shape, dtype=torch.bfloat16, device=cos.device, requires_grad=True)
+        grads = _direct((), (dq, dk, dv))
+        if grads is None or not _tables_ok(grads[0].get_device(), cos, sin):
+            at = torch.zeros(ctx.shape, dtype=torch.bfloat16, device=dq.device, requires_grad=True)
             return (*_plain_backward(ctx.plain, (at,), (dq, dk, dv)), None, None, None, None, None, None)
         dq, dk, dv = grads
         out = torch.empty(ctx.shape, dtype=dq.dtype, device=dq.device)
@@ -165,15 +174,15 @@ class _RopeQkv(torch.autograd.Function):
         return out, None, None, None, None, None, None
 
 
-def _tables_ok(device, *tables) -> bool:
-    return all(type(t) is torch.Tensor and t.dtype == torch.float32 and t.device == device and t.is_contiguous() and not t.requires_grad and t.data_ptr() % 16 == 0
-               for t in tables)
+def _tables_ok(device: int, *tables) -> bool:
+    return all([type(t) is torch.Tensor and t.dtype is torch.float32 and t.get_device() == device and t.is_contiguous() and not t.requires_grad and t.data_ptr() % 16 == 0
+                for t in tables])
 
 
 def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable):
     """Packed [batch * seq, (heads + 2 kv_heads) * head_dim] -> rotated q, k and v as [batch, seq, heads, head_dim]; cos / sin are fp32
     [seq, head_dim / 2] constants. `plain(qkv)` is the same in PyTorch."""
-    if not _usable(qkv) or not _tables_ok(qkv.device, cos, sin):
+    if not _usable(qkv) or not _tables_ok(qkv.get_device(), cos, sin):
         return None
     seq = cos.shape[0] if cos.dim() else 0
     if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
@@ -211,14 +220,14 @@ def swiglu(gu: torch.Tensor, plain: Callable) -> Optional[torch.Tensor]:
 
 
 def xent_usable(logits: torch.Tensor, targets: torch.Tensor) -> bool:
-    return _usable(logits) and logits.dim() == 2 and _plain_tensor(targets) and targets.dtype == torch.int64 and targets.device == logits.device and targets.is_contiguous() \
-        and targets.shape == logits.shape[:1]
+    return _usable(logits) and logits.dim() == 2 and _plain_tensor(targets) and targets.dtype is torch.int64 and targets.get_device() == logits.get_device() \
+        and targets.is_contiguous() and targets.shape == logits.shape[:1]
 
 
 def xent_grad_usable(logits: torch.Tensor, targets: torch.Tensor, g: torch.Tensor) -> bool:
     """Whether the gradient kernel may answer this backward pass: a gradient that is itself differentiated, batched or dual has to see
     the operations."""
-    return not torch.is_grad_enabled() and xent_usable(logits, targets) and _plain_tensor(g) and g.device == logits.device
+    return not torch.is_grad_enabled() and _plain_tensor(g) and g.is_cuda and xent_usable(logits, targets)
 
 
 def xent_row_max(logits: torch.Tensor) -> torch.Tensor:
