@@ -77,13 +77,19 @@ class MoeDispatcher:
         self._tokens = x.shape[0]
         at = (rx.value, rs.value, rc.value, rsrc.value)
         if self._recv is None or self._recv[0] != at:
-            dev = x.device
-            with torch.inference_mode(False):        # kept beyond this call, which may be an inference pass
-                self._recv = (at, _view(rx.value, (self.cap, self.hidden), torch.float8_e4m3fn if self.mxfp8 else torch.bfloat16, dev),
-                              _view(rs.value, (self.cap, self.hidden // 32), torch.uint8, dev) if self.mxfp8 else None,
-                              _view(rc.value, (self.local_experts,), torch.int32, dev), _view(rsrc.value, (self.cap,), torch.int32, dev))
+            if torch.is_inference_mode_enabled():        # the views are kept beyond this call
+                with torch.inference_mode(False):
+                    self._recv = (at, *self._views(at, x.device))
+            else:
+                self._recv = (at, *self._views(at, x.device))
         # new tensors over the same memory on every call (`data`: with a version count of their own), as the caller may do with them what it likes
         return tuple(None if t is None else t.data for t in self._recv[1:])
+
+    def _views(self, at, dev):
+        rx, rs, rc, rsrc = at
+        return (_view(rx, (self.cap, self.hidden), torch.float8_e4m3fn if self.mxfp8 else torch.bfloat16, dev),
+                _view(rs, (self.cap, self.hidden // 32), torch.uint8, dev) if self.mxfp8 else None,
+                _view(rc, (self.local_experts,), torch.int32, dev), _view(rsrc, (self.cap,), torch.int32, dev))
 
     def combine(self, topk_weights: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
         assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
