@@ -261,3 +261,33 @@ def test_one_rank_routing_table_that_is_not_16_byte_aligned(T, E, K):
         d.close()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("nranks,T,E,K,H", [(2, 40, 8, 2, 256), (4, 128, 64, 8, 1024)])
+def test_ids_outside_the_experts_among_ranks(nranks, T, E, K, H):
+    """The same with several ranks and identity experts: a token comes back as the sum of its valid entries' weights times itself, in the
+    second routing too, which masks entries that had rows in the first."""
+    from hccl_b200.ops import moe
+    from hccl_b200.utils import emu
+    l = moe._decl()
+    cfg = moe.HcclMoeConfig(E, K, H, T, nranks * T * K, 0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    xs = [torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16) for _ in range(nranks)]
+    idxs = [torch.randint(0, E, (T, K), generator=g, device="cuda").to(torch.int32) for _ in range(nranks)]
+    ws = [torch.rand(T, K, generator=g, device="cuda") for _ in range(nranks)]
+    outs = [torch.zeros(T, H, dtype=torch.bfloat16, device="cuda") for _ in range(nranks)]
+    counts = [torch.zeros(E // nranks, dtype=torch.int32, device="cuda") for _ in range(nranks)]
+    with emu.EmuWorld(nranks, 1 << 20, arena_bytes=4 * nranks * T * K * H * 2 + (8 << 20)) as w:
+        arr = lambda ts: (ctypes.c_void_p * nranks)(*[t.data_ptr() for t in ts])
+        for step in range(2):
+            if step:
+                for r, idx in enumerate(idxs):
+                    idx[torch.rand(T, K, generator=g, device="cuda") < 0.3] = -1 if r % 2 else E
+                    idx[r] = -1
+            assert l.HcclEmuMoeRoundTrip(w._h, ctypes.byref(cfg), arr(xs), arr(idxs), arr(ws), arr(outs), T, arr(counts), max(1, min(16, 148 // nranks))) == 0
+            torch.cuda.synchronize()
+            ok = [(i >= 0) & (i < E) for i in idxs]
+            assert torch.equal(torch.cat(counts).long(), sum(torch.bincount(i[o].long(), minlength=E) for i, o in zip(idxs, ok)))
+            for x, o, wt, out in zip(xs, ok, ws, outs):
+                ref = x.double() * torch.where(o, wt, 0.0).double().sum(1, keepdim=True)
+                assert bool(((out.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + K * 2.0 ** -23) + 1e-30).all())
