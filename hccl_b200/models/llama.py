@@ -187,7 +187,7 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
     def backward(ctx, g):
         if ctx.fused:
             logits, targets, mx, packed = ctx.saved_tensors
-            if _block.xent_grad_usable(logits, targets, g):
+            if _block.xent_grad_usable(logits, targets, mx, packed, g):
                 return _block.xent_grad(logits, targets, ctx.vocab_start, mx, packed, g), None, None, None
             with torch.no_grad():                                           # what the plain form keeps
                 p = (logits.float() - mx[:, None]).exp() / packed[0][:, None]

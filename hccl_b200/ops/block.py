@@ -67,6 +67,12 @@ def _usable(*ts: torch.Tensor) -> bool:
     return all([_operand(t, device) for t in ts])
 
 
+def _floats_ok(device: int, *ts) -> bool:
+    """fp32 constants on that GPU, contiguous and 16-byte aligned."""
+    return all([type(t) is torch.Tensor and t.dtype is torch.float32 and t.get_device() == device and t.is_contiguous() and not t.requires_grad and t.data_ptr() % 16 == 0
+                for t in ts])
+
+
 def _plain_backward(plain: Callable, inputs, grads):
     """Gradients of `plain(*inputs)` by the single operations, a differentiable function of inputs and grads under create_graph."""
     again = torch.is_grad_enabled()
@@ -120,7 +126,7 @@ class _RmsNorm(torch.autograd.Function):
         if dy is None:
             return dxk, dwk, None, None
         grads = _direct((x, w), (dy,))
-        if grads is None:
+        if grads is None or x.shape != dy.shape or not _floats_ok(x.get_device(), rstd):
             dx, dw = _plain_backward(ctx.plain, (x, w), dy)
         else:
             dy, = grads
@@ -164,7 +170,7 @@ class _RopeQkv(torch.autograd.Function):
     def backward(ctx, dq, dk, dv):
         cos, sin = ctx.saved_tensors
         grads = _direct((), (dq, dk, dv))
-        if grads is None or not _tables_ok(grads[0].get_device(), cos, sin):
+        if grads is None or not _floats_ok(grads[0].get_device(), cos, sin):
             at = torch.zeros(ctx.shape, dtype=torch.bfloat16, device=dq.device, requires_grad=True)
             return (*_plain_backward(ctx.plain, (at,), (dq, dk, dv)), None, None, None, None, None, None)
         dq, dk, dv = grads
@@ -174,15 +180,10 @@ class _RopeQkv(torch.autograd.Function):
         return out, None, None, None, None, None, None
 
 
-def _tables_ok(device: int, *tables) -> bool:
-    return all([type(t) is torch.Tensor and t.dtype is torch.float32 and t.get_device() == device and t.is_contiguous() and not t.requires_grad and t.data_ptr() % 16 == 0
-                for t in tables])
-
-
 def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable):
     """Packed [batch * seq, (heads + 2 kv_heads) * head_dim] -> rotated q, k and v as [batch, seq, heads, head_dim]; cos / sin are fp32
     [seq, head_dim / 2] constants. `plain(qkv)` is the same in PyTorch."""
-    if not _usable(qkv) or not _tables_ok(qkv.get_device(), cos, sin):
+    if not _usable(qkv) or not _floats_ok(qkv.get_device(), cos, sin):
         return None
     seq = cos.shape[0] if cos.dim() else 0
     if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
@@ -204,7 +205,7 @@ class _SwiGlu(torch.autograd.Function):
     def backward(ctx, dh):
         gu, = ctx.saved_tensors
         grads = _direct((gu,), (dh,))
-        if grads is None:
+        if grads is None or gu.numel() != 2 * dh.numel():
             return (*_plain_backward(ctx.plain, (gu,), dh), None)
         dh, = grads
         out = torch.empty_like(gu)
@@ -224,10 +225,10 @@ def xent_usable(logits: torch.Tensor, targets: torch.Tensor) -> bool:
         and targets.is_contiguous() and targets.shape == logits.shape[:1]
 
 
-def xent_grad_usable(logits: torch.Tensor, targets: torch.Tensor, g: torch.Tensor) -> bool:
+def xent_grad_usable(logits: torch.Tensor, targets: torch.Tensor, mx: torch.Tensor, packed: torch.Tensor, g: torch.Tensor) -> bool:
     """Whether the gradient kernel may answer this backward pass: a gradient that is itself differentiated, batched or dual has to see
-    the operations."""
-    return not torch.is_grad_enabled() and _plain_tensor(g) and g.is_cuda and xent_usable(logits, targets)
+    the operations, and so has a saved tensor that came back as something else."""
+    return not torch.is_grad_enabled() and _plain_tensor(g) and g.is_cuda and xent_usable(logits, targets) and _floats_ok(logits.get_device(), mx, packed)
 
 
 def xent_row_max(logits: torch.Tensor) -> torch.Tensor:
@@ -244,7 +245,7 @@ def xent_sums(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, mx:
 
 
 def xent_grad(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, mx: torch.Tensor, packed: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
-    out, packed, g = torch.empty_like(logits), packed.contiguous(), g.float()
+    out, g = torch.empty_like(logits), g.float()
     check(_decl().HcclXent(2, logits.data_ptr(), targets.data_ptr(), vocab_start, mx.data_ptr(), packed.data_ptr(), g.data_ptr(), out.data_ptr(), *logits.shape,
                            _stream(logits)), "HcclXent")
     return out

@@ -174,3 +174,23 @@ def test_rotary_embedding_keeps_nothing_of_the_projection():
     c = torch.randn(leaf.shape, device="cuda").to(torch.bfloat16)
     for a, b in zip(torch.autograd.grad(got, ups, c), torch.autograd.grad(ref, ups, c)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["rms_norm", "rope", "swiglu", "xent"])
+def test_saved_tensors_that_come_back_changed(name):
+    """Hooks that keep 32-bit tensors in 16 bits (and hand those back), or everything transposed: the backward kernels read nothing whose
+    type or layout is not what the forward pass saved."""
+    from hccl_b200.models.llama import _VocabParallelCrossEntropy as X
+    if name == "xent":
+        logits, targets, _, _ = _logits()
+        f, ins = lambda t: X.apply(t, targets, _OneRank, 0), [logits]
+    else:
+        f, _, ins = _op(name)
+    ref = torch.autograd.grad(_outs(f(*ins)), ins, [torch.ones_like(o) for o in _outs(f(*ins))])
+    narrow = (lambda t: t.to(torch.bfloat16) if t.dtype == torch.float32 else t, lambda t: t)
+    turned = (lambda t: t.t().contiguous() if t.dim() == 2 else t, lambda t: t.t() if t.dim() == 2 else t)
+    for pack, unpack in (narrow, turned):
+        with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+            out = _outs(f(*ins))
+        for a, b in zip(torch.autograd.grad(out, ins, [torch.ones_like(o) for o in out]), ref):
+            assert (a.double() - b.double()).norm() <= 2.0 ** -5 * b.double().norm()
