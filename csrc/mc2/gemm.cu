@@ -7,6 +7,7 @@
 #include "gemm_sm100.cuh"
 #include "gemm_sm100_2cta.cuh"
 #include "gemm_splitk_launch.cuh"
+#include "gemm_wide_launch.cuh"
 #include <cstdlib>
 #include "hccl/hccl_mc2.h"
 
@@ -223,43 +224,54 @@ bool Gemm2CtaEnabled()
     return v != 0;
 }
 
-// A CTA pair with tiles of that width (192, 224, otherwise 256).
-static HcclResult LaunchPlain2Cta(uint32_t bn, const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
+// A CTA pair with tiles of that width: 192, 224 and 256 with two accumulators, wider ones as two halves.
+static HcclResult LaunchPair(uint32_t bn, const void *a, const void *b, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
 {
     if (bn == 192) return LaunchPlain2CtaT<192>(a, b, c, M, N, K, outFp32, s);
     if (bn == 224) return LaunchPlain2CtaT<224>(a, b, c, M, N, K, outFp32, s);
+    if (bn > 256) return LaunchWide<false>(bn, a, b, c, M, N, K, outFp32, GroupMOverride(8), s);
     return LaunchPlain2CtaT<256>(a, b, c, M, N, K, outFp32, s);
 }
 
-// Which tile kernel: waves of tiles times what a wave of that kernel takes, relative to a wave of 256 x 256 pair tiles. The weights are
-// measured on one B200 at K = 4096 (time of 1 ... 3 waves): pair 224 wide 0.87, 192 wide 0.80 (160 and 128 wide, 0.67 and 0.64, never won
-// a shape by more than 2 %), one CTA 256 wide 1.42 (3336 x 15080 x 2696: 321 us in 11 waves against 247 in 12 of
-// pairs), 128 wide 0.75, 64 wide 0.62. They serve every K: of 70 random products with K = 64 ... 2048 and 78 of 65 ... 256 rows none was slower
-// than by the rule that counted 128 x 256 tiles. What the weights decide, us with 256-wide pairs / chosen: 1000 x 6144 x 4096
-// 48.1 / 39.5 (192), 700 x 8192 x 2048 29.6 / 23.7 (192), 2048 x 14336 x 4096 180 / 158 (224), 2048 x 28672 x 4096 310 / 300 (224); and
-// 1500 x 3000 x 3000 takes 31.5 on pairs against 48 on one-CTA tiles, which the count had picked.
-// Narrower pair tiles read more of A per result, so they have to win by 3 %.
+// Which tile kernel: waves of tiles times what a wave of that kernel takes. Half of the cost counts whole waves and half the fraction of the
+// GPU that the tiles fill, since idle SMs leave power to the others. A wave per 4096 of K takes the tile's columns (pairs) or 0.9 of them (one
+// CTA) plus what its loads of A and B hold it up, which is more where K is no multiple of 64: its rows then straddle 128-byte lines. The
+// constants are fitted to 124 random products on one B200 (64 to 8192 rows, N 512 to 28672, K 512 to 16384; every width timed in random
+// order, each after 30 to 50 ms of its own): the choice is 0.3 % slower than the best width on average. The widths above 256 and these
+// costs against 192 / 224 / 256 chosen by waves alone: 1473 x 17784 x 9608 496 / 420 us (512 columns), 3882 x 18048 x 6664 957 / 814 (512),
+// 2115 x 2304 x 2344 31.6 / 24.2 (288), 7073 x 6152 x 5992 598 / 425 (480), 2048 x 4096 x 14336 195 / 181 (480), 1000 x 6144 x 4096 43.0 / 42.1 (352),
+// 8192 x 8192 x 28672 3133 / 2867 (512).
 struct TileChoice { bool pair; uint32_t bn; };
-static TileChoice ChooseTile(uint64_t m, uint64_t n, bool transposedB)
+static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposedB)
 {
     const uint64_t sms = (uint64_t)SmCount(), pairs = sms / 2, rows = (m + kBM - 1) / kBM, rowPairs = (rows + 1) / 2;
-    auto waves = [](uint64_t tiles, uint64_t slots) { return (tiles + slots - 1) / slots; };
-    TileChoice best{false, 64};
-    uint64_t cost = waves(rows * ((n + 63) / 64), sms) * 62;
-    auto offer = [&](bool pair, uint32_t bn, uint64_t tiles, uint64_t weight, uint64_t percent) {
-        const uint64_t c = waves(tiles, pair ? pairs : sms) * weight;
-        if (c * 100 <= cost * percent) { best = {pair, bn}; cost = c; }
+    const double k4 = (double)k / 4096;
+    const bool straddle = k % 64 != 0;
+    auto filled = [](uint64_t tiles, uint64_t slots) { return std::max(1.0, (double)tiles / (double)slots); };
+    auto waves = [](uint64_t tiles, uint64_t slots) { return (double)((tiles + slots - 1) / slots); };
+    auto one = [&](uint32_t bn) {
+        const uint64_t tiles = rows * ((n + bn - 1) / bn);
+        return (0.8 * waves(tiles, sms) + 0.2 * filled(tiles, sms)) * (20 + k4 * (0.9 * bn + (straddle ? 170 : 130)));
     };
-    offer(false, 128, rows * ((n + 127) / 128), 75, 100);
-    // 256-wide one-CTA tiles where N is made of them, which takes one wave of up to 148 for two of 128-wide tiles: 128 x 28672 x 8192 81.5 us, 89.2
-    // on 128-wide tiles (N = 28664); 128 x 21504 x 4096 38.6 and 43.5; level at K <= 1024. Another N keeps the 128-wide ones, not measured against
-    // 256-wide tiles with a ragged last column
-    if (!transposedB && n % 256 == 0) offer(false, 256, rows * ((n + 255) / 256), 142, 100);
+    auto pair = [&](uint32_t bn) {
+        const uint64_t tiles = rowPairs * ((n + bn - 1) / bn);
+        return 10 + 0.5 * (waves(tiles, pairs) + filled(tiles, pairs)) * ((bn > 256 ? 20 : 0) + k4 * (bn + (straddle ? 200 : 90)));
+    };
+    TileChoice best{false, 64};
+    double cost = one(64);
+    auto offer = [&](bool isPair, uint32_t bn, double c) { if (c <= cost) { best = {isPair, bn}; cost = c; } };
+    offer(false, 128, one(128));
+    // 256-wide one-CTA tiles where N is made of them (another N was not measured)
+    if (!transposedB && n % 256 == 0) offer(false, 256, one(256));
     if (!Gemm2CtaEnabled()) return best;
-    offer(true, 256, rowPairs * ((n + 255) / 256), 100, 100);
-    if (transposedB) return best;                // its tiles are whole 64-column boxes per CTA, and it has no 256-wide one-CTA form
-    offer(true, 224, rowPairs * ((n + 223) / 224), 87, 97);
-    offer(true, 192, rowPairs * ((n + 191) / 192), 80, 97);
+    offer(true, 256, pair(256));
+    if (transposedB) {           // its tiles are whole 64-column boxes per CTA; 2048 x 4096 x 28672 387 / 379 us (256 / 512), 4096 x 4096 x 14336 394 / 373
+        offer(true, 512, pair(512) / 0.96);          // 2048 x 14336 x 4096, 3 % cheaper by this count, takes 186 / 204
+        return best;
+    }
+    offer(true, 224, pair(224));
+    offer(true, 192, pair(192));
+    for (uint32_t bn = 288; bn <= 512; bn += 32) offer(true, bn, pair(bn));
     return best;
 }
 
@@ -283,25 +295,25 @@ HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint6
         const SplitKChoice sk = ChooseSplitK(m, n, k, 0);
         if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
-    const TileChoice t = ChooseTile(m, n, false);
+    const TileChoice t = ChooseTile(m, n, k, false);
     if (!t.pair && t.bn < 256) {
         const SplitKChoice sk = ChooseSplitK(m, n, k, ((m + 127) / 128) * ((n + t.bn - 1) / t.bn));
         if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
-    if (t.pair) return LaunchPlain2Cta(t.bn, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    if (t.pair) return LaunchPair(t.bn, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.bn == 256) return LaunchPlain<256>(a, b, c, m, n, k, outFp32 != 0, stream);
     if (t.bn == 128) return LaunchPlain<128>(a, b, c, m, n, k, outFp32 != 0, stream);
     return LaunchPlain<64>(a, b, c, m, n, k, outFp32 != 0, stream);
 }
 
-// variant 2 or 256 = 256 x 256 tiles on CTA pairs (cta_group::2), 192 / 224 = pair tiles of that width, 1000 * S + BT = the split-K
-// kernel with BT rows of A per tile and S CTAs along K; anything else = automatic choice
+// variant 2 or 256 = 256 x 256 tiles on CTA pairs (cta_group::2), 192 / 224 and 288 ... 512 in steps of 32 = pair tiles of that width,
+// 1000 * S + BT = the split-K kernel with BT rows of A per tile and S CTAs along K; anything else = automatic choice
 HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, int variant, cudaStream_t stream)
 {
-    if (variant == 2 || variant == 192 || variant == 224 || variant == 256) {
+    if (variant == 2 || variant == 192 || variant == 224 || variant == 256 || (variant >= 288 && variant <= 512 && variant % 32 == 0)) {
         if (!a || !b || !c) return HCCL_E_PTR;
         if (m == 0 || n == 0 || k == 0 || (k % 8) || (n % 8) || m > 0x7fffffff || n > 0x7fffffff || k > 0x7fffffff) return HCCL_E_PARA;
-        return LaunchPlain2Cta((uint32_t)variant, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+        return LaunchPair((uint32_t)variant, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
     if (variant >= 1000) {
         if (!a || !b || !c) return HCCL_E_PTR;
@@ -319,7 +331,8 @@ HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uin
         HCCL_ERROR("HcclGemmBf16Nn: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    const TileChoice t = ChooseTile(m, n, true);
+    const TileChoice t = ChooseTile(m, n, k, true);
+    if (t.pair && t.bn == 512) return LaunchWide<true>(512, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, GroupMOverride(8), stream);
     if (t.pair) return LaunchPlain2CtaT<256, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.bn == 128) return LaunchPlain<128, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     return LaunchPlain<64, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);

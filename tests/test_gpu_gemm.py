@@ -114,6 +114,42 @@ def test_gemm_pair_tile_widths(shape, variant, out_dtype):
     assert bool((out[M] == 7.0).all())
 
 
+@pytest.mark.parametrize("shape,variant", [((256, 288, 64), 288), ((8, 8, 8), 512), ((257, 520, 200), 320), ((1000, 6144, 264), 352), ((300, 1000, 136), 416), ((520, 448, 328), 448),
+                                           ((700, 3000, 1032), 480), ((2048, 5120, 320), 512), ((2115, 2304, 2344), 0), ((1000, 6144, 4096), 0)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_wide_tiles(shape, variant, out_dtype):
+    """Pair tiles of two halves: unequal halves, one k-block and fewer k-blocks than half 0 runs ahead, a second half past the edge, several tiles per
+    pair, and shapes for which the automatic choice picks them (bound as above)."""
+    from hccl_b200.ops import gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=out_dtype)
+    gemm.gemm_bf16(a, w, out[:M], variant=variant)
+    torch.cuda.synchronize()
+    gemm.check_error()
+    ref, mag = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out[:M].double() - ref).abs() <= bound + 1e-30).all())
+    assert bool((out[M] == 7.0).all())
+
+
+@pytest.mark.parametrize("shape", [(2000, 4096, 14344), (4096, 4096, 4104)])
+def test_gemm_nn_wide_tiles(shape):
+    """B stored [K, N] in 512-wide pair tiles, where the automatic choice takes them; one and two waves (bound as above)."""
+    from hccl_b200.ops import gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(K, N, generator=g, device="cuda").to(torch.bfloat16)
+    out = gemm.gemm_bf16_nn(a, w)
+    torch.cuda.synchronize()
+    gemm.check_error()
+    ref, mag = a.double() @ w.double(), a.double().abs() @ w.double().abs()
+    assert bool(((out.double() - ref).abs() <= mag * K * 2.0 ** -24 + ref.abs() * 2.0 ** -8 + 1e-30).all())
+
+
 @pytest.mark.parametrize("pairs", ["", "0"])
 def test_pairs_can_be_switched_off(pairs):
     """HCCL_GEMM_2CTA=0 keeps both operand layouts off the CTA-pair kernels (the variable is read once per process)."""
