@@ -48,9 +48,11 @@ template <int TPR> __device__ __forceinline__ float RowSum(float v, float *red)
     return s;
 }
 
-// y = x * rsqrt(mean(x^2) + eps) * w. A row is shared by TPR threads; the second pass over it hits L1 / L2. KEEP: x and w are copied on
-// the way for a backward pass that may come after they were changed.
-template <int TPR, bool KEEP>
+// y = x * rsqrt(mean(x^2) + eps) * w. A row is shared by TPR threads. Up to two vectors per thread (NV) stay in registers between the sum and the
+// result; wider rows (NV = 0) are read again from L1 / L2, which leaves the registers to more rows in flight. KEEP: x and w are copied on the
+// way for a backward pass that may come after they were changed. Bound by memory: 2048 x 4096 with copies (48 MB) on one B200 14.3 us from a cold L2,
+// 16.4 with a second load of the row; 1000 x 8192 without copies 12.3 with it, 14.2 from registers.
+template <int TPR, int NV, bool KEEP>
 __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ y,
                                                          float *__restrict__ rstd, __nv_bfloat16 *__restrict__ xKept, __nv_bfloat16 *__restrict__ wKept, uint32_t T,
                                                          uint32_t H, float eps)
@@ -59,35 +61,49 @@ __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *_
     const uint32_t row = blockIdx.x * (kThreads / TPR) + threadIdx.x / TPR, lane = threadIdx.x % TPR;
     if (row >= T) return;                                // whole warps (TPR = 32) or no thread at all (one row per block)
     const uint4 *xr = (const uint4 *)(x + (size_t)row * H), *wr = (const uint4 *)w;
+    uint4 xv[NV ? NV : 1];
     float s = 0.f;
-    for (uint32_t v = lane; v < H / 8; v += TPR) {
-        const uint4 raw = xr[v];
+    auto square = [&](uint32_t v, const uint4 &raw) {
         if (KEEP) ((uint4 *)(xKept + (size_t)row * H))[v] = raw;
         float f[8];
         Unpack8(raw, f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) s += f[j] * f[j];
+    };
+    if (NV) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) if (lane + i * TPR < H / 8) xv[i] = xr[lane + i * TPR];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) if (lane + i * TPR < H / 8) square(lane + i * TPR, xv[i]);
+    } else {
+        for (uint32_t v = lane; v < H / 8; v += TPR) square(v, xr[v]);
     }
     const float r = rsqrtf(RowSum<TPR>(s, red) / (float)H + eps);
     if (lane == 0) rstd[row] = r;
     uint4 *yr = (uint4 *)(y + (size_t)row * H);
-    for (uint32_t v = lane; v < H / 8; v += TPR) {
+    auto scale = [&](uint32_t v, const uint4 &raw) {
         const uint4 wv = wr[v];
         if (KEEP && row == 0) ((uint4 *)wKept)[v] = wv;
         float f[8], g[8];
-        Unpack8(xr[v], f);
+        Unpack8(raw, f);
         Unpack8(wv, g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
         yr[v] = Pack8(f);
+    };
+    if (NV) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) if (lane + i * TPR < H / 8) scale(lane + i * TPR, xv[i]);
+    } else {
+        for (uint32_t v = lane; v < H / 8; v += TPR) scale(v, xr[v]);
     }
 }
 
 // dx = r * (dy * w - xhat * mean(dy * w * xhat)), xhat = x * r; dw = sum over rows of dy * xhat. A thread owns NV vectors of columns of
 // every row its block walks over (with a stride of the grid): x, dy and w of a row are loaded once and stay in registers between the
-// row sum and the result, and so does the thread's part of dw, which goes to partial[block] at the end. A second kernel adds the
-// blocks in order: the same bits on every run. 2048 x 4096 on one B200: 18.4 us, 27.5 with dw in shared memory and a
-// second load of the row.
+// row sum and the result, and so does the thread's part of dw, which goes to partial[block] at the end; the next row is on its way
+// meanwhile. A second kernel adds the blocks in a fixed order: the same bits on every run. 2048 x 4096 on one B200, both kernels from a cold L2:
+// 23.3 us, 31.6 without the early loads, with three blocks per SM and the sums below at one column per thread.
 template <int TPR, int NV>
 __global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16 *__restrict__ dy, const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
                                                             const float *__restrict__ rstd, __nv_bfloat16 *__restrict__ dx, float *__restrict__ partial, uint32_t T,
@@ -106,16 +122,29 @@ __global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16
 #pragma unroll
         for (int j = 0; j < 8; ++j) part[i][j] = 0.f;
     }
-    for (uint32_t row = blockIdx.x * kRows + group; row < T; row += gridDim.x * kRows) {
+    uint4 nx[NV], nd[NV];
+    float nr = 0.f;
+    auto fetch = [&](uint32_t row) {
         const uint4 *xr = (const uint4 *)(x + (size_t)row * H), *dr = (const uint4 *)(dy + (size_t)row * H);
-        uint4 xv[NV], dv[NV];
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const uint32_t v = lane + i * TPR;
-            xv[i] = v < H / 8 ? xr[v] : make_uint4(0, 0, 0, 0);
-            dv[i] = v < H / 8 ? dr[v] : make_uint4(0, 0, 0, 0);
+            nx[i] = v < H / 8 ? xr[v] : make_uint4(0, 0, 0, 0);
+            nd[i] = v < H / 8 ? dr[v] : make_uint4(0, 0, 0, 0);
         }
-        const float r = rstd[row];
+        nr = rstd[row];
+    };
+    constexpr bool kEarly = NV <= 4;                     // more would not fit the registers
+    const uint32_t step = gridDim.x * kRows;
+    uint32_t row = blockIdx.x * kRows + group;
+    if (kEarly && row < T) fetch(row);
+    for (; row < T; row += step) {
+        uint4 xv[NV], dv[NV];
+        if (!kEarly) fetch(row);
+        const float r = nr;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) { xv[i] = nx[i]; dv[i] = nd[i]; }
+        if (kEarly && row + step < T) fetch(row + step);
         float s = 0.f;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
@@ -167,21 +196,26 @@ __global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16
     }
 }
 
-// out[c] = sum over parts of partial[part][c]: 32 columns per block, 8 threads per column, added up in a fixed order.
+// out[c] = sum over parts of partial[part][c]: 32 columns per block, four per load, 32 threads per column group, added up in a fixed order.
 __global__ void __launch_bounds__(kThreads) SumPartsKernel(const float *__restrict__ partial, __nv_bfloat16 *__restrict__ out, uint32_t parts, uint32_t H)
 {
-    __shared__ float sm[8][32];
-    const uint32_t c = blockIdx.x * 32 + (threadIdx.x & 31), q = threadIdx.x >> 5;
-    float s = 0.f;
-    if (c < H)
-        for (uint32_t p = q; p < parts; p += 8) s += partial[(size_t)p * H + c];
-    sm[q][threadIdx.x & 31] = s;
+    __shared__ float4 sm[32][8];
+    const uint32_t g = threadIdx.x & 7, q = threadIdx.x >> 3, c = blockIdx.x * 32 + g * 4;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < H) {                                         // H is a multiple of 8: whole groups
+#pragma unroll 4
+        for (uint32_t p = q; p < parts; p += 32) {
+            const float4 v = *(const float4 *)(partial + (size_t)p * H + c);
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+    }
+    sm[q][g] = s;
     __syncthreads();
-    if (q == 0 && c < H) {
+    if (threadIdx.x < 32 && blockIdx.x * 32 + threadIdx.x < H) {
         float t = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) t += sm[j][threadIdx.x];
-        out[c] = __float2bfloat16(t);
+        for (int j = 0; j < 32; ++j) t += ((const float *)sm[j])[threadIdx.x];
+        out[blockIdx.x * 32 + threadIdx.x] = __float2bfloat16(t);
     }
 }
 
@@ -229,20 +263,28 @@ __global__ void __launch_bounds__(kThreads) RopeQkvKernel(__nv_bfloat16 *__restr
 }
 
 // gu = [T, 2F] (gate | up): h = silu(gate) * up. silu is rounded to bf16 before the product, as two separate operations round it: the
-// forward pass keeps the bits of the plain form.
+// forward pass keeps the bits of the plain form. The product of two bf16 values is exact in 32 bits, so a packed multiplication rounds it
+// the same way. What bounds it is instructions: 2048 x 14336 on one B200 from a cold L2 38.9 us, 48.1 with index divisions in 64 bits and the products in
+// 32 (memory alone 27); 4096 x 28672 131, 166. Index is 64 bits wide where the vectors need it.
+template <class Index>
 __global__ void __launch_bounds__(kThreads) SwiGluKernel(const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ h, uint64_t vecs, uint32_t F)
 {
-    const uint64_t idx = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    const Index idx = (Index)blockIdx.x * kThreads + threadIdx.x;
     if (idx >= vecs) return;
     const uint32_t per = F / 8;
-    const uint64_t t = idx / per, j = idx % per;
-    const uint4 *row = (const uint4 *)(gu + t * 2 * F);
-    float g[8], u[8];
-    Unpack8(row[j], g);
-    Unpack8(row[per + j], u);
+    const Index t = idx / per, j = idx - t * per;
+    const uint4 *row = (const uint4 *)gu + (uint64_t)t * 2 * per;
+    const uint4 gv = row[j], uv = row[per + j];
+    float g[8];
+    Unpack8(gv, g);
+    const __nv_bfloat162 *u = (const __nv_bfloat162 *)&uv;
+    uint4 o;
+    __nv_bfloat162 *ov = (__nv_bfloat162 *)&o;
 #pragma unroll
-    for (int x = 0; x < 8; ++x) g[x] = __bfloat162float(__float2bfloat16(g[x] / (1.f + expf(-g[x])))) * u[x];
-    ((uint4 *)h)[idx] = Pack8(g);
+    for (int x = 0; x < 8; ++x) g[x] = g[x] / (1.f + expf(-g[x]));
+#pragma unroll
+    for (int x = 0; x < 4; ++x) ov[x] = __hmul2_rn(__floats2bfloat162_rn(g[2 * x], g[2 * x + 1]), u[x]);
+    ((uint4 *)h)[idx] = o;
 }
 
 __global__ void __launch_bounds__(kThreads) SwiGluBwdKernel(const __nv_bfloat16 *__restrict__ dh, const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ dgu,
@@ -366,6 +408,13 @@ void LaunchRmsNormBwd(const void *dy, const void *x, const void *w, const float 
     RmsNormBwdKernel<TPR, NV><<<parts, kThreads, 0, s>>>((const __nv_bfloat16 *)dy, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, rstd, (__nv_bfloat16 *)dx, partial, T, H);
 }
 
+// 16-byte vectors of a row per thread
+uint32_t NormVecs(uint32_t H)
+{
+    const uint32_t threads = H <= kWarpRowMax ? 32 : kThreads;
+    return (H / 8 + threads - 1) / threads;
+}
+
 bool NormShapeOk(uint64_t T, uint64_t H) { return T > 0 && T <= 0x7fffffff && H > 0 && H % 8 == 0 && H <= kNormMax; }
 
 HcclResult LaunchRmsNorm(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
@@ -374,9 +423,18 @@ HcclResult LaunchRmsNorm(const void *x, const void *w, void *y, float *rstd, voi
     if (!NormShapeOk(rows, hidden) || !Aligned16(x) || !Aligned16(w) || !Aligned16(y) || !Aligned16(xKept) || !Aligned16(wKept)) return HCCL_E_PARA;
     const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden;
     const bool warp = hidden <= kWarpRowMax;
-    auto kern = warp ? (xKept ? RmsNormKernel<32, true> : RmsNormKernel<32, false>) : (xKept ? RmsNormKernel<kThreads, true> : RmsNormKernel<kThreads, false>);
-    kern<<<warp ? (T + 7) / 8 : T, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, (__nv_bfloat16 *)xKept,
-                                                         (__nv_bfloat16 *)wKept, T, H, eps);
+    auto launch = [&](auto plain, auto keep) {
+        auto kern = xKept ? keep : plain;
+        kern<<<warp ? (T + 7) / 8 : T, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, (__nv_bfloat16 *)xKept,
+                                                             (__nv_bfloat16 *)wKept, T, H, eps);
+    };
+    const uint32_t nv = NormVecs(H);
+    if (warp && nv == 1) launch(RmsNormKernel<32, 1, false>, RmsNormKernel<32, 1, true>);
+    else if (warp && nv == 2) launch(RmsNormKernel<32, 2, false>, RmsNormKernel<32, 2, true>);
+    else if (warp) launch(RmsNormKernel<32, 0, false>, RmsNormKernel<32, 0, true>);
+    else if (nv == 1) launch(RmsNormKernel<kThreads, 1, false>, RmsNormKernel<kThreads, 1, true>);
+    else if (nv == 2) launch(RmsNormKernel<kThreads, 2, false>, RmsNormKernel<kThreads, 2, true>);
+    else launch(RmsNormKernel<kThreads, 0, false>, RmsNormKernel<kThreads, 0, true>);
     return Launched("RMSNorm");
 }
 
@@ -402,8 +460,8 @@ HcclResult HcclRmsNormKeep(const void *x, const void *w, void *y, float *rstd, v
 
 uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden)
 {
-    const uint64_t perBlock = hidden <= kWarpRowMax ? kThreads / 32 : 1;
-    return std::min<uint64_t>((rows + perBlock - 1) / perBlock, (uint64_t)Sms() * 3);
+    const uint64_t perBlock = hidden <= kWarpRowMax ? kThreads / 32 : 1, nv = hidden ? NormVecs((uint32_t)hidden) : 1;
+    return std::min<uint64_t>((rows + perBlock - 1) / perBlock, (uint64_t)Sms() * (nv == 1 ? 3 : nv == 2 ? 2 : 1));   // what the registers let an SM hold
 }
 
 HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, void *dw, float *partial, uint64_t rows, uint64_t hidden,
@@ -413,7 +471,7 @@ HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const fl
     if (!NormShapeOk(rows, hidden) || !Aligned16(dy) || !Aligned16(x) || !Aligned16(w) || !Aligned16(dx)) return HCCL_E_PARA;
     const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden, parts = (uint32_t)HcclRmsNormBwdParts(rows, hidden);
     auto launch = [&](auto kern) { kern(dy, x, w, rstd, dx, partial, T, H, parts, stream); };
-    const uint32_t nv = (H / 8 + (hidden <= kWarpRowMax ? 31 : kThreads - 1)) / (hidden <= kWarpRowMax ? 32 : kThreads);
+    const uint32_t nv = NormVecs(H);
     if (hidden <= kWarpRowMax) launch(nv == 1 ? LaunchRmsNormBwd<32, 1> : nv == 2 ? LaunchRmsNormBwd<32, 2> : LaunchRmsNormBwd<32, 4>);
     else launch(nv == 1 ? LaunchRmsNormBwd<kThreads, 1> : nv == 2 ? LaunchRmsNormBwd<kThreads, 2> : nv <= 4 ? LaunchRmsNormBwd<kThreads, 4> : LaunchRmsNormBwd<kThreads, 6>);
     CHK_RET(Launched("RMSNorm backward"));
@@ -440,7 +498,8 @@ HcclResult HcclSwiGlu(const void *gateUp, void *h, uint64_t rows, uint64_t ffn, 
     if (!gateUp || !h) return HCCL_E_PTR;
     const uint64_t vecs = rows * (ffn / 8), blocks = (vecs + kThreads - 1) / kThreads;
     if (rows == 0 || ffn == 0 || ffn % 8 || ffn > 0x7fffffff || blocks > 0x7fffffff || !Aligned16(gateUp) || !Aligned16(h)) return HCCL_E_PARA;
-    SwiGluKernel<<<(uint32_t)blocks, kThreads, 0, stream>>>((const __nv_bfloat16 *)gateUp, (__nv_bfloat16 *)h, vecs, (uint32_t)ffn);
+    auto kern = (blocks + 1) * kThreads <= 0xffffffffull ? SwiGluKernel<uint32_t> : SwiGluKernel<uint64_t>;
+    kern<<<(uint32_t)blocks, kThreads, 0, stream>>>((const __nv_bfloat16 *)gateUp, (__nv_bfloat16 *)h, vecs, (uint32_t)ffn);
     return Launched("SwiGLU");
 }
 
