@@ -238,10 +238,12 @@ c10::intrusive_ptr<c10d::Backend> createProcessGroupHCCL(const c10::intrusive_pt
 }  // namespace
 
 void BindFusedOps(py::module &m);   // fused_ops.cc
+void BindBlockOps(py::module &m);   // block_ops.cc
 
 PYBIND11_MODULE(hccl_b200_torch, m)
 {
     m.doc() = "torch.distributed backend and matmul operators on the hccl_b200 C API";
     BindFusedOps(m);
+    BindBlockOps(m);
     m.def("create_process_group", &createProcessGroupHCCL, py::arg("store"), py::arg("rank"), py::arg("size"), py::arg("timeout"));
 }

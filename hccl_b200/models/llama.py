@@ -10,6 +10,7 @@ benchmarks that exercise the TP / DP paths the communication library is written 
 """
 from __future__ import annotations
 
+import functools
 import math
 from dataclasses import dataclass
 from typing import Optional
@@ -65,15 +66,19 @@ class RMSNorm(nn.Module):
 
     def forward(self, x):
         if not torch.jit.is_scripting():
-            y = _block.rms_norm(x, self.weight, self.eps, self._plain)
+            y = _block.rms_norm(x, self.weight, self.eps, functools.partial(_plain_rms_norm, eps=self.eps))
             if y is not None:
                 return y
         return self._plain(x, self.weight)
 
     def _plain(self, x, w):
-        v = x.float()
-        v = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)
-        return (v * w.float()).to(x.dtype)
+        return _plain_rms_norm(x, w, self.eps)
+
+
+def _plain_rms_norm(x, w, eps: float):
+    v = x.float()
+    v = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + eps)
+    return (v * w.float()).to(x.dtype)
 
 
 def _rope_tables(seq: int, head_dim: int, theta: float, device):
@@ -114,7 +119,7 @@ class Attention(nn.Module):
 
     def forward(self, x_local, batch: int, seq: int, cos, sin):
         qkv = self.qkv(x_local)                                            # [B*S, (hl + 2 kvl) * hd]
-        plain = lambda t: self._rotated(t, batch, seq, cos, sin)
+        plain = functools.partial(_rotated, batch=batch, seq=seq, heads=self.h_local, kv_heads=self.kv_local, hd=self.hd, cos=cos, sin=sin)
         out = _block.rope_qkv(qkv, cos, sin, batch, self.h_local, self.kv_local, self.hd, plain)
         q, k, v = (t.transpose(1, 2) for t in (plain(qkv) if out is None else out))
         o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.h_local != self.kv_local)
@@ -122,10 +127,14 @@ class Attention(nn.Module):
         return self.out(o)                                                  # [B*S / tp, hidden]
 
     def _rotated(self, qkv, batch, seq, cos, sin):
-        q, k, v = qkv.split([self.h_local * self.hd, self.kv_local * self.hd, self.kv_local * self.hd], dim=-1)
-        q = _apply_rope(q.reshape(batch, seq, self.h_local, self.hd), cos, sin)
-        k = _apply_rope(k.reshape(batch, seq, self.kv_local, self.hd), cos, sin)
-        return q, k, v.reshape(batch, seq, self.kv_local, self.hd)
+        return _rotated(qkv, batch, seq, self.h_local, self.kv_local, self.hd, cos, sin)
+
+
+def _rotated(qkv, batch, seq, heads, kv_heads, hd, cos, sin):
+    q, k, v = qkv.split([heads * hd, kv_heads * hd, kv_heads * hd], dim=-1)
+    q = _apply_rope(q.reshape(batch, seq, heads, hd), cos, sin)
+    k = _apply_rope(k.reshape(batch, seq, kv_heads, hd), cos, sin)
+    return q, k, v.reshape(batch, seq, kv_heads, hd)
 
 
 class Block(nn.Module):
@@ -189,14 +198,31 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
             logits, targets, mx, packed = ctx.saved_tensors
             if _block.xent_grad_usable(logits, targets, mx, packed, g):
                 return _block.xent_grad(logits, targets, ctx.vocab_start, mx, packed, g), None, None, None
-            with torch.no_grad():                                           # what the plain form keeps
-                p = (logits.float() - mx[:, None]).exp() / packed[0][:, None]
-                mine, idx = _owned(targets, ctx.vocab_start, logits.shape[-1])
-        else:
-            p, mine, idx = ctx.saved_tensors
-        grad = p.clone()
-        grad[torch.arange(p.shape[0], device=p.device)[mine], idx[mine]] -= 1.0
-        return (grad * (g / p.shape[0])).to(torch.bfloat16 if p.is_cuda else torch.float32), None, None, None
+            return *_xent_backward(ctx.vocab_start, logits, targets, mx, packed, g), None, None, None
+        return _xent_gradient(*ctx.saved_tensors, g), None, None, None
+
+
+def _xent_gradient(p, mine, idx, g):
+    grad = p.clone()
+    grad[torch.arange(p.shape[0], device=p.device)[mine], idx[mine]] -= 1.0
+    return (grad * (g / p.shape[0])).to(torch.bfloat16 if p.is_cuda else torch.float32)
+
+
+def _xent_backward(vocab_start, logits, targets, mx, packed, g):
+    with torch.no_grad():                                                   # what the plain form keeps
+        p = (logits.float() - mx[:, None]).exp() / packed[0][:, None]
+        mine, idx = _owned(targets, vocab_start, logits.shape[-1])
+    return (_xent_gradient(p, mine, idx, g),)
+
+
+_block.PYTHON_BACKWARD["xent"] = _xent_backward
+
+
+def _cross_entropy(logits_local, targets, comm, vocab_start):
+    """On one rank a native node with the same kernels, where it applies."""
+    n = _block.native_nodes(logits_local) if comm.size == 1 else None
+    loss = None if n is None else n.xent(logits_local, targets, vocab_start)
+    return _VocabParallelCrossEntropy.apply(logits_local, targets, comm, vocab_start) if loss is None else loss
 
 
 def _sync(comm, t):
@@ -240,7 +266,7 @@ class Llama(nn.Module):
         if targets is None:
             return logits
         vloc = self.cfg.vocab_size // tp
-        return _VocabParallelCrossEntropy.apply(logits, targets.reshape(-1), self.comm, rank * vloc)
+        return _cross_entropy(logits, targets.reshape(-1), self.comm, rank * vloc)
 
     def sync_replicated_grads(self) -> None:
         """Parameters replicated across the tensor-parallel group (embedding, norm scales) see only this rank's tokens:

@@ -5,6 +5,9 @@ Each function returns None where its kernel does not apply (another type or devi
 tracing or dispatch mode) and the caller keeps its plain PyTorch form. The same plain form computes the gradient of a gradient,
 and the gradient where the incoming one is batched or dual or something watches the backward pass. What the backward kernels read
 is not changed by a caller that writes its tensors in between.
+
+The autograd functions exist twice: as nodes in native code (csrc/torch/block_ops.cc), which the extension brings, and as the Python
+functions below for another flavor of the library. The native nodes hand an unusual backward pass to `PYTHON_BACKWARD`.
 """
 from __future__ import annotations
 
@@ -13,7 +16,10 @@ from typing import Callable, Optional
 
 import torch
 
+from .._ext import ops as _extension
 from .._lib import check, lib
+
+PYTHON_BACKWARD: dict = {}      # kind -> backward pass by single operations, for the native nodes
 
 
 def _decl():
@@ -104,6 +110,36 @@ def _aligned(t: torch.Tensor) -> torch.Tensor:
     return t.clone() if t.data_ptr() % 16 else t
 
 
+_NODES = False
+
+
+def nodes():
+    """The extension with the native autograd nodes, or None where it is not in use."""
+    global _NODES
+    if _NODES is False:
+        n = _extension()
+        if n is not None:
+            n.block_init(torch.Tensor, torch.nn.Parameter, check, _watched, lambda kind, *args: PYTHON_BACKWARD[kind](*args))
+        _NODES = n
+    return _NODES
+
+
+def native_nodes(t: torch.Tensor):
+    """The native nodes for an operation on t, or None where the Python form has to answer (symbolic tracing meets the type first)."""
+    return nodes() if (type(t) is torch.Tensor or type(t) is torch.nn.Parameter) and not _watched() and t.is_cuda else None
+
+
+PYTHON_BACKWARD["rms_norm"] = lambda plain, x, w, dy: _plain_backward(plain, (x, w), dy)
+PYTHON_BACKWARD["swiglu"] = lambda plain, gu, dh: _plain_backward(plain, (gu,), dh)
+
+
+def _rope_backward(plain, shape, dq, dk, dv):
+    return _plain_backward(plain, (torch.zeros(shape, dtype=torch.bfloat16, device=dq.device, requires_grad=True),), (dq, dk, dv))
+
+
+PYTHON_BACKWARD["rope_qkv"] = _rope_backward
+
+
 class _RmsNorm(torch.autograd.Function):
     """-> (y, x, w). The backward pass reads copies of x and w that the kernel makes on its way, since the caller may change both before it
     (x += f(norm(x)), an optimizer step). The copies are outputs, so that the gradient of a gradient finds its way to x and w."""
@@ -140,7 +176,11 @@ class _RmsNorm(torch.autograd.Function):
 
 
 def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> Optional[torch.Tensor]:
-    """x * rsqrt(mean(x^2) + eps) * w over the last dimension; `plain(x, w)` is the same in PyTorch."""
+    """x * rsqrt(mean(x^2) + eps) * w over the last dimension; `plain(x, w)` is the same in PyTorch. What `plain` refers to lives as long as
+    the graph does."""
+    n = native_nodes(x)
+    if n is not None:
+        return n.rms_norm(x, w, eps, plain)
     if not _usable(x, w):
         return None
     h = x.shape[-1] if x.dim() else 0
@@ -171,8 +211,7 @@ class _RopeQkv(torch.autograd.Function):
         cos, sin = ctx.saved_tensors
         grads = _direct((), (dq, dk, dv))
         if grads is None or not _floats_ok(grads[0].get_device(), cos, sin):
-            at = torch.zeros(ctx.shape, dtype=torch.bfloat16, device=dq.device, requires_grad=True)
-            return (*_plain_backward(ctx.plain, (at,), (dq, dk, dv)), None, None, None, None, None, None)
+            return (*_rope_backward(ctx.plain, ctx.shape, dq, dk, dv), None, None, None, None, None, None)
         dq, dk, dv = grads
         out = torch.empty(ctx.shape, dtype=dq.dtype, device=dq.device)
         check(_decl().HcclRopeQkv(out.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cos.data_ptr(), sin.data_ptr(), ctx.shape[0], cos.shape[0], *ctx.dims, 1,
@@ -183,6 +222,9 @@ class _RopeQkv(torch.autograd.Function):
 def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable):
     """Packed [batch * seq, (heads + 2 kv_heads) * head_dim] -> rotated q, k and v as [batch, seq, heads, head_dim]; cos / sin are fp32
     [seq, head_dim / 2] constants. `plain(qkv)` is the same in PyTorch."""
+    n = native_nodes(qkv)
+    if n is not None:
+        return n.rope_qkv(qkv, cos, sin, batch, heads, kv_heads, head_dim, plain)
     if not _usable(qkv) or not _floats_ok(qkv.get_device(), cos, sin):
         return None
     seq = cos.shape[0] if cos.dim() else 0
@@ -215,6 +257,9 @@ class _SwiGlu(torch.autograd.Function):
 
 def swiglu(gu: torch.Tensor, plain: Callable) -> Optional[torch.Tensor]:
     """silu(gate) * up for gu = [rows, gate | up]; `plain(gu)` is the same in PyTorch."""
+    n = native_nodes(gu)
+    if n is not None:
+        return n.swiglu(gu, plain)
     if not _usable(gu) or gu.dim() != 2 or gu.shape[1] % 16:
         return None
     return _SwiGlu.apply(gu, plain)

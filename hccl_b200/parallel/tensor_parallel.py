@@ -35,6 +35,7 @@ def use_native_gemm(flag: bool) -> None:
     """False routes the non-fused matmuls (weight gradients) to torch.matmul; used by the NCCL + cuBLAS baseline arm."""
     global _NATIVE_GEMM
     _NATIVE_GEMM = flag
+    _tell_nodes()
 
 
 def _mm_nt(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
@@ -57,6 +58,15 @@ def use_native_wgrad(flag: bool) -> None:
     that reads B MN-major is used for input gradients only); the default leaves this plain, collective-free GEMM with transposed operands to cuBLAS."""
     global _NATIVE_WGRAD
     _NATIVE_WGRAD = flag
+    _tell_nodes()
+
+
+def _tell_nodes() -> None:
+    """The native layers have copies of the switches."""
+    n = _block.nodes()
+    if n is not None:
+        n.set_native_gemm(_NATIVE_GEMM)
+        n.set_native_wgrad(_NATIVE_WGRAD)
 
 
 def _wgrad(dy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
@@ -120,14 +130,16 @@ class _ColumnSeqParallel(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        gathered, w = ctx.saved_tensors
-        dy = dy.contiguous()
-        if _nn_ok(ctx.comm, dy, w):
-            dx = _gemm.gemm_bf16_nn(dy, w.contiguous())
-        else:
-            dx = matmul_reduce_scatter(ctx.comm, dy, w.t().contiguous())      # RS(dy @ W): the mirror of the forward
-        dw = _wgrad(dy, gathered)                                               # dy^T @ AG(x)
-        return dx, dw, None
+        return (*_column_backward(ctx.comm, *ctx.saved_tensors, dy), None)
+
+
+def _column_backward(comm, gathered, w, dy):
+    dy = dy.contiguous()
+    if _nn_ok(comm, dy, w):
+        dx = _gemm.gemm_bf16_nn(dy, w.contiguous())
+    else:
+        dx = matmul_reduce_scatter(comm, dy, w.t().contiguous())              # RS(dy @ W): the mirror of the forward
+    return dx, _wgrad(dy, gathered)                                             # dy^T @ AG(x)
 
 
 class _RowSeqParallel(torch.autograd.Function):
@@ -141,14 +153,28 @@ class _RowSeqParallel(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy_local):
-        x, w = ctx.saved_tensors
-        dyg = dy_local.contiguous()
-        if _nn_ok(ctx.comm, dyg, w):
-            dx = _gemm.gemm_bf16_nn(dyg, w.contiguous())
-        else:
-            dx, dyg = all_gather_matmul(ctx.comm, dyg, w.t().contiguous(), want_gathered=True)                 # AG(dy) @ W
-        dw = _wgrad(dyg, x)                                                                                    # AG(dy)^T @ x
-        return dx, dw, None
+        return (*_row_backward(ctx.comm, *ctx.saved_tensors, dy_local), None)
+
+
+def _row_backward(comm, x, w, dy_local):
+    dyg = dy_local.contiguous()
+    if _nn_ok(comm, dyg, w):
+        dx = _gemm.gemm_bf16_nn(dyg, w.contiguous())
+    else:
+        dx, dyg = all_gather_matmul(comm, dyg, w.t().contiguous(), want_gathered=True)                         # AG(dy) @ W
+    return dx, _wgrad(dyg, x)                                                                                  # AG(dy)^T @ x
+
+
+_block.PYTHON_BACKWARD["column"] = _column_backward
+_block.PYTHON_BACKWARD["row"] = _row_backward
+
+
+def _one_rank_linear(x: torch.Tensor, w: torch.Tensor, comm, column: bool):
+    """The sequence-parallel layer of one rank as one native node (the same kernels), or None where it does not apply."""
+    if comm.size != 1 or not _NATIVE_GEMM or not getattr(comm, "fused", True):
+        return None
+    n = _block.native_nodes(x)
+    return None if n is None else n.linear(x, w, comm, comm.handle, column)
 
 
 class _RowAllReduce(torch.autograd.Function):
@@ -185,6 +211,11 @@ class _ColumnReplicatedInput(torch.autograd.Function):
         return dx, _wgrad(dy, x), None
 
 
+def _rows(x: torch.Tensor, width: int) -> torch.Tensor:
+    """x as a matrix of rows of that width; a tensor that is one already needs no view of itself."""
+    return x if type(x) is torch.Tensor and x.dim() == 2 and x.shape[1] == width else x.reshape(-1, width)
+
+
 # ---- modules -------------------------------------------------------------------------------------------------------
 class ColumnParallelLinear(nn.Module):
     """Weight [out_features / tp, in_features]. sequence_parallel=True: input [tokens / tp, in] -> output [tokens, out / tp]."""
@@ -200,13 +231,11 @@ class ColumnParallelLinear(nn.Module):
         self.weight = nn.Parameter(w)
 
     def forward(self, x):
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
-        fn = _ColumnSeqParallel if self.sequence_parallel else _ColumnReplicatedInput
-        y = fn.apply(x2, self.weight, self.comm)
+        lead, x2 = x.shape[:-1], _rows(x, self.in_features)
         if self.sequence_parallel:
-            return y
-        return y.reshape(*lead, -1)
+            y = _one_rank_linear(x2, self.weight, self.comm, True)
+            return _ColumnSeqParallel.apply(x2, self.weight, self.comm) if y is None else y
+        return _ColumnReplicatedInput.apply(x2, self.weight, self.comm).reshape(*lead, -1)
 
 
 class RowParallelLinear(nn.Module):
@@ -223,13 +252,11 @@ class RowParallelLinear(nn.Module):
         self.weight = nn.Parameter(w)
 
     def forward(self, x):
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features // self.comm.size)
-        fn = _RowSeqParallel if self.sequence_parallel else _RowAllReduce
-        y = fn.apply(x2, self.weight, self.comm)
+        lead, x2 = x.shape[:-1], _rows(x, self.in_features // self.comm.size)
         if self.sequence_parallel:
-            return y
-        return y.reshape(*lead, -1)
+            y = _one_rank_linear(x2, self.weight, self.comm, False)
+            return _RowSeqParallel.apply(x2, self.weight, self.comm) if y is None else y
+        return _RowAllReduce.apply(x2, self.weight, self.comm).reshape(*lead, -1)
 
 
 def _init_shard(w: torch.Tensor, std: float, seed: Optional[int], rank: int, dim: int, full: int) -> None:
@@ -266,9 +293,10 @@ class TensorParallelMLP(nn.Module):
 
     def forward(self, x_local):
         gu = self.gate_up(x_local)
-        h = _block.swiglu(gu, self._plain)
-        return self.down(self._plain(gu) if h is None else h)
+        h = _block.swiglu(gu, _plain_swiglu)
+        return self.down(_plain_swiglu(gu) if h is None else h)
 
-    def _plain(self, gu):
-        g, u = gu[:, : self.ffn_local], gu[:, self.ffn_local:]
-        return torch.nn.functional.silu(g) * u
+
+def _plain_swiglu(gu):
+    ffn = gu.shape[1] // 2
+    return torch.nn.functional.silu(gu[:, :ffn]) * gu[:, ffn:]
