@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include "../kernels/primitives.cuh"
+#include "sm100_ptx.cuh"
 
 namespace hccl {
 namespace moe {
@@ -27,6 +28,7 @@ struct MoeArgs {
     uint32_t T, K, H, E, cap, mxfp8;
     uint64_t wsOff;            // workspace offset in every heap
     MoeLayout L;
+    uint32_t segVecs;          // combine: 16-byte vectors of an output row per warp (a multiple of 32)
     uint32_t identity;         // emulation: copy recvX -> yBuf at the end of dispatch
 };
 
@@ -63,6 +65,29 @@ __device__ __forceinline__ uint8_t ToE4m3(float v)
     return (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
 }
 
+// Eight bf16 values of a 1 x 32 block that four neighbouring lanes share -> e4m3 values and the block's scale. Called by whole warps.
+__device__ __forceinline__ uint2 QuantizeVec(const uint4 &raw, uint8_t *scale)
+{
+    const __nv_bfloat162 *h = (const __nv_bfloat162 *)&raw;
+    float f[8], amax = 0.f;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        const float2 p = __bfloat1622float2(h[x]);
+        f[2 * x] = p.x; f[2 * x + 1] = p.y;
+        amax = fmaxf(amax, fmaxf(fabsf(p.x), fabsf(p.y)));
+    }
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    *scale = E8m0For(amax);
+    const float inv = exp2f((float)(127 - (int)*scale));
+    uint32_t b[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+        b[x] = (uint32_t)ToE4m3(f[4 * x] * inv) | (uint32_t)ToE4m3(f[4 * x + 1] * inv) << 8 | (uint32_t)ToE4m3(f[4 * x + 2] * inv) << 16 |
+               (uint32_t)ToE4m3(f[4 * x + 3] * inv) << 24;
+    return make_uint2(b[0], b[1]);
+}
+
 // Slot of an entry that has no row (its expert id lies outside [0, numExperts), or nothing was sent because a receive buffer is too small):
 // a row of zeros behind the own expert-output rows, so that the combine needs no test (one per load: 4096 tokens, top-8 106 us
 // for 90; 2048 tokens, top-16 58 us for 53).
@@ -70,12 +95,13 @@ __device__ __forceinline__ uint64_t NoSlot(uint32_t me, uint32_t cap) { return (
 
 constexpr int kMoeWarps = kMoeThreads / 32;
 constexpr uint32_t kSegVecs = 128;                    // 16-byte vectors of a token row that one warp moves at a time (2 KB)
+constexpr uint32_t kSegVecsFew = 32;                  // the same where tokens are few: 512 bytes, one load per lane
 
-// A (token, 2 KB segment) range of the grid's CTA `cta`: contiguous, so a CTA meets few tokens and every row is spread over
+// A (token, segment) range of the grid's CTA `cta`: contiguous, so a CTA meets few tokens and every row is spread over
 // as many CTAs as there are when tokens are few.
-__device__ __forceinline__ void MoeItems(const MoeArgs &A, uint32_t cta, uint32_t G, uint32_t *segs, uint64_t *lo, uint64_t *hi)
+__device__ __forceinline__ void MoeItems(const MoeArgs &A, uint32_t segVecs, uint32_t cta, uint32_t G, uint32_t *segs, uint64_t *lo, uint64_t *hi)
 {
-    *segs = (A.H / 8 + kSegVecs - 1) / kSegVecs;
+    *segs = (A.H / 8 + segVecs - 1) / segVecs;
     const uint64_t items = (uint64_t)A.T * *segs;
     *lo = items * cta / G;
     *hi = items * (cta + 1) / G;
@@ -114,9 +140,10 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
     __shared__ uint32_t sWarp[kMoeWarps][kMaxExperts]; // per warp: entries of e in the current batch, then the first row of the warp's entries
     __shared__ uint32_t sRow[kMoeThreads];             // destination row of the batch's entries
 
+    if (SOLO) { sm100::LetDependentsStart(); sm100::DependencyWait(); }
     uint32_t segs;
     uint64_t itemLo, itemHi;
-    MoeItems(A, cta, G, &segs, &itemLo, &itemHi);
+    MoeItems(A, kSegVecs, cta, G, &segs, &itemLo, &itemHi);
     const uint32_t tLo = (uint32_t)(itemLo / segs), tHi = (uint32_t)((itemHi + segs - 1) / segs);    // tokens this CTA touches
 
     // 1. histogram of this rank's entries
@@ -243,24 +270,7 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (v0 + j * 32 >= rowVecs) break;                     // rows are multiples of 32 vectors: whole warps take this
-                    const __nv_bfloat162 *h = (const __nv_bfloat162 *)&r[j];
-                    float f[8], amax = 0.f;
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) {
-                        const float2 p = __bfloat1622float2(h[x]);
-                        f[2 * x] = p.x; f[2 * x + 1] = p.y;
-                        amax = fmaxf(amax, fmaxf(fabsf(p.x), fabsf(p.y)));
-                    }
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                    se[j] = E8m0For(amax);
-                    const float inv = exp2f((float)(127 - (int)se[j]));
-                    uint32_t b[2];
-#pragma unroll
-                    for (int x = 0; x < 2; ++x)
-                        b[x] = (uint32_t)ToE4m3(f[4 * x] * inv) | (uint32_t)ToE4m3(f[4 * x + 1] * inv) << 8 | (uint32_t)ToE4m3(f[4 * x + 2] * inv) << 16 |
-                               (uint32_t)ToE4m3(f[4 * x + 3] * inv) << 24;
-                    q[j] = make_uint2(b[0], b[1]);
+                    q[j] = QuantizeVec(r[j], &se[j]);
                 }
             }
             for (uint32_t kk = 0; kk < K; ++kk) {
@@ -331,6 +341,114 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
     }
 }
 
+// Dispatch of few tokens on one rank. The general kernel's time is then its chain of steps, some twenty block-wide barriers from the
+// histogram to the rows. Here the row of an entry is counted directly: how many entries go to an earlier expert, or to the same one before
+// it. Every CTA holds all entries in its threads' registers (at most kFewEntries) and counts for its own few (at most kFewOwn) with one
+// warp-wide sum each, while the first pieces of its rows are already on their way. The CTA behind the last one with rows counts the
+// experts' totals.
+constexpr uint32_t kFewEntries = 8 * kMoeThreads, kFewOwn = 64;
+inline uint32_t FewOwn(const MoeArgs &A, uint32_t G)     // bound on the entries of one CTA's tokens
+{
+    const uint64_t segs = (A.H / 8 + kSegVecsFew - 1) / kSegVecsFew, items = ((uint64_t)A.T * segs + G - 1) / G;
+    return (uint32_t)((items + segs - 2) / segs + 1) * A.K;
+}
+__global__ void __launch_bounds__(kMoeThreads) MoeDispatchFewKernel(const DevComm *c, const __grid_constant__ MoeArgs A)
+{
+    __shared__ uint32_t sOwn[kFewOwn], sRow[kFewOwn], sCnt[kMoeWarps][kFewOwn + 1], sTotal[kMaxExperts];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = A.K, E = A.E, entries = A.T * K;
+    const uint32_t G = gridDim.x - 1, cta = blockIdx.x, rowVecs = A.H / 8;
+    sm100::LetDependentsStart();
+    sm100::DependencyWait();
+    char *ws = c->heap[0] + A.wsOff;
+    uint64_t *slotMap = (uint64_t *)(ws + A.L.slotMap);
+    const uint64_t noSlot = NoSlot(0, A.cap);
+    uint32_t e[kFewEntries / kMoeThreads];
+#pragma unroll
+    for (uint32_t r = 0; r < kFewEntries / kMoeThreads; ++r) {
+        const uint32_t i = r * kMoeThreads + tid;
+        e[r] = i < entries ? (uint32_t)A.topkIdx[i] : 0xffffffffu;
+        if (e[r] >= E) e[r] = 0xffffffffu;               // no row: behind all experts
+    }
+    if (cta == G) {
+        for (uint32_t x = tid; x < E; x += kMoeThreads) sTotal[x] = 0;
+        for (uint32_t v = tid; v < rowVecs; v += kMoeThreads) ((uint4 *)(ws + A.L.yBuf + (uint64_t)A.cap * A.H * 2))[v] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+#pragma unroll
+        for (uint32_t r = 0; r < kFewEntries / kMoeThreads; ++r) if (e[r] < E) atomicAdd(&sTotal[e[r]], 1u);
+        __syncthreads();
+        for (uint32_t x = tid; x < E; x += kMoeThreads) ((int32_t *)(ws + A.L.recvCounts))[x] = (int32_t)sTotal[x];
+        return;
+    }
+    uint32_t segs;
+    uint64_t itemLo, itemHi;
+    MoeItems(A, kSegVecsFew, cta, G, &segs, &itemLo, &itemHi);
+    const uint32_t tLo = (uint32_t)(itemLo / segs), tHi = (uint32_t)((itemHi + segs - 1) / segs), first = tLo * K, own = (tHi - tLo) * K;
+    auto piece = [&](uint64_t it) {
+        const uint32_t v = (uint32_t)(it % segs) * kSegVecsFew + lane;
+        return v < rowVecs ? ((const uint4 *)((const char *)A.x + it / segs * A.H * 2))[v] : make_uint4(0, 0, 0, 0);
+    };
+    uint4 next = itemLo + warp < itemHi ? piece(itemLo + warp) : make_uint4(0, 0, 0, 0);
+    if (tid < own) {
+        const uint32_t x = (uint32_t)A.topkIdx[first + tid];
+        sOwn[tid] = x < E ? x : 0xffffffffu;
+    }
+    __syncthreads();
+    const uint32_t rounds = (entries + kMoeThreads - 1) / kMoeThreads;
+    for (uint32_t j = 0; j <= own; ++j) {                // j = own: all entries that have a row
+        const uint32_t mine = j < own ? sOwn[j] : 0xffffffffu, at = j < own ? first + j : 0;
+        uint32_t n = 0;
+#pragma unroll
+        for (uint32_t r = 0; r < kFewEntries / kMoeThreads; ++r)
+            if (r < rounds) n += e[r] < mine || (e[r] == mine && r * kMoeThreads + tid < at);
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) sCnt[warp][j] = n;
+    }
+    __syncthreads();
+    uint32_t total = 0;
+#pragma unroll
+    for (int w = 0; w < kMoeWarps; ++w) total += sCnt[w][own];
+    if (tid < own) {
+        uint32_t row = 0;
+#pragma unroll
+        for (int w = 0; w < kMoeWarps; ++w) row += sCnt[w][tid];
+        sRow[tid] = row;
+    }
+    __syncthreads();
+    if (total > A.cap) {                                 // receive buffer too small: report, move nothing
+        if (cta == 0 && tid == 0) {
+            DevStatus *st = c->status;
+            st->rank = 0; st->observed = total; st->expected = A.cap; st->phase = 62;
+            __threadfence_system();
+            *((volatile uint32_t *)&st->code) = 2u;
+        }
+        if (tid < own) slotMap[first + tid] = noSlot;
+        return;
+    }
+    for (uint64_t it = itemLo + warp; it < itemHi; it += kMoeWarps) {
+        const uint4 r = next;
+        if (it + kMoeWarps < itemHi) next = piece(it + kMoeWarps);
+        const uint32_t t = (uint32_t)(it / segs), seg = (uint32_t)(it % segs), v = seg * kSegVecsFew + lane;
+        uint2 q;
+        uint8_t se;
+        if (A.mxfp8) q = QuantizeVec(r, &se);
+        for (uint32_t kk = 0; kk < K; ++kk) {
+            const uint32_t j = (t - tLo) * K + kk, ex = sOwn[j], row = sRow[j];
+            const bool has = ex < E;                     // and row < total <= cap
+            if (seg == 0 && lane == 0) {
+                slotMap[first + j] = has ? row : noSlot;
+                if (has) ((int32_t *)(ws + A.L.recvSrc))[row] = (int32_t)t;
+            }
+            if (!has || v >= rowVecs) continue;
+            if (!A.mxfp8) {
+                ((uint4 *)(ws + A.L.recvX + (uint64_t)row * A.H * 2))[v] = r;
+            } else {
+                ((uint2 *)(ws + A.L.recvX + (uint64_t)row * A.H))[v] = q;
+                if ((lane & 3) == 0) ((uint8_t *)(ws + A.L.recvScales + (uint64_t)row * (A.H / 32)))[v / 4] = se;
+            }
+        }
+    }
+}
+
 // Combine: out[t] = sum over k, in order, of weight * expert row (zeros for an entry without one). Bound by reading topK rows per token. KMAX (8 or 16) keeps
 // the row addresses and weights of a token in registers; a warp takes 2 KB of the output row at a time, all KMAX source rows
 // of a vector in flight. 2048 tokens of hidden 4096, top-16 (128 registers, 24 bytes spilled): 137 us, now 53 (rows alone 44).
@@ -342,6 +460,7 @@ __global__ void __launch_bounds__(kMoeThreads) MoeCombineKernel(const DevComm *c
     const int me = SOLO ? 0 : c->rank;
     char *ws = c->heap[me] + A.wsOff;
     const uint64_t *slotMap = (const uint64_t *)(ws + A.L.slotMap);
+    if (SOLO) { sm100::LetDependentsStart(); sm100::DependencyWait(); }
     if (!SOLO) {
         // every rank's expert outputs are complete once it has entered this kernel
         if (blockIdx.x == 0) {
@@ -355,7 +474,7 @@ __global__ void __launch_bounds__(kMoeThreads) MoeCombineKernel(const DevComm *c
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = A.K, rowVecs = A.H / 8;
     uint32_t segs;
     uint64_t itemLo, itemHi;
-    MoeItems(A, blockIdx.x, gridDim.x, &segs, &itemLo, &itemHi);
+    MoeItems(A, A.segVecs, blockIdx.x, gridDim.x, &segs, &itemLo, &itemHi);
     for (uint64_t it = itemLo + warp; it < itemHi; it += kMoeWarps) {
         const uint32_t t = (uint32_t)(it / segs), seg = (uint32_t)(it % segs);
         const uint4 *rows[KMAX];
@@ -368,8 +487,8 @@ __global__ void __launch_bounds__(kMoeThreads) MoeCombineKernel(const DevComm *c
                 w[j] = A.weights[t * K + j];
             }
         uint4 *dst = (uint4 *)((char *)A.out + (uint64_t)t * A.H * 2);
-        const uint32_t vEnd = (seg + 1) * kSegVecs < rowVecs ? (seg + 1) * kSegVecs : rowVecs;
-        for (uint32_t v = seg * kSegVecs + lane; v < vEnd; v += 32) {
+        const uint32_t vEnd = (seg + 1) * A.segVecs < rowVecs ? (seg + 1) * A.segVecs : rowVecs;
+        for (uint32_t v = seg * A.segVecs + lane; v < vEnd; v += 32) {
             float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             uint4 raw[KMAX];
 #pragma unroll

@@ -67,14 +67,30 @@ MoeArgs MakeArgs(const HcclMoeConfig &cfg, const MoeLayout &L, uint64_t wsOff, u
     a.T = T; a.K = cfg.topK; a.H = cfg.hidden; a.E = cfg.numExperts; a.cap = Capacity(cfg); a.mxfp8 = cfg.mxfp8;
     a.wsOff = wsOff;
     a.L = L;
+    a.segVecs = kSegVecs;
     return a;
 }
 
-// One rank: no more CTAs than 2 KB pieces of token rows (every CTA of the dispatch counts all entries first).
-uint32_t SoloCtas(const MoeArgs &a, uint32_t ctas)
+// One rank: no more CTAs than pieces of token rows (every CTA of the dispatch counts all entries first).
+uint32_t SoloCtas(const MoeArgs &a, uint32_t segVecs, uint32_t ctas)
 {
-    const uint64_t items = (uint64_t)a.T * ((a.H / 8 + kSegVecs - 1) / kSegVecs);
+    const uint64_t items = (uint64_t)a.T * ((a.H / 8 + segVecs - 1) / segVecs);
     return (uint32_t)std::min<uint64_t>(ctas, items);
+}
+
+// One rank: a plain launch that may start while the kernel before it drains.
+cudaError_t LaunchSolo(const void *fn, void **params, uint32_t ctas, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kMoeThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, params);
 }
 
 // solo: a communicator of one rank needs no barrier among CTAs, so the kernel is launched without the cooperative constraint.
@@ -87,7 +103,7 @@ template <bool EMU> HcclResult LaunchMoe(bool dispatch, const DevComm *comms, co
     if (!EMU && solo) {
         const void *fn = dispatch ? (const void *)MoeDispatchKernel<false, true>
                                   : a.K <= 8 ? (const void *)MoeCombineKernel<false, true, 8> : (const void *)MoeCombineKernel<false, true, 16>;
-        e = cudaLaunchKernel(fn, dim3(ctas), dim3(kMoeThreads), params, 0, s);
+        e = LaunchSolo(fn, params, ctas, s);
     } else {
         const void *fn = dispatch ? (const void *)MoeDispatchKernel<EMU, false>
                                   : a.K <= 8 ? (const void *)MoeCombineKernel<EMU, false, 8> : (const void *)MoeCombineKernel<EMU, false, 16>;
@@ -151,7 +167,15 @@ HcclResult HcclMoeDispatch(HcclMoeHandle handle, const void *x, const int32_t *t
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.x = x;
     a.topkIdx = topkIdx;
-    CHK_RET(LaunchMoe<false>(true, c->devCommPtr, a, nullptr, st->solo ? SoloCtas(a, st->ctas) : st->ctas, 1, stream, st->solo));
+    const uint32_t fewCtas = SoloCtas(a, kSegVecsFew, st->ctas);
+    if (st->solo && (uint64_t)a.T * a.K <= kFewEntries && FewOwn(a, fewCtas) <= kFewOwn) {
+        const DevComm *comms = c->devCommPtr;
+        void *params[] = {(void *)&comms, (void *)&a};
+        const cudaError_t e = LaunchSolo((const void *)MoeDispatchFewKernel, params, fewCtas + 1, stream);
+        if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u)", cudaGetErrorString(e), fewCtas + 1); return HCCL_E_RUNTIME; }
+    } else {
+        CHK_RET(LaunchMoe<false>(true, c->devCommPtr, a, nullptr, st->solo ? SoloCtas(a, kSegVecs, st->ctas) : st->ctas, 1, stream, st->solo));
+    }
     st->lastTokens = numTokens;
     c->counters.kernelsLaunched++;
     CountLaunch();
@@ -182,7 +206,9 @@ HcclResult HcclMoeCombine(HcclMoeHandle handle, const float *topkWeights, void *
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.weights = topkWeights;
     a.out = out;
-    CHK_RET(LaunchMoe<false>(false, c->devCommPtr, a, nullptr, st->solo ? SoloCtas(a, st->combineCtas) : st->ctas, 1, stream, st->solo));
+    // few tokens on one rank: small pieces, so that a warp has one load of each row to wait for
+    if (st->solo && (uint64_t)a.T * (a.H / 8) <= (uint64_t)st->combineCtas * kMoeWarps * 2 * kSegVecsFew) a.segVecs = kSegVecsFew;
+    CHK_RET(LaunchMoe<false>(false, c->devCommPtr, a, nullptr, st->solo ? SoloCtas(a, a.segVecs, st->combineCtas) : st->ctas, 1, stream, st->solo));
     c->counters.kernelsLaunched++;
     CountLaunch();
     c->counters.ops++;

@@ -291,3 +291,48 @@ def test_ids_outside_the_experts_among_ranks(nranks, T, E, K, H):
             for x, o, wt, out in zip(xs, ok, ws, outs):
                 ref = x.double() * torch.where(o, wt, 0.0).double().sum(1, keepdim=True)
                 assert bool(((out.double() - ref).abs() <= ref.abs() * (2.0 ** -8 + K * 2.0 ** -23) + 1e-30).all())
+
+
+@pytest.mark.parametrize("T,E,K,H,mxfp8,ctas", [(512, 256, 8, 256, False, ""), (513, 256, 8, 256, False, ""), (4096, 320, 1, 512, True, ""), (4097, 7, 1, 256, False, ""), (1, 3, 2, 7168, True, ""),
+                                                (256, 64, 16, 2304, True, ""), (100, 16, 8, 512, False, "5"), (40, 16, 8, 512, True, "40")])
+def test_one_rank_few_tokens(T, E, K, H, mxfp8, ctas, monkeypatch):
+    """Both sides of the lines between the dispatch that counts rows directly and the general one (entries in all, entries per CTA), some entries
+    without a row: the general kernel's layout, and a combine over it."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    if ctas:
+        monkeypatch.setenv("HCCL_MOE_CTAS", ctas)
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(T + K)
+        x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+        idx = torch.randint(0, E, (T, K), generator=g, device="cuda").to(torch.int32)
+        idx[torch.rand(T, K, generator=g, device="cuda") < 0.05] = -1
+        w = torch.rand(T, K, generator=g, device="cuda")
+        d = MoeDispatcher(comm, E, K, H, T, max_recv_rows=T * K, mxfp8=mxfp8)
+        rx, rs, counts, src = d.dispatch(x, idx)
+        y = torch.randn(T * K, H, generator=g, device="cuda").to(torch.bfloat16)
+        d.expert_out.copy_(y)
+        out = d.combine(w)
+        torch.cuda.synchronize()
+        flat, ok = idx.flatten().long(), (idx >= 0)
+        n = int(ok.sum())
+        order = torch.argsort(torch.where(ok.flatten(), flat, E), stable=True)[:n]
+        assert torch.equal(counts.long(), torch.bincount(flat[ok.flatten()], minlength=E))
+        assert torch.equal(src[:n].long(), order // K)
+        rows = x[order // K]
+        if mxfp8:
+            amax = rows.float().view(n, H // 32, 32).abs().amax(2)
+            assert torch.equal(rs[:n].long(), torch.ceil(torch.log2(amax.double() / 448)).long() + 127)
+            scaled = rows.float().view(n, H // 32, 32) * torch.exp2(127 - rs[:n].float())[..., None]
+            assert torch.equal(rx[:n].view(torch.uint8), scaled.to(torch.float8_e4m3fn).view(n, H).view(torch.uint8))
+        else:
+            assert torch.equal(rx[:n], rows)
+        slot = torch.zeros(T * K, dtype=torch.long, device="cuda")
+        slot[order] = torch.arange(n, device="cuda")
+        terms = torch.where(ok[..., None], w.double()[..., None] * y[slot.view(T, K)].double(), 0.0)
+        ref = terms.sum(1)
+        assert bool(((out.double() - ref).abs() <= terms.abs().sum(1) * K * 2.0 ** -23 + ref.abs() * 2.0 ** -8).all())
+        d.close()
+    finally:
+        comm.destroy()
