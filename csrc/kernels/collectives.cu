@@ -45,9 +45,11 @@ template <typename T, int OP, bool EMU> __device__ void AllReduceOneShotBody(KCt
     const uint64_t slot = Up128(A.bytes);
     Part p = PartOf(A.bytes, gridDim.x, blockIdx.x);
     const char *in = (const char *)A.in + p.off;
-    for (int d = 0; d < n; ++d) {
-        int r = (k.rank + d) % n;
-        BlockCopy(k.Ccl(r) + (uint64_t)k.rank * slot + p.off, in, p.len);
+    for (int d0 = 0; d0 < n; d0 += kCopyGroup) {
+        CopyPart c[kCopyGroup];
+#pragma unroll
+        for (int q = 0; q < kCopyGroup; ++q) c[q] = {k.Ccl((k.rank + d0 + q) % n) + (uint64_t)k.rank * slot + p.off, in, p.len};
+        BlockCopies(c, n - d0 < kCopyGroup ? n - d0 : kCopyGroup);
     }
     if (!ChannelBarrier(k, 1)) return;
     const char *slots[kMaxRanks];
@@ -62,10 +64,15 @@ template <typename T, int OP> __device__ void AllReduceTwoShotCore(KCtx &k, cons
 {
     const int n = k.nranks;
     const uint64_t slice = Up128((bytes + n - 1) / n);
-    for (int d = 0; d < n; ++d) {
-        int r = (k.rank + d) % n;
-        Part p = PartOf(SliceLen(bytes, slice, r), k.vGrid, k.vBlock);
-        BlockCopy(k.Ccl(r) + (uint64_t)k.rank * slice + p.off, in + (uint64_t)r * slice + p.off, p.len);
+    for (int d0 = 0; d0 < n; d0 += kCopyGroup) {
+        CopyPart c[kCopyGroup];
+#pragma unroll
+        for (int q = 0; q < kCopyGroup; ++q) {
+            const int r = (k.rank + d0 + q) % n;
+            const Part p = PartOf(SliceLen(bytes, slice, r), k.vGrid, k.vBlock);
+            c[q] = {k.Ccl(r) + (uint64_t)k.rank * slice + p.off, in + (uint64_t)r * slice + p.off, p.len};
+        }
+        BlockCopies(c, n - d0 < kCopyGroup ? n - d0 : kCopyGroup);
     }
     if (!ChannelBarrier(k, 1)) return;
     {
@@ -76,10 +83,15 @@ template <typename T, int OP> __device__ void AllReduceTwoShotCore(KCtx &k, cons
         ReduceSlots<T, OP, kMaxRanks>((T *)(out + (uint64_t)k.rank * slice + p.off), res, slots, n, p.len / sizeof(T));
     }
     if (!ChannelBarrier(k, 2)) return;
-    for (int d = 1; d < n; ++d) {
-        int r = (k.rank + d) % n;
-        Part p = PartOf(SliceLen(bytes, slice, r), k.vGrid, k.vBlock);
-        BlockCopy(out + (uint64_t)r * slice + p.off, k.Ccl(r) + (uint64_t)n * slice + p.off, p.len);
+    for (int d0 = 1; d0 < n; d0 += kCopyGroup) {
+        CopyPart c[kCopyGroup];
+#pragma unroll
+        for (int q = 0; q < kCopyGroup; ++q) {
+            const int r = (k.rank + d0 + q) % n;
+            const Part p = PartOf(SliceLen(bytes, slice, r), k.vGrid, k.vBlock);
+            c[q] = {out + (uint64_t)r * slice + p.off, k.Ccl(r) + (uint64_t)n * slice + p.off, p.len};
+        }
+        BlockCopies(c, n - d0 < kCopyGroup ? n - d0 : kCopyGroup);
     }
 }
 template <typename T, int OP, bool EMU> __device__ void AllReduceTwoShotBody(KCtx &k, const CollArgs &A)
@@ -645,9 +657,12 @@ template <bool EMU> __device__ void BroadcastZcNvlsBody(KCtx &k, const CollArgs 
 #include "pipelined.cuh"
 
 // ================================================================================================ kernels
-#define COLL_KERNEL_TYPED(NAME, BODY)                                                                                  \
+#define COLL_KERNEL_TYPED(NAME, BODY) COLL_KERNEL_TYPED_BOUNDS(NAME, BODY, __launch_bounds__(kThreads))
+// two CTAs of these stay on an SM (emulated ranks and concurrent operators count on it), whatever the loads in flight would take
+#define COLL_KERNEL_TYPED_TWO(NAME, BODY) COLL_KERNEL_TYPED_BOUNDS(NAME, BODY, __launch_bounds__(kThreads, 2))
+#define COLL_KERNEL_TYPED_BOUNDS(NAME, BODY, BOUNDS)                                                                   \
     template <typename T, bool EMU>                                                                                    \
-    __global__ void __launch_bounds__(kThreads) NAME(const DevComm *comms, const __grid_constant__ CollArgs a, const CollArgs *emuArgs) \
+    __global__ void BOUNDS NAME(const DevComm *comms, const __grid_constant__ CollArgs a, const CollArgs *emuArgs) \
     {                                                                                                                  \
         KCtx k = EnterCollective<EMU>(comms);                                                                          \
         const CollArgs &A = ArgsOf<EMU>(a, emuArgs);                                                                   \
@@ -659,8 +674,8 @@ template <bool EMU> __device__ void BroadcastZcNvlsBody(KCtx &k, const CollArgs 
         }                                                                                                              \
         LeaveCollective(k);                                                                                            \
     }
-COLL_KERNEL_TYPED(KAllReduceOneShot, AllReduceOneShotBody)
-COLL_KERNEL_TYPED(KAllReduceTwoShot, AllReduceTwoShotBody)
+COLL_KERNEL_TYPED_TWO(KAllReduceOneShot, AllReduceOneShotBody)
+COLL_KERNEL_TYPED_TWO(KAllReduceTwoShot, AllReduceTwoShotBody)
 COLL_KERNEL_TYPED(KReduceScatterV, ReduceScatterVBody)
 COLL_KERNEL_TYPED(KReduce, ReduceBody)
 template <typename T, int OP, bool EMU> __device__ void AllReducePipePlainBody(KCtx &k, const CollArgs &A) { pipe::AllReduceBody<T, OP, EMU, false>(k, A); }
@@ -671,15 +686,16 @@ template <bool EMU> __device__ void AllGatherPipePlainBody(KCtx &k, const CollAr
 template <bool EMU> __device__ void AllGatherPipeNvlsBody(KCtx &k, const CollArgs &A) { pipe::AllGatherBody<EMU, true>(k, A); }
 template <bool EMU> __device__ void AlltoAllPipeBody(KCtx &k, const CollArgs &A) { pipe::AllGatherBody<EMU, false, true>(k, A); }
 COLL_KERNEL_TYPED(KAllReduceRing, AllReduceRingBody)
-COLL_KERNEL_TYPED(KAllReduceConcurrentPlain, AllReduceConcurrentPlainBody)
+COLL_KERNEL_TYPED_TWO(KAllReduceConcurrentPlain, AllReduceConcurrentPlainBody)
 COLL_KERNEL_TYPED(KAllReduceZc, AllReduceZcPlainBody)
 COLL_KERNEL_TYPED(KReduceScatterZc, ReduceScatterZcPlainBody)
 COLL_KERNEL_TYPED(KAllReducePipe, AllReducePipePlainBody)
 COLL_KERNEL_TYPED(KReduceScatterPipe, ReduceScatterPipePlainBody)
 
-#define COLL_KERNEL_NVLS(NAME, BODY)                                                                                   \
+#define COLL_KERNEL_NVLS(NAME, BODY) COLL_KERNEL_NVLS_BOUNDS(NAME, BODY, __launch_bounds__(kThreads))
+#define COLL_KERNEL_NVLS_BOUNDS(NAME, BODY, BOUNDS)                                                                    \
     template <typename T, int OP, bool EMU>                                                                            \
-    __global__ void __launch_bounds__(kThreads) NAME(const DevComm *comms, const __grid_constant__ CollArgs a, const CollArgs *emuArgs) \
+    __global__ void BOUNDS NAME(const DevComm *comms, const __grid_constant__ CollArgs a, const CollArgs *emuArgs) \
     {                                                                                                                  \
         KCtx k = EnterCollective<EMU>(comms);                                                                          \
         BODY<T, OP, EMU>(k, ArgsOf<EMU>(a, emuArgs));                                                                  \
@@ -689,7 +705,7 @@ COLL_KERNEL_NVLS(KAllReduceNvlsOneShot, AllReduceNvlsOneShotBody)
 COLL_KERNEL_NVLS(KAllReduceNvlsTwoShot, AllReduceNvlsTwoShotBody)
 COLL_KERNEL_NVLS(KReduceScatterNvls, ReduceScatterNvlsBody)
 COLL_KERNEL_NVLS(KAllReducePipeNvls, AllReducePipeNvlsBody)
-COLL_KERNEL_NVLS(KAllReduceConcurrentNvls, AllReduceConcurrentNvlsBody)
+COLL_KERNEL_NVLS_BOUNDS(KAllReduceConcurrentNvls, AllReduceConcurrentNvlsBody, __launch_bounds__(kThreads, 2))
 COLL_KERNEL_NVLS(KAllReduceZcNvls, AllReduceZcNvlsBody)
 COLL_KERNEL_NVLS(KReduceScatterZcNvls, ReduceScatterZcNvlsBody)
 COLL_KERNEL_NVLS(KReduceScatterPipeNvls, ReduceScatterPipeNvlsBody)

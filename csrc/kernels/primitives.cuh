@@ -335,6 +335,37 @@ __device__ __forceinline__ void BlockCopy(void *dst, const void *src, uint64_t n
     }
 }
 
+// `n` copies at once (at most kCopyGroup): a thread's loads from all sources are in flight together, where one copy after the other waits for
+// each. Falls back to that where a side is not 16-byte aligned.
+constexpr int kCopyGroup = 4;
+struct CopyPart { void *dst; const void *src; uint64_t len; };
+__device__ __forceinline__ void BlockCopies(const CopyPart (&p)[kCopyGroup], int n)
+{
+    uint64_t nvec[kCopyGroup], most = 0;
+    uintptr_t any = 0;
+#pragma unroll
+    for (int q = 0; q < kCopyGroup; ++q) {
+        nvec[q] = q < n ? p[q].len >> 4 : 0;
+        if (nvec[q] > most) most = nvec[q];
+        if (q < n) any |= (uintptr_t)p[q].dst | (uintptr_t)p[q].src | (HCCL_RANGE_OK(p[q].dst, p[q].len) && HCCL_RANGE_OK(p[q].src, p[q].len) ? 0u : 1u);
+    }
+    if (any & 15u) {                                     // a range that is not in order is reported and skipped there
+        for (int q = 0; q < n; ++q) BlockCopy(p[q].dst, p[q].src, p[q].len);
+        return;
+    }
+    for (uint64_t i = threadIdx.x; i < most; i += blockDim.x) {
+        uint4 v[kCopyGroup];
+#pragma unroll
+        for (int q = 0; q < kCopyGroup; ++q) if (i < nvec[q]) v[q] = ((const uint4 *)p[q].src)[i];
+#pragma unroll
+        for (int q = 0; q < kCopyGroup; ++q) if (i < nvec[q]) ((uint4 *)p[q].dst)[i] = v[q];
+    }
+#pragma unroll
+    for (int q = 0; q < kCopyGroup; ++q)
+        if (q < n)
+            for (uint64_t i = (nvec[q] << 4) + threadIdx.x; i < p[q].len; i += blockDim.x) ((char *)p[q].dst)[i] = ((const char *)p[q].src)[i];
+}
+
 // ---------------------------------------------------------------------------------------------- typed reduction
 template <typename T> struct Acc { using type = T; };
 template <> struct Acc<__half> { using type = float; };
@@ -367,19 +398,21 @@ __device__ __forceinline__ void ReduceSlots(T *out, T *out2, const char *const *
     if (!HCCL_RANGE_OK(out, nElems * sizeof(T)) || (out2 && !HCCL_RANGE_OK(out2, nElems * sizeof(T)))) return;
     bool vecOk = (((uintptr_t)out | (uintptr_t)out2) & 15u) == 0;
     uint64_t nvec = vecOk ? nElems / VE : 0;
+    // the vectors of up to four slots are in flight together; what is added to what, and in which order, does not depend on it
+    constexpr int G = 4;
     for (uint64_t i = threadIdx.x; i < nvec; i += blockDim.x) {
         A acc[VE];
-        {
-            uint4 raw = ((const uint4 *)slotBase[0])[i];
-            const T *e = (const T *)&raw;
+        for (int r0 = 0; r0 < nslots; r0 += G) {
+            uint4 raw[G];
 #pragma unroll
-            for (int j = 0; j < VE; ++j) acc[j] = ToAcc<T>(e[j]);
-        }
-        for (int r = 1; r < nslots; ++r) {
-            uint4 raw = ((const uint4 *)slotBase[r])[i];
-            const T *e = (const T *)&raw;
+            for (int g = 0; g < G; ++g) if (r0 + g < nslots) raw[g] = ((const uint4 *)slotBase[r0 + g])[i];
 #pragma unroll
-            for (int j = 0; j < VE; ++j) acc[j] = Combine<OP, A>(acc[j], ToAcc<T>(e[j]));
+            for (int g = 0; g < G; ++g) {
+                if (r0 + g >= nslots) break;
+                const T *e = (const T *)&raw[g];
+#pragma unroll
+                for (int j = 0; j < VE; ++j) acc[j] = r0 + g == 0 ? ToAcc<T>(e[j]) : Combine<OP, A>(acc[j], ToAcc<T>(e[j]));
+            }
         }
         uint4 res;
         T *e = (T *)&res;
