@@ -76,6 +76,23 @@ def test_gemm_split_k(shape, bt, split, out_dtype):
     assert bool((out[M] == 7.0).all())
 
 
+@pytest.mark.parametrize("shape", [(65, 4088, 5128), (128, 8200, 5000), (129, 1744, 5240), (200, 520, 2048), (257, 3704, 5128), (512, 1448, 5128), (512, 2824, 2048), (300, 5408, 2056)])
+def test_gemm_split_k_of_65_to_512_rows(shape):
+    """Products that the automatic choice sends to 64-, 128- and 256-row split-K tiles, and the first beyond its lines (bound as above)."""
+    from hccl_b200.ops import gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    gemm.gemm_bf16(a, w, out[:M])
+    torch.cuda.synchronize()
+    gemm.check_error()
+    ref, mag = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    assert bool(((out[:M].double() - ref).abs() <= mag * K * 2.0 ** -24 + ref.abs() * 2.0 ** -8 + 1e-30).all())
+    assert bool((out[M] == 7.0).all())
+
+
 @pytest.mark.parametrize("shape", [(1, 8, 8), (128, 64, 64), (100, 72, 200), (1000, 264, 520), (384, 768, 1600), (2048, 4104, 1032), (4096, 2560, 264)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 def test_gemm_nn(shape, out_dtype):
