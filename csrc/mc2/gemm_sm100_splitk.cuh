@@ -54,6 +54,7 @@ struct SplitKParams {
     uint32_t *errorWord;
     const uint8_t *sfB, *sfA;     // block-scaled form: scale atoms [rows / 128][K / 128][512]
     uint32_t sfAtomsA;            // 128-row atoms A's scale array holds
+    uint32_t earlyB;              // the kernel before this one wrote A only: B may be read while it runs
 };
 
 namespace splitk {
@@ -106,14 +107,23 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
     TcFenceAfter();
     const uint32_t tmemBase = *tmemPtr;
     LetDependentsStart();
-    DependencyWait();                        // up to here nothing touched global memory but the kernel's own parameters
+    const uint8_t *sfB = MX ? p.sfB + (uint64_t)(n0 / 128) * kTotal * kSfAtomBytes : nullptr;
+    auto loadB = [&](uint32_t kb, uint32_t stage) {
+        MbarExpectTx(&full[stage], S::kBBytes + S::kABytes + S::kSfBytes);
+        TmaLoad2D(sB + stage * S::kBBytes, &p.tmapB, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)n0);
+        if (MX) BulkLoadG2S(sSF + stage * S::kSfBytes, sfB + (uint64_t)kb * kSfAtomBytes, kSfAtomBytes, &full[stage]);
+    };
+    const uint32_t early = !p.earlyB ? 0 : kHi - kLo < (uint32_t)STAGES ? kHi - kLo : (uint32_t)STAGES;
+    if (warp == 0 && ElectOne())
+        for (uint32_t i = 0; i < early; ++i) loadB(kLo + i, i);
+    __syncwarp();
+    DependencyWait();                        // up to here nothing touched global memory but the kernel's own parameters and, where allowed, B
 
     if (warp == 0) {
         if (ElectOne()) {
             uint32_t stage = 0, phase = 0;
-            const uint8_t *sfB = nullptr, *sfA[2] = {nullptr, nullptr};
+            const uint8_t *sfA[2] = {nullptr, nullptr};
             if (MX) {
-                sfB = p.sfB + (uint64_t)(n0 / 128) * kTotal * kSfAtomBytes;
 #pragma unroll
                 for (int j = 0; j < S::kAtomsA; ++j) {
                     uint32_t atom = m0 / 128 + j;                            // rows past M: any finite scales do (their operands are zero)
@@ -123,12 +133,10 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
             }
             for (uint32_t kb = kLo; kb < kHi; ++kb) {
                 if (!MbarWaitRelaxed(&empty[stage], phase ^ 1, abortWord, 0)) break;
-                MbarExpectTx(&full[stage], S::kBBytes + S::kABytes + S::kSfBytes);
-                TmaLoad2D(sB + stage * S::kBBytes, &p.tmapB, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)n0);
+                if (kb - kLo >= early) loadB(kb, stage);
                 TmaLoad2D(sA + stage * S::kABytes, &p.tmapA, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)m0);
                 if (MX) {
                     uint8_t *sf = sSF + stage * S::kSfBytes;
-                    BulkLoadG2S(sf, sfB + (uint64_t)kb * kSfAtomBytes, kSfAtomBytes, &full[stage]);
 #pragma unroll
                     for (int j = 0; j < S::kAtomsA; ++j) BulkLoadG2S(sf + (1 + j) * kSfAtomBytes, sfA[j] + (uint64_t)kb * kSfAtomBytes, kSfAtomBytes, &full[stage]);
                 }

@@ -44,7 +44,7 @@ inline SplitKChoice ChooseSplitK(uint64_t m, uint64_t n, uint64_t k, bool mx)
 
 template <int BT, bool MX>
 HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, uint32_t split, bool outFp32,
-                         cudaStream_t s)
+                         bool earlyB, cudaStream_t s)
 {
     using S = GemmSplitKSmem<BT, MX>;
     SplitKParams p{};
@@ -52,7 +52,7 @@ HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const vo
     CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * elem, 128, boxK, elem));
     CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * elem, BT, boxK, elem));
     p.C = c; p.M = M; p.N = N; p.K = K; p.split = split; p.outFp32 = outFp32; p.errorWord = GemmErrorWord();
-    p.sfA = (const uint8_t *)sfa; p.sfB = (const uint8_t *)sfb; p.sfAtomsA = (M + 127) / 128;
+    p.sfA = (const uint8_t *)sfa; p.sfB = (const uint8_t *)sfb; p.sfAtomsA = (M + 127) / 128; p.earlyB = earlyB;
     static std::atomic<bool> attrSet{false};
     auto kern = GemmKernelSplitK<BT, MX>;
     const size_t smem = S::kTotal + 1024;
@@ -79,9 +79,10 @@ HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const vo
     return HCCL_SUCCESS;
 }
 
+// earlyB: the kernel before this one in the stream wrote nothing but A, and itself waited for all before it
 template <bool MX>
 HcclResult LaunchSplitK(SplitKChoice ch, const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32,
-                        cudaStream_t s)
+                        cudaStream_t s, bool earlyB = false)
 {
     if (((uintptr_t)c | (uintptr_t)sfa | (uintptr_t)sfb) & 15u) {           // four results per store, 16-byte bulk copies of the scales
         HCCL_ERROR("split-K GEMM: result %p and block scales %p, %p must be 16-byte aligned", c, sfa, sfb);
@@ -92,11 +93,11 @@ HcclResult LaunchSplitK(SplitKChoice ch, const void *a, const void *sfa, const v
     // block-scaled tiles have to start on a scale atom
     if (ch.split == 0 || ch.split > 8 || ch.split > kBlocks || (MX && ch.bt < 64 && M > ch.bt)) return HCCL_E_PARA;
     switch (ch.bt) {
-        case 16: return LaunchSplitKT<16, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, s);
-        case 32: return LaunchSplitKT<32, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, s);
-        case 64: return LaunchSplitKT<64, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, s);
-        case 128: return LaunchSplitKT<128, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, s);
-        case 256: return LaunchSplitKT<256, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, s);
+        case 16: return LaunchSplitKT<16, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 32: return LaunchSplitKT<32, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 64: return LaunchSplitKT<64, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 128: return LaunchSplitKT<128, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 256: return LaunchSplitKT<256, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
         default: return HCCL_E_PARA;
     }
 }

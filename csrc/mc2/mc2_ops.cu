@@ -491,6 +491,16 @@ HcclResult HcclAllGatherMatmulMxfp8(const void *aLocal, const void *sfaLocal, co
     return RunFused(AGMM, c, aLocal, b, out, nullptr, mLocal, n, k, stream, sfaLocal, sfb);
 }
 
+// One rank: the three block-scaled operators are the product itself; activations given in bf16 are quantised on the way.
+HcclResult HcclQuantizeMatmulMxfp8(const void *a, void *payload, void *scales, const void *b, const void *sfb, void *out, uint64_t m, uint64_t n, uint64_t k, HcclComm comm,
+                                   cudaStream_t stream)
+{
+    Comm *c = CommFromHandle(comm);
+    if (!c) return HCCL_E_PTR;
+    if (c->nranks != 1) { HCCL_ERROR("HcclQuantizeMatmulMxfp8 takes a communicator of one rank"); return HCCL_E_NOT_SUPPORT; }
+    return HcclQuantizeGemmMxfp8(a, payload, scales, b, sfb, out, m, n, k, 0, stream);
+}
+
 HcclResult HcclMatmulReduceScatterMxfp8(const void *a, const void *sfa, const void *b, const void *sfb, void *out, uint64_t m, uint64_t n, uint64_t kLocal,
                                         HcclComm comm, cudaStream_t stream)
 {

@@ -35,7 +35,8 @@ def _decl():
         l.HcclAllGatherMatmulMxfp8.argtypes = [vp, vp, vp, vp, vp, u64, u64, u64, vp, vp]
         l.HcclMatmulReduceScatterMxfp8.argtypes = [vp, vp, vp, vp, vp, u64, u64, u64, vp, vp]
         l.HcclMatmulAllReduceMxfp8.argtypes = [vp, vp, vp, vp, vp, u64, u64, u64, vp, vp]
-        for f in (l.HcclQuantizeMxfp8, l.HcclGemmMxfp8Variant, l.HcclAllGatherMatmulMxfp8, l.HcclMatmulReduceScatterMxfp8, l.HcclMatmulAllReduceMxfp8):
+        l.HcclQuantizeMatmulMxfp8.argtypes = [vp, vp, vp, vp, vp, vp, u64, u64, u64, vp, vp]
+        for f in (l.HcclQuantizeMxfp8, l.HcclQuantizeMatmulMxfp8, l.HcclGemmMxfp8Variant, l.HcclAllGatherMatmulMxfp8, l.HcclMatmulReduceScatterMxfp8, l.HcclMatmulAllReduceMxfp8):
             f.restype = ctypes.c_int
         l._mx_declared = True
     return l
@@ -53,10 +54,14 @@ def empty_like_quantized(rows: int, k: int, device) -> MxTensor:
     return MxTensor(torch.empty((rows, k), dtype=torch.uint8, device=device), torch.empty(scale_bytes(rows, k), dtype=torch.uint8, device=device), rows, k)
 
 
-def quantize(x: torch.Tensor, out: Optional[MxTensor] = None, stream=None) -> MxTensor:
-    """bf16 [rows, K] (K % 128 == 0) -> MxTensor, on the GPU."""
+def _check_quantizable(x: torch.Tensor) -> None:
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.dim() == 2):
         raise ValueError("quantize takes a contiguous 2-D bf16 CUDA tensor")
+
+
+def quantize(x: torch.Tensor, out: Optional[MxTensor] = None, stream=None) -> MxTensor:
+    """bf16 [rows, K] (K % 128 == 0) -> MxTensor, on the GPU."""
+    _check_quantizable(x)
     rows, k = x.shape
     if out is None:
         out = empty_like_quantized(rows, k, x.device)
@@ -112,13 +117,29 @@ def _as_mx_fresh(x, stream=None) -> MxTensor:
 def _as_mx(x, stream=None) -> MxTensor:
     if isinstance(x, MxTensor):
         return x
+    return quantize(x, out=_act_buffer(x, stream), stream=stream)
+
+
+def _act_buffer(x: torch.Tensor, stream) -> MxTensor:
     key = (x.shape[0], x.shape[1], x.device, _stream(stream))
     buf = _ACT_BUFFERS.get(key)
     if buf is None:
         if len(_ACT_BUFFERS) >= 16:
             _ACT_BUFFERS.clear()
         buf = _ACT_BUFFERS[key] = empty_like_quantized(x.shape[0], x.shape[1], x.device)
-    return quantize(x, out=buf, stream=stream)
+    return buf
+
+
+def _one_rank(comm, a: torch.Tensor, w, out: Optional[torch.Tensor], stream) -> torch.Tensor:
+    """The three operators on one rank with activations in bf16: the product alone, quantisation in the same call."""
+    _check_quantizable(a)
+    buf, w = _act_buffer(a, stream), _as_mx_fresh(w, stream)
+    m, k = a.shape
+    if out is None:
+        out = torch.empty((m, w.rows), dtype=torch.bfloat16, device=a.device)
+    check(_decl().HcclQuantizeMatmulMxfp8(a.data_ptr(), buf.payload.data_ptr(), buf.scales.data_ptr(), w.payload.data_ptr(), w.scales.data_ptr(), out.data_ptr(), m, w.rows, k,
+                                          comm.handle, _stream(stream)), "HcclQuantizeMatmulMxfp8")
+    return out
 
 
 def gemm(a, w, out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16, tile_n: int = 0, stream=None) -> torch.Tensor:
@@ -134,6 +155,8 @@ def gemm(a, w, out: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torc
 
 def all_gather_matmul(comm, a_local, w, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """out[size*m, N] = all_gather(a_local[m, K]) @ w[N, K]^T; the gather moves e4m3 bytes and scales."""
+    if comm.size == 1 and not isinstance(a_local, MxTensor):
+        return _one_rank(comm, a_local, w, out, stream)
     a, w = _as_mx(a_local, stream), _as_mx_fresh(w, stream)
     if out is None:
         out = torch.empty((a.rows * comm.size, w.rows), dtype=torch.bfloat16, device=a.payload.device)
@@ -144,6 +167,8 @@ def all_gather_matmul(comm, a_local, w, out: Optional[torch.Tensor] = None, stre
 
 def matmul_reduce_scatter(comm, a, w, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
     """out[M/size, N] = reduce_scatter_rows(a[M, Klocal] @ w[N, Klocal]^T); partials travel as bf16, summed in rank order."""
+    if comm.size == 1 and not isinstance(a, MxTensor):
+        return _one_rank(comm, a, w, out, stream)
     a, w = _as_mx(a, stream), _as_mx_fresh(w, stream)
     if out is None:
         out = torch.empty((a.rows // comm.size, w.rows), dtype=torch.bfloat16, device=a.payload.device)
@@ -153,6 +178,8 @@ def matmul_reduce_scatter(comm, a, w, out: Optional[torch.Tensor] = None, stream
 
 
 def matmul_all_reduce(comm, a, w, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
+    if comm.size == 1 and not isinstance(a, MxTensor):
+        return _one_rank(comm, a, w, out, stream)
     a, w = _as_mx(a, stream), _as_mx_fresh(w, stream)
     if out is None:
         out = torch.empty((a.rows, w.rows), dtype=torch.bfloat16, device=a.payload.device)

@@ -80,6 +80,9 @@ HcclResult HcclQuantizeMxfp8(const void *in, void *payload, void *scales, uint64
 /* C[m,n] = A[m,k] * B[n,k]^T on one GPU, both operands block-scaled, bf16 (or fp32) result. */
 HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
                          cudaStream_t stream);
+/* The same with A in bf16: quantised into payload and scales first, the product may read B while that runs. */
+HcclResult HcclQuantizeGemmMxfp8(const void *a, void *payload, void *scales, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
+                                 cudaStream_t stream);
 /* tileN 128, 192 or 256 forces the tile width, 2192 / 2256 CTA pairs of that width, 100000 + 1000 * S + BT split-K (0 = automatic). */
 HcclResult HcclGemmMxfp8Variant(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
                                 int tileN, cudaStream_t stream);
@@ -91,6 +94,9 @@ HcclResult HcclMatmulReduceScatterMxfp8(const void *a, const void *sfa, const vo
                                         HcclComm comm, cudaStream_t stream);
 HcclResult HcclMatmulAllReduceMxfp8(const void *a, const void *sfa, const void *b, const void *sfb, void *out, uint64_t m, uint64_t n, uint64_t kLocal,
                                     HcclComm comm, cudaStream_t stream);
+/* Any of the three on a communicator of one rank, activations in bf16 (quantised into payload and scales in the same call). */
+HcclResult HcclQuantizeMatmulMxfp8(const void *a, void *payload, void *scales, const void *b, const void *sfb, void *out, uint64_t m, uint64_t n, uint64_t k, HcclComm comm,
+                                   cudaStream_t stream);
 
 #ifdef __cplusplus
 }

@@ -143,3 +143,29 @@ def test_block_scaled_split_k(m, n, k, bt, split):
     torch.cuda.synchronize()
     g.check_error()
     assert bool(((out.double() - ref).abs() <= mag * k * 2.0 ** -24 + 1e-30).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 512, 512), (32, 8192, 1024), (64, 264, 14336), (300, 1024, 2048), (2048, 512, 256)])
+def test_one_rank_operators_quantise_in_the_call(m, n, k):
+    """bf16 activations on one rank: the bits of quantising first, also where the weights were written by the kernel right before the call
+    (the product may read them while the activations are quantised) and where the buffers are reused by the next call."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops import mxfp8
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        xs = [_wild((m, k), 3 + i).to(torch.bfloat16) for i in range(3)]
+        ws = [mxfp8.quantize(_wild((n, k), 9 + i).to(torch.bfloat16)) for i in range(3)]
+        refs = [mxfp8.gemm(mxfp8.quantize(x), w) for x, w in zip(xs, ws)]
+        shared = mxfp8.MxTensor(torch.zeros_like(ws[0].payload), torch.zeros_like(ws[0].scales), n, k)
+        torch.cuda.synchronize()
+        outs = []
+        for op in (mxfp8.matmul_all_reduce, mxfp8.all_gather_matmul, mxfp8.matmul_reduce_scatter):
+            for x, w in zip(xs, ws):
+                shared.scales.copy_(w.scales)
+                shared.payload.copy_(w.payload)
+                outs.append(op(comm, x, shared))
+        torch.cuda.synchronize()
+        for i, out in enumerate(outs):
+            assert torch.equal(out, refs[i % 3])
+    finally:
+        comm.destroy()
