@@ -111,7 +111,9 @@ struct OpNode : Node {
         } catch (py::error_already_set &e) {                 // an exception of the Python form keeps its type on its way through the engine
             py::gil_scoped_acquire gil;
             e.restore();
-            throw_python_error();
+            python_error err;
+            err.persist();
+            throw err;
         }
     }
     void release_variables() override
