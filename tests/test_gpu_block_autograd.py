@@ -194,3 +194,85 @@ def test_saved_tensors_that_come_back_changed(name):
             out = _outs(f(*ins))
         for a, b in zip(torch.autograd.grad(out, ins, [torch.ones_like(o) for o in out]), ref):
             assert (a.double() - b.double()).norm() <= 2.0 ** -5 * b.double().norm()
+
+
+def _tiny(seed=3):
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.models.llama import Llama, LlamaConfig
+    torch.zeros(1, device="cuda")
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    return comm, Llama(LlamaConfig.tiny(), comm, dtype=torch.bfloat16, device="cuda", seed=seed)
+
+
+@pytest.mark.parametrize("tokens", [(2, 128), (1, 100)])
+def test_native_nodes_give_the_bits_of_the_python_functions(tokens, monkeypatch):
+    """A whole decoder through both: loss and gradients, on rows that the fused linear takes and on rows that it does not; saved tensors on the
+    CPU, a recomputed block, a graph run twice."""
+    from torch.utils.checkpoint import checkpoint
+    from hccl_b200.models.llama import _rope_tables
+    from hccl_b200.ops import block
+    comm, model = _tiny()
+    try:
+        t = torch.randint(0, 512, (tokens[0], tokens[1] + 1), device="cuda")
+        params = list(model.parameters())
+
+        def step():
+            loss = model(t[:, :-1].contiguous(), t[:, 1:].contiguous())
+            first = torch.autograd.grad(loss, params, retain_graph=True)
+            return [loss.detach(), *first, *torch.autograd.grad(loss, params)]
+
+        native = step()
+        with torch.autograd.graph.save_on_cpu():
+            loss = model(t[:, :-1].contiguous(), t[:, 1:].contiguous())
+        offloaded = torch.autograd.grad(loss, params)
+        x = torch.randn(tokens[0] * tokens[1], 256, device="cuda").to(torch.bfloat16).requires_grad_()
+        rope = _rope_tables(tokens[1], 32, 500000.0, "cuda")
+        args = (x, *tokens, *rope)
+        plain, = torch.autograd.grad(model.blocks[0](*args).sum(), x)
+        again, = torch.autograd.grad(checkpoint(model.blocks[0], *args, use_reentrant=False).sum(), x)
+        assert torch.equal(plain, again)
+        monkeypatch.setattr(block, "_NODES", None)
+        for a, b in zip(native, step()):
+            assert torch.equal(a, b)
+        for a, b in zip(native[1:], offloaded):
+            assert torch.equal(a, b)
+    finally:
+        comm.destroy()
+
+
+def test_native_nodes_keep_the_engine_s_rules():
+    """A graph that was freed and a weight that changed in place are refused; an error of the Python form keeps its type; a module that holds its
+    own output is collected."""
+    import gc
+    import weakref
+    from hccl_b200.models.llama import RMSNorm, _rope_tables
+    from hccl_b200.ops import block
+    comm, model = _tiny()
+    try:
+        x = torch.randn(256, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+        run = lambda: model.blocks[0](x, 2, 128, *_rope_tables(128, 32, 500000.0, "cuda")).sum()
+        out = run()
+        out.backward()
+        with pytest.raises(RuntimeError, match="second time"):
+            out.backward()
+        out = run()
+        with torch.no_grad():
+            model.blocks[0].mlp.down.weight.mul_(1)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            out.backward()
+
+        def failing(x, w):
+            raise LookupError("plain form")
+
+        w = torch.ones(256, device="cuda", dtype=torch.bfloat16).requires_grad_()
+        y = block.rms_norm(x, w, 1e-5, failing)
+        with pytest.raises(LookupError, match="plain form"):
+            torch.autograd.grad(y.sum(), x, create_graph=True)
+        norm = RMSNorm(256, 1e-5, torch.bfloat16, "cuda")
+        norm.kept = norm(x)
+        gone = weakref.ref(norm)
+        del norm
+        gc.collect()
+        assert gone() is None
+    finally:
+        comm.destroy()
