@@ -233,14 +233,15 @@ static HcclResult LaunchPair(uint32_t bn, const void *a, const void *b, void *c,
     return LaunchPlain2CtaT<256>(a, b, c, M, N, K, outFp32, s);
 }
 
-// Which tile kernel: waves of tiles times what a wave of that kernel takes. Half of the cost counts whole waves and half the fraction of the
-// GPU that the tiles fill, since idle SMs leave power to the others. A wave per 4096 of K takes the tile's columns (pairs) or 0.9 of them (one
-// CTA) plus what its loads of A and B hold it up, which is more where K is no multiple of 64: its rows then straddle 128-byte lines. The
-// constants are fitted to 124 random products on one B200 (64 to 8192 rows, N 512 to 28672, K 512 to 16384; every width timed in random
-// order, each after 30 to 50 ms of its own): the choice is 0.3 % slower than the best width on average. The widths above 256 and these
-// costs against 192 / 224 / 256 chosen by waves alone: 1473 x 17784 x 9608 496 / 420 us (512 columns), 3882 x 18048 x 6664 957 / 814 (512),
+// Which tile kernel: waves of tiles times what a wave of that kernel takes, plus 40 for the launch of clusters. A part of the cost counts whole
+// waves and the rest the fraction of the GPU that the tiles fill, since idle SMs leave power to the others. A wave per 4096 of K takes the tile's
+// columns (pairs) or 0.9 of them (one CTA) plus what its loads of A and B hold it up, which is more where K is no multiple of 64: its rows then
+// straddle 128-byte lines. The constants are fitted to 130 random products on one B200 (64 to 8192 rows, N 512 to 28672, K 512 to 16384; every
+// width timed in random order, each after 30 to 50 ms of its own): the choice is 0.3 to 0.5 % slower than the best width on average. The widths above
+// 256 and these costs against 192 / 224 / 256 chosen by waves alone: 1473 x 17784 x 9608 496 / 420 us (512 columns), 3882 x 18048 x 6664 957 / 814 (512),
 // 2115 x 2304 x 2344 31.6 / 24.2 (288), 7073 x 6152 x 5992 598 / 425 (480), 2048 x 4096 x 14336 195 / 181 (480), 1000 x 6144 x 4096 43.0 / 42.1 (352),
-// 8192 x 8192 x 28672 3133 / 2867 (512).
+// 8192 x 8192 x 28672 3133 / 2867 (512). Wide tiles where K is made of 64s pay for their exposed start only in few waves or with a long K: 8100 x 28032 x 2624 takes
+// 947 with 512 columns and 856 with 256.
 struct TileChoice { bool pair; uint32_t bn; };
 static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposedB)
 {
@@ -251,11 +252,12 @@ static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposed
     auto waves = [](uint64_t tiles, uint64_t slots) { return (double)((tiles + slots - 1) / slots); };
     auto one = [&](uint32_t bn) {
         const uint64_t tiles = rows * ((n + bn - 1) / bn);
-        return (0.8 * waves(tiles, sms) + 0.2 * filled(tiles, sms)) * (20 + k4 * (0.9 * bn + (straddle ? 170 : 130)));
+        return (0.8 * waves(tiles, sms) + 0.2 * filled(tiles, sms)) * (20 + k4 * (0.9 * bn + (straddle ? 170 : 95)));
     };
     auto pair = [&](uint32_t bn) {
         const uint64_t tiles = rowPairs * ((n + bn - 1) / bn);
-        return 10 + 0.5 * (waves(tiles, pairs) + filled(tiles, pairs)) * ((bn > 256 ? 20 : 0) + k4 * (bn + (straddle ? 200 : 90)));
+        const double whole = straddle ? 0.5 : 0.7, start = bn <= 256 ? 0 : straddle ? 20 : 45;
+        return 40 + (whole * waves(tiles, pairs) + (1 - whole) * filled(tiles, pairs)) * (start + k4 * (bn + (straddle ? 200 : 45)));
     };
     TileChoice best{false, 64};
     double cost = one(64);
@@ -266,7 +268,7 @@ static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposed
     if (!Gemm2CtaEnabled()) return best;
     offer(true, 256, pair(256));
     if (transposedB) {           // its tiles are whole 64-column boxes per CTA; 2048 x 4096 x 28672 387 / 379 us (256 / 512), 4096 x 4096 x 14336 394 / 373
-        offer(true, 512, pair(512) / 0.96);          // 2048 x 14336 x 4096, 3 % cheaper by this count, takes 186 / 204
+        if (k >= 8192) offer(true, 512, pair(512));  // not with a short K: 2986 x 16472 x 3712 303 / 330, 2048 x 14336 x 4096 186 / 204
         return best;
     }
     offer(true, 224, pair(224));
