@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -102,8 +103,24 @@ variable_list FromPython(const py::object &r, size_t n)
 
 struct OpNode : Node {
     std::unique_ptr<PyRef> held;               // what the Python form's backward pass needs beside tensors
+    struct Saved { SavedVariable *v; bool output; };
     virtual variable_list Backward(variable_list &&g) = 0;
-    virtual void Release() = 0;
+    virtual std::vector<Saved> Keeps() = 0;
+    // Compiled autograd traces the backward pass: it runs on stand-ins, which the Python form takes. Its graph holds what `held` refers to
+    // as constants, so no graph is taken for another node.
+    void compiled_args(torch::dynamo::autograd::CompiledNodeArgs &args) const override
+    {
+        static std::atomic<int64_t> count{0};
+        for (const Saved &k : const_cast<OpNode *>(this)->Keeps()) args.collect(*k.v, k.output);
+        args.collect(count++);
+    }
+    variable_list apply_with_saved(const variable_list &inputs, torch::dynamo::autograd::SwapSavedVariables &saved) override
+    {
+        for (const Saved &k : Keeps()) saved.before(*k.v);
+        variable_list r = apply(variable_list(inputs));
+        for (const Saved &k : Keeps()) saved.after(*k.v);
+        return r;
+    }
     variable_list apply(variable_list &&g) final
     {
         try {
@@ -119,7 +136,7 @@ struct OpNode : Node {
     void release_variables() override
     {
         std::lock_guard<std::mutex> lock(mutex_);
-        Release();
+        for (const Saved &k : Keeps()) k.v->reset_data();
     }
     // the saved tensors; not locked longer, since the Python form may run other graphs
     template <class... S> std::tuple<std::conditional_t<true, at::Tensor, S>...> Unpack(const S &...saved)
@@ -154,7 +171,7 @@ c10::DeviceIndex DeviceOf(const at::Tensor &t) { return t.is_cuda() ? t.device()
 struct RmsNormNode : OpNode {
     SavedVariable x, w, rstd;
     std::string name() const override { return "_RmsNormBackward"; }
-    void Release() override { x.reset_data(); w.reset_data(); rstd.reset_data(); }
+    std::vector<Saved> Keeps() override { return {{&x, true}, {&w, true}, {&rstd, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         if (!g[0].defined()) return {g[1], g[2]};
@@ -227,7 +244,7 @@ struct RopeNode : OpNode {
     uint32_t heads = 0, kvHeads = 0, headDim = 0;
     at::TensorOptions options;
     std::string name() const override { return "_RopeQkvBackward"; }
-    void Release() override { cos.reset_data(); sin.reset_data(); }
+    std::vector<Saved> Keeps() override { return {{&cos, false}, {&sin, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         const auto [c, s] = Unpack(cos, sin);
@@ -288,7 +305,7 @@ py::object RopeQkv(py::handle qkvh, py::handle cosh, py::handle sinh, int64_t ba
 struct SwiGluNode : OpNode {
     SavedVariable gu;
     std::string name() const override { return "_SwiGluBackward"; }
-    void Release() override { gu.reset_data(); }
+    std::vector<Saved> Keeps() override { return {{&gu, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         const auto [in] = Unpack(gu);
@@ -335,7 +352,7 @@ struct LinearNode : OpNode {
     at::TensorOptions options;
     bool column = false;
     std::string name() const override { return column ? "_ColumnSeqParallelBackward" : "_RowSeqParallelBackward"; }
-    void Release() override { x.reset_data(); w.reset_data(); }
+    std::vector<Saved> Keeps() override { return {{&x, false}, {&w, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         const auto [xv, wv] = Unpack(x, w);
@@ -399,7 +416,7 @@ struct XentNode : OpNode {
     int64_t vocabStart = 0;
     at::TensorOptions options;
     std::string name() const override { return "_VocabParallelCrossEntropyBackward"; }
-    void Release() override { logits.reset_data(); targets.reset_data(); mx.reset_data(); packed.reset_data(); }
+    std::vector<Saved> Keeps() override { return {{&logits, false}, {&targets, false}, {&mx, false}, {&packed, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         const auto [l, t, m, p] = Unpack(logits, targets, mx, packed);

@@ -165,8 +165,13 @@ def _row_backward(comm, x, w, dy_local):
     return dx, _wgrad(dyg, x)                                                                                  # AG(dy)^T @ x
 
 
-_block.PYTHON_BACKWARD["column"] = _column_backward
-_block.PYTHON_BACKWARD["row"] = _row_backward
+def _one_rank_backward(backward):
+    """The products by single operations where a tensor is a stand-in (a traced or batched one has no memory for the kernels)."""
+    return lambda comm, x, w, dy: backward(comm, x, w, dy) if all([_block._plain_tensor(t) for t in (x, w, dy)]) else (dy @ w, dy.t() @ x)
+
+
+_block.PYTHON_BACKWARD["column"] = _one_rank_backward(_column_backward)
+_block.PYTHON_BACKWARD["row"] = _one_rank_backward(_row_backward)
 
 
 def _one_rank_linear(x: torch.Tensor, w: torch.Tensor, comm, column: bool):
