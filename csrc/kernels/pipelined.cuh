@@ -1,6 +1,6 @@
 // Warp-specialised, software-pipelined collectives for payloads of any size in ONE launch.
 //
-// The plain kernels of collectives.cu run "stage in -> synchronise -> move over NVLink -> synchronise -> copy out" as
+// The plain kernels of collectives.cuh run "stage in -> synchronise -> move over NVLink -> synchronise -> copy out" as
 // consecutive phases of the whole CTA, so the local staging copies and the NVLink traffic never overlap and the payload
 // of a launch is bounded by the scratch size. Here the CTA's warps split into role groups that work on different
 // sub-chunks at the same time, connected by counting flags in the symmetric heap:

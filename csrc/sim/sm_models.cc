@@ -1,6 +1,6 @@
 // Schedule models of the SM / NVLS collective kernels, in the IR the offline checker consumes.
 //
-// The kernels in csrc/kernels/collectives.cu are not issued task by task, so they have no schedule of their own to check.
+// The kernels in csrc/kernels/collectives.cuh are not issued task by task, so they have no schedule of their own to check.
 // Each model here restates one kernel body as IR, with the same arithmetic (128-byte aligned slots and slices, PartOf
 // splitting over channels, rank rotation) and the same synchronisation points: a channel is a queue, a channel barrier
 // is a POST to and a WAIT for every peer on that channel's slot, a plain peer store / load is a WRITE / READ, a rank-ordered
