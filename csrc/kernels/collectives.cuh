@@ -47,65 +47,48 @@ __device__ __forceinline__ uint64_t SliceLen(uint64_t total, uint64_t slice, int
 // ================================================================================================ AllReduce one-shot
 // Every rank pushes its part into slot[rank] of every rank's scratch; after the channel barrier each rank reduces the
 // n local slots in rank order.
-template <typename T, int OP, bool EMU> __device__ void AllReduceOneShotBody(KCtx &k, const CollArgs &A)
+template <typename T, bool EMU> __device__ void AllReduceOneShotBody(KCtx &k, const CollArgs &A)
 {
     const int n = k.nranks;
     const uint64_t slot = Up128(A.bytes);
     Part p = PartOf(A.bytes, gridDim.x, blockIdx.x);
-    const char *in = (const char *)A.in + p.off;
-    for (int d0 = 0; d0 < n; d0 += kCopyGroup) {
-        CopyPart c[kCopyGroup];
-#pragma unroll
-        for (int q = 0; q < kCopyGroup; ++q) c[q] = {k.Ccl((k.rank + d0 + q) % n) + (uint64_t)k.rank * slot + p.off, in, p.len};
-        BlockCopies(c, n - d0 < kCopyGroup ? n - d0 : kCopyGroup);
-    }
+    BlockCopyToAll(n, [&](int d) { return k.Ccl((k.rank + d) % n) + (uint64_t)k.rank * slot + p.off; }, (const char *)A.in + p.off, p.len);
     if (!ChannelBarrier(k, 1)) return;
-    const char *slots[kMaxRanks];
-    for (int r = 0; r < n; ++r) slots[r] = k.Ccl(k.rank) + (uint64_t)r * slot + p.off;
-    ReduceSlots<T, OP, kMaxRanks>((T *)((char *)A.out + p.off), (T *)nullptr, slots, n, p.len / sizeof(T));
+    ReduceSlotsBy<T>(A.op, (T *)((char *)A.out + p.off), (T *)nullptr, k.Ccl(k.rank) + p.off, slot, n, p.len / sizeof(T));
 }
 
 // ================================================================================================ AllReduce two-shot
 // Reduce-scatter by push (slice j of every rank lands in rank j's slots), ordered reduce of the own slice, all-gather
-// by pull from the owners' result regions. Small slices are bound by the latency of loads, so copies to and from several ranks, and the slots of
-// the reduction, have their loads in flight together: four emulated ranks, 1000003 bf16 values, 16 CTAs each, 56.0 -> 49.1 us a pass on one B200.
-template <typename T, int OP> __device__ void AllReduceTwoShotCore(KCtx &k, const char *in, char *out, uint64_t bytes)
+// by pull from the owners' result regions. Bound by the latency of loads: a thread has four in flight from the first copy to the last, and one from each of
+// four slots in the reduction. Emulated ranks on one B200, 256 CTAs in all at most, 16 MB of bf16 per rank, us per call for 2 / 4 / 5 / 8 ranks: 60.9 / 85.2 / 102.5 /
+// 137.2; with one copy after the other and one slot after the other 63.1 / 93.6 / 105.1 / 146.5; with groups of four copies and one load of each in flight
+// 70.0 / 91.7 / 115.7 / 149.6; with the copies taking turns by vector 65.6 / 85.4 / 104.2 / 136.8. Not measured on several GPUs.
+template <typename T> __device__ __forceinline__ void AllReduceTwoShotCore(KCtx &k, const char *in, char *out, uint64_t bytes, uint32_t op)
 {
     const int n = k.nranks;
     const uint64_t slice = Up128((bytes + n - 1) / n);
-    for (int d0 = 0; d0 < n; d0 += kCopyGroup) {
-        CopyPart c[kCopyGroup];
-#pragma unroll
-        for (int q = 0; q < kCopyGroup; ++q) {
-            const int r = (k.rank + d0 + q) % n;
-            const Part p = PartOf(SliceLen(bytes, slice, r), k.vGrid, k.vBlock);
-            c[q] = {k.Ccl(r) + (uint64_t)k.rank * slice + p.off, in + (uint64_t)r * slice + p.off, p.len};
-        }
-        BlockCopies(c, n - d0 < kCopyGroup ? n - d0 : kCopyGroup);
-    }
+    auto part = [&](int r) { return PartOf(SliceLen(bytes, slice, r), k.vGrid, k.vBlock); };
+    BlockCopiesOf(n, [&](int d) {
+        const int r = (k.rank + d) % n;
+        const Part p = part(r);
+        return CopyPart{k.Ccl(r) + (uint64_t)k.rank * slice + p.off, in + (uint64_t)r * slice + p.off, p.len};
+    });
     if (!ChannelBarrier(k, 1)) return;
     {
-        Part p = PartOf(SliceLen(bytes, slice, k.rank), k.vGrid, k.vBlock);
-        const char *slots[kMaxRanks];
-        for (int r = 0; r < n; ++r) slots[r] = k.Ccl(k.rank) + (uint64_t)r * slice + p.off;
+        const Part p = part(k.rank);
         T *res = (T *)(k.Ccl(k.rank) + (uint64_t)n * slice + p.off);
-        ReduceSlots<T, OP, kMaxRanks>((T *)(out + (uint64_t)k.rank * slice + p.off), res, slots, n, p.len / sizeof(T));
+        ReduceSlotsBy<T>(op, (T *)(out + (uint64_t)k.rank * slice + p.off), res, k.Ccl(k.rank) + p.off, slice, n, p.len / sizeof(T));
     }
     if (!ChannelBarrier(k, 2)) return;
-    for (int d0 = 1; d0 < n; d0 += kCopyGroup) {
-        CopyPart c[kCopyGroup];
-#pragma unroll
-        for (int q = 0; q < kCopyGroup; ++q) {
-            const int r = (k.rank + d0 + q) % n;
-            const Part p = PartOf(SliceLen(bytes, slice, r), k.vGrid, k.vBlock);
-            c[q] = {out + (uint64_t)r * slice + p.off, k.Ccl(r) + (uint64_t)n * slice + p.off, p.len};
-        }
-        BlockCopies(c, n - d0 < kCopyGroup ? n - d0 : kCopyGroup);
-    }
+    BlockCopiesOf(n - 1, [&](int d) {
+        const int r = (k.rank + 1 + d) % n;
+        const Part p = part(r);
+        return CopyPart{out + (uint64_t)r * slice + p.off, k.Ccl(r) + (uint64_t)n * slice + p.off, p.len};
+    });
 }
-template <typename T, int OP, bool EMU> __device__ void AllReduceTwoShotBody(KCtx &k, const CollArgs &A)
+template <typename T, bool EMU> __device__ void AllReduceTwoShotBody(KCtx &k, const CollArgs &A)
 {
-    AllReduceTwoShotCore<T, OP>(k, (const char *)A.in, (char *)A.out, A.bytes);
+    AllReduceTwoShotCore<T>(k, (const char *)A.in, (char *)A.out, A.bytes, A.op);
 }
 
 // ================================================================================================ AllReduce ring
@@ -287,23 +270,24 @@ template <typename T, int OP, bool EMU> __device__ void AllReduceNvlsTwoShotBody
 // executors split one payload between two planes by HCCL_ALG_MULTIPLE_DIMENSION_SPLIT_RATIO; reference:
 // src/ops/all_reduce/executor/ins_v2_all_reduce_concurrent_executor.cc:159,479-487). Without a multicast mapping both parts
 // run the peer-store algorithm. Channels are CTA indices, so the two parts never share a flag word.
-template <typename T, int OP, bool EMU, bool NVLS> __device__ void AllReduceConcurrentBody(KCtx &k, const CollArgs &A)
+template <typename T, bool EMU, bool NVLS, int NVLS_OP = HCCL_REDUCE_SUM> __device__ void AllReduceConcurrentBody(KCtx &k, const CollArgs &A)
 {
     const uint64_t bytesA = A.splitBytes;
     const uint32_t ctasA = A.splitCtas;
     const int n = k.nranks;
-    if (blockIdx.x < ctasA) {
-        k.vGrid = ctasA; k.vBlock = blockIdx.x; k.cclShift = 0;
-        if constexpr (NVLS) AllReduceNvlsTwoShotCore<T, OP>(k, (const char *)A.in, (char *)A.out, bytesA);
-        else AllReduceTwoShotCore<T, OP>(k, (const char *)A.in, (char *)A.out, bytesA);
-    } else {
-        k.vGrid = gridDim.x - ctasA; k.vBlock = blockIdx.x - ctasA;
-        k.cclShift = 2ull * (uint64_t)n * Up128((bytesA + n - 1) / n);          // past the larger of the two layouts of part A
-        AllReduceTwoShotCore<T, OP>(k, (const char *)A.in + bytesA, (char *)A.out + bytesA, A.bytes - bytesA);
+    const bool first = blockIdx.x < ctasA;
+    k.vGrid = first ? ctasA : gridDim.x - ctasA;
+    k.vBlock = first ? blockIdx.x : blockIdx.x - ctasA;
+    k.cclShift = first ? 0 : 2ull * (uint64_t)n * Up128((bytesA + n - 1) / n);      // past the larger of the two layouts of part A
+    if (NVLS && first) {
+        if constexpr (NVLS) AllReduceNvlsTwoShotCore<T, NVLS_OP>(k, (const char *)A.in, (char *)A.out, bytesA);
+        return;
     }
+    const uint64_t off = first ? 0 : bytesA;
+    AllReduceTwoShotCore<T>(k, (const char *)A.in + off, (char *)A.out + off, first ? bytesA : A.bytes - bytesA, A.op);
 }
-template <typename T, int OP, bool EMU> __device__ void AllReduceConcurrentNvlsBody(KCtx &k, const CollArgs &A) { AllReduceConcurrentBody<T, OP, EMU, true>(k, A); }
-template <typename T, int OP, bool EMU> __device__ void AllReduceConcurrentPlainBody(KCtx &k, const CollArgs &A) { AllReduceConcurrentBody<T, OP, EMU, false>(k, A); }
+template <typename T, int OP, bool EMU> __device__ void AllReduceConcurrentNvlsBody(KCtx &k, const CollArgs &A) { AllReduceConcurrentBody<T, EMU, true, OP>(k, A); }
+template <typename T, bool EMU> __device__ void AllReduceConcurrentPlainBody(KCtx &k, const CollArgs &A) { AllReduceConcurrentBody<T, EMU, false>(k, A); }
 
 // Latency end of the pull kernels: one pass in which every thread has a 16-byte load from EACH peer in flight, instead of
 // one peer after the other (n - 1 dependent round trips when a CTA's share per peer is a few KB). kG bounds the registers.
@@ -367,7 +351,7 @@ template <bool EMU> __device__ void AllGatherVBody(KCtx &k, const CollArgs &A)
 }
 
 // ================================================================================================ ReduceScatter(V), push
-template <typename T, int OP, bool EMU> __device__ void ReduceScatterVBody(KCtx &k, const CollArgs &A)
+template <typename T, bool EMU> __device__ void ReduceScatterVBody(KCtx &k, const CollArgs &A)
 {
     const int n = k.nranks;
     uint64_t slot = 0;
@@ -380,9 +364,7 @@ template <typename T, int OP, bool EMU> __device__ void ReduceScatterVBody(KCtx 
     }
     if (!ChannelBarrier(k, 1)) return;
     Part p = PartOf(A.sendBytes[k.rank], gridDim.x, blockIdx.x);
-    const char *slots[kMaxRanks];
-    for (int r = 0; r < n; ++r) slots[r] = k.Ccl(k.rank) + (uint64_t)r * slot + p.off;
-    ReduceSlots<T, OP, kMaxRanks>((T *)((char *)A.out + p.off), (T *)nullptr, slots, n, p.len / sizeof(T));
+    ReduceSlotsBy<T>(A.op, (T *)((char *)A.out + p.off), (T *)nullptr, k.Ccl(k.rank) + p.off, slot, n, p.len / sizeof(T));
 }
 
 template <typename T, int OP, bool EMU> __device__ void ReduceScatterNvlsBody(KCtx &k, const CollArgs &A)
@@ -435,7 +417,7 @@ template <bool EMU> __device__ void BroadcastNvlsBody(KCtx &k, const CollArgs &A
 }
 
 // ================================================================================================ Reduce (to root)
-template <typename T, int OP, bool EMU> __device__ void ReduceBody(KCtx &k, const CollArgs &A)
+template <typename T, bool EMU> __device__ void ReduceBody(KCtx &k, const CollArgs &A)
 {
     const int n = k.nranks, root = (int)A.root;
     const uint64_t slot = Up128(A.bytes);
@@ -443,9 +425,7 @@ template <typename T, int OP, bool EMU> __device__ void ReduceBody(KCtx &k, cons
     BlockCopy(k.Ccl(root) + (uint64_t)k.rank * slot + p.off, (const char *)A.in + p.off, p.len);
     if (!ChannelBarrier(k, 1)) return;
     if (k.rank != root) return;
-    const char *slots[kMaxRanks];
-    for (int r = 0; r < n; ++r) slots[r] = k.Ccl(root) + (uint64_t)r * slot + p.off;
-    ReduceSlots<T, OP, kMaxRanks>((T *)((char *)A.out + p.off), (T *)nullptr, slots, n, p.len / sizeof(T));
+    ReduceSlotsBy<T>(A.op, (T *)((char *)A.out + p.off), (T *)nullptr, k.Ccl(root) + p.off, slot, n, p.len / sizeof(T));
 }
 
 // ================================================================================================ Scatter (pull from root)
@@ -666,12 +646,9 @@ template <bool EMU> __device__ void BroadcastZcNvlsBody(KCtx &k, const CollArgs 
 #include "pipelined.cuh"
 
 // ================================================================================================ kernels
-#define COLL_KERNEL_TYPED(NAME, BODY) COLL_KERNEL_TYPED_BOUNDS(NAME, BODY, __launch_bounds__(kThreads))
-// two CTAs of these stay on an SM (emulated ranks and concurrent operators count on it), whatever the loads in flight would take
-#define COLL_KERNEL_TYPED_TWO(NAME, BODY) COLL_KERNEL_TYPED_BOUNDS(NAME, BODY, __launch_bounds__(kThreads, 2))
-#define COLL_KERNEL_TYPED_BOUNDS(NAME, BODY, BOUNDS)                                                                   \
+#define COLL_KERNEL_TYPED(NAME, BODY)                                                                                  \
     template <typename T, bool EMU>                                                                                    \
-    __global__ void BOUNDS NAME(const DevComm *comms, const __grid_constant__ CollArgs a, const CollArgs *emuArgs) \
+    __global__ void __launch_bounds__(kThreads) NAME(const DevComm *comms, const __grid_constant__ CollArgs a, const CollArgs *emuArgs) \
     {                                                                                                                  \
         KCtx k = EnterCollective<EMU>(comms);                                                                          \
         const CollArgs &A = ArgsOf<EMU>(a, emuArgs);                                                                   \
@@ -683,10 +660,19 @@ template <bool EMU> __device__ void BroadcastZcNvlsBody(KCtx &k, const CollArgs 
         }                                                                                                              \
         LeaveCollective(k);                                                                                            \
     }
+// The body takes the reduction at run time. Two CTAs stay on an SM: emulated ranks and concurrent operators count on it.
+#define COLL_KERNEL_TYPED_TWO(NAME, BODY)                                                                              \
+    template <typename T, bool EMU>                                                                                    \
+    __global__ void __launch_bounds__(kThreads, 2) NAME(const DevComm *comms, const __grid_constant__ CollArgs a, const CollArgs *emuArgs) \
+    {                                                                                                                  \
+        KCtx k = EnterCollective<EMU>(comms);                                                                          \
+        BODY<T, EMU>(k, ArgsOf<EMU>(a, emuArgs));                                                                      \
+        LeaveCollective(k);                                                                                            \
+    }
 COLL_KERNEL_TYPED_TWO(KAllReduceOneShot, AllReduceOneShotBody)
 COLL_KERNEL_TYPED_TWO(KAllReduceTwoShot, AllReduceTwoShotBody)
-COLL_KERNEL_TYPED(KReduceScatterV, ReduceScatterVBody)
-COLL_KERNEL_TYPED(KReduce, ReduceBody)
+COLL_KERNEL_TYPED_TWO(KReduceScatterV, ReduceScatterVBody)
+COLL_KERNEL_TYPED_TWO(KReduce, ReduceBody)
 template <typename T, int OP, bool EMU> __device__ void AllReducePipePlainBody(KCtx &k, const CollArgs &A) { pipe::AllReduceBody<T, OP, EMU, false>(k, A); }
 template <typename T, int OP, bool EMU> __device__ void AllReducePipeNvlsBody(KCtx &k, const CollArgs &A) { pipe::AllReduceBody<T, OP, EMU, true>(k, A); }
 template <typename T, int OP, bool EMU> __device__ void ReduceScatterPipePlainBody(KCtx &k, const CollArgs &A) { pipe::ReduceScatterBody<T, OP, EMU, false>(k, A); }

@@ -335,35 +335,79 @@ __device__ __forceinline__ void BlockCopy(void *dst, const void *src, uint64_t n
     }
 }
 
-// `n` copies at once (at most kCopyGroup): a thread's loads from all sources are in flight together, where one copy after the other waits for
-// each. Falls back to that where a side is not 16-byte aligned.
-constexpr int kCopyGroup = 4;
-struct CopyPart { void *dst; const void *src; uint64_t len; };
-__device__ __forceinline__ void BlockCopies(const CopyPart (&p)[kCopyGroup], int n)
+// Copies to or from n ranks, described in shared memory, one after the other. Every thread keeps four 16-byte loads in flight across their ends,
+// where a copy by itself leaves the loads of its last vectors to wait for one another. Sides that are not 16-byte aligned are copied by
+// themselves.
+struct CopyPart { char *dst; const char *src; uint64_t len; };
+__device__ __forceinline__ void BlockCopies(const CopyPart *parts, int n)
 {
-    uint64_t nvec[kCopyGroup], most = 0;
+    uint64_t most = 0;
     uintptr_t any = 0;
-#pragma unroll
-    for (int q = 0; q < kCopyGroup; ++q) {
-        nvec[q] = q < n ? p[q].len >> 4 : 0;
-        if (nvec[q] > most) most = nvec[q];
-        if (q < n) any |= (uintptr_t)p[q].dst | (uintptr_t)p[q].src | (HCCL_RANGE_OK(p[q].dst, p[q].len) && HCCL_RANGE_OK(p[q].src, p[q].len) ? 0u : 1u);
+    for (int q = 0; q < n; ++q) {                        // a range that is not in order is reported and skipped by BlockCopy
+        const CopyPart p = parts[q];
+        if (p.len > most) most = p.len;
+        if (p.len) any |= (uintptr_t)p.dst | (uintptr_t)p.src | (HCCL_RANGE_OK(p.dst, p.len) && HCCL_RANGE_OK(p.src, p.len) ? 0u : 1u);
     }
-    if (any & 15u) {                                     // a range that is not in order is reported and skipped there
-        for (int q = 0; q < n; ++q) BlockCopy(p[q].dst, p[q].src, p[q].len);
+    if (any & 15u) {
+        for (int q = 0; q < n; ++q) BlockCopy(parts[q].dst, parts[q].src, parts[q].len);
         return;
     }
-    for (uint64_t i = threadIdx.x; i < most; i += blockDim.x) {
-        uint4 v[kCopyGroup];
+    constexpr int U = 4;
+    const uint64_t end = ((most >> 4) + blockDim.x - 1) / blockDim.x * blockDim.x;       // all threads take as many turns per copy
+    uint64_t i = threadIdx.x;
+    for (int q = 0; q < n && end;) {
+        uint4 v[U], *d[U];
 #pragma unroll
-        for (int q = 0; q < kCopyGroup; ++q) if (i < nvec[q]) v[q] = ((const uint4 *)p[q].src)[i];
+        for (int u = 0; u < U; ++u) {
+            d[u] = nullptr;
+            if (q < n && i < parts[q].len >> 4) {
+                v[u] = ((const uint4 *)parts[q].src)[i];
+                d[u] = (uint4 *)parts[q].dst + i;
+            }
+            if ((i += blockDim.x) >= end) { i = threadIdx.x; ++q; }
+        }
 #pragma unroll
-        for (int q = 0; q < kCopyGroup; ++q) if (i < nvec[q]) ((uint4 *)p[q].dst)[i] = v[q];
+        for (int u = 0; u < U; ++u) if (d[u]) *d[u] = v[u];
     }
+    for (int q = 0; q < n; ++q)
+        for (uint64_t i = (parts[q].len & ~15ull) + threadIdx.x; i < parts[q].len; i += blockDim.x) parts[q].dst[i] = parts[q].src[i];
+}
+// The same with part(q) as copy q. Called by all threads; a barrier of the CTA has to lie between two calls.
+template <class F> __device__ __forceinline__ void BlockCopiesOf(int n, F part)
+{
+    __shared__ CopyPart parts[kMaxRanks];
+    if ((int)threadIdx.x < n) parts[threadIdx.x] = part((int)threadIdx.x);
+    __syncthreads();
+    BlockCopies(parts, n);
+}
+
+// One source to n destinations (dst(q)): a vector is loaded once, four at a time.
+template <class F> __device__ __forceinline__ void BlockCopyToAll(int n, F dst, const char *src, uint64_t len)
+{
+    __shared__ char *to[kMaxRanks];
+    if ((int)threadIdx.x < n) to[threadIdx.x] = dst((int)threadIdx.x);
+    __syncthreads();
+    uintptr_t any = (uintptr_t)src;
+    for (int q = 0; q < n; ++q) any |= (uintptr_t)to[q] | (HCCL_RANGE_OK(to[q], len) && HCCL_RANGE_OK(src, len) ? 0u : 1u);
+    if (any & 15u) {
+        for (int q = 0; q < n; ++q) BlockCopy(to[q], src, len);
+        return;
+    }
+    constexpr int U = 4;
+    const uint64_t vecs = len >> 4;
+    for (uint64_t i = threadIdx.x; i < vecs; i += (uint64_t)blockDim.x * U) {
+        uint4 v[U];
 #pragma unroll
-    for (int q = 0; q < kCopyGroup; ++q)
-        if (q < n)
-            for (uint64_t i = (nvec[q] << 4) + threadIdx.x; i < p[q].len; i += blockDim.x) ((char *)p[q].dst)[i] = ((const char *)p[q].src)[i];
+        for (int u = 0; u < U; ++u) if (i + (uint64_t)u * blockDim.x < vecs) v[u] = ((const uint4 *)src)[i + (uint64_t)u * blockDim.x];
+#pragma unroll 1
+        for (int q = 0; q < n; ++q) {
+            uint4 *d = (uint4 *)to[q] + i;
+#pragma unroll
+            for (int u = 0; u < U; ++u) if (i + (uint64_t)u * blockDim.x < vecs) d[(uint64_t)u * blockDim.x] = v[u];
+        }
+    }
+    for (int q = 0; q < n; ++q)
+        for (uint64_t i = (vecs << 4) + threadIdx.x; i < len; i += blockDim.x) to[q][i] = src[i];
 }
 
 // ---------------------------------------------------------------------------------------------- typed reduction
@@ -388,24 +432,26 @@ template <int OP, typename A> __device__ __forceinline__ A Combine(A a, A b)
 
 // out[i] = slot_0[i] (op) slot_1[i] ... (op) slot_{n-1}[i], slots in rank order (the same order on every rank, so
 // every rank that reduces the same data obtains identical bits). Half-precision types accumulate in fp32.
-// slot r lives at slotBase[r] (local or peer memory), all 16-byte aligned. `out2` optionally receives a second copy.
-template <typename T, int OP, int MAXR>
-__device__ __forceinline__ void ReduceSlots(T *out, T *out2, const char *const *slotBase, int nslots, uint64_t nElems)
+// slot r lives at slots + r * stride (local or peer memory), all 16-byte aligned. `out2` optionally receives a second copy.
+template <typename T, int OP>
+__device__ __forceinline__ void ReduceSlots(T *out, T *out2, const char *slots, uint64_t stride, int nslots, uint64_t nElems)
 {
     using A = typename Acc<T>::type;
     constexpr int VE = 16 / sizeof(T);
-    for (int r = 0; r < nslots; ++r) if (!HCCL_RANGE_OK(slotBase[r], nElems * sizeof(T))) return;
+    for (int r = 0; r < nslots; ++r) if (!HCCL_RANGE_OK(slots + r * stride, nElems * sizeof(T))) return;
     if (!HCCL_RANGE_OK(out, nElems * sizeof(T)) || (out2 && !HCCL_RANGE_OK(out2, nElems * sizeof(T)))) return;
     bool vecOk = (((uintptr_t)out | (uintptr_t)out2) & 15u) == 0;
     uint64_t nvec = vecOk ? nElems / VE : 0;
     // the vectors of up to four slots are in flight together; what is added to what, and in which order, does not depend on it
     constexpr int G = 4;
+#pragma unroll 1
     for (uint64_t i = threadIdx.x; i < nvec; i += blockDim.x) {
         A acc[VE];
+#pragma unroll 1
         for (int r0 = 0; r0 < nslots; r0 += G) {
             uint4 raw[G];
 #pragma unroll
-            for (int g = 0; g < G; ++g) if (r0 + g < nslots) raw[g] = ((const uint4 *)slotBase[r0 + g])[i];
+            for (int g = 0; g < G; ++g) if (r0 + g < nslots) raw[g] = ((const uint4 *)(slots + (r0 + g) * stride))[i];
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 if (r0 + g >= nslots) break;
@@ -422,11 +468,23 @@ __device__ __forceinline__ void ReduceSlots(T *out, T *out2, const char *const *
         if (out2) ((uint4 *)out2)[i] = res;
     }
     for (uint64_t i = nvec * VE + threadIdx.x; i < nElems; i += blockDim.x) {
-        A acc = ToAcc<T>(((const T *)slotBase[0])[i]);
-        for (int r = 1; r < nslots; ++r) acc = Combine<OP, A>(acc, ToAcc<T>(((const T *)slotBase[r])[i]));
+        const char *s = slots + i * sizeof(T);
+        A acc = ToAcc<T>(*(const T *)s);
+        for (int r = 1; r < nslots; ++r) acc = Combine<OP, A>(acc, ToAcc<T>(*(const T *)(s += stride)));
         T v = FromAcc<T>(acc);
         out[i] = v;
         if (out2) out2[i] = v;
+    }
+}
+
+// The same for a reduction that is known at run time: the copies around it are compiled once for all of them.
+template <typename T> __device__ __forceinline__ void ReduceSlotsBy(uint32_t op, T *out, T *out2, const char *slots, uint64_t stride, int nslots, uint64_t nElems)
+{
+    switch (op) {
+        case HCCL_REDUCE_SUM: ReduceSlots<T, HCCL_REDUCE_SUM>(out, out2, slots, stride, nslots, nElems); break;
+        case HCCL_REDUCE_PROD: ReduceSlots<T, HCCL_REDUCE_PROD>(out, out2, slots, stride, nslots, nElems); break;
+        case HCCL_REDUCE_MAX: ReduceSlots<T, HCCL_REDUCE_MAX>(out, out2, slots, stride, nslots, nElems); break;
+        default: ReduceSlots<T, HCCL_REDUCE_MIN>(out, out2, slots, stride, nslots, nElems); break;
     }
 }
 

@@ -78,6 +78,27 @@ def test_allreduce_dtypes_ops(emu_mod, dtype, op):
                     assert torch.equal(o.to(torch.int64), ref.to(dtype).to(torch.int64))
 
 
+@pytest.mark.parametrize("nranks", [2, 3, 5, 6, 8])
+@pytest.mark.parametrize("alg", ["SmAllReduceMesh1DOneShot", "SmAllReduceMesh1DTwoShot", "SmAllReduceConcurrent"])
+def test_allreduce_groups_of_copies(emu_mod, nranks, alg):
+    """A CTA's copies to and from all ranks run together, four vectors per thread: shares of fewer, exactly and more vectors than that, ends inside a
+    vector and inside a thread's turn, buffers that are not 16-byte aligned, in place. Bits of a sum in 32 bits in rank order."""
+    full = 512 * 8                                          # elements that one vector of each thread covers
+    with emu_mod.EmuWorld(nranks, 4 << 20) as w:
+        for count, off, inplace in ((3, 0, False), (full, 0, False), (full * nranks, 0, True), (4 * full * nranks + 8, 0, False), (5 * full + 13, 0, False),
+                                    (2 * full * nranks + 1, 1, False), (full + 9, 4, True)):
+            bufs = [_rand(count + off, torch.bfloat16, 31 * count + r)[off:] for r in range(nranks)]
+            ref = bufs[0].float()
+            for b in bufs[1:]:
+                ref = ref + b.float()
+            ref = ref.to(torch.bfloat16)
+            outs = bufs if inplace else [torch.zeros(count + 2 * off + 8, dtype=torch.bfloat16, device="cuda")[off:] for _ in range(nranks)]
+            assert w.run(CMD["ALLREDUCE"], alg, bufs, outs, count, torch.bfloat16, max_ctas=2) == 0
+            for o in outs:
+                assert torch.equal(o[:count], ref)
+                assert not o[count:].any()
+
+
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.uint16, torch.uint32])
 def test_allreduce_unsigned(emu_mod, dtype):
     nranks, count = 4, 2051
