@@ -183,7 +183,8 @@ struct RmsNormNode : OpNode {
             py::gil_scoped_acquire gil;
             if (direct) {
                 const auto dev = DeviceOf(g[0]);
-                direct = !Watched() && PlainGrad(g[0]) && Operand(xv, dev) && Operand(wv, dev) && Floats(r, dev) && xv.sizes() == g[0].sizes();
+                direct = !Watched() && PlainGrad(g[0]) && Operand(xv, dev) && Operand(wv, dev) && Floats(r, dev) && xv.sizes() == g[0].sizes() && wv.dim() == 1 &&
+                         wv.size(0) == xv.size(-1) && r.numel() * wv.size(0) == xv.numel();
             }
             if (!direct) out = FromPython((*g_env.backward)("rms_norm", held->o, xv, wv, g[0]), 2);
         }
@@ -255,7 +256,8 @@ struct RopeNode : OpNode {
             py::gil_scoped_acquire gil;
             if (direct) {
                 const auto dev = DeviceOf(dq);
-                direct = !Watched() && PlainGrad(dq) && PlainGrad(dk) && PlainGrad(dv) && Floats(c, dev) && Floats(s, dev);
+                direct = !Watched() && PlainGrad(dq) && PlainGrad(dk) && PlainGrad(dv) && Floats(c, dev) && Floats(s, dev) && c.sizes() == at::IntArrayRef({q[1], headDim / 2}) &&
+                         s.sizes() == c.sizes();
             }
             if (!direct) return FromPython((*g_env.backward)("rope_qkv", held->o, py::cast(in), dq, dk, dv), 1);
         }
@@ -314,7 +316,7 @@ struct SwiGluNode : OpNode {
         bool direct = !at::GradMode::is_enabled();
         {
             py::gil_scoped_acquire gil;
-            if (direct) direct = !Watched() && PlainGrad(dh) && Operand(in, DeviceOf(dh)) && in.numel() == 2 * dh.numel();
+            if (direct) direct = !Watched() && PlainGrad(dh) && Operand(in, DeviceOf(dh)) && in.dim() == 2 && dh.dim() == 2 && in.size(0) == dh.size(0) && in.size(1) == 2 * dh.size(1);
             if (!direct) return FromPython((*g_env.backward)("swiglu", held->o, in, dh), 1);
         }
         const at::Tensor d = Aligned(dh), out = at::empty_like(in);
@@ -363,8 +365,8 @@ struct LinearNode : OpNode {
             py::gil_scoped_acquire gil;
             if (direct) {
                 const auto dev = DeviceOf(dy);
-                direct = !Watched() && PlainGrad(dy) && dy.dim() == 2 && Operand(xv, dev) && Operand(wv, dev) && dy.numel() > 0 && dy.size(0) == xv.size(0) &&
-                         dy.size(1) == wv.size(0) && py::getattr(held->o, "fused", py::bool_(true)).cast<bool>();
+                direct = !Watched() && PlainGrad(dy) && dy.dim() == 2 && Operand(xv, dev) && Operand(wv, dev) && xv.dim() == 2 && wv.dim() == 2 && dy.numel() > 0 &&
+                         dy.size(0) == xv.size(0) && dy.size(1) == wv.size(0) && wv.size(1) == xv.size(1) && xv.size(1) % 8 == 0 && py::getattr(held->o, "fused", py::bool_(true)).cast<bool>();
             }
             if (!direct) return FromPython((*g_env.backward)(column ? "column" : "row", held->o, xv, wv, dy), 2);
         }
@@ -428,7 +430,7 @@ struct XentNode : OpNode {
             if (direct) {
                 const auto dev = c10::cuda::current_device();
                 direct = !Watched() && Plain(up) && up.is_cuda() && Operand(l, dev) && l.dim() == 2 && Plain(t) && t.scalar_type() == at::kLong && t.device() == l.device() &&
-                         t.is_contiguous() && t.dim() == 1 && t.size(0) == l.size(0) && Floats(m, dev) && Floats(p, dev);
+                         t.is_contiguous() && t.dim() == 1 && t.size(0) == l.size(0) && Floats(m, dev) && m.numel() == l.size(0) && Floats(p, dev) && p.numel() == 2 * l.size(0);
             }
             if (!direct) return FromPython((*g_env.backward)("xent", held->o, l, t, m, p, up), 1);
         }

@@ -162,7 +162,7 @@ class _RmsNorm(torch.autograd.Function):
         if dy is None:
             return dxk, dwk, None, None
         grads = _direct((x, w), (dy,))
-        if grads is None or x.shape != dy.shape or not _floats_ok(x.get_device(), rstd):
+        if grads is None or x.shape != dy.shape or w.shape != x.shape[-1:] or not _floats_ok(x.get_device(), rstd) or rstd.numel() * w.numel() != x.numel():
             dx, dw = _plain_backward(ctx.plain, (x, w), dy)
         else:
             dy, = grads
@@ -203,14 +203,14 @@ class _RopeQkv(torch.autograd.Function):
         check(_decl().HcclRopeQkv(qkv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), t, seq, heads, kv_heads, head_dim, 0,
                                   _stream(qkv)), "HcclRopeQkv")
         ctx.save_for_backward(cos, sin)                # the rotation is linear: its gradient does not depend on qkv
-        ctx.shape, ctx.dims, ctx.plain = qkv.shape, (heads, kv_heads, head_dim), plain
+        ctx.shape, ctx.dims, ctx.table, ctx.plain = qkv.shape, (heads, kv_heads, head_dim), cos.shape, plain
         return q, k, v
 
     @staticmethod
     def backward(ctx, dq, dk, dv):
         cos, sin = ctx.saved_tensors
         grads = _direct((), (dq, dk, dv))
-        if grads is None or not _floats_ok(grads[0].get_device(), cos, sin):
+        if grads is None or not _floats_ok(grads[0].get_device(), cos, sin) or not cos.shape == sin.shape == ctx.table:
             return (*_rope_backward(ctx.plain, ctx.shape, dq, dk, dv), None, None, None, None, None, None)
         dq, dk, dv = grads
         out = torch.empty(ctx.shape, dtype=dq.dtype, device=dq.device)
@@ -247,7 +247,7 @@ class _SwiGlu(torch.autograd.Function):
     def backward(ctx, dh):
         gu, = ctx.saved_tensors
         grads = _direct((gu,), (dh,))
-        if grads is None or gu.numel() != 2 * dh.numel():
+        if grads is None or gu.shape != (dh.shape[0], 2 * dh.shape[1]):
             return (*_plain_backward(ctx.plain, (gu,), dh), None)
         dh, = grads
         out = torch.empty_like(gu)
@@ -273,7 +273,8 @@ def xent_usable(logits: torch.Tensor, targets: torch.Tensor) -> bool:
 def xent_grad_usable(logits: torch.Tensor, targets: torch.Tensor, mx: torch.Tensor, packed: torch.Tensor, g: torch.Tensor) -> bool:
     """Whether the gradient kernel may answer this backward pass: a gradient that is itself differentiated, batched or dual has to see
     the operations, and so has a saved tensor that came back as something else."""
-    return not torch.is_grad_enabled() and _plain_tensor(g) and g.is_cuda and xent_usable(logits, targets) and _floats_ok(logits.get_device(), mx, packed)
+    return not torch.is_grad_enabled() and _plain_tensor(g) and g.is_cuda and xent_usable(logits, targets) and _floats_ok(logits.get_device(), mx, packed) \
+        and mx.shape == logits.shape[:1] and packed.shape == (2, logits.shape[0])
 
 
 def xent_row_max(logits: torch.Tensor) -> torch.Tensor:

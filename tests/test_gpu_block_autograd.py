@@ -196,6 +196,64 @@ def test_saved_tensors_that_come_back_changed(name):
             assert (a.double() - b.double()).norm() <= 2.0 ** -5 * b.double().norm()
 
 
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("name", ["rms_norm", "rope", "swiglu", "xent", "column", "row"])
+def test_saved_tensors_of_another_size(name, native, monkeypatch):
+    """A hook hands one saved tensor back wider, longer or shorter than it was: the backward pass gives the gradient of what it still knows, or an
+    error, and no kernel reads or writes by the sizes of the forward pass."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.models.llama import _cross_entropy
+    from hccl_b200.ops import block
+    from hccl_b200.parallel import tensor_parallel as tp
+    comm = None
+    assert block.nodes() is not None
+    if not native:
+        monkeypatch.setattr(block, "_NODES", None)
+    try:
+        if name == "xent":
+            logits, targets, _, _ = _logits()
+            f, ins = lambda t: _cross_entropy(t, targets, _OneRank, 0), [logits]
+        elif name in ("column", "row"):
+            torch.zeros(1, device="cuda")
+            comm = Communicator.from_root_info(1, get_root_info(), 0)
+            ins = [torch.randn(*s, device="cuda").to(torch.bfloat16).requires_grad_() for s in ((128, 64), (128, 64))]
+            cls = tp._ColumnSeqParallel if name == "column" else tp._RowSeqParallel
+
+            def f(x, w):
+                y = tp._one_rank_linear(x, w, comm, name == "column")
+                assert (y is not None) == native
+                return cls.apply(x, w, comm) if y is None else y
+        else:
+            f, _, ins = _op(name)
+        ups = [torch.ones_like(o) for o in _outs(f(*ins))]
+        ref = torch.autograd.grad(_outs(f(*ins)), ins, ups)
+        saved = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append(t.shape) or t, lambda t: t):
+            f(*ins)
+        changes = (lambda t: torch.cat([t, t], -1), lambda t: torch.cat([t, t]), lambda t: t[..., :-8].contiguous() if t.shape[-1] > 8 else t[..., :2].contiguous(),
+                   lambda t: t[:-1].clone())
+        for at in range(len(saved)):
+            for change in changes:
+                count = [0]
+
+                def pack(t):
+                    count[0] += 1
+                    return count[0] - 1, t
+
+                with torch.autograd.graph.saved_tensors_hooks(pack, lambda p: change(p[1]) if p[0] == at else p[1]):
+                    out = _outs(f(*ins))
+                try:
+                    got = torch.autograd.grad(out, ins, ups)
+                except (RuntimeError, IndexError, ValueError, AssertionError):
+                    continue
+                for a, b in zip(got, ref):
+                    assert a.shape == b.shape and (a.double() - b.double()).norm() <= 2.0 ** -5 * b.double().norm()
+        torch.cuda.synchronize()
+    finally:
+        if comm is not None:
+            comm.destroy()
+
+
 def _tiny(seed=3):
     from hccl_b200.comm import Communicator, get_root_info
     from hccl_b200.models.llama import Llama, LlamaConfig
