@@ -196,8 +196,9 @@ __global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16
     }
 }
 
-// out[c] = sum over parts of partial[part][c]: 32 columns per block, four per load, 32 threads per column group, added up in a fixed order.
-__global__ void __launch_bounds__(kThreads) SumPartsKernel(const float *__restrict__ partial, __nv_bfloat16 *__restrict__ out, uint32_t parts, uint32_t H)
+// out[c] = sum over parts of partial[part][c]: 32 columns per block, four per load (VEC: 16-byte aligned) or turn, 32 threads per column group, added up in a
+// fixed order.
+template <bool VEC> __global__ void __launch_bounds__(kThreads) SumPartsKernel(const float *__restrict__ partial, __nv_bfloat16 *__restrict__ out, uint32_t parts, uint32_t H)
 {
     __shared__ float4 sm[32][8];
     const uint32_t g = threadIdx.x & 7, q = threadIdx.x >> 3, c = blockIdx.x * 32 + g * 4;
@@ -205,7 +206,8 @@ __global__ void __launch_bounds__(kThreads) SumPartsKernel(const float *__restri
     if (c < H) {                                         // H is a multiple of 8: whole groups
 #pragma unroll 4
         for (uint32_t p = q; p < parts; p += 32) {
-            const float4 v = *(const float4 *)(partial + (size_t)p * H + c);
+            const float *at = partial + (size_t)p * H + c;
+            const float4 v = VEC ? *(const float4 *)at : make_float4(at[0], at[1], at[2], at[3]);
             s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
         }
     }
@@ -469,13 +471,15 @@ HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const fl
 {
     if (!dy || !x || !w || !rstd || !dx || !dw || !partial) return HCCL_E_PTR;
     if (!NormShapeOk(rows, hidden) || !Aligned16(dy) || !Aligned16(x) || !Aligned16(w) || !Aligned16(dx)) return HCCL_E_PARA;
+    const bool vec = Aligned16(partial);                 // rows up to kWarpRowMax are also taken with a workspace that is aligned to its elements alone
+    if (((uintptr_t)partial & 3u) || (!vec && hidden > kWarpRowMax)) return HCCL_E_PARA;
     const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden, parts = (uint32_t)HcclRmsNormBwdParts(rows, hidden);
     auto launch = [&](auto kern) { kern(dy, x, w, rstd, dx, partial, T, H, parts, stream); };
     const uint32_t nv = NormVecs(H);
     if (hidden <= kWarpRowMax) launch(nv == 1 ? LaunchRmsNormBwd<32, 1> : nv == 2 ? LaunchRmsNormBwd<32, 2> : LaunchRmsNormBwd<32, 4>);
     else launch(nv == 1 ? LaunchRmsNormBwd<kThreads, 1> : nv == 2 ? LaunchRmsNormBwd<kThreads, 2> : nv <= 4 ? LaunchRmsNormBwd<kThreads, 4> : LaunchRmsNormBwd<kThreads, 6>);
     CHK_RET(Launched("RMSNorm backward"));
-    SumPartsKernel<<<(H + 31) / 32, kThreads, 0, stream>>>(partial, (__nv_bfloat16 *)dw, parts, H);
+    (vec ? SumPartsKernel<true> : SumPartsKernel<false>)<<<(H + 31) / 32, kThreads, 0, stream>>>(partial, (__nv_bfloat16 *)dw, parts, H);
     return Launched("RMSNorm weight gradient");
 }
 

@@ -16,7 +16,7 @@ extern "C" {
 HcclResult HcclRmsNorm(const void *x, const void *w, void *y, float *rstd, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
 /* The same, and copies of x and w: what the backward pass reads where x or w may be changed in between. */
 HcclResult HcclRmsNormKeep(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
-/* Rows of the fp32 workspace `partial` [parts, hidden] that HcclRmsNormBwd needs. */
+/* Rows of the fp32 workspace `partial` [parts, hidden] that HcclRmsNormBwd needs. Up to 1024 columns it may also be aligned to 4 bytes alone. */
 uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden);
 HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, void *dw, float *partial, uint64_t rows, uint64_t hidden,
                           cudaStream_t stream);

@@ -254,6 +254,25 @@ def test_saved_tensors_of_another_size(name, native, monkeypatch):
             comm.destroy()
 
 
+@pytest.mark.parametrize("rows,hidden", [(5, 8), (700, 256), (70, 1000)])
+def test_norm_workspace_aligned_to_its_elements(rows, hidden):
+    """Up to 1024 columns the backward pass takes a workspace at any multiple of four bytes: the same bits as on whole vectors."""
+    from hccl_b200.ops import block
+    l = block._decl()
+    x, dy, w = [torch.randn(*s, device="cuda").to(torch.bfloat16) for s in ((rows, hidden), (rows, hidden), (hidden,))]
+    rstd = torch.rsqrt(x.float().square().mean(1) + 1e-5)
+    parts = l.HcclRmsNormBwdParts(rows, hidden)
+
+    def run(offset):
+        dx, dw, partial = torch.empty_like(x), torch.empty_like(w), torch.empty(parts * hidden + 4, device="cuda")
+        assert l.HcclRmsNormBwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), dx.data_ptr(), dw.data_ptr(), partial.data_ptr() + offset, rows, hidden,
+                                torch.cuda.current_stream().cuda_stream) == 0
+        return dx, dw
+
+    for offset in (4, 8, 12):
+        assert all(torch.equal(a, b) for a, b in zip(run(0), run(offset)))
+
+
 def _tiny(seed=3):
     from hccl_b200.comm import Communicator, get_root_info
     from hccl_b200.models.llama import Llama, LlamaConfig

@@ -126,3 +126,12 @@ def test_one_rank_moe_kernels_do_not_use_the_registered_communicator():
     for line in solo.splitlines():
         if "HCCL_RANGE_OK" in line or "HCCL_CHECK_RANGE" in line or "BlockCopy(" in line:
             assert "SOLO ?" in line, line
+
+
+def test_norm_backward_refuses_a_workspace_that_its_loads_cannot_take():
+    """Pointers are checked before anything is launched: 2 bytes off everywhere, 4 bytes off where rows are wider than 1024 columns."""
+    from hccl_b200.ops import block
+    from hccl_b200.types import Result
+    at = 1 << 20
+    for hidden, partial in ((256, at + 2), (1032, at + 4), (4096, at + 8)):
+        assert block._decl().HcclRmsNormBwd(at, at, at, at, at, at, partial, 8, hidden, None) == Result.E_PARA, (hidden, partial)
