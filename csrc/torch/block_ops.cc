@@ -105,19 +105,26 @@ variable_list FromPython(const py::object &r, size_t n)
 struct OpNode : Node {
     std::unique_ptr<PyRef> held;               // what the Python form's backward pass needs beside tensors
     struct Saved { SavedVariable *v; bool output; };
+    bool traced = false;                       // compiled autograd runs this backward pass, on stand-ins
     virtual variable_list Backward(variable_list &&g) = 0;
     virtual std::vector<Saved> Keeps() = 0;
-    // Compiled autograd traces the backward pass: it runs on stand-ins, which the Python form takes. Its graph holds what `held` refers to
-    // as constants, so no graph is taken for another node.
+    // What the traced single operations depend on beside the node's tensors and its type.
+    virtual void Constants(torch::dynamo::autograd::CompiledNodeArgs &) const {}
+    // Compiled autograd takes one traced graph for all nodes that collect the same, so nothing traced may come from `held`. It cannot run a
+    // backward pass inside another: the traced forms are written out.
     void compiled_args(torch::dynamo::autograd::CompiledNodeArgs &args) const override
     {
-        static std::atomic<int64_t> count{0};
         for (const Saved &k : const_cast<OpNode *>(this)->Keeps()) args.collect(*k.v, k.output);
-        args.collect(count++);
+        Constants(args);
     }
     variable_list apply_with_saved(const variable_list &inputs, torch::dynamo::autograd::SwapSavedVariables &saved) override
     {
         for (const Saved &k : Keeps()) saved.before(*k.v);
+        struct Tracing {
+            bool &on;
+            explicit Tracing(bool &t) : on(t) { on = true; }
+            ~Tracing() { on = false; }
+        } tracing(traced);
         variable_list r = apply(variable_list(inputs));
         for (const Saved &k : Keeps()) saved.after(*k.v);
         return r;
@@ -178,7 +185,7 @@ struct RmsNormNode : OpNode {
         if (!g[0].defined()) return {g[1], g[2]};
         const auto [xv, wv, r] = Unpack(x, w, rstd);
         variable_list out(2);
-        bool direct = !at::GradMode::is_enabled();
+        bool direct = !traced && !at::GradMode::is_enabled();
         {
             py::gil_scoped_acquire gil;
             if (direct) {
@@ -186,7 +193,8 @@ struct RmsNormNode : OpNode {
                 direct = !Watched() && PlainGrad(g[0]) && Operand(xv, dev) && Operand(wv, dev) && Floats(r, dev) && xv.sizes() == g[0].sizes() && wv.dim() == 1 &&
                          wv.size(0) == xv.size(-1) && r.numel() * wv.size(0) == xv.numel();
             }
-            if (!direct) out = FromPython((*g_env.backward)("rms_norm", held->o, xv, wv, g[0]), 2);
+            if (traced) out = FromPython((*g_env.backward)("rms_norm traced", xv, wv, r, g[0]), 2);
+            else if (!direct) out = FromPython((*g_env.backward)("rms_norm", held->o, xv, wv, g[0]), 2);
         }
         if (direct) {
             const at::Tensor dy = Aligned(g[0]);
@@ -246,12 +254,16 @@ struct RopeNode : OpNode {
     uint32_t heads = 0, kvHeads = 0, headDim = 0;
     at::TensorOptions options;
     std::string name() const override { return "_RopeQkvBackward"; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override
+    {
+        for (const std::vector<int64_t> *v : {&in, &q, &kv}) args.collect(*v);
+    }
     std::vector<Saved> Keeps() override { return {{&cos, false}, {&sin, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         const auto [c, s] = Unpack(cos, sin);
         const at::Tensor dq = ZerosWhereUndefined(g[0], q, options), dk = ZerosWhereUndefined(g[1], kv, options), dv = ZerosWhereUndefined(g[2], kv, options);
-        bool direct = !at::GradMode::is_enabled();
+        bool direct = !traced && !at::GradMode::is_enabled();
         {
             py::gil_scoped_acquire gil;
             if (direct) {
@@ -259,6 +271,7 @@ struct RopeNode : OpNode {
                 direct = !Watched() && PlainGrad(dq) && PlainGrad(dk) && PlainGrad(dv) && Floats(c, dev) && Floats(s, dev) && c.sizes() == at::IntArrayRef({q[1], headDim / 2}) &&
                          s.sizes() == c.sizes();
             }
+            if (traced) return FromPython((*g_env.backward)("rope_qkv traced", c, s, py::cast(in), dq, dk, dv), 1);
             if (!direct) return FromPython((*g_env.backward)("rope_qkv", held->o, py::cast(in), dq, dk, dv), 1);
         }
         const at::Tensor a = Aligned(dq), b = Aligned(dk), v = Aligned(dv), out = at::empty(in, a.options());
@@ -313,9 +326,10 @@ struct SwiGluNode : OpNode {
     {
         const auto [in] = Unpack(gu);
         const at::Tensor dh = g[0].defined() ? g[0] : at::zeros({in.size(0), in.size(1) / 2}, in.options());
-        bool direct = !at::GradMode::is_enabled();
+        bool direct = !traced && !at::GradMode::is_enabled();
         {
             py::gil_scoped_acquire gil;
+            if (traced) return FromPython((*g_env.backward)("swiglu traced", in, dh), 1);
             if (direct) direct = !Watched() && PlainGrad(dh) && Operand(in, DeviceOf(dh)) && in.dim() == 2 && dh.dim() == 2 && in.size(0) == dh.size(0) && in.size(1) == 2 * dh.size(1);
             if (!direct) return FromPython((*g_env.backward)("swiglu", held->o, in, dh), 1);
         }
@@ -355,12 +369,13 @@ struct LinearNode : OpNode {
     at::TensorOptions options;
     bool column = false;
     std::string name() const override { return column ? "_ColumnSeqParallelBackward" : "_RowSeqParallelBackward"; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(shape); }
     std::vector<Saved> Keeps() override { return {{&x, false}, {&w, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         const auto [xv, wv] = Unpack(x, w);
         at::Tensor dy = ZerosWhereUndefined(g[0], shape, options);
-        bool direct = !at::GradMode::is_enabled() && g_nativeGemm && !g_nativeWgrad;
+        bool direct = !traced && !at::GradMode::is_enabled() && g_nativeGemm && !g_nativeWgrad;
         {
             py::gil_scoped_acquire gil;
             if (direct) {
@@ -368,6 +383,7 @@ struct LinearNode : OpNode {
                 direct = !Watched() && PlainGrad(dy) && dy.dim() == 2 && Operand(xv, dev) && Operand(wv, dev) && xv.dim() == 2 && wv.dim() == 2 && dy.numel() > 0 &&
                          dy.size(0) == xv.size(0) && dy.size(1) == wv.size(0) && wv.size(1) == xv.size(1) && xv.size(1) % 8 == 0 && py::getattr(held->o, "fused", py::bool_(true)).cast<bool>();
             }
+            if (traced) return FromPython((*g_env.backward)("linear traced", xv, wv, dy), 2);
             if (!direct) return FromPython((*g_env.backward)(column ? "column" : "row", held->o, xv, wv, dy), 2);
         }
         dy = Aligned(dy);
@@ -419,12 +435,13 @@ struct XentNode : OpNode {
     int64_t vocabStart = 0;
     at::TensorOptions options;
     std::string name() const override { return "_VocabParallelCrossEntropyBackward"; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(vocabStart); }
     std::vector<Saved> Keeps() override { return {{&logits, false}, {&targets, false}, {&mx, false}, {&packed, false}}; }
     variable_list Backward(variable_list &&g) override
     {
         const auto [l, t, m, p] = Unpack(logits, targets, mx, packed);
         const at::Tensor up = ZerosWhereUndefined(g[0], {}, options);
-        bool direct = !at::GradMode::is_enabled();
+        bool direct = !traced && !at::GradMode::is_enabled();
         {
             py::gil_scoped_acquire gil;
             if (direct) {
@@ -432,6 +449,7 @@ struct XentNode : OpNode {
                 direct = !Watched() && Plain(up) && up.is_cuda() && Operand(l, dev) && l.dim() == 2 && Plain(t) && t.scalar_type() == at::kLong && t.device() == l.device() &&
                          t.is_contiguous() && t.dim() == 1 && t.size(0) == l.size(0) && Floats(m, dev) && m.numel() == l.size(0) && Floats(p, dev) && p.numel() == 2 * l.size(0);
             }
+            if (traced) return FromPython((*g_env.backward)("xent traced", held->o, l, t, m, p, up), 1);
             if (!direct) return FromPython((*g_env.backward)("xent", held->o, l, t, m, p, up), 1);
         }
         const at::Tensor out = at::empty_like(l), scale = up.to(at::kFloat);

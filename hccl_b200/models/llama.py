@@ -215,7 +215,15 @@ def _xent_backward(vocab_start, logits, targets, mx, packed, g):
     return (_xent_gradient(p, mine, idx, g),)
 
 
+def _xent_traced(vocab_start, logits, targets, mx, packed, g):
+    """Under compiled autograd, where no shape may depend on the targets."""
+    hot = torch.arange(logits.shape[-1], device=logits.device) == (targets - vocab_start)[:, None]
+    p = (logits.float() - mx[:, None]).exp() / packed[0][:, None]
+    return ((torch.where(hot, p - 1.0, p) * (g / p.shape[0])).to(logits.dtype),)
+
+
 _block.PYTHON_BACKWARD["xent"] = _xent_backward
+_block.PYTHON_BACKWARD["xent traced"] = _xent_traced
 
 
 def _cross_entropy(logits_local, targets, comm, vocab_start):

@@ -140,6 +140,36 @@ def _rope_backward(plain, shape, dq, dk, dv):
 PYTHON_BACKWARD["rope_qkv"] = _rope_backward
 
 
+# The same under compiled autograd, which traces a backward pass on stand-ins: written out, from the saved tensors alone.
+def _rms_norm_traced(x, w, rstd, dy):
+    r = rstd.reshape(*x.shape[:-1], 1)
+    xhat, d = x.float() * r, dy.float()
+    g = d * w.float()
+    dx = r * (g - xhat * (g * xhat).mean(-1, keepdim=True))
+    return dx.to(x.dtype), (d * xhat).flatten(0, -2).sum(0).to(w.dtype) if x.dim() > 1 else (d * xhat).to(w.dtype)
+
+
+def _rope_traced(cos, sin, shape, dq, dk, dv):
+    def turned_back(d):
+        a, b = d.float().chunk(2, -1)
+        c, s = cos[:, None], sin[:, None]
+        return torch.cat([a * c + b * s, b * c - a * s], -1).to(d.dtype)
+
+    return (torch.cat([t.flatten(2) for t in (turned_back(dq), turned_back(dk), dv)], -1).reshape(shape),)
+
+
+def _swiglu_traced(gu, dh):
+    g, u = gu.float().chunk(2, -1)
+    d, s = dh.float(), torch.sigmoid(g)
+    return (torch.cat([d * u * s * (1 + g * (1 - s)), d * (g * s)], -1).to(gu.dtype),)
+
+
+PYTHON_BACKWARD["rms_norm traced"] = _rms_norm_traced
+PYTHON_BACKWARD["rope_qkv traced"] = _rope_traced
+PYTHON_BACKWARD["swiglu traced"] = _swiglu_traced
+PYTHON_BACKWARD["linear traced"] = lambda x, w, dy: (dy @ w, dy.t() @ x)
+
+
 class _RmsNorm(torch.autograd.Function):
     """-> (y, x, w). The backward pass reads copies of x and w that the kernel makes on its way, since the caller may change both before it
     (x += f(norm(x)), an optimizer step). The copies are outputs, so that the gradient of a gradient finds its way to x and w."""

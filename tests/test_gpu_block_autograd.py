@@ -273,6 +273,64 @@ def test_norm_workspace_aligned_to_its_elements(rows, hidden):
         assert all(torch.equal(a, b) for a, b in zip(run(0), run(offset)))
 
 
+@pytest.mark.parametrize("name", ["rms_norm", "rope", "swiglu", "xent", "column", "row"])
+def test_compiled_autograd_traces_a_node_once(name):
+    """The same step several times under compiled autograd, on new values: the gradients of the single operations and one trace in all. Another first class
+    of a vocabulary shard is another trace; the norm's epsilon and the rotary tables are inputs of it."""
+    from torch._dynamo import compiled_autograd
+    from torch._dynamo.utils import counters
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.models.llama import RMSNorm, _rope_tables, _rotated
+    from hccl_b200.ops import block
+    from hccl_b200.parallel import tensor_parallel as tp
+    nodes = block.nodes()
+    assert nodes is not None
+    torch.zeros(1, device="cuda")
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    draw = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16).requires_grad_()
+    try:
+        def case(step):
+            """fused outputs, inputs, plain outputs (or gradients) of one step; step 3 has another constant"""
+            if name == "rms_norm":
+                norm, ins = RMSNorm(64, 1e-5 if step < 3 else 0.5, torch.bfloat16, "cuda"), [draw(5, 64), draw(64)]
+                return block.rms_norm(*ins, norm.eps, norm._plain), ins, norm._plain
+            if name == "rope":
+                cos, sin = _rope_tables(3, 16, 10000.0 + 5000 * step, "cuda")
+                plain = lambda t: _rotated(t, 2, 3, 4, 2, 16, cos, sin)
+                ins = [draw(6, 128)]
+                return block.rope_qkv(*ins, cos, sin, 2, 4, 2, 16, plain), ins, plain
+            if name == "swiglu":
+                plain, ins = lambda t: torch.nn.functional.silu(t[:, :32]) * t[:, 32:], [draw(5, 64)]
+                return block.swiglu(*ins, plain), ins, plain
+            if name == "xent":
+                ins, targets, start = [draw(6, 24)], torch.randint(0, 24, (6,), device="cuda"), 0 if step < 3 else 4
+
+                def plain(t):
+                    lse, mine, idx = t.float().logsumexp(-1), (targets >= start) & (targets < start + 24), (targets - start).clamp(0, 23)
+                    return (lse - torch.where(mine, t.float().gather(1, idx[:, None])[:, 0], torch.zeros_like(lse))).mean()
+
+                return nodes.xent(*ins, targets, start), ins, plain
+            ins = [draw(128, 64), draw(192, 64)]
+            return tp._one_rank_linear(*ins, comm, name == "column"), ins, lambda x, w: x @ w.t()
+
+        def run(step):
+            out, ins, plain = case(step)
+            ups = [torch.randn_like(o) for o in _outs(out)]
+            before = counters["compiled_autograd"]["captures"]
+            with compiled_autograd._enable(torch.compile(backend="eager")):
+                torch.autograd.backward(_outs(out), ups)
+            ref = torch.autograd.grad(_outs(plain(*ins)), ins, ups)
+            for t, r in zip(ins, ref):
+                assert (t.grad.double() - r.double()).norm() <= 2.0 ** -7 * r.double().norm()
+            return counters["compiled_autograd"]["captures"] - before
+
+        counts = [run(step) for step in range(4)]
+        assert counts[0] == 1 and counts[1] == 0 and counts[2] == 0, counts
+        assert counts[3] == (1 if name == "xent" else 0), counts
+    finally:
+        comm.destroy()
+
+
 def _tiny(seed=3):
     from hccl_b200.comm import Communicator, get_root_info
     from hccl_b200.models.llama import Llama, LlamaConfig
