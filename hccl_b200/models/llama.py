@@ -203,8 +203,8 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
 
 
 def _xent_gradient(p, mine, idx, g):
-    hot = (torch.arange(p.shape[1], device=p.device) == idx[:, None]) & mine[:, None]
-    grad = torch.where(hot, p - 1.0, p)
+    grad = p.clone()
+    grad[torch.arange(p.shape[0], device=p.device)[mine], idx[mine]] -= 1.0
     return (grad * (g / p.shape[0])).to(torch.bfloat16 if p.is_cuda else torch.float32)
 
 

@@ -98,3 +98,31 @@ def test_rms_norm_can_be_scripted():
     norm = RMSNorm(64, 1e-5, torch.bfloat16, "cpu")
     x = torch.randn(3, 64, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
     assert torch.equal(torch.jit.script(norm)(x), norm(x))
+
+
+def test_plain_cross_entropy_gradient_passes_over_the_probabilities_once():
+    """The gradient by single operations: one copy of the probabilities, corrected at the targets, scaled; no matrix of targets beside it."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from hccl_b200.models.llama import _xent_gradient
+    p = torch.softmax(torch.randn(6, 40), 1)
+    targets = torch.tensor([0, 39, 7, 100, -3, 12])
+    mine = (targets >= 0) & (targets < 40)
+
+    class Matrices(TorchDispatchMode):
+        made = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            out = func(*args, **(kwargs or {}))
+            if isinstance(out, torch.Tensor) and out.numel() == p.numel() and not any(out is a for a in args):
+                self.made += 1
+            return out
+
+    with Matrices() as m:
+        got = _xent_gradient(p, mine, targets.clamp(0, 39), torch.tensor(3.0))
+    want = p.clone()
+    for r in range(6):
+        if mine[r]:
+            want[r, targets[r]] -= 1.0
+    assert torch.equal(got, want * (3.0 / 6))
+    assert m.made <= 3, m.made
