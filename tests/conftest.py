@@ -33,12 +33,13 @@ def pytest_collection_modifyitems(config, items):
 
 @pytest.fixture(scope="session", autouse=True)
 def _native_lib():
-    """Build the native library once per session if it is missing (nvcc cross-compiles without a GPU)."""
-    from hccl_b200 import _lib
+    """Build the native library and the torch extension once per session if one is missing (nvcc cross-compiles without a GPU)."""
+    from hccl_b200 import _ext, _lib
+    from hccl_b200.utils import build
 
     if not _lib.LIB_PATH.exists():
-        from hccl_b200.utils import build
-
         build.build_native()
+    if not os.environ.get("HCCL_B200_LIB") and not _ext.EXT_PATH.exists():
+        build.build_torch_ext()
     os.environ.setdefault("HCCL_DEVICE_WAIT_TIMEOUT_MS", "20000")
     return _lib.lib()

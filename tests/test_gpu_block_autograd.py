@@ -1,8 +1,23 @@
 """The one-kernel parts of a decoder block under autograd: what the plain operations took has to be taken, with the same meaning."""
+import os
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+
+def _native_nodes():
+    """The extension with the native autograd nodes; without it a test of them would compare the Python functions with themselves."""
+    from hccl_b200.ops import block
+    if os.environ.get("HCCL_B200_LIB"):
+        pytest.skip("another flavor of the library runs the Python functions")
+    assert block.nodes() is not None
+    return block.nodes()
+
+
+def _is_native(t):
+    return t.grad_fn is not None and not isinstance(t.grad_fn, torch.autograd.function.BackwardCFunction)
 
 
 class _OneRank:
@@ -206,7 +221,7 @@ def test_saved_tensors_of_another_size(name, native, monkeypatch):
     from hccl_b200.ops import block
     from hccl_b200.parallel import tensor_parallel as tp
     comm = None
-    assert block.nodes() is not None
+    _native_nodes()
     if not native:
         monkeypatch.setattr(block, "_NODES", None)
     try:
@@ -283,8 +298,7 @@ def test_compiled_autograd_traces_a_node_once(name):
     from hccl_b200.models.llama import RMSNorm, _rope_tables, _rotated
     from hccl_b200.ops import block
     from hccl_b200.parallel import tensor_parallel as tp
-    nodes = block.nodes()
-    assert nodes is not None
+    nodes = _native_nodes()
     torch.zeros(1, device="cuda")
     comm = Communicator.from_root_info(1, get_root_info(), 0)
     draw = lambda *s: torch.randn(*s, device="cuda").to(torch.bfloat16).requires_grad_()
@@ -346,6 +360,7 @@ def test_native_nodes_give_the_bits_of_the_python_functions(tokens, monkeypatch)
     from torch.utils.checkpoint import checkpoint
     from hccl_b200.models.llama import _rope_tables
     from hccl_b200.ops import block
+    _native_nodes()
     comm, model = _tiny()
     try:
         t = torch.randint(0, 512, (tokens[0], tokens[1] + 1), device="cuda")
@@ -353,6 +368,7 @@ def test_native_nodes_give_the_bits_of_the_python_functions(tokens, monkeypatch)
 
         def step():
             loss = model(t[:, :-1].contiguous(), t[:, 1:].contiguous())
+            assert _is_native(loss) == (block.nodes() is not None)
             first = torch.autograd.grad(loss, params, retain_graph=True)
             return [loss.detach(), *first, *torch.autograd.grad(loss, params)]
 
@@ -382,6 +398,7 @@ def test_native_nodes_keep_the_engine_s_rules():
     import weakref
     from hccl_b200.models.llama import RMSNorm, _rope_tables
     from hccl_b200.ops import block
+    _native_nodes()
     comm, model = _tiny()
     try:
         x = torch.randn(256, 256, device="cuda").to(torch.bfloat16).requires_grad_()
@@ -401,6 +418,7 @@ def test_native_nodes_keep_the_engine_s_rules():
 
         w = torch.ones(256, device="cuda", dtype=torch.bfloat16).requires_grad_()
         y = block.rms_norm(x, w, 1e-5, failing)
+        assert _is_native(y)
         with pytest.raises(LookupError, match="plain form"):
             torch.autograd.grad(y.sum(), x, create_graph=True)
         norm = RMSNorm(256, 1e-5, torch.bfloat16, "cuda")
