@@ -36,9 +36,8 @@ inline SplitKChoice ChooseSplitK(uint64_t m, uint64_t n, uint64_t k, bool mx)
     const uint64_t tiles = nt * ((m + bt - 1) / bt), ctas = k > 6144 || m > 64 ? 256 : 148;
     const SplitKChoice narrow{bt, parts(ctas / tiles)};
     if (m <= 64 || mx || narrow.split >= 6 || (k < 5000 && narrow.split >= 3)) return narrow;
-    if (m <= 128) return k >= 4096 && 256 / nt >= 2 ? SplitKChoice{128, parts(256 / nt)} : SplitKChoice{};     // 72 x 7192 x 2576: 11.6, tiles 10.6
+    if (m <= 128) return k >= 4096 ? SplitKChoice{128, parts(256 / nt)} : SplitKChoice{};     // 72 x 7192 x 2576: 11.6, tiles 10.6
     const uint64_t t256 = nt * ((m + 255) / 256), s = 148 / t256;
-    if (t256 > 60) return {};
     return {256, parts(s > 4 ? std::max<uint64_t>(4, 120 / t256) : std::max<uint64_t>(3, s))};
 }
 
