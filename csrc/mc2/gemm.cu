@@ -8,6 +8,7 @@
 #include "gemm_sm100_2cta.cuh"
 #include "gemm_splitk_launch.cuh"
 #include "gemm_wide_launch.cuh"
+#include "tile_choice.h"
 #include <cstdlib>
 #include "hccl/hccl_mc2.h"
 
@@ -233,50 +234,6 @@ static HcclResult LaunchPair(uint32_t bn, const void *a, const void *b, void *c,
     return LaunchPlain2CtaT<256>(a, b, c, M, N, K, outFp32, s);
 }
 
-// Which tile kernel: waves of tiles times what a wave of that kernel takes, plus 40 for the launch of clusters. A part of the cost counts whole
-// waves and the rest the fraction of the GPU that the tiles fill, since idle SMs leave power to the others. A wave per 4096 of K takes the tile's
-// columns (pairs) or 0.9 of them (one CTA) plus what its loads of A and B hold it up, which is more where K is no multiple of 64: its rows then
-// straddle 128-byte lines. The constants are fitted to 130 random products on one B200 (64 to 8192 rows, N 512 to 28672, K 512 to 16384; every
-// width timed in random order, each after 30 to 50 ms of its own): the choice is 0.3 to 0.5 % slower than the best width on average. The widths above
-// 256 and these costs against 192 / 224 / 256 chosen by waves alone: 1473 x 17784 x 9608 496 / 420 us (512 columns), 3882 x 18048 x 6664 957 / 814 (512),
-// 2115 x 2304 x 2344 31.6 / 24.2 (288), 7073 x 6152 x 5992 598 / 425 (480), 2048 x 4096 x 14336 195 / 181 (480), 1000 x 6144 x 4096 43.0 / 42.1 (352),
-// 8192 x 8192 x 28672 3133 / 2867 (512). Wide tiles where K is made of 64s pay for their exposed start only in few waves or with a long K: 8100 x 28032 x 2624 takes
-// 947 with 512 columns and 856 with 256.
-struct TileChoice { bool pair; uint32_t bn; };
-static TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposedB)
-{
-    const uint64_t sms = (uint64_t)SmCount(), pairs = sms / 2, rows = (m + kBM - 1) / kBM, rowPairs = (rows + 1) / 2;
-    const double k4 = (double)k / 4096;
-    const bool straddle = k % 64 != 0;
-    auto filled = [](uint64_t tiles, uint64_t slots) { return std::max(1.0, (double)tiles / (double)slots); };
-    auto waves = [](uint64_t tiles, uint64_t slots) { return (double)((tiles + slots - 1) / slots); };
-    auto one = [&](uint32_t bn) {
-        const uint64_t tiles = rows * ((n + bn - 1) / bn);
-        return (0.8 * waves(tiles, sms) + 0.2 * filled(tiles, sms)) * (20 + k4 * (0.9 * bn + (straddle ? 170 : 95)));
-    };
-    auto pair = [&](uint32_t bn) {
-        const uint64_t tiles = rowPairs * ((n + bn - 1) / bn);
-        const double whole = straddle ? 0.5 : 0.7, start = bn <= 256 ? 0 : straddle ? 20 : 45;
-        return 40 + (whole * waves(tiles, pairs) + (1 - whole) * filled(tiles, pairs)) * (start + k4 * (bn + (straddle ? 200 : 45)));
-    };
-    TileChoice best{false, 64};
-    double cost = one(64);
-    auto offer = [&](bool isPair, uint32_t bn, double c) { if (c <= cost) { best = {isPair, bn}; cost = c; } };
-    offer(false, 128, one(128));
-    // 256-wide one-CTA tiles where N is made of them (another N was not measured)
-    if (!transposedB && n % 256 == 0) offer(false, 256, one(256));
-    if (!Gemm2CtaEnabled()) return best;
-    offer(true, 256, pair(256));
-    if (transposedB) {           // its tiles are whole 64-column boxes per CTA; 2048 x 4096 x 28672 387 / 379 us (256 / 512), 4096 x 4096 x 14336 394 / 373
-        if (k >= 8192) offer(true, 512, pair(512));  // not with a short K: 2986 x 16472 x 3712 303 / 330, 2048 x 14336 x 4096 186 / 204
-        return best;
-    }
-    offer(true, 224, pair(224));
-    offer(true, 192, pair(192));
-    for (uint32_t bn = 288; bn <= 512; bn += 32) offer(true, bn, pair(bn));
-    return best;
-}
-
 }  // namespace mc2
 }  // namespace hccl
 
@@ -295,7 +252,7 @@ HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint6
     }
     const SplitKChoice sk = ChooseSplitK(m, n, k, false);
     if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
-    const TileChoice t = ChooseTile(m, n, k, false);
+    const TileChoice t = ChooseTile(m, n, k, false, SmCount(), Gemm2CtaEnabled());
     if (t.pair) return LaunchPair(t.bn, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.bn == 256) return LaunchPlain<256>(a, b, c, m, n, k, outFp32 != 0, stream);
     if (t.bn == 128) return LaunchPlain<128>(a, b, c, m, n, k, outFp32 != 0, stream);
@@ -327,7 +284,7 @@ HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uin
         HCCL_ERROR("HcclGemmBf16Nn: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    const TileChoice t = ChooseTile(m, n, k, true);
+    const TileChoice t = ChooseTile(m, n, k, true, SmCount(), Gemm2CtaEnabled());
     if (t.pair && t.bn == 512) return LaunchWide<true>(512, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, GroupMOverride(8), stream);
     if (t.pair) return LaunchPlain2CtaT<256, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.bn == 128) return LaunchPlain<128, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);

@@ -1,0 +1,36 @@
+"""The choice of a tile kernel for plain bf16 products, compiled as host code, against measured times."""
+import subprocess
+from pathlib import Path
+
+ROOT = Path(__file__).resolve().parents[1]
+WIDTHS = (192, 224, 256, 288, 320, 352, 384, 416, 448, 480, 512)
+# (m, n, k) and the time of every pair width in us, medians of five runs on one B200. K is made of 64s, of 16s or of neither
+MEASURED = [
+    ((3448, 12576, 6360), (611.6, 586.7, 578.1, 534.1, 540.1, 507.8, 501.8, 485.3, 495.4, 499.5, 450.3)),
+    ((1358, 12120, 4480), (133.7, 133.8, 113.9, 134.1, 160.7, 124.5, 145.2, 149.4, 161.1, 168.7, 129.5)),
+    ((1012, 8200, 4104), (82.6, 67.5, 71.0, 73.0, 83.7, 85.6, 94.4, 89.2, 92.7, 58.6, 59.2)),
+    ((8119, 560, 4720), (50.4, 54.3, 58.3, 40.3, 44.0, 47.3, 49.3, 54.5, 56.8, 57.7, 60.3)),
+    ((957, 24464, 2480), (98.3, 95.6, 106.6, 113.1, 121.6, 115.5, 118.4, 125.5, 107.7, 121.1, 119.1)),
+    ((1180, 13120, 5408), (135.4, 130.9, 146.6, 182.8, 152.7, 157.7, 167.7, 178.7, 194.0, 142.4, 148.4)),
+    ((998, 9128, 5104), (84.0, 89.7, 68.2, 83.2, 93.1, 88.0, 99.8, 107.6, 109.8, 123.5, 76.4)),
+    ((3963, 12056, 720), (75.0, 77.0, 75.5, 85.4, 88.5, 85.2, 81.9, 86.8, 88.3, 90.2, 86.0)),
+    ((3039, 3016, 11624), (248.5, 261.4, 205.8, 231.8, 211.1, 223.9, 236.5, 238.4, 253.5, 267.7, 145.3)),
+    ((5200, 24872, 864), (203.5, 210.1, 195.3, 248.9, 250.1, 245.7, 257.4, 247.2, 270.8, 242.1, 274.1)),
+    ((7082, 896, 3936), (41.2, 48.6, 51.8, 60.1, 59.2, 65.5, 69.9, 72.8, 47.0, 47.4, 52.4)),
+]
+
+
+def _choose(tmp_path, products):
+    src = tmp_path / "choose.cc"
+    src.write_text('#include <cstdio>\n#include "mc2/tile_choice.h"\nint main() { unsigned long long m, n, k; while (scanf("%llu %llu %llu", &m, &n, &k) == 3) { '
+                   'auto t = hccl::mc2::ChooseTile(m, n, k, false, 148, true); printf("%d %u\\n", (int)t.pair, t.bn); } }\n')
+    exe = tmp_path / "choose"
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'csrc'}", str(src), "-o", str(exe)], check=True, timeout=120)
+    out = subprocess.run([str(exe)], input="".join(f"{m} {n} {k}\n" for m, n, k in products), capture_output=True, text=True, check=True, timeout=60)
+    return [tuple(int(v) for v in line.split()) for line in out.stdout.splitlines()]
+
+
+def test_chosen_width_is_within_the_noise_of_the_best(tmp_path):
+    """Runs of one width differed by up to 8 % where these were measured."""
+    for (shape, us), (pair, width) in zip(MEASURED, _choose(tmp_path, [p for p, _ in MEASURED])):
+        assert pair and us[WIDTHS.index(width)] <= 1.08 * min(us), (shape, width, us)
