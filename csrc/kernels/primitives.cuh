@@ -381,33 +381,43 @@ template <class F> __device__ __forceinline__ void BlockCopiesOf(int n, F part)
     BlockCopies(parts, n);
 }
 
-// One source to n destinations (dst(q)): a vector is loaded once, four at a time.
+// One source to n destinations (dst(q)), by the widest of 16, 4 and 1 bytes that all sides are aligned to: loaded once, four at a time.
+template <typename V> __device__ __forceinline__ void StoreToAll(char *const *to, int n, const char *src, uint64_t len)
+{
+    constexpr int U = 4;
+    const uint64_t vecs = len / sizeof(V);
+    for (uint64_t i = threadIdx.x; i < vecs; i += (uint64_t)blockDim.x * U) {
+        V v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) if (i + (uint64_t)u * blockDim.x < vecs) v[u] = ((const V *)src)[i + (uint64_t)u * blockDim.x];
+#pragma unroll 1
+        for (int q = 0; q < n; ++q) {
+            V *d = (V *)to[q] + i;
+#pragma unroll
+            for (int u = 0; u < U; ++u) if (i + (uint64_t)u * blockDim.x < vecs) d[(uint64_t)u * blockDim.x] = v[u];
+        }
+    }
+    for (int q = 0; q < n; ++q)
+        for (uint64_t i = vecs * sizeof(V) + threadIdx.x; i < len; i += blockDim.x) to[q][i] = src[i];
+}
 template <class F> __device__ __forceinline__ void BlockCopyToAll(int n, F dst, const char *src, uint64_t len)
 {
     __shared__ char *to[kMaxRanks];
     if ((int)threadIdx.x < n) to[threadIdx.x] = dst((int)threadIdx.x);
     __syncthreads();
     uintptr_t any = (uintptr_t)src;
-    for (int q = 0; q < n; ++q) any |= (uintptr_t)to[q] | (HCCL_RANGE_OK(to[q], len) && HCCL_RANGE_OK(src, len) ? 0u : 1u);
-    if (any & 15u) {
+    bool ok = HCCL_RANGE_OK(src, len);
+    for (int q = 0; q < n; ++q) {
+        any |= (uintptr_t)to[q];
+        ok = ok && HCCL_RANGE_OK(to[q], len);
+    }
+    if (!ok) {                                           // reported, and skipped there
         for (int q = 0; q < n; ++q) BlockCopy(to[q], src, len);
         return;
     }
-    constexpr int U = 4;
-    const uint64_t vecs = len >> 4;
-    for (uint64_t i = threadIdx.x; i < vecs; i += (uint64_t)blockDim.x * U) {
-        uint4 v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) if (i + (uint64_t)u * blockDim.x < vecs) v[u] = ((const uint4 *)src)[i + (uint64_t)u * blockDim.x];
-#pragma unroll 1
-        for (int q = 0; q < n; ++q) {
-            uint4 *d = (uint4 *)to[q] + i;
-#pragma unroll
-            for (int u = 0; u < U; ++u) if (i + (uint64_t)u * blockDim.x < vecs) d[(uint64_t)u * blockDim.x] = v[u];
-        }
-    }
-    for (int q = 0; q < n; ++q)
-        for (uint64_t i = (vecs << 4) + threadIdx.x; i < len; i += blockDim.x) to[q][i] = src[i];
+    if ((any & 15u) == 0) StoreToAll<uint4>(to, n, src, len);
+    else if ((any & 3u) == 0) StoreToAll<uint32_t>(to, n, src, len);
+    else StoreToAll<char>(to, n, src, len);
 }
 
 // ---------------------------------------------------------------------------------------------- typed reduction
