@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
 // it. Every CTA holds all entries in its threads' registers (at most kFewEntries) and counts for its own few (at most kFewOwn) with one
 // warp-wide sum each, while the first pieces of its rows are already on their way. The CTA behind the last one with rows counts the
 // experts' totals. 100 tokens of hidden 7168, 256 experts, top-8, block-scaled, dispatch and combine among others on one B200: 18.4 us with the general
-// kernel and 2 KB pieces in the combine, 13.9 with this one, 512-byte pieces and launches that overlap.
+// kernel and 2 KB pieces in the combine, 14.9 with this one, 512-byte pieces and launches that overlap; mostly the host's part of the
+// calls, so runs differ by 0.7.
 constexpr uint32_t kFewEntries = 8 * kMoeThreads, kFewOwn = 64;
 inline uint32_t FewOwn(const MoeArgs &A, uint32_t G)     // bound on the entries of one CTA's tokens
 {

@@ -37,7 +37,7 @@ def check_result(t: torch.Tensor, elems: int, dtypes, what: str = "out") -> None
 def gemm_bf16(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, out_dtype: torch.dtype = torch.bfloat16,
               stream=None, variant: int = 0) -> torch.Tensor:
     """a: [M, K] bf16, w: [N, K] bf16 (both row-major) -> [M, N] in `out_dtype` (bf16 or fp32).
-    variant: 0 automatic, 2 CTA-pair (cta_group::2) 256 x 256 tiles, 192 / 224 pair tiles of that width, 1000 * S + BT split-K with BT rows of
+    variant: 0 automatic, 2 CTA-pair (cta_group::2) 256 x 256 tiles, 192 / 224 and 288 ... 512 in steps of 32 pair tiles of that width, 1000 * S + BT split-K with BT rows of
     a per tile and S CTAs along K."""
     if not (a.is_cuda and w.is_cuda):
         raise RuntimeError("gemm_bf16 needs CUDA tensors (the tcgen05 kernel has no CPU path)")

@@ -49,7 +49,7 @@ typedef struct HcclOpResCtxDef {
 /* ---- Part 2: fused operators (bf16 here, block-scaled fp8 in part 3; weights are [N, K] row-major, i.e. K contiguous) ---------------------------- */
 /* C[M,N] = A[M,K] * B[N,K]^T on one GPU (the building block; also the N = 1 degenerate case of the fused ops). */
 HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream);
-/* variant 2 = 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2), 192 / 224 / 256 = pair tiles of that width, 1000 * S + BT = split-K with
+/* variant 2 = 256 x 256 tiles on CTA pairs (tcgen05 cta_group::2), 192 / 224 / 256 and 288 ... 512 in steps of 32 = pair tiles of that width, 1000 * S + BT = split-K with
  * BT (16 ... 256) rows of A per tile and S (1 ... 8) CTAs along K; anything else = automatic */
 HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, int variant, cudaStream_t stream);
 /* C[M,N] = A[M,K] * B[K,N], both row-major: the input gradient of a linear layer from its [K, N] weight as stored. */

@@ -221,8 +221,9 @@ def test_saved_tensors_of_another_size(name, native, monkeypatch):
     from hccl_b200.ops import block
     from hccl_b200.parallel import tensor_parallel as tp
     comm = None
-    _native_nodes()
-    if not native:
+    if native:
+        _native_nodes()
+    else:
         monkeypatch.setattr(block, "_NODES", None)
     try:
         if name == "xent":
