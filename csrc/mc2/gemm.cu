@@ -250,9 +250,8 @@ HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint6
         HCCL_ERROR("HcclGemmBf16: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    const SplitKChoice sk = ChooseSplitK(m, n, k, false);
+    const auto [sk, t] = ChoosePlain(m, n, k, SmCount(), Gemm2CtaEnabled());
     if (sk.split) return LaunchSplitK<false>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
-    const TileChoice t = ChooseTile(m, n, k, false, SmCount(), Gemm2CtaEnabled());
     if (t.pair) return LaunchPair(t.bn, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.bn == 256) return LaunchPlain<256>(a, b, c, m, n, k, outFp32 != 0, stream);
     if (t.bn == 128) return LaunchPlain<128>(a, b, c, m, n, k, outFp32 != 0, stream);

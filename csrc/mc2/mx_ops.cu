@@ -149,7 +149,7 @@ HcclResult GemmMxfp8(const void *a, const void *sfa, const void *b, const void *
     }
     const char *tileEnv = getenv("HCCL_MX_TILE_N");
     if (!tileEnv) {
-        const SplitKChoice sk = ChooseSplitK(m, n, k, true);
+        const SplitKChoice sk = ChooseSplitK(m, n, k, true, false);
         if (sk.split) return LaunchSplitK<true>(sk, a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream, earlyB);
     }
     // CTA pairs when the product about fills the GPU with pair tiles (HCCL_MX_PAIR=0 keeps the one-CTA kernels): 192-wide tiles with two

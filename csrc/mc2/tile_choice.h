@@ -1,4 +1,4 @@
-// Tile kernel of a plain bf16 product. Host arithmetic alone, so that the choice can be tested without a GPU.
+// Kernel of a plain product. Host arithmetic alone, so that the choice can be tested without a GPU.
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -51,6 +51,62 @@ inline TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposed
     for (uint32_t bn = 288; bn <= 512; bn += 32)
         if (pair(bn) <= limit) offer(true, bn, pair(bn));
     return best;
+}
+
+// bt rows of A per tile (16, 32, 64, 128, 256), split CTAs along K per tile (1 ... 8)
+struct SplitKChoice { uint32_t bt = 0, split = 0; };
+
+// Clusters of 1 ... 8 CTAs that run at once with one CTA on an SM: SMs come in groups that a cluster does not cross. Read off the step in time over
+// 967 products: with one cluster more than fit the product takes 1.4 times as long on average as with one CTA less along K.
+constexpr uint32_t kClustersAtOnce[9] = {0, 148, 71, 44, 33, 26, 22, 15, 15};
+
+// Whether the split-K form is the better one for this product, and its shape. narrowWave: the best tiles are 64 wide on one CTA and take one wave of at
+// least 90 CTAs.
+// Measured on one B200 with weights that rotate through more than L2, us per product in a graph of many (tile kernels / split-K):
+//   rows <= 64, K >= 2048: split-K wins or ties. m x n x k = 4 x 4096 x 4096: 25.2 / 10.3; 16 x 4096 x 14336: 42.3 / 22.9; 1 x 512 x 16384:
+//     47.8 / 11.1; 8 x 28672 x 4096: 50.5 / 40.6; 64 x 128256 x 4096: 195.8 / 171; 64 x 28672 x 8192: 81.3 / 79.8. With K = 1024 it
+//     wins with up to 16 rows (16 x 8192 x 1024: 9.8 / 7.1) and not with 64 (64 x 4096 x 1024: 7.2 / 7.4).
+//   more rows: where the tile kernels leave the GPU partly empty (200 x 1024 x 8192: 26.1 / 13.4; 512 x 1024 x 4096: 15.4 / 12.2), not
+//     where they have about as many CTAs as SMs (128 x 8192 x 1024: 8.1 / 10.3). One wave of 64-wide tiles is better up to K = 3700 (2400 where K straddles
+//     sectors, which costs tiles more), and for every K where 257 to 384 rows leave the second 256-row tile half empty and two CTAs along
+//     K: 193 x 4512 x 2624 11.0 / 12.7, 349 x 2216 x 2056 13.1 / 17.5, 365 x 3120 x 2880 11.7 / 16.6. Of 489 such products the choice takes 1.020 of the
+//     best kernel's time on average; split-K for all of them 1.30.
+//   CTAs in all: about one per SM while K is short (32 tiles, K 4096: split 4 10.3, 8 11.0; 64 tiles, K 1024: 2 7.1, 4 7.9), two per SM for a
+//     long K (64 tiles, K 8192: 2 27.6, 4 25.9) or several row tiles (100 x 4096 x 4096: 3 14.2, 4 13.5).
+//   65 to 512 rows, bf16, us with 64-row tiles / chosen (split x rows): one tile of 128 rows in two CTAs per SM 88 x 10120 x 7160 74 / 39 (3 x 128),
+//     122 x 10368 x 13952 91 / 56 (3 x 128), 69 x 4088 x 13504 30.7 / 24.3 (8 x 128); 256-row tiles, one CTA per SM, as many along K as run at once:
+//     336 x 3704 x 15208 143 / 76 (3 x 256 although two would run at once, 91: K straddles sectors). 64-row tiles stay where six CTAs share one
+//     (109 x 2088 x 15896 26.5 / 31.7 with 6 x 128) or three to five share a short K (229 x 1552 x 2464 9.1 / 10.0 with 8 x 256).
+//   Over 967 random products of 65 to 512 rows the choice takes 1.030 of the best kernel's time on average; without 128- and 256-row tiles 1.075; with
+//     four CTAs along K wherever 148 SMs have room for them, and tiles counted 128 wide, 1.041 and up to 1.95.
+inline SplitKChoice ChooseSplitK(uint64_t m, uint64_t n, uint64_t k, bool mx, bool narrowWave)
+{
+    const uint64_t nt = (n + 127) / 128, tileCtas = (m + 127) / 128 * nt;       // tileCtas: CTAs that 128-wide tiles would use
+    if (m <= 64 ? (k < 2048 && (m > 16 || k < 512)) : (k < 2048 || m > 512 || tileCtas >= 90 || (narrowWave && k < (k % 16 ? 2400 : 3700)))) return {};
+    auto parts = [&](uint64_t s) { return (uint32_t)std::min<uint64_t>(8, std::min<uint64_t>(std::max<uint64_t>(1, s), k / 256)); };
+    const uint32_t bt = m <= 16 ? 16 : m <= 32 ? 32 : 64;
+    const uint64_t tiles = nt * ((m + bt - 1) / bt), ctas = k > 6144 || m > 64 ? 256 : 148;
+    const SplitKChoice narrow{bt, parts(ctas / tiles)};
+    if (m <= 64 || mx || narrow.split >= 6 || (k < 5000 && narrow.split >= 3)) return narrow;
+    if (m <= 128) return k >= 4096 ? SplitKChoice{128, parts(256 / nt)} : SplitKChoice{};     // 72 x 7192 x 2576: 11.6, tiles 10.6
+    const uint64_t t256 = nt * ((m + 255) / 256);
+    uint64_t s = 8;
+    while (s > 1 && t256 > kClustersAtOnce[s]) --s;
+    if (s == 2 && narrowWave) return {};
+    return {256, parts(s == 2 && k % 16 ? 3 : s)};
+}
+
+// The kernel of C = A * B^T in bf16: split-K where `split` is not 0, else the tile.
+struct PlainChoice { SplitKChoice splitK; TileChoice tile; };
+inline PlainChoice ChoosePlain(uint64_t m, uint64_t n, uint64_t k, uint64_t sms, bool pairsEnabled)
+{
+    if (m <= 64) {
+        const SplitKChoice sk = ChooseSplitK(m, n, k, false, false);
+        if (sk.split) return {sk, {false, 64}};
+    }
+    const TileChoice t = ChooseTile(m, n, k, false, sms, pairsEnabled);
+    const uint64_t narrow = !t.pair && t.bn == 64 ? (m + 127) / 128 * ((n + 63) / 64) : 0;
+    return {m <= 64 ? SplitKChoice{} : ChooseSplitK(m, n, k, false, narrow >= 90 && narrow <= sms), t};
 }
 
 }  // namespace mc2
