@@ -112,21 +112,18 @@ __device__ __forceinline__ void MoeItems(const MoeArgs &A, uint32_t segVecs, uin
 //   1. every CTA counts ALL routed entries itself, split into those before its first token and the others (shared-memory
 //      atomics; 32768 entries are 16 loads of four per thread). That replaces a per-CTA histogram in global memory, a grid-wide
 //      barrier and the walk over all CTAs' counts.
-//   2. with several ranks CTA 0 publishes the rank's totals and the grid waits for everyone's; with one rank (SOLO) the
-//      totals are already here and the kernel is launched without any grid barrier.
+//   2. CTA 0 publishes the rank's totals and the grid waits for everyone's.
 //   3. base rows by one prefix sum over the experts; the ordinal of an entry among those of its expert (token order) from
 //      __match_any_sync within a warp and a running count over the warps: the layout is a function of the routing alone.
 //   4. a warp reads a 2 KB piece of a token row ONCE, quantises it once (block-scaled form: four lanes share a 1 x 32 block,
 //      so loads and stores stay coalesced) and writes it to all topK destinations.
-// One B200, one rank, 256 experts, top-8, hidden 7168, 4096 tokens, bf16: dispatch + combine took 530 us, now 206 (dispatch 111, combine
-// 92; reading and writing the rows alone 81 each). Where rows are
-// short the counting outweighs them, 32768 tokens of hidden 256, top-8: 560 us, now 80 (rows alone 23).
-template <bool EMU, bool SOLO>
+// One rank needs no barrier and has a kernel of its own (moe_bulk.cuh).
+template <bool EMU>
 __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *comms, const __grid_constant__ MoeArgs av, const MoeArgs *emuArgs)
 {
     const DevComm *c = EMU ? &comms[blockIdx.y] : comms;
     const MoeArgs &A = EMU ? emuArgs[blockIdx.y] : av;
-    const int n = SOLO ? 1 : c->nranks, me = SOLO ? 0 : c->rank;
+    const int n = c->nranks, me = c->rank;
     char *ws = c->heap[me] + A.wsOff;
     const uint32_t E = A.E, EL = E / n, K = A.K, entries = A.T * K;
     const uint32_t G = gridDim.x, cta = blockIdx.x;
@@ -140,7 +137,6 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
     __shared__ uint32_t sWarp[kMoeWarps][kMaxExperts]; // per warp: entries of e in the current batch, then the first row of the warp's entries
     __shared__ uint32_t sRow[kMoeThreads];             // destination row of the batch's entries
 
-    if (SOLO) { sm100::LetDependentsStart(); sm100::DependencyWait(); }
     uint32_t segs;
     uint64_t itemLo, itemHi;
     MoeItems(A, kSegVecs, cta, G, &segs, &itemLo, &itemHi);
@@ -176,30 +172,25 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
     __syncthreads();
 
     // 2. everyone's totals
-    KCtx k;
-    if (!SOLO) {
-        k = MoeEnter(c, 0);
-        if (cta == 0) {
-            for (uint32_t e = tid; e < E; e += kMoeThreads)
-                for (int r = 0; r < n; ++r) FlagsOf(c->heap[r])->moeCount[me][e] = sTotal[e];
-            ChannelBarrier(k, 61);
-            __threadfence();
-        }
-        cg::this_grid().sync();
+    KCtx k = MoeEnter(c, 0);
+    if (cta == 0) {
+        for (uint32_t e = tid; e < E; e += kMoeThreads)
+            for (int r = 0; r < n; ++r) FlagsOf(c->heap[r])->moeCount[me][e] = sTotal[e];
+        ChannelBarrier(k, 61);
+        __threadfence();
     }
+    cg::this_grid().sync();
 
     // 3. first row of every expert at its destination: rows of the rank's earlier experts + rows of earlier sources
     const uint32_t e0 = tid;
     uint32_t all = 0, earlier = 0;
     static_assert(kMaxExperts <= kMoeThreads, "one thread per expert");
     if (e0 < E) {
-        if (SOLO) all = sTotal[e0];
-        else
-            for (int s = 0; s < n; ++s) {
-                const uint32_t v = k.flags->moeCount[s][e0];
-                all += v;
-                if (s < me) earlier += v;
-            }
+        for (int s = 0; s < n; ++s) {
+            const uint32_t v = k.flags->moeCount[s][e0];
+            all += v;
+            if (s < me) earlier += v;
+        }
         sScan[0][e0] = all;
     }
     __syncthreads();
@@ -281,8 +272,7 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
                 }
                 const uint32_t d = ex / EL, row = sRow[(t - tb) * K + kk];
                 char *dws = c->heap[d] + A.wsOff;
-                // one rank: the debug flavor's heap check reads the communicator that MoeEnter registers, which this form does not call
-                if (SOLO ? row >= A.cap : !HCCL_RANGE_OK(dws + A.L.recvX + (uint64_t)row * (A.mxfp8 ? A.H : rowBytes), A.mxfp8 ? A.H : rowBytes)) {
+                if (!HCCL_RANGE_OK(dws + A.L.recvX + (uint64_t)row * (A.mxfp8 ? A.H : rowBytes), A.mxfp8 ? A.H : rowBytes)) {
                     if (seg == 0 && lane == 0) slotMap[i] = noSlot;
                     continue;
                 }
@@ -308,7 +298,6 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
         }
         __syncthreads();
     }
-    if (SOLO) return;
     __threadfence_system();
     cg::this_grid().sync();
     // 5. everyone has finished writing: after this barrier the received rows are visible
@@ -341,119 +330,9 @@ __global__ void __launch_bounds__(kMoeThreads) MoeDispatchKernel(const DevComm *
     }
 }
 
-// Dispatch of few tokens on one rank. The general kernel's time is then its chain of steps, some twenty block-wide barriers from the
-// histogram to the rows. Here the row of an entry is counted directly: how many entries go to an earlier expert, or to the same one before
-// it. Every CTA holds all entries in its threads' registers (at most kFewEntries) and counts for its own few (at most kFewOwn) with one
-// warp-wide sum each, while the first pieces of its rows are already on their way. The CTA behind the last one with rows counts the
-// experts' totals. 100 tokens of hidden 7168, 256 experts, top-8, block-scaled, dispatch and combine among others on one B200: 18.4 us with the general
-// kernel and 2 KB pieces in the combine, 14.9 with this one, 512-byte pieces and launches that overlap; mostly the host's part of the
-// calls, so runs differ by 0.7.
-constexpr uint32_t kFewEntries = 8 * kMoeThreads, kFewOwn = 64;
-inline uint32_t FewOwn(const MoeArgs &A, uint32_t G)     // bound on the entries of one CTA's tokens
-{
-    const uint64_t segs = (A.H / 8 + kSegVecsFew - 1) / kSegVecsFew, items = ((uint64_t)A.T * segs + G - 1) / G;
-    return (uint32_t)((items + segs - 2) / segs + 1) * A.K;
-}
-__global__ void __launch_bounds__(kMoeThreads) MoeDispatchFewKernel(const DevComm *c, const __grid_constant__ MoeArgs A)
-{
-    __shared__ uint32_t sOwn[kFewOwn], sRow[kFewOwn], sCnt[kMoeWarps][kFewOwn + 1], sTotal[kMaxExperts];
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = A.K, E = A.E, entries = A.T * K;
-    const uint32_t G = gridDim.x - 1, cta = blockIdx.x, rowVecs = A.H / 8;
-    sm100::LetDependentsStart();
-    sm100::DependencyWait();
-    char *ws = c->heap[0] + A.wsOff;
-    uint64_t *slotMap = (uint64_t *)(ws + A.L.slotMap);
-    const uint64_t noSlot = NoSlot(0, A.cap);
-    uint32_t e[kFewEntries / kMoeThreads];
-#pragma unroll
-    for (uint32_t r = 0; r < kFewEntries / kMoeThreads; ++r) {
-        const uint32_t i = r * kMoeThreads + tid;
-        e[r] = i < entries ? (uint32_t)A.topkIdx[i] : 0xffffffffu;
-        if (e[r] >= E) e[r] = 0xffffffffu;               // no row: behind all experts
-    }
-    if (cta == G) {
-        for (uint32_t x = tid; x < E; x += kMoeThreads) sTotal[x] = 0;
-        for (uint32_t v = tid; v < rowVecs; v += kMoeThreads) ((uint4 *)(ws + A.L.yBuf + (uint64_t)A.cap * A.H * 2))[v] = make_uint4(0, 0, 0, 0);
-        __syncthreads();
-#pragma unroll
-        for (uint32_t r = 0; r < kFewEntries / kMoeThreads; ++r) if (e[r] < E) atomicAdd(&sTotal[e[r]], 1u);
-        __syncthreads();
-        for (uint32_t x = tid; x < E; x += kMoeThreads) ((int32_t *)(ws + A.L.recvCounts))[x] = (int32_t)sTotal[x];
-        return;
-    }
-    uint32_t segs;
-    uint64_t itemLo, itemHi;
-    MoeItems(A, kSegVecsFew, cta, G, &segs, &itemLo, &itemHi);
-    const uint32_t tLo = (uint32_t)(itemLo / segs), tHi = (uint32_t)((itemHi + segs - 1) / segs), first = tLo * K, own = (tHi - tLo) * K;
-    auto piece = [&](uint64_t it) {
-        const uint32_t v = (uint32_t)(it % segs) * kSegVecsFew + lane;
-        return v < rowVecs ? ((const uint4 *)((const char *)A.x + it / segs * A.H * 2))[v] : make_uint4(0, 0, 0, 0);
-    };
-    uint4 next = itemLo + warp < itemHi ? piece(itemLo + warp) : make_uint4(0, 0, 0, 0);
-    if (tid < own) {
-        const uint32_t x = (uint32_t)A.topkIdx[first + tid];
-        sOwn[tid] = x < E ? x : 0xffffffffu;
-    }
-    __syncthreads();
-    const uint32_t rounds = (entries + kMoeThreads - 1) / kMoeThreads;
-    for (uint32_t j = 0; j <= own; ++j) {                // j = own: all entries that have a row
-        const uint32_t mine = j < own ? sOwn[j] : 0xffffffffu, at = j < own ? first + j : 0;
-        uint32_t n = 0;
-#pragma unroll
-        for (uint32_t r = 0; r < kFewEntries / kMoeThreads; ++r)
-            if (r < rounds) n += e[r] < mine || (e[r] == mine && r * kMoeThreads + tid < at);
-        n = __reduce_add_sync(0xffffffffu, n);
-        if (lane == 0) sCnt[warp][j] = n;
-    }
-    __syncthreads();
-    uint32_t total = 0;
-#pragma unroll
-    for (int w = 0; w < kMoeWarps; ++w) total += sCnt[w][own];
-    if (tid < own) {
-        uint32_t row = 0;
-#pragma unroll
-        for (int w = 0; w < kMoeWarps; ++w) row += sCnt[w][tid];
-        sRow[tid] = row;
-    }
-    __syncthreads();
-    if (total > A.cap) {                                 // receive buffer too small: report, move nothing
-        if (cta == 0 && tid == 0) {
-            DevStatus *st = c->status;
-            st->rank = 0; st->observed = total; st->expected = A.cap; st->phase = 62;
-            __threadfence_system();
-            *((volatile uint32_t *)&st->code) = 2u;
-        }
-        if (tid < own) slotMap[first + tid] = noSlot;
-        return;
-    }
-    for (uint64_t it = itemLo + warp; it < itemHi; it += kMoeWarps) {
-        const uint4 r = next;
-        if (it + kMoeWarps < itemHi) next = piece(it + kMoeWarps);
-        const uint32_t t = (uint32_t)(it / segs), seg = (uint32_t)(it % segs), v = seg * kSegVecsFew + lane;
-        uint2 q;
-        uint8_t se;
-        if (A.mxfp8) q = QuantizeVec(r, &se);
-        for (uint32_t kk = 0; kk < K; ++kk) {
-            const uint32_t j = (t - tLo) * K + kk, ex = sOwn[j], row = sRow[j];
-            const bool has = ex < E;                     // and row < total <= cap
-            if (seg == 0 && lane == 0) {
-                slotMap[first + j] = has ? row : noSlot;
-                if (has) ((int32_t *)(ws + A.L.recvSrc))[row] = (int32_t)t;
-            }
-            if (!has || v >= rowVecs) continue;
-            if (!A.mxfp8) {
-                ((uint4 *)(ws + A.L.recvX + (uint64_t)row * A.H * 2))[v] = r;
-            } else {
-                ((uint2 *)(ws + A.L.recvX + (uint64_t)row * A.H))[v] = q;
-                if ((lane & 3) == 0) ((uint8_t *)(ws + A.L.recvScales + (uint64_t)row * (A.H / 32)))[v / 4] = se;
-            }
-        }
-    }
-}
-
 // Combine: out[t] = sum over k, in order, of weight * expert row (zeros for an entry without one). Bound by reading topK rows per token. KMAX (8 or 16) keeps
 // the row addresses and weights of a token in registers; a warp takes 2 KB of the output row at a time, all KMAX source rows
-// of a vector in flight. 2048 tokens of hidden 4096, top-16 (128 registers, 24 bytes spilled): 137 us, now 53 (rows alone 44).
+// of a vector in flight. One rank (SOLO): few tokens only, in pieces of 512 bytes; moe_bulk.cuh has the kernel for more.
 template <bool EMU, bool SOLO, int KMAX>
 __global__ void __launch_bounds__(kMoeThreads) MoeCombineKernel(const DevComm *comms, const __grid_constant__ MoeArgs av, const MoeArgs *emuArgs)
 {

@@ -6,7 +6,7 @@
 #include "../core/comm.h"
 #include "../kernels/emu_world.h"
 #include "hccl/hccl_moe.h"
-#include "moe_kernels.cuh"
+#include "moe_bulk.cuh"
 
 namespace hccl {
 namespace moe {
@@ -49,7 +49,7 @@ struct MoeState {
     uint64_t wsOff = 0;
     uint32_t ctas = 0;
     bool solo = false;
-    uint32_t combineCtas = 0;     // one rank: its registers allow one CTA per SM, a second wave costs 4 % (94.5 / 91 us at 4096 tokens)
+    uint32_t bulkCtas = 0;        // one rank: CTAs of the kernels that fill an SM
     uint32_t lastTokens = 0;
 };
 
@@ -71,44 +71,50 @@ MoeArgs MakeArgs(const HcclMoeConfig &cfg, const MoeLayout &L, uint64_t wsOff, u
     return a;
 }
 
-// One rank: no more CTAs than pieces of token rows (every CTA of the dispatch counts all entries first).
+// One rank: no more CTAs than pieces of token rows.
 uint32_t SoloCtas(const MoeArgs &a, uint32_t segVecs, uint32_t ctas)
 {
     const uint64_t items = (uint64_t)a.T * ((a.H / 8 + segVecs - 1) / segVecs);
     return (uint32_t)std::min<uint64_t>(ctas, items);
 }
 
-// One rank: a plain launch that may start while the kernel before it drains.
-cudaError_t LaunchSolo(const void *fn, void **params, uint32_t ctas, cudaStream_t s)
+// The shared memory of the one-rank kernels, on the current device.
+bool RingsAllowed()
 {
+    auto allow = [](const void *fn, uint32_t bytes) { return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess; };
+    return allow((const void *)MoeDispatchBulkKernel<false>, kDispatchRing) && allow((const void *)MoeDispatchBulkKernel<true>, kDispatchRing) &&
+           allow(CombineBulk(1), kCombineSmem) && allow(CombineBulk(4), kCombineSmem) && allow(CombineBulk(8), kCombineSmem) && allow(CombineBulk(16), kCombineSmem);
+}
+
+// One rank: a plain launch that may start while the kernel before it drains.
+HcclResult LaunchSolo(const void *fn, const DevComm *comms, const MoeArgs &a, uint32_t ctas, uint32_t threads, uint32_t smem, cudaStream_t s)
+{
+    MoeArgs av = a;
+    const MoeArgs *none = nullptr;
+    void *params[] = {(void *)&comms, (void *)&av, (void *)&none};
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(kMoeThreads);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, fn, params);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, params);
+    if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u)", cudaGetErrorString(e), ctas); return HCCL_E_RUNTIME; }
+    return HCCL_SUCCESS;
 }
 
-// solo: a communicator of one rank needs no barrier among CTAs, so the kernel is launched without the cooperative constraint.
-template <bool EMU> HcclResult LaunchMoe(bool dispatch, const DevComm *comms, const MoeArgs &a, const MoeArgs *emuArgs, uint32_t ctas, uint32_t ranksY, cudaStream_t s,
-                                         bool solo = false)
+// Several ranks: cooperative, since CTAs wait for one another.
+template <bool EMU> HcclResult LaunchMoe(bool dispatch, const DevComm *comms, const MoeArgs &a, const MoeArgs *emuArgs, uint32_t ctas, uint32_t ranksY, cudaStream_t s)
 {
     MoeArgs av = a;
     void *params[] = {(void *)&comms, (void *)&av, (void *)&emuArgs};
-    cudaError_t e;
-    if (!EMU && solo) {
-        const void *fn = dispatch ? (const void *)MoeDispatchKernel<false, true>
-                                  : a.K <= 8 ? (const void *)MoeCombineKernel<false, true, 8> : (const void *)MoeCombineKernel<false, true, 16>;
-        e = LaunchSolo(fn, params, ctas, s);
-    } else {
-        const void *fn = dispatch ? (const void *)MoeDispatchKernel<EMU, false>
-                                  : a.K <= 8 ? (const void *)MoeCombineKernel<EMU, false, 8> : (const void *)MoeCombineKernel<EMU, false, 16>;
-        e = cudaLaunchCooperativeKernel(fn, dim3(ctas, ranksY), dim3(kMoeThreads), params, 0, s);
-    }
+    const void *fn = dispatch ? (const void *)MoeDispatchKernel<EMU>
+                              : a.K <= 8 ? (const void *)MoeCombineKernel<EMU, false, 8> : (const void *)MoeCombineKernel<EMU, false, 16>;
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(ctas, ranksY), dim3(kMoeThreads), params, 0, s);
     if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u x %u)", cudaGetErrorString(e), ctas, ranksY); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
@@ -135,9 +141,9 @@ HcclResult HcclMoeCreate(HcclComm comm, const HcclMoeConfig *config, HcclMoeHand
     st->ctas = (uint32_t)std::min(SmCountNow(), 64);
     // one rank: the rows stay in this GPU's memory, 64 SMs do not keep HBM busy and no CTA waits for another
     st->solo = c->nranks == 1;
-    if (st->solo) st->ctas = (uint32_t)SmCountNow() * 2;
-    st->combineCtas = st->solo ? (uint32_t)SmCountNow() : st->ctas;
-    if (const char *e = getenv("HCCL_MOE_CTAS")) { int v = atoi(e); if (v > 0 && v <= SmCountNow()) st->ctas = st->combineCtas = (uint32_t)v; }
+    st->bulkCtas = (uint32_t)SmCountNow();
+    if (const char *e = getenv("HCCL_MOE_CTAS")) { int v = atoi(e); if (v > 0 && v <= SmCountNow()) st->ctas = st->bulkCtas = (uint32_t)v; }
+    if (st->solo && !RingsAllowed()) { HCCL_ERROR("MoE: %u bytes of shared memory per CTA are not available", kCombineSmem); delete st; return HCCL_E_RUNTIME; }
     st->L = MakeLayout(*config);
     HcclResult r = SymAlloc(c, st->L.total, &st->ws);
     if (r != HCCL_SUCCESS) { delete st; return r; }
@@ -167,14 +173,11 @@ HcclResult HcclMoeDispatch(HcclMoeHandle handle, const void *x, const int32_t *t
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.x = x;
     a.topkIdx = topkIdx;
-    const uint32_t fewCtas = SoloCtas(a, kSegVecsFew, st->ctas);
-    if (st->solo && (uint64_t)a.T * a.K <= kFewEntries && FewOwn(a, fewCtas) <= kFewOwn) {
-        const DevComm *comms = c->devCommPtr;
-        void *params[] = {(void *)&comms, (void *)&a};
-        const cudaError_t e = LaunchSolo((const void *)MoeDispatchFewKernel, params, fewCtas + 1, stream);
-        if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u)", cudaGetErrorString(e), fewCtas + 1); return HCCL_E_RUNTIME; }
+    if (st->solo) {
+        const void *fn = a.mxfp8 ? (const void *)MoeDispatchBulkKernel<true> : (const void *)MoeDispatchBulkKernel<false>;
+        CHK_RET(LaunchSolo(fn, c->devCommPtr, a, SoloCtas(a, kSegVecs, st->bulkCtas), kMoeThreads, kDispatchRing, stream));
     } else {
-        CHK_RET(LaunchMoe<false>(true, c->devCommPtr, a, nullptr, st->solo ? SoloCtas(a, kSegVecs, st->ctas) : st->ctas, 1, stream, st->solo));
+        CHK_RET(LaunchMoe<false>(true, c->devCommPtr, a, nullptr, st->ctas, 1, stream));
     }
     st->lastTokens = numTokens;
     c->counters.kernelsLaunched++;
@@ -206,9 +209,17 @@ HcclResult HcclMoeCombine(HcclMoeHandle handle, const float *topkWeights, void *
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.weights = topkWeights;
     a.out = out;
-    // few tokens on one rank: small pieces, so that a warp has one load of each row to wait for
-    if (st->solo && (uint64_t)a.T * (a.H / 8) <= (uint64_t)st->combineCtas * kMoeWarps * 2 * kSegVecsFew) a.segVecs = kSegVecsFew;
-    CHK_RET(LaunchMoe<false>(false, c->devCommPtr, a, nullptr, st->solo ? SoloCtas(a, a.segVecs, st->combineCtas) : st->ctas, 1, stream, st->solo));
+    if (!st->solo) {
+        CHK_RET(LaunchMoe<false>(false, c->devCommPtr, a, nullptr, st->ctas, 1, stream));
+    } else if ((uint64_t)a.T * (a.H / 8) <= (uint64_t)st->bulkCtas * kMoeWarps * 2 * kSegVecsFew) {
+        // Up to two pieces per warp: the kernel that loads into registers has no tables to fill first. Us with it / with the ring, top-8, 256 experts, hidden
+        // 7168: 64 tokens 3.0 / 3.6, 128 4.0 / 4.4, 256 6.5 / 6.4, 512 14.6 / 12.9; 4000 x 1024 top-1 7.0 / 6.4.
+        a.segVecs = kSegVecsFew;
+        const void *fn = a.K <= 8 ? (const void *)MoeCombineKernel<false, true, 8> : (const void *)MoeCombineKernel<false, true, 16>;
+        CHK_RET(LaunchSolo(fn, c->devCommPtr, a, SoloCtas(a, a.segVecs, st->bulkCtas), kMoeThreads, 0, stream));
+    } else {
+        CHK_RET(LaunchSolo(CombineBulk(a.K), c->devCommPtr, a, SoloCtas(a, 32, st->bulkCtas), CombineWarps(a.K) * 32, CombineBytes(a.K), stream));
+    }
     c->counters.kernelsLaunched++;
     CountLaunch();
     c->counters.ops++;

@@ -336,3 +336,49 @@ def test_one_rank_few_tokens(T, E, K, H, mxfp8, ctas, monkeypatch):
         d.close()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("T,E,K,H,mxfp8,ctas", [(700, 64, 16, 512, False, "3"), (700, 64, 14, 768, True, "3"), (513, 320, 13, 256, False, "2"), (4097, 9, 1, 1280, True, "2"), (900, 32, 5, 2304, False, "7"),
+                                                (300, 8, 2, 7168, True, ""), (2500, 60, 6, 1024, False, ""), (333, 256, 7, 4352, True, "")])
+def test_one_rank_rings(T, E, K, H, mxfp8, ctas, monkeypatch):
+    """The rings of the one-rank kernels: several batches of entries per CTA in both directions, every depth, a last piece that is not whole, ragged
+    ranges, some entries without a row. Rows and scales are bytes; the combine adds at most 16 products in 32 bits and rounds once."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    if ctas:
+        monkeypatch.setenv("HCCL_MOE_CTAS", ctas)
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(T + K)
+        x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+        idx = torch.randint(0, E, (T, K), generator=g, device="cuda").to(torch.int32)
+        idx[torch.rand(T, K, generator=g, device="cuda") < 0.05] = E
+        w = torch.rand(T, K, generator=g, device="cuda")
+        d = MoeDispatcher(comm, E, K, H, T, max_recv_rows=T * K, mxfp8=mxfp8)
+        rx, rs, counts, src = d.dispatch(x, idx)
+        y = torch.randn(T * K, H, generator=g, device="cuda").to(torch.bfloat16)
+        d.expert_out.copy_(y)
+        out = d.combine(w)
+        torch.cuda.synchronize()
+        flat, ok = idx.flatten().long(), idx < E
+        n = int(ok.sum())
+        order = torch.argsort(flat, stable=True)[:n]
+        assert torch.equal(counts.long(), torch.bincount(flat[ok.flatten()], minlength=E))
+        assert torch.equal(src[:n].long(), order // K)
+        rows = x[order // K]
+        if mxfp8:
+            _, q, se = _moe_quant_reference(rows)
+            assert torch.equal(rx[:n].view(torch.uint8), q) and torch.equal(rs[:n], se)
+        else:
+            assert torch.equal(rx[:n], rows)
+        slot = torch.zeros(T * K, dtype=torch.long, device="cuda")
+        slot[order] = torch.arange(n, device="cuda")
+        ref, bound = torch.zeros(T, H, dtype=torch.float64, device="cuda"), torch.zeros(T, H, dtype=torch.float64, device="cuda")
+        for j in range(K):
+            term = torch.where(ok[:, j, None], w[:, j, None].double() * y[slot.view(T, K)[:, j]].double(), 0.0)
+            ref += term
+            bound += term.abs()
+        assert bool(((out.double() - ref).abs() <= bound * K * 2.0 ** -23 + ref.abs() * 2.0 ** -8).all())
+        d.close()
+    finally:
+        comm.destroy()
