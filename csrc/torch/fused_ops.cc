@@ -1,4 +1,4 @@
-// Native face of the matmul operators for PyTorch: argument checks, result allocation, the current stream and the C call in one
+// Native face of the matmul, block-scaled and MoE operators for PyTorch: argument checks, result allocation, the current stream and the C call in one
 // step. A decode-sized product takes under ten microseconds on the device; the same steps in Python and ctypes took
 // longer than that, so the GPU waited for the host between such calls.
 #include <c10/cuda/CUDAStream.h>
@@ -6,6 +6,7 @@
 #include <torch/extension.h>
 
 #include "hccl/hccl_mc2.h"
+#include "hccl/hccl_moe.h"
 
 namespace {
 
@@ -60,10 +61,75 @@ std::pair<int, at::Tensor> Fused(uint64_t comm, int kind, int64_t ranks, const a
     return {(int)r, std::move(o)};
 }
 
+// Memory of a call's own that it uses on a stream other than the one it was allocated for.
+void UsedOn(const at::Tensor &t, cudaStream_t s)
+{
+    const auto current = c10::cuda::getCurrentCUDAStream(t.device().index());
+    if (s != current.stream()) t.record_stream(c10::cuda::getStreamFromExternal(s, t.device().index()).unwrap());
+}
+
+// The quantised activations live for the call alone, in the order of its stream: nothing is shared between threads or kept between calls, and a captured
+// graph has them in its own pool.
+std::pair<int, at::Tensor> MxMatmul(uint64_t comm, const at::Tensor &a, const at::Tensor &payload, const at::Tensor &scales, int64_t n, const std::optional<at::Tensor> &out,
+                                    std::optional<uint64_t> stream)
+{
+    py::gil_scoped_release nogil;
+    const int64_t m = a.size(0), k = a.size(1);
+    at::Tensor o = out ? *out : at::empty({m, n}, a.options());
+    cudaStream_t s = StreamOf(stream);
+    const at::Tensor act = at::empty({m * k + (int64_t)HcclMxfp8ScaleBytes(m, k)}, a.options().dtype(at::kByte));
+    uint8_t *q = act.numel() ? act.data_ptr<uint8_t>() : nullptr;
+    const HcclResult r = HcclQuantizeMatmulMxfp8(a.data_ptr(), q, q + m * k, payload.data_ptr(), scales.data_ptr(), o.data_ptr(), m, n, k, (HcclComm)(uintptr_t)comm, s);
+    if (stream) UsedOn(act, s);
+    return {(int)r, std::move(o)};
+}
+
+std::tuple<int, at::Tensor, at::Tensor> MxQuantize(const at::Tensor &x, const std::optional<at::Tensor> &payload, const std::optional<at::Tensor> &scales,
+                                                   std::optional<uint64_t> stream)
+{
+    py::gil_scoped_release nogil;
+    const int64_t rows = x.size(0), k = x.size(1);
+    at::Tensor p = payload ? *payload : at::empty({rows, k}, x.options().dtype(at::kByte));
+    at::Tensor f = scales ? *scales : at::empty({(int64_t)HcclMxfp8ScaleBytes(rows, k)}, x.options().dtype(at::kByte));
+    const HcclResult r = HcclQuantizeMxfp8(x.data_ptr(), p.data_ptr(), f.data_ptr(), rows, k, StreamOf(stream));
+    return {(int)r, std::move(p), std::move(f)};
+}
+
+// `kept` holds the tensors over the receive buffers that the caller made for the addresses `at`. -> (HcclResult, addresses, new tensors over the same memory with a
+// version count of their own, or None where the addresses are others)
+py::tuple MoeDispatch(uint64_t handle, const at::Tensor &x, const at::Tensor &idx, std::optional<uint64_t> stream, const py::object &at, const py::tuple &kept)
+{
+    void *rx = nullptr, *rs = nullptr;
+    int32_t *rc = nullptr, *src = nullptr;
+    HcclResult r;
+    {
+        py::gil_scoped_release nogil;
+        r = HcclMoeDispatch((HcclMoeHandle)(uintptr_t)handle, x.data_ptr(), idx.data_ptr<int32_t>(), (uint32_t)x.size(0), &rx, &rs, &rc, &src, StreamOf(stream));
+    }
+    const py::tuple now = py::make_tuple((uint64_t)(uintptr_t)rx, (uint64_t)(uintptr_t)rs, (uint64_t)(uintptr_t)rc, (uint64_t)(uintptr_t)src);
+    if (r != HCCL_SUCCESS || !now.equal(at)) return py::make_tuple((int)r, now, py::none());
+    py::tuple out(kept.size());
+    for (size_t i = 0; i < kept.size(); ++i) out[i] = kept[i].is_none() ? py::object(py::none()) : py::cast(kept[i].cast<at::Tensor>().variable_data());
+    return py::make_tuple((int)r, now, out);
+}
+
+std::pair<int, at::Tensor> MoeCombine(uint64_t handle, const at::Tensor &weights, int64_t tokens, int64_t hidden, const std::optional<at::Tensor> &out,
+                                      std::optional<uint64_t> stream)
+{
+    py::gil_scoped_release nogil;
+    at::Tensor o = out ? *out : at::empty({tokens, hidden}, weights.options().dtype(at::kBFloat16));
+    const HcclResult r = HcclMoeCombine((HcclMoeHandle)(uintptr_t)handle, weights.data_ptr<float>(), o.data_ptr(), (uint32_t)tokens, StreamOf(stream));
+    return {(int)r, std::move(o)};
+}
+
 }  // namespace
 
 void BindFusedOps(py::module &m)
 {
     m.def("gemm", &Gemm);
     m.def("fused", &Fused);
+    m.def("mx_matmul", &MxMatmul);
+    m.def("mx_quantize", &MxQuantize);
+    m.def("moe_dispatch", &MoeDispatch);
+    m.def("moe_combine", &MoeCombine);
 }

@@ -6,6 +6,7 @@ from typing import Optional, Tuple
 
 import torch
 
+from .._ext import ops as _native
 from .._lib import check, lib
 
 
@@ -70,20 +71,29 @@ class MoeDispatcher:
 
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor, stream=None) -> Tuple[torch.Tensor, Optional[torch.Tensor], torch.Tensor, torch.Tensor]:
         assert x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and topk_idx.dtype == torch.int32 and topk_idx.is_contiguous()
-        s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) if stream is None else stream.cuda_stream
-        rx, rs, rc, rsrc = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
-        check(_decl().HcclMoeDispatch(self._h, x.data_ptr(), topk_idx.data_ptr(), x.shape[0], ctypes.byref(rx), ctypes.byref(rs), ctypes.byref(rc),
-                                      ctypes.byref(rsrc), s), "HcclMoeDispatch")
-        self._tokens = x.shape[0]
-        at = (rx.value, rs.value, rc.value, rsrc.value)
+        n = _native()
+        if n is not None:
+            rc, at, recv = n.moe_dispatch(self._h.value if self._h else 0, x, topk_idx, None if stream is None else stream.cuda_stream, *(((), ()) if self._recv is None else self._recv))
+            if rc:
+                check(rc, "HcclMoeDispatch")
+            self._tokens = x.shape[0]
+            if recv is not None:
+                return recv
+        else:
+            s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) if stream is None else stream.cuda_stream
+            rx, rs, rc, rsrc = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
+            check(_decl().HcclMoeDispatch(self._h, x.data_ptr(), topk_idx.data_ptr(), x.shape[0], ctypes.byref(rx), ctypes.byref(rs), ctypes.byref(rc),
+                                          ctypes.byref(rsrc), s), "HcclMoeDispatch")
+            self._tokens = x.shape[0]
+            at = tuple(p.value or 0 for p in (rx, rs, rc, rsrc))
         if self._recv is None or self._recv[0] != at:
             if torch.is_inference_mode_enabled():        # the views are kept beyond this call
                 with torch.inference_mode(False):
-                    self._recv = (at, *self._views(at, x.device))
+                    self._recv = (at, self._views(at, x.device))
             else:
-                self._recv = (at, *self._views(at, x.device))
+                self._recv = (at, self._views(at, x.device))
         # new tensors over the same memory on every call (`data`: with a version count of their own), as the caller may do with them what it likes
-        return tuple(None if t is None else t.data for t in self._recv[1:])
+        return tuple(None if t is None else t.data for t in self._recv[1])
 
     def _views(self, at, dev):
         rx, rs, rc, rsrc = at
@@ -93,6 +103,12 @@ class MoeDispatcher:
 
     def combine(self, topk_weights: torch.Tensor, out: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
         assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
+        n = _native()
+        if n is not None:
+            rc, out = n.moe_combine(self._h.value if self._h else 0, topk_weights, self._tokens, self.hidden, out, None if stream is None else stream.cuda_stream)
+            if rc:
+                check(rc, "HcclMoeCombine")
+            return out
         if out is None:
             out = torch.empty((self._tokens, self.hidden), dtype=torch.bfloat16, device=topk_weights.device)
         s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) if stream is None else stream.cuda_stream

@@ -13,6 +13,7 @@ from typing import Optional
 
 import torch
 
+from .._ext import ops as _native
 from .._lib import check, lib
 
 
@@ -63,6 +64,12 @@ def quantize(x: torch.Tensor, out: Optional[MxTensor] = None, stream=None) -> Mx
     """bf16 [rows, K] (K % 128 == 0) -> MxTensor, on the GPU."""
     _check_quantizable(x)
     rows, k = x.shape
+    n = _native()
+    if n is not None:
+        rc, payload, scales = n.mx_quantize(x, None if out is None else out.payload, None if out is None else out.scales, None if stream is None else stream.cuda_stream)
+        if rc:
+            check(rc, "HcclQuantizeMxfp8")
+        return MxTensor(payload, scales, rows, k) if out is None else out
     if out is None:
         out = empty_like_quantized(rows, k, x.device)
     check(_decl().HcclQuantizeMxfp8(x.data_ptr(), out.payload.data_ptr(), out.scales.data_ptr(), rows, k, _stream(stream)), "HcclQuantizeMxfp8")
@@ -133,7 +140,14 @@ def _act_buffer(x: torch.Tensor, stream) -> MxTensor:
 def _one_rank(comm, a: torch.Tensor, w, out: Optional[torch.Tensor], stream) -> torch.Tensor:
     """The three operators on one rank with activations in bf16: the product alone, quantisation in the same call."""
     _check_quantizable(a)
-    buf, w = _act_buffer(a, stream), _as_mx_fresh(w, stream)
+    w = _as_mx_fresh(w, stream)
+    n = _native()
+    if n is not None:
+        rc, out = n.mx_matmul(comm.handle, a, w.payload, w.scales, w.rows, out, None if stream is None else stream.cuda_stream)
+        if rc:
+            check(rc, "HcclQuantizeMatmulMxfp8")
+        return out
+    buf = _act_buffer(a, stream)
     m, k = a.shape
     if out is None:
         out = torch.empty((m, w.rows), dtype=torch.bfloat16, device=a.device)

@@ -169,3 +169,32 @@ def test_one_rank_operators_quantise_in_the_call(m, n, k):
             assert torch.equal(out, refs[i % 3])
     finally:
         comm.destroy()
+
+
+def test_one_rank_calls_keep_their_activations_apart():
+    """Calls of one shape on two streams and from two threads, back to back: every one has its own quantised activations. Whole bytes and one kernel, so the results are
+    those of a call by itself."""
+    import threading
+
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops import mxfp8
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        w = mxfp8.quantize(torch.randn(1024, 512, device="cuda").to(torch.bfloat16))
+        xs = [torch.randn(48, 512, device="cuda").to(torch.bfloat16) for _ in range(16)]
+        want = [mxfp8.gemm(mxfp8.quantize(x), w) for x in xs]
+        torch.cuda.synchronize()
+        streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], [None] * 16
+
+        def calls(part):
+            for i in range(part, 16, 2):
+                with torch.cuda.stream(streams[i // 2 % 2]):
+                    got[i] = mxfp8.matmul_all_reduce(comm, xs[i], w, stream=streams[i // 4 % 2] if i % 3 == 0 else None)
+
+        threads = [threading.Thread(target=calls, args=(p,)) for p in range(2)]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    finally:
+        comm.destroy()
