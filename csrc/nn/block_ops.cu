@@ -33,6 +33,17 @@ __device__ __forceinline__ uint4 Pack8(const float (&f)[8])
     return o;
 }
 
+// a + b, each sum rounded to bf16
+__device__ __forceinline__ uint4 Add8(const uint4 &a, const uint4 &b)
+{
+    float f[8], g[8];
+    Unpack8(a, f);
+    Unpack8(b, g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] += g[j];
+    return Pack8(f);
+}
+
 // Sum over the TPR threads that share a row: a warp (TPR = 32) or the whole block.
 template <int TPR> __device__ __forceinline__ float RowSum(float v, float *red)
 {
@@ -50,18 +61,19 @@ template <int TPR> __device__ __forceinline__ float RowSum(float v, float *red)
 
 // y = x * rsqrt(mean(x^2) + eps) * w. A row is shared by TPR threads. Up to two vectors per thread (NV) stay in registers between the sum and the
 // result; wider rows (NV = 0) are read again from L1 / L2, which leaves the registers to more rows in flight. KEEP: x and w are copied on the
-// way for a backward pass that may come after they were changed. Bound by memory: 2048 x 4096 with copies (48 MB) on one B200 14.3 us from a cold L2,
+// way for a backward pass that may come after they were changed. ADD: the row is x + d, rounded to bf16 as an addition by itself rounds it, and its copy is
+// the sum (the residual stream of a decoder goes on with it). Bound by memory: 2048 x 4096 with copies (48 MB) on one B200 14.3 us from a cold L2,
 // 16.4 with a second load of the row; 1000 x 8192 without copies 12.3 with it, 14.2 from registers.
-template <int TPR, int NV, bool KEEP>
-__global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ y,
-                                                         float *__restrict__ rstd, __nv_bfloat16 *__restrict__ xKept, __nv_bfloat16 *__restrict__ wKept, uint32_t T,
+template <int TPR, int NV, bool KEEP, bool ADD = false>
+__global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ d, const __nv_bfloat16 *__restrict__ w,
+                                                         __nv_bfloat16 *__restrict__ y, float *__restrict__ rstd, __nv_bfloat16 *xKept, __nv_bfloat16 *__restrict__ wKept, uint32_t T,
                                                          uint32_t H, float eps)
 {
     __shared__ float red[kThreads / 32];
     const uint32_t row = blockIdx.x * (kThreads / TPR) + threadIdx.x / TPR, lane = threadIdx.x % TPR;
     if (row >= T) return;                                // whole warps (TPR = 32) or no thread at all (one row per block)
-    const uint4 *xr = (const uint4 *)(x + (size_t)row * H), *wr = (const uint4 *)w;
-    uint4 xv[NV ? NV : 1];
+    const uint4 *xr = (const uint4 *)(x + (size_t)row * H), *dr = (const uint4 *)(d + (size_t)row * H), *wr = (const uint4 *)w;
+    uint4 xv[NV ? NV : 1], dv[NV ? NV : 1];
     float s = 0.f;
     auto square = [&](uint32_t v, const uint4 &raw) {
         if (KEEP) ((uint4 *)(xKept + (size_t)row * H))[v] = raw;
@@ -72,12 +84,20 @@ __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *_
     };
     if (NV) {
 #pragma unroll
-        for (int i = 0; i < NV; ++i) if (lane + i * TPR < H / 8) xv[i] = xr[lane + i * TPR];
+        for (int i = 0; i < NV; ++i)
+            if (lane + i * TPR < H / 8) {
+                xv[i] = xr[lane + i * TPR];
+                if (ADD) dv[i] = dr[lane + i * TPR];
+            }
 #pragma unroll
-        for (int i = 0; i < NV; ++i) if (lane + i * TPR < H / 8) square(lane + i * TPR, xv[i]);
+        for (int i = 0; i < NV; ++i)
+            if (lane + i * TPR < H / 8) {
+                if (ADD) xv[i] = Add8(xv[i], dv[i]);
+                square(lane + i * TPR, xv[i]);
+            }
     } else {
         for (uint32_t v = lane; v < H / 8; v += TPR) {
-            const uint4 raw = xr[v];                     // a value: 9000 x 8192 without copies 45.4 us, 55.6 with a reference to memory handed on
+            const uint4 raw = ADD ? Add8(xr[v], dr[v]) : xr[v];   // a value: 9000 x 8192 without copies 45.4 us, 55.6 with a reference to memory handed on
             square(v, raw);
         }
     }
@@ -86,7 +106,7 @@ __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *_
     uint4 *yr = (uint4 *)(y + (size_t)row * H);
     auto scale = [&](uint32_t v, const uint4 &raw) {
         const uint4 wv = wr[v];
-        if (KEEP && row == 0) ((uint4 *)wKept)[v] = wv;
+        if (KEEP && wKept && row == 0) ((uint4 *)wKept)[v] = wv;
         float f[8], g[8];
         Unpack8(raw, f);
         Unpack8(wv, g);
@@ -99,7 +119,7 @@ __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *_
         for (int i = 0; i < NV; ++i) if (lane + i * TPR < H / 8) scale(lane + i * TPR, xv[i]);
     } else {
         for (uint32_t v = lane; v < H / 8; v += TPR) {
-            const uint4 raw = xr[v];
+            const uint4 raw = ADD ? ((const uint4 *)(xKept + (size_t)row * H))[v] : xr[v];       // its own store of the first pass
             scale(v, raw);
         }
     }
@@ -108,11 +128,11 @@ __global__ void __launch_bounds__(kThreads) RmsNormKernel(const __nv_bfloat16 *_
 // dx = r * (dy * w - xhat * mean(dy * w * xhat)), xhat = x * r; dw = sum over rows of dy * xhat. A thread owns NV vectors of columns of
 // every row its block walks over (with a stride of the grid): x, dy and w of a row are loaded once and stay in registers between the
 // row sum and the result, and so does the thread's part of dw, which goes to partial[block] at the end; the next row is on its way
-// meanwhile. A second kernel adds the blocks in a fixed order: the same bits on every run. 2048 x 4096 on one B200, both kernels from a cold L2:
+// meanwhile. ADD: dx + res, the gradient that reached x by another way, rounded as an addition by itself rounds it. A second kernel adds the blocks in a fixed order: the same bits on every run. 2048 x 4096 on one B200, both kernels from a cold L2:
 // 23.3 us, 31.6 without the early loads, with three blocks per SM and the sums below at one column per thread.
-template <int TPR, int NV>
+template <int TPR, int NV, bool ADD>
 __global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16 *__restrict__ dy, const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
-                                                            const float *__restrict__ rstd, __nv_bfloat16 *__restrict__ dx, float *__restrict__ partial, uint32_t T,
+                                                            const float *__restrict__ rstd, const __nv_bfloat16 *__restrict__ res, __nv_bfloat16 *__restrict__ dx, float *__restrict__ partial, uint32_t T,
                                                             uint32_t H)
 {
     __shared__ float red[kThreads / 32];
@@ -150,6 +170,12 @@ __global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16
         const float r = nr;
 #pragma unroll
         for (int i = 0; i < NV; ++i) { xv[i] = nx[i]; dv[i] = nd[i]; }
+        uint4 rv[NV];
+        if (ADD) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                if (lane + i * TPR < H / 8) rv[i] = ((const uint4 *)(res + (size_t)row * H))[lane + i * TPR];
+        }
         if (kEarly && row + step < T) fetch(row + step);
         float s = 0.f;
 #pragma unroll
@@ -175,7 +201,7 @@ __global__ void __launch_bounds__(kThreads) RmsNormBwdKernel(const __nv_bfloat16
                 f[j] = r * (d[j] * g[j] - xh * m);
                 part[i][j] += d[j] * xh;
             }
-            if (lane + i * TPR < H / 8) o[lane + i * TPR] = Pack8(f);
+            if (lane + i * TPR < H / 8) o[lane + i * TPR] = ADD ? Add8(Pack8(f), rv[i]) : Pack8(f);
         }
     }
     float *out = partial + (size_t)blockIdx.x * H;
@@ -411,9 +437,10 @@ constexpr uint64_t kWarpRowMax = 1024;     // rows up to this wide are handled b
 constexpr uint64_t kNormMax = 12288;       // widest row: six vectors per thread of a block
 
 template <int TPR, int NV>
-void LaunchRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, float *partial, uint32_t T, uint32_t H, uint32_t parts, cudaStream_t s)
+void LaunchRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, const void *res, void *dx, float *partial, uint32_t T, uint32_t H, uint32_t parts, cudaStream_t s)
 {
-    RmsNormBwdKernel<TPR, NV><<<parts, kThreads, 0, s>>>((const __nv_bfloat16 *)dy, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, rstd, (__nv_bfloat16 *)dx, partial, T, H);
+    auto kern = res ? RmsNormBwdKernel<TPR, NV, true> : RmsNormBwdKernel<TPR, NV, false>;
+    kern<<<parts, kThreads, 0, s>>>((const __nv_bfloat16 *)dy, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, rstd, (const __nv_bfloat16 *)res, (__nv_bfloat16 *)dx, partial, T, H);
 }
 
 // 16-byte vectors of a row per thread
@@ -425,24 +452,25 @@ uint32_t NormVecs(uint32_t H)
 
 bool NormShapeOk(uint64_t T, uint64_t H) { return T > 0 && T <= 0x7fffffff && H > 0 && H % 8 == 0 && H <= kNormMax; }
 
-HcclResult LaunchRmsNorm(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
+// d: what is added to x first, or null
+HcclResult LaunchRmsNorm(const void *x, const void *d, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
 {
     if (!x || !w || !y || !rstd) return HCCL_E_PTR;
-    if (!NormShapeOk(rows, hidden) || !Aligned16(x) || !Aligned16(w) || !Aligned16(y) || !Aligned16(xKept) || !Aligned16(wKept)) return HCCL_E_PARA;
+    if (!NormShapeOk(rows, hidden) || !Aligned16(x) || !Aligned16(d) || !Aligned16(w) || !Aligned16(y) || !Aligned16(xKept) || !Aligned16(wKept)) return HCCL_E_PARA;
     const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden;
     const bool warp = hidden <= kWarpRowMax;
-    auto launch = [&](auto plain, auto keep) {
-        auto kern = xKept ? keep : plain;
-        kern<<<warp ? (T + 7) / 8 : T, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd, (__nv_bfloat16 *)xKept,
-                                                             (__nv_bfloat16 *)wKept, T, H, eps);
+    auto launch = [&](auto plain, auto keep, auto add) {
+        auto kern = d ? add : xKept ? keep : plain;
+        kern<<<warp ? (T + 7) / 8 : T, kThreads, 0, stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)d, (const __nv_bfloat16 *)w, (__nv_bfloat16 *)y, rstd,
+                                                             (__nv_bfloat16 *)xKept, (__nv_bfloat16 *)wKept, T, H, eps);
     };
     const uint32_t nv = NormVecs(H);
-    if (warp && nv == 1) launch(RmsNormKernel<32, 1, false>, RmsNormKernel<32, 1, true>);
-    else if (warp && nv == 2) launch(RmsNormKernel<32, 2, false>, RmsNormKernel<32, 2, true>);
-    else if (warp) launch(RmsNormKernel<32, 0, false>, RmsNormKernel<32, 0, true>);
-    else if (nv == 1) launch(RmsNormKernel<kThreads, 1, false>, RmsNormKernel<kThreads, 1, true>);
-    else if (nv == 2) launch(RmsNormKernel<kThreads, 2, false>, RmsNormKernel<kThreads, 2, true>);
-    else launch(RmsNormKernel<kThreads, 0, false>, RmsNormKernel<kThreads, 0, true>);
+    if (warp && nv == 1) launch(RmsNormKernel<32, 1, false>, RmsNormKernel<32, 1, true>, RmsNormKernel<32, 1, true, true>);
+    else if (warp && nv == 2) launch(RmsNormKernel<32, 2, false>, RmsNormKernel<32, 2, true>, RmsNormKernel<32, 2, true, true>);
+    else if (warp) launch(RmsNormKernel<32, 0, false>, RmsNormKernel<32, 0, true>, RmsNormKernel<32, 0, true, true>);
+    else if (nv == 1) launch(RmsNormKernel<kThreads, 1, false>, RmsNormKernel<kThreads, 1, true>, RmsNormKernel<kThreads, 1, true, true>);
+    else if (nv == 2) launch(RmsNormKernel<kThreads, 2, false>, RmsNormKernel<kThreads, 2, true>, RmsNormKernel<kThreads, 2, true, true>);
+    else launch(RmsNormKernel<kThreads, 0, false>, RmsNormKernel<kThreads, 0, true>, RmsNormKernel<kThreads, 0, true, true>);
     return Launched("RMSNorm");
 }
 
@@ -457,13 +485,19 @@ extern "C" {
 
 HcclResult HcclRmsNorm(const void *x, const void *w, void *y, float *rstd, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
 {
-    return LaunchRmsNorm(x, w, y, rstd, nullptr, nullptr, rows, hidden, eps, stream);
+    return LaunchRmsNorm(x, nullptr, w, y, rstd, nullptr, nullptr, rows, hidden, eps, stream);
 }
 
 HcclResult HcclRmsNormKeep(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
 {
     if (!xKept || !wKept) return HCCL_E_PTR;
-    return LaunchRmsNorm(x, w, y, rstd, xKept, wKept, rows, hidden, eps, stream);
+    return LaunchRmsNorm(x, nullptr, w, y, rstd, xKept, wKept, rows, hidden, eps, stream);
+}
+
+HcclResult HcclRmsNormAdd(const void *x, const void *d, const void *w, void *sum, void *y, float *rstd, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream)
+{
+    if (!d || !sum) return HCCL_E_PTR;
+    return LaunchRmsNorm(x, d, w, y, rstd, sum, wKept, rows, hidden, eps, stream);
 }
 
 uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden)
@@ -475,12 +509,18 @@ uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden)
 HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, void *dw, float *partial, uint64_t rows, uint64_t hidden,
                           cudaStream_t stream)
 {
+    return HcclRmsNormBwdAdd(dy, x, w, rstd, nullptr, dx, dw, partial, rows, hidden, stream);
+}
+
+HcclResult HcclRmsNormBwdAdd(const void *dy, const void *x, const void *w, const float *rstd, const void *dSum, void *dx, void *dw, float *partial, uint64_t rows,
+                             uint64_t hidden, cudaStream_t stream)
+{
     if (!dy || !x || !w || !rstd || !dx || !dw || !partial) return HCCL_E_PTR;
-    if (!NormShapeOk(rows, hidden) || !Aligned16(dy) || !Aligned16(x) || !Aligned16(w) || !Aligned16(dx)) return HCCL_E_PARA;
+    if (!NormShapeOk(rows, hidden) || !Aligned16(dy) || !Aligned16(x) || !Aligned16(w) || !Aligned16(dSum) || !Aligned16(dx)) return HCCL_E_PARA;
     const bool vec = Aligned16(partial);                 // rows up to kWarpRowMax are also taken with a workspace that is aligned to its elements alone
     if (((uintptr_t)partial & 3u) || (!vec && hidden > kWarpRowMax)) return HCCL_E_PARA;
     const uint32_t T = (uint32_t)rows, H = (uint32_t)hidden, parts = (uint32_t)HcclRmsNormBwdParts(rows, hidden);
-    auto launch = [&](auto kern) { kern(dy, x, w, rstd, dx, partial, T, H, parts, stream); };
+    auto launch = [&](auto kern) { kern(dy, x, w, rstd, dSum, dx, partial, T, H, parts, stream); };
     const uint32_t nv = NormVecs(H);
     if (hidden <= kWarpRowMax) launch(nv == 1 ? LaunchRmsNormBwd<32, 1> : nv == 2 ? LaunchRmsNormBwd<32, 2> : LaunchRmsNormBwd<32, 4>);
     else launch(nv == 1 ? LaunchRmsNormBwd<kThreads, 1> : nv == 2 ? LaunchRmsNormBwd<kThreads, 2> : nv <= 4 ? LaunchRmsNormBwd<kThreads, 4> : LaunchRmsNormBwd<kThreads, 6>);

@@ -175,55 +175,66 @@ c10::DeviceIndex DeviceOf(const at::Tensor &t) { return t.is_cuda() ? t.device()
 
 // ---- RMSNorm ---------------------------------------------------------------------------------------------------------
 // Outputs y and the copies of x and w that the kernel makes on its way: the backward pass reads the values that the forward pass saw, and the
-// gradient of a gradient finds its way to x and w through them.
+// gradient of a gradient finds its way to x and w through them. With `added` the input is x + d and the copy is that sum. The copy may be used further, as the
+// residual stream of a decoder: the gradient that comes back by it is added in the same kernel.
 struct RmsNormNode : OpNode {
     SavedVariable x, w, rstd;
+    bool added = false;
     std::string name() const override { return "_RmsNormBackward"; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(added); }
+    variable_list Inputs(at::Tensor dx, at::Tensor dw) const { return added ? variable_list{dx, dx, dw} : variable_list{dx, dw}; }
     std::vector<Saved> Keeps() override { return {{&x, true}, {&w, true}, {&rstd, false}}; }
     variable_list Backward(variable_list &&g) override
     {
-        if (!g[0].defined()) return {g[1], g[2]};
+        if (!g[0].defined()) return Inputs(g[1], g[2]);
         const auto [xv, wv, r] = Unpack(x, w, rstd);
         variable_list out(2);
-        bool direct = !traced && !at::GradMode::is_enabled();
+        bool together = false, direct = !traced && !at::GradMode::is_enabled();
         {
             py::gil_scoped_acquire gil;
             if (direct) {
                 const auto dev = DeviceOf(g[0]);
                 direct = !Watched() && PlainGrad(g[0]) && Operand(xv, dev) && Operand(wv, dev) && Floats(r, dev) && xv.sizes() == g[0].sizes() && wv.dim() == 1 &&
                          wv.size(0) == xv.size(-1) && r.numel() * wv.size(0) == xv.numel();
+                together = direct && g[1].defined() && PlainGrad(g[1]) && g[1].device() == g[0].device() && g[1].sizes() == g[0].sizes();
             }
             if (traced) out = FromPython((*g_env.backward)("rms_norm traced", xv, wv, r, g[0]), 2);
             else if (!direct) out = FromPython((*g_env.backward)("rms_norm", held->o, xv, wv, g[0]), 2);
         }
         if (direct) {
-            const at::Tensor dy = Aligned(g[0]);
+            const at::Tensor dy = Aligned(g[0]), past = together ? Aligned(g[1]) : at::Tensor();
             const int64_t h = xv.size(-1), rows = r.numel();
             out[0] = at::empty_like(xv);
             out[1] = at::empty_like(wv);
             const at::Tensor partial = at::empty({(int64_t)HcclRmsNormBwdParts((uint64_t)rows, (uint64_t)h), h}, r.options());
-            Check(HcclRmsNormBwd(dy.data_ptr(), xv.data_ptr(), wv.data_ptr(), r.data_ptr<float>(), out[0].data_ptr(), out[1].data_ptr(), partial.data_ptr<float>(), rows, h,
-                                 Stream(xv)), "HcclRmsNormBwd");
+            Check(HcclRmsNormBwdAdd(dy.data_ptr(), xv.data_ptr(), wv.data_ptr(), r.data_ptr<float>(), together ? past.data_ptr() : nullptr, out[0].data_ptr(), out[1].data_ptr(),
+                                    partial.data_ptr<float>(), rows, h, Stream(xv)), "HcclRmsNormBwdAdd");
         }
-        for (int i = 0; i < 2; ++i)
+        for (int i = together ? 1 : 0; i < 2; ++i)
             if (g[i + 1].defined()) out[i] = out[i].defined() ? out[i] + g[i + 1] : g[i + 1];
-        return out;
+        return Inputs(out[0], out[1]);
     }
 };
 
-py::object RmsNorm(py::handle xh, py::handle wh, double eps, py::object plain)
+bool NormOperands(const at::Tensor &x, const at::Tensor &w)
+{
+    if (!x.defined() || !w.defined() || x.dim() == 0) return false;
+    const int64_t h = x.size(-1);
+    return h % 8 == 0 && h <= 12288 && w.dim() == 1 && w.size(0) == h;
+}
+
+// y; with `kept` (y, the copy of x) where a gradient may be asked for, (y, x) where not
+py::object RmsNorm(py::handle xh, py::handle wh, double eps, py::object plain, bool kept)
 {
     const at::Tensor x = OperandArg(xh), w = OperandArg(wh);
-    if (!x.defined() || !w.defined() || x.dim() == 0) return py::none();
+    if (!NormOperands(x, w)) return py::none();
     const int64_t h = x.size(-1);
-    if (h % 8 || h > 12288 || w.dim() != 1 || w.size(0) != h) return py::none();
-    at::Tensor y;
+    at::Tensor y, rstd, xk, wk;
+    const bool wanted = OpNode::Wanted({x, w});
     {
-        const bool wanted = OpNode::Wanted({x, w});
         auto node = wanted ? MakeNode<RmsNormNode>(std::move(plain), x, w) : nullptr;
         py::gil_scoped_release nogil;
         const uint64_t rows = (uint64_t)(x.numel() / h);
-        at::Tensor rstd, xk, wk;
         {
             at::NoGradGuard noGrad;
             y = at::empty_like(x);
@@ -244,7 +255,41 @@ py::object RmsNorm(py::handle xh, py::handle wh, double eps, py::object plain)
             node->rstd = SavedVariable(rstd, false);
         }
     }
-    return py::cast(y);
+    if (!kept) return py::cast(y);
+    return py::make_tuple(y, wanted ? py::cast(xk) : py::reinterpret_borrow<py::object>(xh));
+}
+
+// (the norm of x + d, x + d)
+py::object RmsNormAdd(py::handle xh, py::handle dh, py::handle wh, double eps, py::object plain)
+{
+    const at::Tensor x = OperandArg(xh), d = OperandArg(dh), w = OperandArg(wh);
+    if (!NormOperands(x, w) || !d.defined() || x.sizes() != d.sizes()) return py::none();
+    const int64_t h = x.size(-1);
+    at::Tensor y, sum;
+    {
+        const bool wanted = OpNode::Wanted({x, d, w});
+        auto node = wanted ? MakeNode<RmsNormNode>(std::move(plain), x, d, w) : nullptr;
+        py::gil_scoped_release nogil;
+        const uint64_t rows = (uint64_t)(x.numel() / h);
+        at::Tensor rstd, wk;
+        {
+            at::NoGradGuard noGrad;
+            y = at::empty_like(x);
+            sum = at::empty_like(x);
+            rstd = at::empty({(int64_t)rows}, x.options().dtype(at::kFloat));
+            if (wanted) wk = at::empty_like(w);
+            Check(HcclRmsNormAdd(x.data_ptr(), d.data_ptr(), w.data_ptr(), sum.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(), wanted ? wk.data_ptr() : nullptr, rows, h,
+                                 (float)eps, Stream(x)), "HcclRmsNormAdd");
+        }
+        if (wanted) {
+            torch::autograd::set_history({y, sum, wk}, node);
+            node->added = true;
+            node->x = SavedVariable(sum, true);
+            node->w = SavedVariable(wk, true);
+            node->rstd = SavedVariable(rstd, false);
+        }
+    }
+    return py::make_tuple(y, sum);
 }
 
 // ---- rotary embedding --------------------------------------------------------------------------------------------------
@@ -362,7 +407,7 @@ py::object SwiGlu(py::handle guh, py::object plain)
 }
 
 // ---- linear layers of one rank -------------------------------------------------------------------------------------------
-// y = x @ w^T. The column-parallel layer keeps the gathered activations, on one rank a copy of x; the row-parallel one keeps x.
+// y = x @ w^T. The column-parallel layer keeps the gathered activations, on one rank a copy of x unless the caller gives x away; the row-parallel one keeps x.
 struct LinearNode : OpNode {
     SavedVariable x, w;
     std::vector<int64_t> shape;
@@ -393,13 +438,14 @@ struct LinearNode : OpNode {
     }
 };
 
-// column: all_gather_matmul, else matmul_reduce_scatter; `comm` is the communicator (one rank) and `handle` its address
-py::object Linear(py::handle xh, py::handle wh, py::object comm, uint64_t handle, bool column)
+// column: all_gather_matmul, else matmul_reduce_scatter; `comm` is the communicator (one rank) and `handle` its address. own: nobody else has x, so the
+// column-parallel layer needs no copy of it. Any number of rows: one rank has no tiles to agree on with others.
+py::object Linear(py::handle xh, py::handle wh, py::object comm, uint64_t handle, bool column, bool own)
 {
     const at::Tensor x = OperandArg(xh), w = OperandArg(wh);
     if (!x.defined() || !w.defined() || x.dim() != 2 || w.dim() != 2) return py::none();
     const int64_t m = x.size(0), k = x.size(1), n = w.size(0);
-    if (w.size(1) != k || m % 128 || m > 8192 || k % 8 || n % 8) return py::none();
+    if (w.size(1) != k || k % 8 || n % 8) return py::none();
     at::Tensor y;
     {
         const bool wanted = OpNode::Wanted({x, w});
@@ -411,15 +457,15 @@ py::object Linear(py::handle xh, py::handle wh, py::object comm, uint64_t handle
             y = at::empty({m, n}, x.options());
             HcclComm c = (HcclComm)(uintptr_t)handle;
             if (column) {
-                gathered = at::empty({m, k}, x.options());
-                Check(HcclAllGatherMatmul(x.data_ptr(), w.data_ptr(), y.data_ptr(), gathered.data_ptr(), m, n, k, HCCL_DATA_TYPE_BFP16, c, Stream(x)), "HcclAllGatherMatmul");
+                if (wanted && !own) gathered = at::empty({m, k}, x.options());
+                Check(HcclAllGatherMatmul(x.data_ptr(), w.data_ptr(), y.data_ptr(), gathered.defined() ? gathered.data_ptr() : nullptr, m, n, k, HCCL_DATA_TYPE_BFP16, c, Stream(x)), "HcclAllGatherMatmul");
             } else {
                 Check(HcclMatmulReduceScatter(x.data_ptr(), w.data_ptr(), y.data_ptr(), m, n, k, HCCL_DATA_TYPE_BFP16, c, Stream(x)), "HcclMatmulReduceScatter");
             }
         }
         if (wanted) {
             node->column = column;
-            node->x = SavedVariable(column ? gathered : x, false);
+            node->x = SavedVariable(gathered.defined() ? gathered : x, false);
             node->w = SavedVariable(w, false);
             node->shape = y.sizes().vec();
             node->options = y.options();
@@ -512,6 +558,7 @@ void BindBlockOps(py::module &m)
     m.def("set_native_gemm", [](bool v) { g_nativeGemm = v; });
     m.def("set_native_wgrad", [](bool v) { g_nativeWgrad = v; });
     m.def("rms_norm", &RmsNorm);
+    m.def("rms_norm_add", &RmsNormAdd);
     m.def("rope_qkv", &RopeQkv);
     m.def("swiglu", &SwiGlu);
     m.def("linear", &Linear);

@@ -20,7 +20,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import block as _block
-from ..parallel.tensor_parallel import ColumnParallelLinear, RowParallelLinear, TensorParallelMLP
+from ..parallel.tensor_parallel import ColumnParallelLinear, RowParallelLinear, TensorParallelMLP, column_of_own, mlp_of_own
 
 
 @dataclass
@@ -75,6 +75,20 @@ class RMSNorm(nn.Module):
         return _plain_rms_norm(x, w, self.eps)
 
 
+_NORM_FORWARD = RMSNorm.forward
+
+
+def _normed(norm, x, d=None):
+    """(norm of x, x), or (norm of x + d, x + d), and whether the norm is nobody else's; in one kernel where the module is nothing but a norm."""
+    if _block.native_nodes(x) is not None and _block.bare(norm, RMSNorm, _NORM_FORWARD):
+        plain = functools.partial(_plain_rms_norm, eps=norm.eps)
+        out = _block.rms_norm_kept(x, norm.weight, norm.eps, plain) if d is None else _block.rms_norm_add(x, d, norm.weight, norm.eps, plain)
+        if out is not None:
+            return *out, True
+    x = x if d is None else x + d
+    return norm(x), x, False
+
+
 def _plain_rms_norm(x, w, eps: float):
     v = x.float()
     v = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + eps)
@@ -118,7 +132,10 @@ class Attention(nn.Module):
                 self.qkv.weight.copy_(torch.cat(parts).to(self.qkv.weight.device))
 
     def forward(self, x_local, batch: int, seq: int, cos, sin):
-        qkv = self.qkv(x_local)                                            # [B*S, (hl + 2 kvl) * hd]
+        return self._forward(x_local, batch, seq, cos, sin, False)
+
+    def _forward(self, x_local, batch: int, seq: int, cos, sin, own: bool):
+        qkv = column_of_own(self.qkv, x_local) if own else self.qkv(x_local)                                    # [B*S, (hl + 2 kvl) * hd]
         plain = functools.partial(_rotated, batch=batch, seq=seq, heads=self.h_local, kv_heads=self.kv_local, hd=self.hd, cos=cos, sin=sin)
         out = _block.rope_qkv(qkv, cos, sin, batch, self.h_local, self.kv_local, self.hd, plain)
         q, k, v = (t.transpose(1, 2) for t in (plain(qkv) if out is None else out))
@@ -128,6 +145,9 @@ class Attention(nn.Module):
 
     def _rotated(self, qkv, batch, seq, cos, sin):
         return _rotated(qkv, batch, seq, self.h_local, self.kv_local, self.hd, cos, sin)
+
+
+_ATTENTION_FORWARD = Attention.forward
 
 
 def _rotated(qkv, batch, seq, heads, kv_heads, hd, cos, sin):
@@ -146,8 +166,13 @@ class Block(nn.Module):
         self.mlp = TensorParallelMLP(comm, cfg.hidden, cfg.ffn, dtype=dtype, device=device, seed=seed + 10 if seed is not None else None)
 
     def forward(self, x_local, batch, seq, cos, sin):
-        x_local = x_local + self.attn(self.attn_norm(x_local), batch, seq, cos, sin)
-        return x_local + self.mlp(self.mlp_norm(x_local))
+        y, x_local, own = _normed(self.attn_norm, x_local)
+        if own and _block.bare(self.attn, Attention, _ATTENTION_FORWARD):
+            h = self.attn._forward(y, batch, seq, cos, sin, True)
+        else:
+            h = self.attn(y, batch, seq, cos, sin)
+        y, x_local, own = _normed(self.mlp_norm, x_local, h)
+        return x_local + (mlp_of_own(self.mlp, y) if own else self.mlp(y))
 
 
 def _owned(targets, vocab_start, vloc):
@@ -270,7 +295,8 @@ class Llama(nn.Module):
         cos, sin = self._rope
         for blk in self.blocks:
             x = blk(x, B, S, cos, sin)
-        logits = self.lm_head(self.norm(x))                                # [T, vocab / tp]
+        y, _, own = _normed(self.norm, x)
+        logits = column_of_own(self.lm_head, y) if own else self.lm_head(y)                                     # [T, vocab / tp]
         if targets is None:
             return logits
         vloc = self.cfg.vocab_size // tp

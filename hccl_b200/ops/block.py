@@ -48,6 +48,7 @@ def _stream(t: torch.Tensor) -> int:
 # bound once: every forward and backward pass of a small model goes through the checks below
 _transforms, _modes, _forward_ad = torch._C._functorch.peek_interpreter_stack, torch._C._len_torch_dispatch_stack, torch.autograd.forward_ad
 _has_storage, _BF16 = torch._C._has_storage, torch.bfloat16
+_any_global_hook = torch.nn.modules.module._has_any_global_hook
 
 
 def _watched() -> bool:
@@ -210,7 +211,7 @@ def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> O
     the graph does."""
     n = native_nodes(x)
     if n is not None:
-        return n.rms_norm(x, w, eps, plain)
+        return n.rms_norm(x, w, eps, plain, False)
     if not _usable(x, w):
         return None
     h = x.shape[-1] if x.dim() else 0
@@ -221,6 +222,25 @@ def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable) -> O
     y, rstd = torch.empty_like(x), torch.empty(x.numel() // h, dtype=torch.float32, device=x.device)
     check(_decl().HcclRmsNorm(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), rstd.numel(), h, eps, _stream(x)), "HcclRmsNorm")
     return y
+
+
+def rms_norm_kept(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable):
+    """(norm of x, x as the residual stream goes on with it): the second is the copy that the norm makes for its backward pass, which then adds the gradient of both
+    uses in one kernel. None without the native nodes."""
+    n = native_nodes(x)
+    return None if n is None else n.rms_norm(x, w, eps, plain, True)
+
+
+def rms_norm_add(x: torch.Tensor, d: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable):
+    """(norm of x + d, x + d), the bits of the two operations one after the other. None without the native nodes."""
+    n = native_nodes(x)
+    return None if n is None else n.rms_norm_add(x, d, w, eps, plain)
+
+
+def bare(module: torch.nn.Module, cls: type, forward: Callable) -> bool:
+    """Whether calling the module does what `forward` of its class says and nothing else: no subclass, no replaced method, no hook of its own or of all modules."""
+    return type(module) is cls and cls.forward is forward and "forward" not in module.__dict__ and module._compiled_call_impl is None and not (
+        module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks or _any_global_hook())
 
 
 class _RopeQkv(torch.autograd.Function):

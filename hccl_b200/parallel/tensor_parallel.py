@@ -174,12 +174,13 @@ _block.PYTHON_BACKWARD["column"] = _one_rank_backward(_column_backward)
 _block.PYTHON_BACKWARD["row"] = _one_rank_backward(_row_backward)
 
 
-def _one_rank_linear(x: torch.Tensor, w: torch.Tensor, comm, column: bool):
-    """The sequence-parallel layer of one rank as one native node (the same kernels), or None where it does not apply."""
+def _one_rank_linear(x: torch.Tensor, w: torch.Tensor, comm, column: bool, own: bool = False):
+    """The sequence-parallel layer of one rank as one native node (the same kernels), or None where it does not apply. own: nobody else has x or will
+    change it, so the layer may keep it as it is."""
     if comm.size != 1 or not _NATIVE_GEMM or not getattr(comm, "fused", True):
         return None
     n = _block.native_nodes(x)
-    return None if n is None else n.linear(x, w, comm, comm.handle, column)
+    return None if n is None else n.linear(x, w, comm, comm.handle, column, own)
 
 
 class _RowAllReduce(torch.autograd.Function):
@@ -236,11 +237,22 @@ class ColumnParallelLinear(nn.Module):
         self.weight = nn.Parameter(w)
 
     def forward(self, x):
+        return self._forward(x, False)
+
+    def _forward(self, x, own: bool):
         lead, x2 = x.shape[:-1], _rows(x, self.in_features)
         if self.sequence_parallel:
-            y = _one_rank_linear(x2, self.weight, self.comm, True)
+            y = _one_rank_linear(x2, self.weight, self.comm, True, own)
             return _ColumnSeqParallel.apply(x2, self.weight, self.comm) if y is None else y
         return _ColumnReplicatedInput.apply(x2, self.weight, self.comm).reshape(*lead, -1)
+
+
+_COLUMN_FORWARD = ColumnParallelLinear.forward
+
+
+def column_of_own(layer: nn.Module, x: torch.Tensor) -> torch.Tensor:
+    """layer(x) for an x that the caller has made, gives to nobody else and does not change."""
+    return layer._forward(x, True) if _block.bare(layer, ColumnParallelLinear, _COLUMN_FORWARD) else layer(x)
 
 
 class RowParallelLinear(nn.Module):
@@ -297,9 +309,20 @@ class TensorParallelMLP(nn.Module):
                 self.gate_up.weight.copy_(torch.cat([g, u]).to(self.gate_up.weight.device))
 
     def forward(self, x_local):
-        gu = self.gate_up(x_local)
+        return self._forward(x_local, False)
+
+    def _forward(self, x_local, own: bool):
+        gu = column_of_own(self.gate_up, x_local) if own else self.gate_up(x_local)
         h = _block.swiglu(gu, _plain_swiglu)
         return self.down(_plain_swiglu(gu) if h is None else h)
+
+
+_MLP_FORWARD = TensorParallelMLP.forward
+
+
+def mlp_of_own(mlp: nn.Module, x_local: torch.Tensor) -> torch.Tensor:
+    """mlp(x_local), as `column_of_own`."""
+    return mlp._forward(x_local, True) if _block.bare(mlp, TensorParallelMLP, _MLP_FORWARD) else mlp(x_local)
 
 
 def _plain_swiglu(gu):

@@ -16,10 +16,15 @@ extern "C" {
 HcclResult HcclRmsNorm(const void *x, const void *w, void *y, float *rstd, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
 /* The same, and copies of x and w: what the backward pass reads where x or w may be changed in between. */
 HcclResult HcclRmsNormKeep(const void *x, const void *w, void *y, float *rstd, void *xKept, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
+/* sum = x + d, and the norm of that sum; wKept may be null. */
+HcclResult HcclRmsNormAdd(const void *x, const void *d, const void *w, void *sum, void *y, float *rstd, void *wKept, uint64_t rows, uint64_t hidden, float eps, cudaStream_t stream);
 /* Rows of the fp32 workspace `partial` [parts, hidden] that HcclRmsNormBwd needs. Up to 1024 columns it may also be aligned to 4 bytes alone. */
 uint64_t HcclRmsNormBwdParts(uint64_t rows, uint64_t hidden);
 HcclResult HcclRmsNormBwd(const void *dy, const void *x, const void *w, const float *rstd, void *dx, void *dw, float *partial, uint64_t rows, uint64_t hidden,
                           cudaStream_t stream);
+/* The same with dSum[rows, hidden] added to dx: the gradient that reached x (the sum) past the norm. Null: nothing is added. */
+HcclResult HcclRmsNormBwdAdd(const void *dy, const void *x, const void *w, const float *rstd, const void *dSum, void *dx, void *dw, float *partial, uint64_t rows,
+                             uint64_t hidden, cudaStream_t stream);
 /* qkv[tokens, (qHeads + 2 kvHeads) * headDim] -> q, k rotated (pairs are element j and j + headDim / 2) and v, each
  * [tokens, heads, headDim]; cos / sin: fp32 [seq, headDim / 2], token t takes row t % seq. headDim: a multiple of 16.
  * backward != 0: gradients of q, k, v -> gradient of qkv. */

@@ -430,3 +430,103 @@ def test_native_nodes_keep_the_engine_s_rules():
         assert gone() is None
     finally:
         comm.destroy()
+
+
+def _plain_modules(monkeypatch):
+    """The decoder's norms one operation after the other: what the fused ones have to give, bit for bit."""
+    from hccl_b200.models import llama
+    monkeypatch.setattr(llama, "_normed", lambda norm, x, d=None: ((lambda s: (norm(s), s, False))(x if d is None else x + d)))
+
+
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (9, 264), (300, 1024), (7, 1032), (600, 4096), (5, 4104), (3, 12288)])
+def test_norm_of_a_sum(rows, hidden):
+    """The sum, its norm and the gradients of both, in every width of the kernels: the bits of the addition and the norm one after the other."""
+    from torch._dynamo import compiled_autograd
+    from hccl_b200.models.llama import RMSNorm, _normed
+    _native_nodes()
+    torch._dynamo.reset()                                    # a trace for one row is not one for several
+    compiled_autograd.reset()
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    norm = RMSNorm(hidden, 1e-5, torch.bfloat16, "cuda")
+    with torch.no_grad():
+        norm.weight.copy_(torch.randn(hidden, generator=g, device="cuda"))
+    x, d = [torch.randn(rows, hidden, generator=g, device="cuda").to(torch.bfloat16).requires_grad_() for _ in range(2)]
+    ups = [torch.randn(rows, hidden, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    for add in (None, d):
+        ins = [x, norm.weight] if add is None else [x, d, norm.weight]
+        y, s, own = _normed(norm, x, add)
+        assert own and _is_native(y)
+        ref_s = x * 1 if add is None else x + d
+        ref_y = norm(ref_s)
+        assert torch.equal(y, ref_y) and torch.equal(s, ref_s)
+        for outs, refs, grads in (((y, s), (ref_y, ref_s), ups), ((y,), (ref_y,), ups[:1]), ((s,), (ref_s,), ups[1:])):
+            got = torch.autograd.grad(outs, ins, grads, retain_graph=True, allow_unused=True)
+            ref = torch.autograd.grad(refs, ins, grads, retain_graph=True, allow_unused=True)
+            for a, b in zip(got, ref):
+                assert (a is None) == (b is None) and (a is None or torch.equal(a, b))
+        first = torch.autograd.grad((y, s), ins, ups, create_graph=True)
+        ref1 = torch.autograd.grad((ref_y, ref_s), ins, ups, create_graph=True)
+        for a, b in zip(torch.autograd.grad(sum(t.float().square().sum() for t in first), ins), torch.autograd.grad(sum(t.float().square().sum() for t in ref1), ins)):
+            assert (a.double() - b.double()).norm() <= 2.0 ** -6 * b.double().norm()
+        with compiled_autograd._enable(torch.compile(backend="eager")):        # the traced form keeps 32 bits where the kernel rounds
+            torch.autograd.backward(_normed(norm, x, add)[:2], ups)
+        ref_s = x * 1 if add is None else x + d
+        ref_y = norm(ref_s)
+        for t, b in zip(ins, torch.autograd.grad((ref_y, ref_s), ins, ups)):
+            assert (t.grad.double() - b.double()).norm() <= 2.0 ** -6 * b.double().norm()
+            t.grad = None
+        with torch.no_grad():
+            y, s, _ = _normed(norm, x, add)
+            assert torch.equal(y, ref_y) and torch.equal(s, ref_s)
+
+
+@pytest.mark.parametrize("tokens", [(2, 128), (3, 37), (1, 1)])
+def test_block_with_fused_norms_gives_the_bits_of_the_modules(tokens, monkeypatch):
+    """Loss and gradients of a decoder with and without the fused residual additions; saved tensors on the CPU, hooks on the modules (which are all seen)."""
+    _native_nodes()
+    comm, model = _tiny()
+    try:
+        t = torch.randint(0, 512, (tokens[0], tokens[1] + 1), device="cuda")
+        params = list(model.parameters())
+
+        def step():
+            loss = model(t[:, :-1].contiguous(), t[:, 1:].contiguous())
+            return [loss.detach(), *torch.autograd.grad(loss, params)]
+
+        fused = step()
+        with torch.autograd.graph.save_on_cpu():
+            loss = model(t[:, :-1].contiguous(), t[:, 1:].contiguous())
+        for a, b in zip(torch.autograd.grad(loss, params), fused[1:]):
+            assert torch.equal(a, b)
+        seen = []
+        handles = [m.register_forward_hook(lambda m, i, o: seen.append(m)) for m in model.modules() if m is not model]
+        hooked = step()
+        [h.remove() for h in handles]
+        assert len(seen) == len(list(model.modules())) - 2                      # but for the model and its list of blocks
+        _plain_modules(monkeypatch)
+        plain = step()
+        for a, b, c in zip(fused, hooked, plain):
+            assert torch.equal(a, c) and torch.equal(b, c)
+    finally:
+        comm.destroy()
+
+
+def test_block_input_may_change_after_the_pass():
+    """The block's input, which its caller may write afterwards, is not what the backward pass reads."""
+    from hccl_b200.models.llama import _rope_tables
+    comm, model = _tiny()
+    try:
+        leaf = torch.randn(256, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+        up = torch.randn(256, 256, device="cuda").to(torch.bfloat16)
+
+        def grads(change):
+            x = leaf * 1
+            out = model.blocks[0](x, 2, 128, *_rope_tables(128, 32, 500000.0, "cuda"))
+            if change:
+                x.zero_()
+            return torch.autograd.grad(out, [leaf, *model.blocks[0].parameters()], up)
+
+        for a, b in zip(grads(False), grads(True)):
+            assert torch.equal(a, b)
+    finally:
+        comm.destroy()
