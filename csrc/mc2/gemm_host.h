@@ -19,6 +19,7 @@ HcclResult EncodeTmapSf(CUtensorMap *out, const void *scales, uint64_t atoms);
 uint32_t *GemmErrorWord();      // device word shared by all GEMM launches of this process (per device)
 HcclResult GemmCheckError();    // reads it back (synchronous; tests only)
 int SmCount();
+bool Gemm2CtaEnabled();         // HCCL_GEMM_2CTA
 
 }  // namespace mc2
 }  // namespace hccl

@@ -109,5 +109,27 @@ inline PlainChoice ChoosePlain(uint64_t m, uint64_t n, uint64_t k, uint64_t sms,
     return {m <= 64 ? SplitKChoice{} : ChooseSplitK(m, n, k, false, narrow >= 90 && narrow <= sms), t};
 }
 
+// Pair tile width of the product with SwiGLU in its epilogue (forward: half of it gate, half up; backward: columns of the intermediate gradient), 0 = the product and the
+// element-wise kernel one after the other. Forward: wherever the plain product would not split K (few rows, bound by reading the weights); us separate / fused 60 x 2 x 512
+// x 256 5.5 / 5.2, 200 x 2 x 14336 x 4096 61.2 / 60.9, 300 x 2 x 3584 x 1024 11.5 / 12.2. Backward: above 512 rows (777 x 14336 x 4096 135 / 126, 513 x 2056 x 1032 14.1 / 13.7); up to there
+// one-CTA tiles fill the GPU better: 300 x 7168 x 2048 22.8 / 24.2, 130 x 14336 x 4096 37.0 / 40.1, 256 x 512 x 256 6.3 / 8.5.
+inline uint32_t ChooseSwiGlu(uint64_t m, uint64_t ffn, uint64_t k, bool backward, uint64_t sms, bool pairsEnabled)
+{
+    if (!pairsEnabled || (backward ? m <= 512 : ChoosePlain(m, 2 * ffn, k, sms, true).splitK.split != 0)) return 0;
+    const uint64_t pairs = sms / 2, rowPairs = (m + 255) / 256;
+    const double k4 = (double)k / 4096;
+    uint32_t best = 0;
+    double cost = 0;
+    auto offer = [&](uint32_t bn) {
+        const uint64_t cols = backward ? bn : bn / 2, tiles = rowPairs * ((ffn + cols - 1) / cols);
+        const double whole = (double)((tiles + pairs - 1) / pairs), c = (0.7 * whole + 0.3 * std::max(1.0, (double)tiles / (double)pairs)) * (k4 * (bn + 45) + 20);
+        if (!best || c <= cost) { best = bn; cost = c; }
+    };
+    offer(128);
+    if (!backward) { offer(192); offer(224); }
+    offer(256);
+    return best;
+}
+
 }  // namespace mc2
 }  // namespace hccl

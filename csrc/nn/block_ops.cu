@@ -10,6 +10,7 @@
 #include "../common/launch_count.h"
 #include "../common/log.h"
 #include "hccl/hccl_nn.h"
+#include "swiglu.cuh"
 
 namespace hccl {
 namespace nn {
@@ -17,21 +18,6 @@ namespace nn {
 namespace {
 
 constexpr int kThreads = 256;
-
-__device__ __forceinline__ void Unpack8(const uint4 &r, float (&f)[8])
-{
-    const __nv_bfloat162 *h = (const __nv_bfloat162 *)&r;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { const float2 p = __bfloat1622float2(h[j]); f[2 * j] = p.x; f[2 * j + 1] = p.y; }
-}
-__device__ __forceinline__ uint4 Pack8(const float (&f)[8])
-{
-    uint4 o;
-    __nv_bfloat162 t0 = __floats2bfloat162_rn(f[0], f[1]), t1 = __floats2bfloat162_rn(f[2], f[3]);
-    __nv_bfloat162 t2 = __floats2bfloat162_rn(f[4], f[5]), t3 = __floats2bfloat162_rn(f[6], f[7]);
-    o.x = *(uint32_t *)&t0; o.y = *(uint32_t *)&t1; o.z = *(uint32_t *)&t2; o.w = *(uint32_t *)&t3;
-    return o;
-}
 
 // a + b, each sum rounded to bf16
 __device__ __forceinline__ uint4 Add8(const uint4 &a, const uint4 &b)
@@ -296,10 +282,8 @@ __global__ void __launch_bounds__(kThreads) RopeQkvKernel(__nv_bfloat16 *__restr
     *(uint4 *)(dst + half) = Pack8(o2);
 }
 
-// gu = [T, 2F] (gate | up): h = silu(gate) * up. silu is rounded to bf16 before the product, as two separate operations round it: the
-// forward pass keeps the bits of the plain form. The product of two bf16 values is exact in 32 bits, so a packed multiplication rounds it
-// the same way. What bounds it is instructions: 2048 x 14336 on one B200 from a cold L2 38.9 us, 48.1 with index divisions in 64 bits and the products in
-// 32 (memory alone 27); 4096 x 28672 131, 166. Index is 64 bits wide where the vectors need it.
+// gu = [T, 2F] (gate | up): h = silu(gate) * up, the bits of the plain form. What bounds it is instructions: 2048 x 14336 on one B200 33.1 us, 35.1 with a general division per value (memory
+// alone 27); 4096 x 28672 120, 131. Index divisions in 64 bits cost another fifth. Index is 64 bits wide where the vectors need it.
 template <class Index>
 __global__ void __launch_bounds__(kThreads) SwiGluKernel(const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ h, uint64_t vecs, uint32_t F)
 {
@@ -309,16 +293,7 @@ __global__ void __launch_bounds__(kThreads) SwiGluKernel(const __nv_bfloat16 *__
     const Index t = idx / per, j = idx - t * per;
     const uint4 *row = (const uint4 *)gu + (uint64_t)t * 2 * per;
     const uint4 gv = row[j], uv = row[per + j];
-    float g[8];
-    Unpack8(gv, g);
-    const __nv_bfloat162 *u = (const __nv_bfloat162 *)&uv;
-    uint4 o;
-    __nv_bfloat162 *ov = (__nv_bfloat162 *)&o;
-#pragma unroll
-    for (int x = 0; x < 8; ++x) g[x] = g[x] / (1.f + expf(-g[x]));
-#pragma unroll
-    for (int x = 0; x < 4; ++x) ov[x] = __hmul2_rn(__floats2bfloat162_rn(g[2 * x], g[2 * x + 1]), u[x]);
-    ((uint4 *)h)[idx] = o;
+    ((uint4 *)h)[idx] = SwiGlu8(gv, uv);
 }
 
 __global__ void __launch_bounds__(kThreads) SwiGluBwdKernel(const __nv_bfloat16 *__restrict__ dh, const __nv_bfloat16 *__restrict__ gu, __nv_bfloat16 *__restrict__ dgu,
@@ -330,19 +305,7 @@ __global__ void __launch_bounds__(kThreads) SwiGluBwdKernel(const __nv_bfloat16 
     const uint64_t t = idx / per, j = idx % per;
     const uint4 *row = (const uint4 *)(gu + t * 2 * F);
     uint4 *out = (uint4 *)(dgu + t * 2 * F);
-    float g[8], u[8], d[8];
-    Unpack8(row[j], g);
-    Unpack8(row[per + j], u);
-    Unpack8(((const uint4 *)dh)[idx], d);
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        const float sg = 1.f / (1.f + expf(-g[x])), si = g[x] * sg;
-        const float dg = d[x] * u[x] * sg * (1.f + g[x] * (1.f - sg));
-        u[x] = d[x] * si;
-        g[x] = dg;
-    }
-    out[j] = Pack8(g);
-    out[per + j] = Pack8(u);
+    SwiGluGrad8<false>(((const uint4 *)dh)[idx], row[j], row[per + j], &out[j], &out[per + j]);
 }
 
 // Cross entropy over vocabulary shards, one block per row. STEP 0: row maximum. STEP 1: sum of exp(l - max) and the target's

@@ -475,6 +475,81 @@ py::object Linear(py::handle xh, py::handle wh, py::object comm, uint64_t handle
     return py::cast(y);
 }
 
+// ---- SwiGLU layer of one rank ------------------------------------------------------------------------------------------
+// y = (silu(x Wg^T) * (x Wu^T)) Wd^T with W = [Wg; Wu]: the column-parallel product, SwiGLU and the row-parallel product in one node, whose products have the
+// element-wise part in their epilogues where that is faster.
+struct MlpNode : OpNode {
+    SavedVariable x, w, gu, h, wd;
+    std::vector<int64_t> shape;
+    at::TensorOptions options;
+    std::string name() const override { return "_SwiGluMlpBackward"; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(shape); }
+    std::vector<Saved> Keeps() override { return {{&x, false}, {&w, false}, {&gu, false}, {&h, false}, {&wd, false}}; }
+    variable_list Backward(variable_list &&g) override
+    {
+        const auto [xv, wv, guv, hv, wdv] = Unpack(x, w, gu, h, wd);
+        at::Tensor dy = ZerosWhereUndefined(g[0], shape, options);
+        bool direct = !traced && !at::GradMode::is_enabled() && g_nativeGemm && !g_nativeWgrad;
+        {
+            py::gil_scoped_acquire gil;
+            if (direct) {
+                const auto dev = DeviceOf(dy);
+                direct = !Watched() && PlainGrad(dy) && dy.dim() == 2 && dy.numel() > 0;
+                for (const at::Tensor &t : {xv, wv, guv, hv, wdv}) direct = direct && Operand(t, dev) && t.dim() == 2;
+                direct = direct && dy.size(0) == xv.size(0) && dy.size(1) == wdv.size(0) && wv.size(1) == xv.size(1) && guv.size(0) == xv.size(0) && guv.size(1) == wv.size(0) &&
+                         hv.size(0) == xv.size(0) && 2 * hv.size(1) == wv.size(0) && wdv.size(1) == hv.size(1) && xv.size(1) % 8 == 0 && hv.size(1) % 8 == 0 && dy.size(1) % 8 == 0 &&
+                         py::getattr(held->o, "fused", py::bool_(true)).cast<bool>();
+            }
+            if (traced) return FromPython((*g_env.backward)("mlp traced", xv, wv, guv, hv, wdv, dy), 3);
+            if (!direct) return FromPython((*g_env.backward)("mlp", held->o, xv, wv, guv, hv, wdv, dy), 3);
+        }
+        dy = Aligned(dy);
+        const int64_t m = xv.size(0), f = hv.size(1);
+        at::Tensor dgu = at::empty_like(guv), dh, dx = at::empty_like(xv);
+        if (HcclMatmulSwiGluBwdNeedsDh(m, f, dy.size(1))) dh = at::empty_like(hv);
+        Check(HcclMatmulSwiGluBwd(dy.data_ptr(), wdv.data_ptr(), guv.data_ptr(), dgu.data_ptr(), dh.defined() ? dh.data_ptr() : nullptr, m, f, dy.size(1), Stream(dy)),
+              "HcclMatmulSwiGluBwd");
+        const at::Tensor dwd = at::matmul(dy.t(), hv);
+        Check(HcclGemmBf16Nn(dgu.data_ptr(), wv.data_ptr(), dx.data_ptr(), m, wv.size(1), 2 * f, 0, Stream(dy)), "HcclGemmBf16Nn");
+        return {dx, at::matmul(dgu.t(), xv), dwd};
+    }
+};
+
+py::object Mlp(py::handle xh, py::handle wh, py::handle wdh, py::object comm, uint64_t handle, bool own)
+{
+    const at::Tensor x = OperandArg(xh), w = OperandArg(wh), wd = OperandArg(wdh);
+    if (!x.defined() || !w.defined() || !wd.defined() || x.dim() != 2 || w.dim() != 2 || wd.dim() != 2) return py::none();
+    const int64_t m = x.size(0), k = x.size(1), f = wd.size(1), n = wd.size(0);
+    if (w.size(1) != k || w.size(0) != 2 * f || k % 8 || f % 8 || n % 8) return py::none();
+    at::Tensor y;
+    {
+        const bool wanted = OpNode::Wanted({x, w, wd});
+        auto node = wanted ? MakeNode<MlpNode>(std::move(comm), x, w, wd) : nullptr;
+        py::gil_scoped_release nogil;
+        at::Tensor kept = x, gu, h;
+        {
+            at::NoGradGuard noGrad;
+            if (wanted && !own) kept = x.clone();
+            gu = at::empty({m, 2 * f}, x.options());
+            h = at::empty({m, f}, x.options());
+            y = at::empty({m, n}, x.options());
+            Check(HcclMatmulSwiGlu(x.data_ptr(), w.data_ptr(), gu.data_ptr(), h.data_ptr(), m, f, k, wanted, Stream(x)), "HcclMatmulSwiGlu");
+            Check(HcclMatmulReduceScatter(h.data_ptr(), wd.data_ptr(), y.data_ptr(), m, n, f, HCCL_DATA_TYPE_BFP16, (HcclComm)(uintptr_t)handle, Stream(x)), "HcclMatmulReduceScatter");
+        }
+        if (wanted) {
+            node->x = SavedVariable(kept, false);
+            node->w = SavedVariable(w, false);
+            node->gu = SavedVariable(gu, false);
+            node->h = SavedVariable(h, false);
+            node->wd = SavedVariable(wd, false);
+            node->shape = y.sizes().vec();
+            node->options = y.options();
+            torch::autograd::set_history({y}, node);
+        }
+    }
+    return py::cast(y);
+}
+
 // ---- cross entropy of one rank -------------------------------------------------------------------------------------------
 struct XentNode : OpNode {
     SavedVariable logits, targets, mx, packed;
@@ -562,5 +637,6 @@ void BindBlockOps(py::module &m)
     m.def("rope_qkv", &RopeQkv);
     m.def("swiglu", &SwiGlu);
     m.def("linear", &Linear);
+    m.def("mlp", &Mlp);
     m.def("xent", &Xent);
 }

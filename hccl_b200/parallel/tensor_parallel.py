@@ -183,6 +183,25 @@ def _one_rank_linear(x: torch.Tensor, w: torch.Tensor, comm, column: bool, own: 
     return None if n is None else n.linear(x, w, comm, comm.handle, column, own)
 
 
+def _mlp_backward(comm, x, w, gu, h, wd, dy):
+    """The SwiGLU layer's gradients by its parts; by single operations where something has to see them. What was kept for the kernels alone has no history: a gradient of
+    the gradient starts from the input again."""
+    if torch.is_grad_enabled() or not all([_block._plain_tensor(t) for t in (x, w, gu, h, wd, dy)]):
+        return _block._plain_backward(_plain_mlp, [t if t.requires_grad else t.detach().requires_grad_() for t in (x, w, wd)], dy)
+    dh, dwd = _row_backward(comm, h, wd, dy)
+    dgu, = _block._plain_backward(_plain_swiglu, (gu.detach().requires_grad_(),), dh)
+    return (*_column_backward(comm, x, w, dgu), dwd)
+
+
+def _mlp_traced(x, w, gu, h, wd, dy):
+    dgu, = _block.PYTHON_BACKWARD["swiglu traced"](gu, dy @ wd)
+    return dgu @ w, dgu.t() @ x, dy.t() @ h
+
+
+_block.PYTHON_BACKWARD["mlp"] = _mlp_backward
+_block.PYTHON_BACKWARD["mlp traced"] = _mlp_traced
+
+
 class _RowAllReduce(torch.autograd.Function):
     """y[M, N] = AR(x[M, Kl] @ W[N, Kl]^T): the decode-sized variant without sequence sharding."""
 
@@ -250,9 +269,13 @@ class ColumnParallelLinear(nn.Module):
 _COLUMN_FORWARD = ColumnParallelLinear.forward
 
 
+def _is_column(layer: nn.Module) -> bool:
+    return _block.bare(layer, ColumnParallelLinear, _COLUMN_FORWARD)
+
+
 def column_of_own(layer: nn.Module, x: torch.Tensor) -> torch.Tensor:
     """layer(x) for an x that the caller has made, gives to nobody else and does not change."""
-    return layer._forward(x, True) if _block.bare(layer, ColumnParallelLinear, _COLUMN_FORWARD) else layer(x)
+    return layer._forward(x, True) if _is_column(layer) else layer(x)
 
 
 class RowParallelLinear(nn.Module):
@@ -274,6 +297,9 @@ class RowParallelLinear(nn.Module):
             y = _one_rank_linear(x2, self.weight, self.comm, False)
             return _RowSeqParallel.apply(x2, self.weight, self.comm) if y is None else y
         return _RowAllReduce.apply(x2, self.weight, self.comm).reshape(*lead, -1)
+
+
+_ROW_FORWARD = RowParallelLinear.forward
 
 
 def _init_shard(w: torch.Tensor, std: float, seed: Optional[int], rank: int, dim: int, full: int) -> None:
@@ -311,7 +337,22 @@ class TensorParallelMLP(nn.Module):
     def forward(self, x_local):
         return self._forward(x_local, False)
 
+    def _one_rank(self, x_local, own: bool):
+        """The whole layer as one native node on one rank, or None where it does not apply or a part of it is more than its class says."""
+        up, down, comm = self.gate_up, self.down, self.comm
+        if comm.size != 1 or not _NATIVE_GEMM or not getattr(comm, "fused", True):
+            return None
+        n = _block.native_nodes(x_local)
+        if n is None or not _is_column(up) or not _block.bare(down, RowParallelLinear, _ROW_FORWARD):
+            return None
+        if not (up.sequence_parallel and down.sequence_parallel and up.comm is comm and down.comm is comm):
+            return None
+        return n.mlp(_rows(x_local, up.in_features), up.weight, down.weight, comm, comm.handle, own)
+
     def _forward(self, x_local, own: bool):
+        y = self._one_rank(x_local, own)
+        if y is not None:
+            return y
         gu = column_of_own(self.gate_up, x_local) if own else self.gate_up(x_local)
         h = _block.swiglu(gu, _plain_swiglu)
         return self.down(_plain_swiglu(gu) if h is None else h)
@@ -328,3 +369,7 @@ def mlp_of_own(mlp: nn.Module, x_local: torch.Tensor) -> torch.Tensor:
 def _plain_swiglu(gu):
     ffn = gu.shape[1] // 2
     return torch.nn.functional.silu(gu[:, :ffn]) * gu[:, ffn:]
+
+
+def _plain_mlp(x, w, wd):
+    return _plain_swiglu(x @ w.t()) @ wd.t()

@@ -54,6 +54,13 @@ HcclResult HcclGemmBf16(const void *a, const void *b, void *c, uint64_t m, uint6
 HcclResult HcclGemmBf16Variant(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, int variant, cudaStream_t stream);
 /* C[M,N] = A[M,K] * B[K,N], both row-major: the input gradient of a linear layer from its [K, N] weight as stored. */
 HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream);
+/* The products of a SwiGLU layer with its element-wise part, on one GPU. gateUp[m, 2 ffn] = x[m, k] * w[2 ffn, k]^T, h[m, ffn] = silu(gate) * up; with
+ * keepGateUp = 0 the contents of gateUp are undefined afterwards. k and ffn: multiples of 8. The bits of HcclGemmBf16 and HcclSwiGlu. */
+HcclResult HcclMatmulSwiGlu(const void *x, const void *w, void *gateUp, void *h, uint64_t m, uint64_t ffn, uint64_t k, int keepGateUp, cudaStream_t stream);
+/* dGateUp[m, 2 ffn] from dy[m, k], w[k, ffn] and gateUp: the gradient of the intermediate h = dy * w is not kept, but dh[m, ffn] holds it in between where
+ * HcclMatmulSwiGluBwdNeedsDh(m, ffn, k) is not 0. */
+HcclResult HcclMatmulSwiGluBwd(const void *dy, const void *w, const void *gateUp, void *dGateUp, void *dh, uint64_t m, uint64_t ffn, uint64_t k, cudaStream_t stream);
+int HcclMatmulSwiGluBwdNeedsDh(uint64_t m, uint64_t ffn, uint64_t k);
 HcclResult HcclGemmCheckError(void);
 /* Kernels this library has launched in this process so far (all operators; benchmarks report the delta over a region). */
 uint64_t HcclGetKernelLaunchCount(void);

@@ -530,3 +530,106 @@ def test_block_input_may_change_after_the_pass():
             assert torch.equal(a, b)
     finally:
         comm.destroy()
+
+
+def _swiglu_layer(rows, hidden, ffn, seed=1):
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.parallel.tensor_parallel import TensorParallelMLP
+    torch.zeros(1, device="cuda")
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    torch.manual_seed(seed)
+    mlp = TensorParallelMLP(comm, hidden, ffn, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x, up = [torch.randn(rows, hidden, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    return comm, mlp, x.requires_grad_(), up
+
+
+@pytest.mark.parametrize("rows,hidden,ffn", [(1, 64, 64), (70, 136, 72), (130, 512, 1000), (300, 256, 2056), (513, 520, 1000), (768, 1024, 512), (1030, 264, 3000), (5000, 256, 1536)])
+def test_swiglu_layer_gives_the_bits_of_its_parts(rows, hidden, ffn):
+    """The products with SwiGLU in their epilogues: every tile width, rows and columns that do not fill a tile, both sides of the choices; result and gradients are those
+    of the product and the element-wise kernel one after the other (gate values of all sizes, one of them infinite)."""
+    _native_nodes()
+    comm, mlp, x, up = _swiglu_layer(rows, hidden, ffn)
+    try:
+        with torch.no_grad():
+            mlp.gate_up.weight.mul_(torch.exp(torch.randn(2 * ffn, 1, device="cuda")).to(torch.bfloat16) * 30)
+            mlp.gate_up.weight[0, 0] = float("inf")
+        params = list(mlp.parameters())
+
+        def step():
+            y = mlp(x)
+            return [y.detach(), *torch.autograd.grad(y, [x, *params], up)]
+
+        fused = step()
+        assert mlp(x).grad_fn.name() == "_SwiGluMlpBackward"
+        handle = mlp.gate_up.register_forward_hook(lambda *a: None)
+        parts = step()
+        handle.remove()
+        for a, b in zip(fused, parts):
+            assert torch.equal(a.nan_to_num(3.0, 5.0, 7.0), b.nan_to_num(3.0, 5.0, 7.0))
+        with torch.no_grad():
+            assert torch.equal(mlp(x).nan_to_num(3.0, 5.0, 7.0), parts[0].nan_to_num(3.0, 5.0, 7.0))
+    finally:
+        comm.destroy()
+
+
+def test_swiglu_layer_keeps_the_engine_s_rules():
+    """Input that changes after the pass, a gradient's gradient, compiled autograd, batched gradients, saved tensors of another size or on the CPU, a weight that changes in
+    place, the switch of the weight gradients."""
+    from torch._dynamo import compiled_autograd
+    from hccl_b200.parallel import tensor_parallel as tp
+    _native_nodes()
+    comm, mlp, leaf, up = _swiglu_layer(640, 64, 128)
+    try:
+        ins = [leaf, *mlp.parameters()]
+        ref = torch.autograd.grad(mlp(leaf), ins, up)
+        x = leaf * 1
+        y = mlp(x)
+        x.zero_()
+        for a, b in zip(torch.autograd.grad(y, ins, up), ref):
+            assert torch.equal(a, b)
+        plain = tp._plain_mlp(leaf, mlp.gate_up.weight, mlp.down.weight)
+        close = lambda a, b, steps: (a.double() - b.double()).norm() <= steps * 2.0 ** -8 * b.double().norm()
+        pg = torch.autograd.grad(plain, ins, up, create_graph=True)
+        y = mlp(leaf * 1)
+        got = torch.autograd.grad(y, ins, up, create_graph=True)
+        assert all(close(a, b, 8) for a, b in zip(got, pg))                     # a dozen roundings to bf16 on the way
+        second = torch.autograd.grad(sum(t.float().square().sum() for t in got), ins[1:])
+        for a, b in zip(second, torch.autograd.grad(sum(t.float().square().sum() for t in pg), ins[1:])):
+            assert close(a, b, 16)
+        ups = torch.stack([up, up * 2])
+        batched = torch.autograd.grad(mlp(leaf), ins, ups, is_grads_batched=True)
+        assert all(close(t[0], b, 8) and close(t[1], 2 * b, 8) for t, b in zip(batched, ref))
+        with compiled_autograd._enable(torch.compile(backend="eager")):
+            mlp(leaf).backward(up)
+        for t, b in zip(ins, ref):
+            assert close(t.grad, b, 8)
+            t.grad = None
+        with torch.autograd.graph.save_on_cpu():
+            y = mlp(leaf)
+        assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y, ins, up), ref))
+        for at in range(5):
+            for change in (lambda t: torch.cat([t, t], -1), lambda t: t[:-1].clone(), lambda t: t[:, :-8].contiguous()):
+                count = [0]
+
+                def pack(t):
+                    count[0] += 1
+                    return count[0] - 1, t
+
+                with torch.autograd.graph.saved_tensors_hooks(pack, lambda p: change(p[1]) if p[0] == at else p[1]):
+                    y = mlp(leaf)
+                assert count[0] == 5
+                with pytest.raises((RuntimeError, IndexError, ValueError, AssertionError)):
+                    torch.autograd.grad(y, ins, up)
+        tp.use_native_wgrad(True)
+        assert all(close(a, b, 8) for a, b in zip(torch.autograd.grad(mlp(leaf), ins, up), ref))
+        tp.use_native_wgrad(False)
+        y = mlp(leaf)
+        with torch.no_grad():
+            mlp.down.weight.mul_(1)
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            y.sum().backward()
+        torch.cuda.synchronize()
+    finally:
+        tp.use_native_wgrad(False)
+        comm.destroy()
