@@ -8,6 +8,11 @@
 // functions. A backward pass that something has to see, or whose tensors are not the plain ones that the kernels read, is handed to
 // the Python form's own backward. What a node holds of Python must not lead back to a module: a graph node is invisible to the
 // garbage collector, and a module may hold its own output.
+#include <ATen/Context.h>
+#include <ATen/SDPBackend.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/ops/_fused_sdp_choice.h>
+#include <ATen/ops/_scaled_dot_product_cudnn_attention.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -362,6 +367,89 @@ py::object RopeQkv(py::handle qkvh, py::handle cosh, py::handle sinh, int64_t ba
     return py::make_tuple(q, k, v);
 }
 
+// ---- attention of short sequences ---------------------------------------------------------------------------------------
+// From the packed projection to the attention's output. Forward: the rotary kernel and the library's attention, which the dispatcher would choose as well; backward: one kernel.
+// Keeps the projection, which nobody but the caller's own layer may have.
+struct AttentionNode : OpNode {
+    SavedVariable qkv, o, lse, cos, sin;
+    int64_t batch = 0, heads = 0, kvHeads = 0, headDim = 0;
+    std::string name() const override { return "_AttentionBackward"; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override
+    {
+        for (int64_t v : {batch, heads, kvHeads, headDim}) args.collect(v);
+    }
+    std::vector<Saved> Keeps() override { return {{&qkv, false}, {&o, true}, {&lse, false}, {&cos, false}, {&sin, false}}; }
+    variable_list Backward(variable_list &&g) override
+    {
+        const auto [x, out, l, c, s] = Unpack(qkv, o, lse, cos, sin);
+        const at::Tensor dO = g[0].defined() ? g[0] : at::zeros_like(out);
+        bool direct = !traced && !at::GradMode::is_enabled();
+        {
+            py::gil_scoped_acquire gil;
+            if (direct) {
+                const auto dev = DeviceOf(dO);
+                direct = !Watched() && PlainGrad(dO) && Operand(x, dev) && Operand(out, dev) && Floats(l, dev) && Floats(c, dev) && Floats(s, dev) && c.dim() == 2 && c.sizes() == s.sizes() &&
+                         c.size(1) == headDim / 2 && x.dim() == 2 && x.size(0) == batch * c.size(0) && x.size(1) == (heads + 2 * kvHeads) * headDim && out.dim() == 2 &&
+                         out.size(0) == x.size(0) && out.size(1) == heads * headDim && dO.sizes() == out.sizes() && l.numel() == x.size(0) * heads;
+            }
+            if (traced) return FromPython((*g_env.backward)("attention traced", x, c, s, batch, heads, kvHeads, headDim, dO), 1);
+            if (!direct) return FromPython((*g_env.backward)("attention", held->o, x, dO), 1);
+        }
+        const at::Tensor d = Aligned(dO), dx = at::empty_like(x);
+        Check(HcclAttentionBwd(d.data_ptr(), x.data_ptr(), out.data_ptr(), l.data_ptr<float>(), dx.data_ptr(), c.data_ptr<float>(), s.data_ptr<float>(), batch, c.size(0), heads,
+                               kvHeads, headDim, Stream(x)), "HcclAttentionBwd");
+        return {dx};
+    }
+};
+
+// Whether nothing asks for another attention than the default one.
+bool DefaultAttention()
+{
+    const at::Context &c = at::globalContext();
+    return c.userEnabledFlashSDP() && c.userEnabledMemEfficientSDP() && c.userEnabledMathSDP() && c.userEnabledCuDNNSDP() && !at::autocast::is_autocast_enabled(at::kCUDA);
+}
+
+py::object Attention(py::handle qkvh, py::handle cosh, py::handle sinh, int64_t batch, int64_t heads, int64_t kvHeads, int64_t headDim, py::object plain)
+{
+    const at::Tensor qkv = OperandArg(qkvh);
+    if (!qkv.defined() || Py_TYPE(cosh.ptr()) != g_env.tensor || Py_TYPE(sinh.ptr()) != g_env.tensor || batch <= 0 || heads <= 0 || kvHeads <= 0) return py::none();
+    const at::Tensor cos = THPVariable_Unpack(cosh.ptr()), sin = THPVariable_Unpack(sinh.ptr());
+    const auto dev = qkv.device().index();
+    if (!Floats(cos, dev) || !Floats(sin, dev) || cos.dim() != 2 || qkv.dim() != 2 || cos.sizes() != sin.sizes() || cos.size(1) != headDim / 2) return py::none();
+    const int64_t seq = cos.size(0), tokens = batch * seq;
+    if (qkv.size(0) != tokens || qkv.size(1) != (heads + 2 * kvHeads) * headDim || !DefaultAttention() || !HcclAttentionBwdSuits(batch, seq, heads, kvHeads, headDim)) return py::none();
+    if (!OpNode::Wanted({qkv})) return py::none();
+    at::Tensor o;
+    {
+        auto node = MakeNode<AttentionNode>(std::move(plain), qkv);
+        py::gil_scoped_release nogil;
+        at::Tensor lse;
+        {
+            at::NoGradGuard noGrad;
+            const at::Tensor q = at::empty({batch, seq, heads, headDim}, qkv.options()), k = at::empty({batch, seq, kvHeads, headDim}, qkv.options()), v = at::empty_like(k);
+            const at::Tensor qt = q.transpose(1, 2), kt = k.transpose(1, 2), vt = v.transpose(1, 2);
+            if (at::_fused_sdp_choice(qt, kt, vt, {}, 0.0, true, {}, heads != kvHeads) != (int64_t)at::SDPBackend::cudnn_attention) o = at::Tensor();
+            else {
+                Check(HcclRopeQkv(qkv.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr<float>(), sin.data_ptr<float>(), tokens, seq, heads, kvHeads, headDim, 0,
+                                  Stream(qkv)), "HcclRopeQkv");
+                const auto r = at::_scaled_dot_product_cudnn_attention(qt, kt, vt, {}, true, 0.0, true, false, {});
+                o = std::get<0>(r).transpose(1, 2).reshape({tokens, heads * headDim});
+                lse = std::get<1>(r).reshape({batch, heads, seq}).contiguous();
+            }
+        }
+        if (o.defined()) {
+            torch::autograd::set_history({o}, node);
+            node->qkv = SavedVariable(qkv, false);
+            node->o = SavedVariable(o, true);
+            node->lse = SavedVariable(lse, false);
+            node->cos = SavedVariable(cos, false);
+            node->sin = SavedVariable(sin, false);
+            node->batch = batch; node->heads = heads; node->kvHeads = kvHeads; node->headDim = headDim;
+        }
+    }
+    return o.defined() ? py::cast(o) : py::none();
+}
+
 // ---- SwiGLU ------------------------------------------------------------------------------------------------------------
 struct SwiGluNode : OpNode {
     SavedVariable gu;
@@ -635,6 +723,7 @@ void BindBlockOps(py::module &m)
     m.def("rms_norm", &RmsNorm);
     m.def("rms_norm_add", &RmsNormAdd);
     m.def("rope_qkv", &RopeQkv);
+    m.def("attention", &Attention);
     m.def("swiglu", &SwiGlu);
     m.def("linear", &Linear);
     m.def("mlp", &Mlp);

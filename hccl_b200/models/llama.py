@@ -20,7 +20,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops import block as _block
-from ..parallel.tensor_parallel import ColumnParallelLinear, RowParallelLinear, TensorParallelMLP, column_of_own, mlp_of_own
+from ..parallel.tensor_parallel import ColumnParallelLinear, RowParallelLinear, TensorParallelMLP, column_of_own, is_column, mlp_of_own
 
 
 @dataclass
@@ -136,12 +136,14 @@ class Attention(nn.Module):
 
     def _forward(self, x_local, batch: int, seq: int, cos, sin, own: bool):
         qkv = column_of_own(self.qkv, x_local) if own else self.qkv(x_local)                                    # [B*S, (hl + 2 kvl) * hd]
-        plain = functools.partial(_rotated, batch=batch, seq=seq, heads=self.h_local, kv_heads=self.kv_local, hd=self.hd, cos=cos, sin=sin)
+        dims = dict(batch=batch, seq=seq, heads=self.h_local, kv_heads=self.kv_local, hd=self.hd, cos=cos, sin=sin)
+        if is_column(self.qkv):                                             # nobody else has the projection
+            o = _block.attention(qkv, cos, sin, batch, self.h_local, self.kv_local, self.hd, functools.partial(_plain_attention, **dims))
+            if o is not None:
+                return self.out(o)
+        plain = functools.partial(_rotated, **dims)
         out = _block.rope_qkv(qkv, cos, sin, batch, self.h_local, self.kv_local, self.hd, plain)
-        q, k, v = (t.transpose(1, 2) for t in (plain(qkv) if out is None else out))
-        o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=self.h_local != self.kv_local)
-        o = o.transpose(1, 2).reshape(batch * seq, self.h_local * self.hd)
-        return self.out(o)                                                  # [B*S / tp, hidden]
+        return self.out(_attended(*(plain(qkv) if out is None else out)))   # [B*S / tp, hidden]
 
     def _rotated(self, qkv, batch, seq, cos, sin):
         return _rotated(qkv, batch, seq, self.h_local, self.kv_local, self.hd, cos, sin)
@@ -155,6 +157,16 @@ def _rotated(qkv, batch, seq, heads, kv_heads, hd, cos, sin):
     q = _apply_rope(q.reshape(batch, seq, heads, hd), cos, sin)
     k = _apply_rope(k.reshape(batch, seq, kv_heads, hd), cos, sin)
     return q, k, v.reshape(batch, seq, kv_heads, hd)
+
+
+def _attended(q, k, v):
+    batch, seq, heads, hd = q.shape
+    o = F.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True, enable_gqa=heads != k.shape[2])
+    return o.transpose(1, 2).reshape(batch * seq, heads * hd)
+
+
+def _plain_attention(qkv, batch, seq, heads, kv_heads, hd, cos, sin):
+    return _attended(*_rotated(qkv, batch, seq, heads, kv_heads, hd, cos, sin))
 
 
 class Block(nn.Module):

@@ -32,10 +32,12 @@ def _decl():
         l.HcclRmsNormBwdParts.restype = u64
         l.HcclRmsNormBwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, u64, u64, vp]
         l.HcclRopeQkv.argtypes = [vp, vp, vp, vp, vp, vp, u64, u64, u32, u32, u32, i32, vp]
+        l.HcclAttentionBwdSuits.argtypes = [u64, u64, u32, u32, u32]
+        l.HcclAttentionBwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, u64, u64, u32, u32, u32, vp]
         l.HcclSwiGlu.argtypes = [vp, vp, u64, u64, vp]
         l.HcclSwiGluBwd.argtypes = [vp, vp, vp, u64, u64, vp]
         l.HcclXent.argtypes = [i32, vp, vp, i64, vp, vp, vp, vp, u64, u64, vp]
-        for f in (l.HcclRmsNorm, l.HcclRmsNormKeep, l.HcclRmsNormBwd, l.HcclRopeQkv, l.HcclSwiGlu, l.HcclSwiGluBwd, l.HcclXent):
+        for f in (l.HcclRmsNorm, l.HcclRmsNormKeep, l.HcclRmsNormBwd, l.HcclRopeQkv, l.HcclAttentionBwdSuits, l.HcclAttentionBwd, l.HcclSwiGlu, l.HcclSwiGluBwd, l.HcclXent):
             f.restype = ctypes.c_int
         l._nn_declared = True
     return l
@@ -281,6 +283,77 @@ def rope_qkv(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int
     if head_dim % 16 or qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
         return None
     return _RopeQkv.apply(qkv, cos, sin, heads, kv_heads, head_dim, plain)
+
+
+class _Attention(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, qkv, cos, sin, dims, plain):
+        batch, heads, kv_heads, head_dim = dims
+        q, k, v = _RopeQkv.apply(qkv, cos, sin, heads, kv_heads, head_dim, plain)
+        o, lse = torch.ops.aten._scaled_dot_product_cudnn_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), None, True, 0.0, True, False)[:2]
+        o, lse = o.transpose(1, 2).reshape(qkv.shape[0], heads * head_dim), lse.reshape(batch, heads, -1).contiguous()
+        ctx.save_for_backward(qkv, o, lse, cos, sin)
+        ctx.dims, ctx.seq, ctx.plain = dims, cos.shape[0], plain
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        qkv, o, lse, cos, sin = ctx.saved_tensors
+        batch, heads, kv_heads, head_dim = ctx.dims
+        tokens, grads = batch * ctx.seq, _direct((qkv, o), (do,))
+        if grads is None or qkv.shape != (tokens, (heads + 2 * kv_heads) * head_dim) or o.shape != (tokens, heads * head_dim) or do.shape != o.shape \
+                or not _floats_ok(qkv.get_device(), lse, cos, sin) or lse.numel() != tokens * heads or not cos.shape == sin.shape == (ctx.seq, head_dim // 2):
+            return (*_plain_backward(ctx.plain, (qkv,), do), None, None, None, None)
+        do, = grads
+        out = torch.empty_like(qkv)
+        check(_decl().HcclAttentionBwd(do.data_ptr(), qkv.data_ptr(), o.data_ptr(), lse.data_ptr(), out.data_ptr(), cos.data_ptr(), sin.data_ptr(), batch, ctx.seq, heads, kv_heads,
+                                       head_dim, _stream(qkv)), "HcclAttentionBwd")
+        return out, None, None, None, None
+
+
+def _default_attention() -> bool:
+    b = torch.backends.cuda
+    return b.flash_sdp_enabled() and b.mem_efficient_sdp_enabled() and b.math_sdp_enabled() and b.cudnn_sdp_enabled() and not torch.is_autocast_enabled("cuda")
+
+
+def attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable) -> Optional[torch.Tensor]:
+    """Causal attention from the packed projection, [batch * seq, heads * head_dim], for sequences short enough that the backward kernel is the better choice, where a gradient may be asked for and
+    the library's attention would run anyway; the tables as `rope_qkv`. The projection is kept as it is, so nobody else may change it. `plain(qkv)` is the same in PyTorch."""
+    n = native_nodes(qkv)
+    if n is not None:
+        return n.attention(qkv, cos, sin, batch, heads, kv_heads, head_dim, plain)
+    if not _usable(qkv) or not _floats_ok(qkv.get_device(), cos, sin) or not _default_attention() or not (torch.is_grad_enabled() and qkv.requires_grad):
+        return None
+    seq = cos.shape[0] if cos.dim() else 0
+    if qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
+        return None
+    if not _decl().HcclAttentionBwdSuits(batch, seq, heads, kv_heads, head_dim):
+        return None
+    q, k = (torch.empty(batch, seq, h, head_dim, dtype=qkv.dtype, device=qkv.device).transpose(1, 2) for h in (heads, kv_heads))
+    if torch._fused_sdp_choice(q, k, k, is_causal=True, enable_gqa=heads != kv_heads) != torch.nn.attention.SDPBackend.CUDNN_ATTENTION.value:
+        return None
+    return _Attention.apply(qkv, cos, sin, (batch, heads, kv_heads, head_dim), plain)
+
+
+PYTHON_BACKWARD["attention"] = lambda plain, qkv, do: _plain_backward(plain, (qkv,), do)
+
+
+def _attention_traced(qkv, cos, sin, batch, heads, kv_heads, head_dim, do):
+    seq, half = cos.shape[0], head_dim // 2
+    c, s, group = cos[:, None], sin[:, None], heads // kv_heads
+    q, k, v = qkv.float().reshape(batch, seq, -1, head_dim).split([heads, kv_heads, kv_heads], 2)
+    turned = lambda t, sn: torch.cat([t[..., :half] * c - t[..., half:] * sn, t[..., half:] * c + t[..., :half] * sn], -1)
+    q, k, v, d = (t.transpose(1, 2) for t in (turned(q, s), turned(k, s).repeat_interleave(group, 2), v.repeat_interleave(group, 2), do.float().reshape(batch, seq, heads, head_dim)))
+    hidden = torch.arange(seq, device=qkv.device)[None] > torch.arange(seq, device=qkv.device)[:, None]
+    p = ((q @ k.transpose(2, 3)) * head_dim ** -0.5).masked_fill(hidden, float("-inf")).softmax(-1)
+    dp = d @ v.transpose(2, 3)
+    ds = p * (dp - (p * dp).sum(-1, keepdim=True)) * head_dim ** -0.5
+    per_key = lambda t: t.reshape(batch, kv_heads, group, seq, head_dim).sum(2).transpose(1, 2)
+    parts = turned((ds @ k).transpose(1, 2), -s), turned(per_key(ds.transpose(2, 3) @ q), -s), per_key(p.transpose(2, 3) @ d)
+    return (torch.cat(parts, 2).reshape(qkv.shape).to(qkv.dtype),)
+
+
+PYTHON_BACKWARD["attention traced"] = _attention_traced
 
 
 class _SwiGlu(torch.autograd.Function):

@@ -269,13 +269,14 @@ class ColumnParallelLinear(nn.Module):
 _COLUMN_FORWARD = ColumnParallelLinear.forward
 
 
-def _is_column(layer: nn.Module) -> bool:
+def is_column(layer: nn.Module) -> bool:
+    """A column-parallel layer that is what its class says."""
     return _block.bare(layer, ColumnParallelLinear, _COLUMN_FORWARD)
 
 
 def column_of_own(layer: nn.Module, x: torch.Tensor) -> torch.Tensor:
     """layer(x) for an x that the caller has made, gives to nobody else and does not change."""
-    return layer._forward(x, True) if _is_column(layer) else layer(x)
+    return layer._forward(x, True) if is_column(layer) else layer(x)
 
 
 class RowParallelLinear(nn.Module):
@@ -343,7 +344,7 @@ class TensorParallelMLP(nn.Module):
         if comm.size != 1 or not _NATIVE_GEMM or not getattr(comm, "fused", True):
             return None
         n = _block.native_nodes(x_local)
-        if n is None or not _is_column(up) or not _block.bare(down, RowParallelLinear, _ROW_FORWARD):
+        if n is None or not is_column(up) or not _block.bare(down, RowParallelLinear, _ROW_FORWARD):
             return None
         if not (up.sequence_parallel and down.sequence_parallel and up.comm is comm and down.comm is comm):
             return None

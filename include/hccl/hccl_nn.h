@@ -30,6 +30,12 @@ HcclResult HcclRmsNormBwdAdd(const void *dy, const void *x, const void *w, const
  * backward != 0: gradients of q, k, v -> gradient of qkv. */
 HcclResult HcclRopeQkv(void *qkv, void *q, void *k, void *v, const float *cosT, const float *sinT, uint64_t tokens, uint64_t seq, uint32_t qHeads, uint32_t kvHeads,
                        uint32_t headDim, int backward, cudaStream_t stream);
+/* Gradient of causal attention by the packed projection qkv[batch * seq, (qHeads + 2 kvHeads) * headDim], whose q and k HcclRopeQkv rotates: dQkv from dO and o[batch * seq, qHeads * headDim]
+ * and lse[batch, qHeads, seq], the logarithms of the sums of exp(q k / sqrt(headDim)). Query head h reads key head h / (qHeads / kvHeads). headDim: 32 or 64.
+ * HcclAttentionBwdSuits: whether this kernel, made for short sequences, is the better choice. */
+int HcclAttentionBwdSuits(uint64_t batch, uint64_t seq, uint32_t qHeads, uint32_t kvHeads, uint32_t headDim);
+HcclResult HcclAttentionBwd(const void *dO, const void *qkv, const void *o, const float *lse, void *dQkv, const float *cosT, const float *sinT, uint64_t batch, uint64_t seq,
+                            uint32_t qHeads, uint32_t kvHeads, uint32_t headDim, cudaStream_t stream);
 /* h[rows, ffn] = silu(gate) * up with gateUp[rows, 2 ffn] = [gate | up]. ffn: a multiple of 8. */
 HcclResult HcclSwiGlu(const void *gateUp, void *h, uint64_t rows, uint64_t ffn, cudaStream_t stream);
 HcclResult HcclSwiGluBwd(const void *dh, const void *gateUp, void *dGateUp, uint64_t rows, uint64_t ffn, cudaStream_t stream);

@@ -499,8 +499,14 @@ def test_block_with_fused_norms_gives_the_bits_of_the_modules(tokens, monkeypatc
         for a, b in zip(torch.autograd.grad(loss, params), fused[1:]):
             assert torch.equal(a, b)
         seen = []
-        handles = [m.register_forward_hook(lambda m, i, o: seen.append(m)) for m in model.modules() if m is not model]
+        hook = lambda m: m.register_forward_hook(lambda m, i, o: seen.append(m))
+        projections = [b.attn.qkv for b in model.blocks]
+        handles = [hook(m) for m in model.modules() if m is not model and not any(m is p for p in projections)]
         hooked = step()
+        handles += [hook(m) for m in projections]                              # then the library's backward pass of the attention: sums in another order
+        seen.clear()
+        for a, b in zip(step(), fused):
+            assert (a.double() - b.double()).norm() <= 2.0 ** -5 * b.double().norm() + 1e-12
         [h.remove() for h in handles]
         assert len(seen) == len(list(model.modules())) - 2                      # but for the model and its list of blocks
         _plain_modules(monkeypatch)
@@ -633,3 +639,101 @@ def test_swiglu_layer_keeps_the_engine_s_rules():
     finally:
         tp.use_native_wgrad(False)
         comm.destroy()
+
+
+def _attention_case(batch, seq, heads, kv_heads, hd, seed=2):
+    import functools
+    from hccl_b200.models.llama import _plain_attention, _rope_tables
+    from hccl_b200.ops import block
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    qkv, do = [torch.randn(batch * seq, n * hd, generator=g, device="cuda").to(torch.bfloat16) for n in (heads + 2 * kv_heads, heads)]
+    cos, sin = _rope_tables(seq, hd, 10000.0, "cuda")
+    plain = functools.partial(_plain_attention, batch=batch, seq=seq, heads=heads, kv_heads=kv_heads, hd=hd, cos=cos, sin=sin)
+    return lambda t: block.attention(t, cos, sin, batch, heads, kv_heads, hd, plain), plain, qkv.requires_grad_(), do, cos.double(), sin.double()
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("batch,seq,heads,kv_heads,hd", [(1, 2, 8, 4, 32), (3, 63, 2, 1, 32), (2, 64, 4, 4, 32), (1, 65, 8, 2, 32), (2, 200, 6, 3, 32), (1, 1024, 4, 4, 32), (1, 130, 4, 2, 64),
+                                                         (2, 128, 8, 2, 64)])
+def test_attention_of_short_sequences(batch, seq, heads, kv_heads, hd, native, monkeypatch):
+    """The backward kernel: sequences around whole tiles, grouped queries, both widths, against 64 bits from the rotated values as the kernels round them. What the products read is rounded
+    to bf16 once: probabilities, their gradients and O in the sum of dO * O, at most 2^-8 of the magnitudes that are added up, and each result once more. The same bits on every run."""
+    from hccl_b200.models.llama import _rotated
+    from hccl_b200.ops import block
+    if native:
+        _native_nodes()
+    else:
+        monkeypatch.setattr(block, "_NODES", None)
+    f, _, qkv, do, cos, sin = _attention_case(batch, seq, heads, kv_heads, hd)
+    o = f(qkv)
+    assert o.grad_fn.name().startswith("_Attention") and _is_native(o) == native
+    got, = torch.autograd.grad(o, qkv, do, retain_graph=True)
+    assert torch.equal(got, torch.autograd.grad(o, qkv, do)[0])
+    group, scale = heads // kv_heads, hd ** -0.5
+    q, k, v = (t.double().transpose(1, 2) for t in _rotated(qkv.detach(), batch, seq, heads, kv_heads, hd, cos.float(), sin.float()))
+    k, v = k.repeat_interleave(group, 1), v.repeat_interleave(group, 1)
+    d = do.double().reshape(batch, seq, heads, hd).transpose(1, 2)
+    p = (q @ k.transpose(2, 3) * scale).masked_fill(~torch.ones(seq, seq, dtype=torch.bool, device="cuda").tril(), float("-inf")).softmax(-1)
+    ref = p @ v
+    flat = lambda t: t.transpose(1, 2).reshape(batch * seq, -1)
+    assert bool(((o.double() - flat(ref)).abs() <= flat(p @ v.abs()) * 2.0 ** -8 + flat(ref).abs() * 2.0 ** -8).all())
+    dp, dot = d @ v.transpose(2, 3), (d * ref).sum(-1, keepdim=True)
+    ds, mag = p * (dp - dot) * scale, p * (dp.abs() + (d.abs() * ref.abs()).sum(-1, keepdim=True)) * scale
+    grouped = lambda t: t.reshape(batch, kv_heads, group, seq, hd).sum(2)
+    c, s = cos[None, None], sin[None, None]
+
+    def back(t):
+        a, b = t[..., :hd // 2], t[..., hd // 2:]
+        return torch.cat([a * c + b * s, b * c - a * s], -1)
+
+    def both(t):                                                               # a rotation adds parts of both halves
+        return torch.cat([t[..., :hd // 2] + t[..., hd // 2:]] * 2, -1)
+
+    refs = back(ds @ k), back(grouped(ds.transpose(2, 3) @ q)), grouped(p.transpose(2, 3) @ d)
+    mags = both(mag @ k.abs()), both(grouped(mag.transpose(2, 3) @ q.abs())), grouped(p.transpose(2, 3) @ d.abs())
+    want, bound = torch.cat([flat(t) for t in refs], 1), torch.cat([flat(t) for t in mags], 1)
+    assert bool(((got.double() - want).abs() <= bound * 2.0 ** -7 + want.abs() * 2.0 ** -8 + 1e-6).all())
+
+
+def test_attention_keeps_the_engine_s_rules():
+    """Another attention asked for, a projection that changes in place, saved tensors of another size, batched gradients, compiled autograd: the plain form's answers or errors."""
+    from torch._dynamo import compiled_autograd
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    from hccl_b200.ops import block
+    nodes = _native_nodes()
+    f, plain, qkv, do, _, _ = _attention_case(2, 100, 4, 2, 32)
+    close = lambda a, b: (a.double() - b.double()).norm() <= 2.0 ** -6 * b.double().norm()
+    ref, = torch.autograd.grad(plain(qkv), qkv, do)
+    assert close(torch.autograd.grad(f(qkv), qkv, do)[0], ref)
+    with sdpa_kernel(SDPBackend.MATH):
+        assert f(qkv) is None
+    with torch.autocast("cuda", dtype=torch.float16):
+        assert f(qkv) is None
+    batched, = torch.autograd.grad(f(qkv), qkv, torch.stack([do, 2 * do]), is_grads_batched=True)
+    assert close(batched[0], ref) and close(batched[1], 2 * ref)
+    x = qkv * 1
+    o = f(x)
+    x.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(o, qkv, do)
+    for at in range(5):
+        for change in (lambda t: torch.cat([t, t], -1), lambda t: t[:-1].clone(), lambda t: t[..., :-8].contiguous()):
+            count = [0]
+
+            def pack(t):
+                count[0] += 1
+                return count[0] - 1, t
+
+            with torch.autograd.graph.saved_tensors_hooks(pack, lambda p: change(p[1]) if p[0] == at else p[1]):
+                o = f(qkv)
+            assert count[0] == 5
+            try:
+                got, = torch.autograd.grad(o, qkv, do)
+            except (RuntimeError, IndexError, ValueError, AssertionError):
+                continue
+            assert got.shape == ref.shape and close(got, ref)                  # what the plain form does not read may have changed
+    with compiled_autograd._enable(torch.compile(backend="eager")):
+        f(qkv).backward(do)
+    assert close(qkv.grad, ref)
+    with torch.no_grad():
+        assert f(qkv) is None and nodes is block.nodes()
