@@ -378,6 +378,113 @@ __global__ void __launch_bounds__(kThreads) XentKernel(const __nv_bfloat16 *__re
     }
 }
 
+// The cross entropy of one rank up to the loss of every row: what steps 0 and 1 compute, the rows' losses, and copies of logits and targets for a backward pass that may come after
+// they were changed. The second walk over a row finds it in L2. 2048 x 128256 logits: the copy alone, as an operation of its own, reads and writes 1 GB.
+template <bool VEC>
+__global__ void __launch_bounds__(kThreads) XentLossKernel(const __nv_bfloat16 *__restrict__ logits, const int64_t *__restrict__ targets, int64_t vocabStart, float *__restrict__ mx,
+                                                          float *__restrict__ packed, float *__restrict__ rowLoss, __nv_bfloat16 *__restrict__ kept, int64_t *__restrict__ keptTargets,
+                                                          uint32_t T, uint32_t V)
+{
+    __shared__ float red[kThreads / 32];
+    const uint32_t t = blockIdx.x;
+    const __nv_bfloat16 *row = logits + (size_t)t * V;
+    float m = -INFINITY;
+    bool nan = false;                                    // a NaN logit makes the maximum NaN, as a plain maximum over the row does
+    auto take = [&](float f) { nan |= isnan(f); m = fmaxf(m, f); };
+    if (VEC) {
+        for (uint32_t v = threadIdx.x; v < V / 8; v += kThreads) {
+            const uint4 raw = ((const uint4 *)row)[v];
+            if (kept) ((uint4 *)(kept + (size_t)t * V))[v] = raw;
+            float f[8];
+            Unpack8(raw, f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) take(f[j]);
+        }
+    } else {
+        for (uint32_t v = threadIdx.x; v < V; v += kThreads) {
+            const __nv_bfloat16 raw = row[v];
+            if (kept) kept[(size_t)t * V + v] = raw;
+            take(__bfloat162float(raw));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    const int anyNan = __syncthreads_or(nan ? 1 : 0);
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) m = fmaxf(m, red[w]);
+    if (anyNan) m = NAN;
+    float s = 0.f;
+    if (VEC) {
+        for (uint32_t v = threadIdx.x; v < V / 8; v += kThreads) {
+            float f[8];
+            Unpack8(((const uint4 *)row)[v], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s += expf(f[j] - m);
+        }
+    } else {
+        for (uint32_t v = threadIdx.x; v < V; v += kThreads) s += expf(__bfloat162float(row[v]) - m);
+    }
+    s = RowSum<kThreads>(s, red);
+    if (threadIdx.x == 0) {
+        const int64_t target = targets[t] - vocabStart;
+        const float at = target >= 0 && target < (int64_t)V ? __bfloat162float(row[target]) - m : 0.f;
+        mx[t] = m;
+        packed[t] = s;
+        packed[T + t] = at;
+        rowLoss[t] = logf(s) - at;
+        if (keptTargets) keptTargets[t] = targets[t];
+    }
+}
+
+// The mean over the rows, in a fixed order.
+__global__ void __launch_bounds__(1024) MeanKernel(const float *__restrict__ rows, float *__restrict__ mean, uint32_t T)
+{
+    __shared__ float red[32];
+    float s = 0.f;
+    for (uint32_t t = threadIdx.x; t < T; t += 1024) s += rows[t];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    s = red[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *mean = s / (float)T;
+}
+
+// Gradient of an embedding by its few tokens: the block of a token that is the first of its id adds up the rows of all tokens with that id, in their order and in 32 bits.
+// Every block looks at all ids (16 KB at most), where the general way sorts them in some ten launches.
+constexpr uint32_t kEmbedTokens = 2048;
+__global__ void __launch_bounds__(kThreads) EmbeddingGradKernel(const int64_t *__restrict__ ids, const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ grad, uint32_t T,
+                                                               uint32_t H, int64_t V)
+{
+    __shared__ uint32_t same[kEmbedTokens / 32];
+    const uint32_t i = blockIdx.x;
+    auto idOf = [&](uint32_t t) { const int64_t id = ids[t]; return id < 0 ? id + V : id; };      // as an index from the end
+    const int64_t mine = idOf(i);
+    if (mine < 0 || mine >= V) return;
+    for (uint32_t t0 = 0; t0 < T; t0 += kThreads) {
+        const uint32_t t = t0 + threadIdx.x, word = __ballot_sync(0xffffffffu, t < T && idOf(t) == mine);
+        if ((threadIdx.x & 31) == 0 && t / 32 < kEmbedTokens / 32) same[t / 32] = word;
+    }
+    __syncthreads();
+    for (uint32_t w = 0; w <= i / 32; ++w)
+        if (w < i / 32 ? same[w] != 0 : (same[w] & ((1u << (i % 32)) - 1)) != 0) return;          // an earlier token does it
+    const uint32_t v = blockIdx.y * kThreads + threadIdx.x;
+    if (v >= H / 8) return;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (uint32_t w = i / 32; w < (T + 31) / 32; ++w)
+        for (uint32_t bits = same[w]; bits; bits &= bits - 1) {
+            float f[8];
+            Unpack8(((const uint4 *)(dy + (size_t)(w * 32 + __ffs(bits) - 1) * H))[v], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] += f[j];
+        }
+    ((uint4 *)(grad + (size_t)mine * H))[v] = Pack8(acc);
+}
+
 bool Aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
 HcclResult Launched(const char *what)
@@ -536,6 +643,31 @@ HcclResult HcclXent(int step, const void *logits, const int64_t *targets, int64_
     kern<<<(uint32_t)rows, kThreads, 0, stream>>>((const __nv_bfloat16 *)logits, targets, vocabStart, rowMax, packed, gradOut, (__nv_bfloat16 *)grad, (uint32_t)rows,
                                                  (uint32_t)vocab);
     return Launched("cross entropy");
+}
+
+HcclResult HcclXentLoss(const void *logits, const int64_t *targets, int64_t vocabStart, float *rowMax, float *packed, float *rowLoss, void *keptLogits, int64_t *keptTargets, float *loss,
+                        uint64_t rows, uint64_t vocab, cudaStream_t stream)
+{
+    if (!logits || !targets || !rowMax || !packed || !rowLoss || !loss) return HCCL_E_PTR;
+    if (rows == 0 || rows > 0x7fffffff || vocab == 0 || vocab > 0x7fffffff) return HCCL_E_PARA;
+    auto kern = vocab % 8 == 0 && Aligned16(logits) && Aligned16(keptLogits) ? XentLossKernel<true> : XentLossKernel<false>;
+    kern<<<(uint32_t)rows, kThreads, 0, stream>>>((const __nv_bfloat16 *)logits, targets, vocabStart, rowMax, packed, rowLoss, (__nv_bfloat16 *)keptLogits, keptTargets, (uint32_t)rows,
+                                                 (uint32_t)vocab);
+    CHK_RET(Launched("cross entropy"));
+    MeanKernel<<<1, 1024, 0, stream>>>(rowLoss, loss, (uint32_t)rows);
+    return Launched("cross entropy mean");
+}
+
+uint64_t HcclEmbeddingGradTokens(void) { return kEmbedTokens; }
+
+HcclResult HcclEmbeddingGrad(const int64_t *ids, const void *dy, void *grad, uint64_t tokens, uint64_t hidden, uint64_t vocab, cudaStream_t stream)
+{
+    if (!ids || !dy || !grad) return HCCL_E_PTR;
+    if (tokens == 0 || tokens > kEmbedTokens || hidden == 0 || hidden % 8 || hidden > (1u << 24) || vocab == 0 || vocab > 0x7fffffff || !Aligned16(dy) || !Aligned16(grad)) return HCCL_E_PARA;
+    if (cudaMemsetAsync(grad, 0, vocab * hidden * 2, stream) != cudaSuccess) return HCCL_E_RUNTIME;
+    EmbeddingGradKernel<<<dim3((uint32_t)tokens, (uint32_t)((hidden / 8 + kThreads - 1) / kThreads)), kThreads, 0, stream>>>(ids, (const __nv_bfloat16 *)dy, (__nv_bfloat16 *)grad,
+                                                                                                                       (uint32_t)tokens, (uint32_t)hidden, (int64_t)vocab);
+    return Launched("embedding gradient");
 }
 
 }  // extern "C"

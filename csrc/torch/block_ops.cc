@@ -685,10 +685,11 @@ py::object Xent(py::handle lh, py::handle th, int64_t vocabStart)
             const int64_t rows = l.size(0), vocab = l.size(1);
             mx = at::empty({rows}, l.options().dtype(at::kFloat));
             packed = at::empty({2, rows}, mx.options());
-            Check(HcclXent(0, l.data_ptr(), nullptr, 0, mx.data_ptr<float>(), nullptr, nullptr, nullptr, rows, vocab, Stream(l)), "HcclXent");
-            Check(HcclXent(1, l.data_ptr(), t.data_ptr<int64_t>(), vocabStart, mx.data_ptr<float>(), packed.data_ptr<float>(), nullptr, nullptr, rows, vocab, Stream(l)), "HcclXent");
-            loss = (packed.select(0, 0).log() - packed.select(0, 1)).mean();
-            if (wanted) { lk = l.clone(); tk = t.clone(); }                  // the caller may write its tensors before the backward pass
+            loss = at::empty({}, mx.options());
+            const at::Tensor each = at::empty({rows}, mx.options());
+            if (wanted) { lk = at::empty_like(l); tk = at::empty_like(t); }  // the caller may write its tensors before the backward pass
+            Check(HcclXentLoss(l.data_ptr(), t.data_ptr<int64_t>(), vocabStart, mx.data_ptr<float>(), packed.data_ptr<float>(), each.data_ptr<float>(), wanted ? lk.data_ptr() : nullptr,
+                               wanted ? tk.data_ptr<int64_t>() : nullptr, loss.data_ptr<float>(), rows, vocab, Stream(l)), "HcclXentLoss");
         }
         if (wanted) {
             node->logits = SavedVariable(lk, false);
@@ -701,6 +702,61 @@ py::object Xent(py::handle lh, py::handle th, int64_t vocabStart)
         }
     }
     return py::cast(loss);
+}
+
+// ---- embedding ---------------------------------------------------------------------------------------------------------
+// Rows of w by ids; its gradient by the few tokens' kernel.
+struct EmbeddingNode : OpNode {
+    SavedVariable ids;
+    int64_t vocab = 0, hidden = 0, tokens = 0;
+    at::TensorOptions options;
+    std::string name() const override { return "_EmbeddingBackward"; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override
+    {
+        for (int64_t v : {vocab, hidden, tokens}) args.collect(v);
+    }
+    std::vector<Saved> Keeps() override { return {{&ids, false}}; }
+    variable_list Backward(variable_list &&g) override
+    {
+        const auto [t] = Unpack(ids);
+        const at::Tensor dy = ZerosWhereUndefined(g[0], {tokens, hidden}, options);
+        bool direct = !traced && !at::GradMode::is_enabled();
+        {
+            py::gil_scoped_acquire gil;
+            if (direct)
+                direct = !Watched() && PlainGrad(dy) && Plain(t) && t.scalar_type() == at::kLong && t.device() == dy.device() && t.is_contiguous() && t.dim() == 1 && dy.dim() == 2 &&
+                         dy.size(0) == t.size(0) && dy.size(1) == hidden && t.size(0) > 0 && (uint64_t)t.size(0) <= HcclEmbeddingGradTokens();
+            if (!direct) return FromPython((*g_env.backward)("embedding", t, vocab, hidden, dy), 1);
+        }
+        const at::Tensor d = Aligned(dy), dw = at::empty({vocab, hidden}, options);
+        Check(HcclEmbeddingGrad(t.data_ptr<int64_t>(), d.data_ptr(), dw.data_ptr(), t.size(0), hidden, vocab, Stream(dw)), "HcclEmbeddingGrad");
+        return {dw};
+    }
+};
+
+py::object Embedding(py::handle wh, py::handle ih)
+{
+    const at::Tensor w = OperandArg(wh);
+    if (!w.defined() || w.dim() != 2 || w.size(1) % 8 || !PlainObject(ih.ptr())) return py::none();
+    const at::Tensor t = THPVariable_Unpack(ih.ptr());
+    if (!t.has_storage() || t.scalar_type() != at::kLong || t.device() != w.device() || !t.is_contiguous() || t.dim() != 1 || t.numel() == 0 ||
+        (uint64_t)t.size(0) > HcclEmbeddingGradTokens() || !OpNode::Wanted({w})) return py::none();
+    at::Tensor y;
+    {
+        auto node = MakeNode<EmbeddingNode>(py::none(), w);
+        py::gil_scoped_release nogil;
+        {
+            at::NoGradGuard noGrad;
+            y = at::index(w, {t});
+        }
+        node->ids = SavedVariable(t, false);
+        node->vocab = w.size(0);
+        node->hidden = w.size(1);
+        node->tokens = t.size(0);
+        node->options = w.options().requires_grad(false);
+        torch::autograd::set_history({y}, node);
+    }
+    return py::cast(y);
 }
 
 void Init(py::object tensor, py::object parameter, py::object check, py::object watched, py::object backward)
@@ -728,4 +784,5 @@ void BindBlockOps(py::module &m)
     m.def("linear", &Linear);
     m.def("mlp", &Mlp);
     m.def("xent", &Xent);
+    m.def("embedding", &Embedding);
 }

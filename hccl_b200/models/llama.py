@@ -201,6 +201,12 @@ class _VocabParallelCrossEntropy(torch.autograd.Function):
         from ..types import ReduceOp
         vloc = logits_local.shape[-1]
         ctx.fused = _block.xent_usable(logits_local, targets)
+        if ctx.fused and comm.size == 1:
+            loss, mx, packed, logits, kept = _block.xent_loss(logits_local, targets, vocab_start, ctx.needs_input_grad[0])
+            ctx.vocab_start = vocab_start
+            if ctx.needs_input_grad[0]:
+                ctx.save_for_backward(logits, kept, mx, packed)
+            return loss
         if ctx.fused:
             mx = _block.xent_row_max(logits_local)
         else:
@@ -301,7 +307,10 @@ class Llama(nn.Module):
         T = B * S
         assert T % tp == 0
         flat = tokens.reshape(-1)
-        x = self.embed[flat[rank * (T // tp):(rank + 1) * (T // tp)]]      # this rank's token shard
+        ids = flat if tp == 1 else flat[rank * (T // tp):(rank + 1) * (T // tp)]       # this rank's token shard
+        x = _block.embedding(self.embed, ids)
+        if x is None:
+            x = self.embed[ids]
         if self._rope is None or self._rope[0].shape[0] != S or self._rope[0].device != x.device:
             self._rope = _rope_tables(S, self.cfg.hidden // self.cfg.heads, self.cfg.rope_theta, x.device)
         cos, sin = self._rope

@@ -37,7 +37,10 @@ def _decl():
         l.HcclSwiGlu.argtypes = [vp, vp, u64, u64, vp]
         l.HcclSwiGluBwd.argtypes = [vp, vp, vp, u64, u64, vp]
         l.HcclXent.argtypes = [i32, vp, vp, i64, vp, vp, vp, vp, u64, u64, vp]
-        for f in (l.HcclRmsNorm, l.HcclRmsNormKeep, l.HcclRmsNormBwd, l.HcclRopeQkv, l.HcclAttentionBwdSuits, l.HcclAttentionBwd, l.HcclSwiGlu, l.HcclSwiGluBwd, l.HcclXent):
+        l.HcclXentLoss.argtypes = [vp, vp, i64, vp, vp, vp, vp, vp, vp, u64, u64, vp]
+        l.HcclEmbeddingGradTokens.restype = u64
+        l.HcclEmbeddingGrad.argtypes = [vp, vp, vp, u64, u64, u64, vp]
+        for f in (l.HcclXentLoss, l.HcclEmbeddingGrad, l.HcclRmsNorm, l.HcclRmsNormKeep, l.HcclRmsNormBwd, l.HcclRopeQkv, l.HcclAttentionBwdSuits, l.HcclAttentionBwd, l.HcclSwiGlu, l.HcclSwiGluBwd, l.HcclXent):
             f.restype = ctypes.c_int
         l._nn_declared = True
     return l
@@ -418,3 +421,54 @@ def xent_grad(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, mx:
     check(_decl().HcclXent(2, logits.data_ptr(), targets.data_ptr(), vocab_start, mx.data_ptr(), packed.data_ptr(), g.data_ptr(), out.data_ptr(), *logits.shape,
                            _stream(logits)), "HcclXent")
     return out
+
+
+def xent_loss(logits: torch.Tensor, targets: torch.Tensor, vocab_start: int, kept: bool):
+    """One rank: the mean loss, the row maxima and sums as above, and copies of logits and targets (or None) for a backward pass after they have changed."""
+    rows, vocab = logits.shape
+    mx, packed, each = (torch.empty(*s, dtype=torch.float32, device=logits.device) for s in ((rows,), (2, rows), (rows,)))
+    loss = torch.empty((), dtype=torch.float32, device=logits.device)
+    lk, tk = (torch.empty_like(logits), torch.empty_like(targets)) if kept else (None, None)
+    check(_decl().HcclXentLoss(logits.data_ptr(), targets.data_ptr(), vocab_start, mx.data_ptr(), packed.data_ptr(), each.data_ptr(), lk.data_ptr() if kept else None,
+                               tk.data_ptr() if kept else None, loss.data_ptr(), rows, vocab, _stream(logits)), "HcclXentLoss")
+    return loss, mx, packed, lk, tk
+
+
+def _embedding_backward(ids, vocab, hidden, dy):
+    return (torch.zeros(vocab, hidden, dtype=dy.dtype, device=dy.device).index_put((ids,), dy, accumulate=True),)
+
+
+PYTHON_BACKWARD["embedding"] = _embedding_backward
+
+
+class _Embedding(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, w, ids):
+        ctx.save_for_backward(ids)
+        ctx.shape = tuple(w.shape)
+        return w[ids]
+
+    @staticmethod
+    def backward(ctx, dy):
+        ids, = ctx.saved_tensors
+        vocab, hidden = ctx.shape
+        grads = _direct((), (dy,))
+        if grads is None or not _plain_tensor(ids) or ids.dtype is not torch.int64 or ids.device != dy.device or not ids.is_contiguous() \
+                or dy.shape != (*ids.shape, hidden) or not 0 < ids.numel() <= _decl().HcclEmbeddingGradTokens():
+            return (*_embedding_backward(ids, vocab, hidden, dy), None)
+        dy, = grads
+        dw = torch.empty(ctx.shape, dtype=dy.dtype, device=dy.device)
+        check(_decl().HcclEmbeddingGrad(ids.data_ptr(), dy.data_ptr(), dw.data_ptr(), ids.numel(), hidden, vocab, _stream(dw)), "HcclEmbeddingGrad")
+        return dw, None
+
+
+def embedding(w: torch.Tensor, ids: torch.Tensor) -> Optional[torch.Tensor]:
+    """w[ids] for a vector of few ids, whose gradient then takes one kernel."""
+    n = native_nodes(w)
+    if n is not None:
+        return n.embedding(w, ids)
+    if not _usable(w) or not (torch.is_grad_enabled() and w.requires_grad) or w.dim() != 2 or w.shape[1] % 8 or not _plain_tensor(ids):
+        return None
+    if ids.dtype is not torch.int64 or ids.device != w.device or not ids.is_contiguous() or ids.dim() != 1 or not 0 < ids.numel() <= _decl().HcclEmbeddingGradTokens():
+        return None
+    return _Embedding.apply(w, ids)

@@ -45,6 +45,15 @@ HcclResult HcclSwiGluBwd(const void *dh, const void *gateUp, void *dGateUp, uint
 HcclResult HcclXent(int step, const void *logits, const int64_t *targets, int64_t vocabStart, float *rowMax, float *packed, const float *gradOut, void *grad, uint64_t rows,
                     uint64_t vocab, cudaStream_t stream);
 
+/* The same on one rank, up to the loss: rowMax and packed as steps 0 and 1 leave them, rowLoss[rows] = log(packed[0]) - packed[1], loss = their mean; keptLogits and keptTargets
+ * (either may be null) receive copies. */
+HcclResult HcclXentLoss(const void *logits, const int64_t *targets, int64_t vocabStart, float *rowMax, float *packed, float *rowLoss, void *keptLogits, int64_t *keptTargets, float *loss,
+                        uint64_t rows, uint64_t vocab, cudaStream_t stream);
+/* grad[vocab, hidden] = sums of the rows of dy[tokens, hidden] by their ids (negative ones count from the end; others outside are left out), zeros elsewhere. tokens: at most
+ * HcclEmbeddingGradTokens(); hidden: a multiple of 8. */
+uint64_t HcclEmbeddingGradTokens(void);
+HcclResult HcclEmbeddingGrad(const int64_t *ids, const void *dy, void *grad, uint64_t tokens, uint64_t hidden, uint64_t vocab, cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

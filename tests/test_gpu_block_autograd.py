@@ -737,3 +737,66 @@ def test_attention_keeps_the_engine_s_rules():
     assert close(qkv.grad, ref)
     with torch.no_grad():
         assert f(qkv) is None and nodes is block.nodes()
+
+
+@pytest.mark.parametrize("native", [True, False])
+@pytest.mark.parametrize("tokens,hidden,vocab", [(1, 8, 1), (33, 264, 7), (255, 2056, 300), (257, 256, 512), (2048, 64, 50), (2049, 64, 50)])
+def test_embedding_gradient_of_few_tokens(tokens, hidden, vocab, native, monkeypatch):
+    """Ids that repeat, ids from the end, both sides of the most tokens that the kernel takes: sums in 32 bits, rounded once (the general form rounds every addition). The gradient of
+    the gradient, batched gradients and a changed id buffer are those of the plain index."""
+    from torch._dynamo import compiled_autograd
+    from hccl_b200.ops import block
+    if native:
+        _native_nodes()
+    else:
+        monkeypatch.setattr(block, "_NODES", None)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    w = torch.randn(vocab, hidden, generator=g, device="cuda").to(torch.bfloat16).requires_grad_()
+    ids = torch.randint(-vocab, vocab, (tokens,), generator=g, device="cuda")
+    dy = torch.randn(tokens, hidden, generator=g, device="cuda").to(torch.bfloat16)
+    y = block.embedding(w, ids)
+    if tokens > 2048:
+        assert y is None
+        return
+    assert torch.equal(y, w[ids]) and y.grad_fn.name().startswith("_Embedding") and _is_native(y) == native
+    got, = torch.autograd.grad(y, w, dy, retain_graph=True)
+    ref, mag = (torch.zeros(vocab, hidden, dtype=torch.float64, device="cuda").index_put((ids,), t, accumulate=True) for t in (dy.double(), dy.double().abs()))
+    _close(got, ref, mag, tokens)
+    rows = torch.bincount(ids % vocab, minlength=vocab).max().item()
+    close = lambda a, b: ((a.double() - b.double()).abs() <= (mag * rows + b.double().abs()) * 2.0 ** -8 + 1e-30).all()      # the plain form rounds as often as an id occurs
+    b1, = torch.autograd.grad(y, w, torch.stack([dy, -dy]), is_grads_batched=True, retain_graph=True)
+    assert bool(close(b1[0], ref)) and bool(close(b1[1], -ref))
+    up = dy.clone().requires_grad_()
+    first, = torch.autograd.grad(y, w, up, create_graph=True, retain_graph=True)
+    second, = torch.autograd.grad(first, up, torch.ones_like(first))
+    assert torch.equal(second, torch.ones_like(dy))
+    if native:
+        with compiled_autograd._enable(torch.compile(backend="eager")):
+            block.embedding(w, ids).backward(dy)
+        assert bool(close(w.grad, ref))
+        w.grad = None
+    ids.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(y, w, dy)
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 1), (6, 24), (300, 1000), (1025, 515), (64, 128256)])
+def test_cross_entropy_of_one_rank(rows, vocab):
+    """The loss against 64 bits, by the native node and the Python function alike: 32-bit sums over a row and over the rows."""
+    from hccl_b200.models.llama import _VocabParallelCrossEntropy as X, _cross_entropy
+    _native_nodes()
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    logits = (torch.randn(rows, vocab, generator=g, device="cuda") * 3).to(torch.bfloat16).requires_grad_()
+    targets = torch.randint(0, vocab, (rows,), generator=g, device="cuda")
+    ref = torch.nn.functional.cross_entropy(logits.double(), targets)
+    for loss in (_cross_entropy(logits, targets, _OneRank, 0), X.apply(logits, targets, _OneRank, 0)):
+        assert abs(loss.item() - ref.item()) <= 16 * 2.0 ** -23 * (logits.abs().max().item() + ref.item() + 12)
+        got, = torch.autograd.grad(loss, logits)
+        p = torch.softmax(logits.detach().double(), 1)
+        hot = torch.nn.functional.one_hot(targets, vocab).double()
+        _close(got, (p - hot) / rows, (p + hot) / rows, 64)
+    with torch.no_grad():
+        assert torch.equal(_cross_entropy(logits, targets, _OneRank, 0), loss.detach())
+        bad = logits.detach().clone()
+        bad[rows // 2, vocab // 2] = float("nan")
+        assert _cross_entropy(bad, targets, _OneRank, 0).isnan().item()
