@@ -17,6 +17,7 @@
 #pragma once
 #include "gemm_sm100_2cta.cuh"
 #include "gemm_sm100_mx.cuh"
+#include "mx_quantize.cuh"
 
 namespace hccl {
 namespace mc2 {
@@ -54,6 +55,7 @@ struct SplitKParams {
     uint32_t *errorWord;
     const uint8_t *sfB, *sfA;     // block-scaled form: scale atoms [rows / 128][K / 128][512]
     uint32_t sfAtomsA;            // 128-row atoms A's scale array holds
+    const __nv_bfloat16 *a;       // QUANT: A in bf16
     uint32_t earlyB;              // the kernel before this one wrote A only: B may be read while it runs
 };
 
@@ -68,11 +70,14 @@ __device__ __forceinline__ void ClusterArrive() { asm volatile("barrier.cluster.
 __device__ __forceinline__ void ClusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 }  // namespace splitk
 
-template <int BT_, bool MX>
+// QUANT (block-scaled, up to 32 rows per tile): A is given in bf16. The four epilogue warps, which have nothing to do before the accumulator is complete, turn this CTA's part of it into
+// e4m3 values and scales, straight into the ring, in place of the TMA loads.
+template <int BT_, bool MX, bool QUANT = false>
 __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasPerSm)) GemmKernelSplitK(const __grid_constant__ SplitKParams p)
 {
     using S = GemmSplitKSmem<BT_, MX>;
     constexpr int BT = S::BT, STAGES = S::kStages;
+    static_assert(!QUANT || (MX && BT <= 32 && STAGES >= 4), "rows that an epilogue warp quantises, stages for four of them");
     constexpr uint32_t kIdesc = MakeInstrDesc(FMT_BF16, FMT_BF16, 128, BT);
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
@@ -95,8 +100,8 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
 
     if (threadIdx.x == 0) {
         PrefetchTmap(&p.tmapB);
-        PrefetchTmap(&p.tmapA);
-        for (int s = 0; s < STAGES; ++s) { MbarInit(&full[s], 1); MbarInit(&empty[s], 1); }
+        if (!QUANT) PrefetchTmap(&p.tmapA);
+        for (int s = 0; s < STAGES; ++s) { MbarInit(&full[s], QUANT ? 2 : 1); MbarInit(&empty[s], 1); }
         MbarInit(done, 1);
         *abortWord = 0;
         MbarInitFence();
@@ -109,7 +114,7 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
     LetDependentsStart();
     const uint8_t *sfB = MX ? p.sfB + (uint64_t)(n0 / 128) * kTotal * kSfAtomBytes : nullptr;
     auto loadB = [&](uint32_t kb, uint32_t stage) {
-        MbarExpectTx(&full[stage], S::kBBytes + S::kABytes + S::kSfBytes);
+        MbarExpectTx(&full[stage], QUANT ? S::kBBytes + kSfAtomBytes : S::kBBytes + S::kABytes + S::kSfBytes);
         TmaLoad2D(sB + stage * S::kBBytes, &p.tmapB, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)n0);
         if (MX) BulkLoadG2S(sSF + stage * S::kSfBytes, sfB + (uint64_t)kb * kSfAtomBytes, kSfAtomBytes, &full[stage]);
     };
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
         if (ElectOne()) {
             uint32_t stage = 0, phase = 0;
             const uint8_t *sfA[2] = {nullptr, nullptr};
-            if (MX) {
+            if (MX && !QUANT) {
 #pragma unroll
                 for (int j = 0; j < S::kAtomsA; ++j) {
                     uint32_t atom = m0 / 128 + j;                            // rows past M: any finite scales do (their operands are zero)
@@ -134,8 +139,8 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
             for (uint32_t kb = kLo; kb < kHi; ++kb) {
                 if (!MbarWaitRelaxed(&empty[stage], phase ^ 1, abortWord, 0)) break;
                 if (kb - kLo >= early) loadB(kb, stage);
-                TmaLoad2D(sA + stage * S::kABytes, &p.tmapA, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)m0);
-                if (MX) {
+                if (!QUANT) TmaLoad2D(sA + stage * S::kABytes, &p.tmapA, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)m0);
+                if (MX && !QUANT) {
                     uint8_t *sf = sSF + stage * S::kSfBytes;
 #pragma unroll
                     for (int j = 0; j < S::kAtomsA; ++j) BulkLoadG2S(sf + (1 + j) * kSfAtomBytes, sfA[j] + (uint64_t)kb * kSfAtomBytes, kSfAtomBytes, &full[stage]);
@@ -172,6 +177,47 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
             if (ok) UmmaCommit(done);
+        }
+    }
+    if (QUANT && warp >= 4) {
+        // a warp takes every fourth k-block, so that four are on their way from memory; four lanes per row of 128 values, eight rows at a time
+        constexpr int ITEMS = BT / 8;
+        const uint32_t block = lane & 3, row = lane >> 2;
+        uint4 next[ITEMS][4];
+        auto fetch = [&](uint32_t kb) {
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                const uint32_t r = m0 + row + i * 8;
+                const uint4 *src = (const uint4 *)(p.a + (size_t)r * p.K + (size_t)kb * kMxBK + block * 32);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) next[i][j] = r < p.M ? src[j] : make_uint4(0, 0, 0, 0);
+            }
+        };
+        uint32_t kb = kLo + warp - 4, stage = (warp - 4) % STAGES, phase = (warp - 4) / STAGES & 1;
+        if (kb < kHi) fetch(kb);
+        for (; kb < kHi; kb += 4) {
+            uint4 q[ITEMS][2];
+            uint8_t se[ITEMS];
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                se[i] = QuantizeBlock(next[i], q[i]);
+                if (m0 + row + i * 8 >= p.M) se[i] = 127;
+            }
+            if (kb + 4 < kHi) fetch(kb + 4);
+            if (!MbarWaitRelaxed(&empty[stage], phase ^ 1, abortWord, 0)) break;
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                const uint32_t r = row + i * 8, inAtom = m0 % 128 + r;
+                uint4 *dst = (uint4 *)(sA + stage * S::kABytes + r * 128);        // 128-byte swizzle
+                dst[(block * 2) ^ (r & 7)] = q[i][0];
+                dst[(block * 2 + 1) ^ (r & 7)] = q[i][1];
+                sSF[stage * S::kSfBytes + kSfAtomBytes + (inAtom % 32) * 16 + inAtom / 32 * 4 + block] = se[i];
+            }
+            FenceProxyAsyncShared();
+            __syncwarp();
+            if (lane == 0) MbarArrive(&full[stage]);
+            stage += 4;
+            if (stage >= STAGES) { stage -= STAGES; phase ^= 1; }
         }
     }
     __syncwarp();

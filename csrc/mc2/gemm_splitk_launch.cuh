@@ -11,7 +11,7 @@
 namespace hccl {
 namespace mc2 {
 
-template <int BT, bool MX>
+template <int BT, bool MX, bool QUANT = false>
 HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, uint32_t split, bool outFp32,
                          bool earlyB, cudaStream_t s)
 {
@@ -19,11 +19,12 @@ HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const vo
     SplitKParams p{};
     const uint32_t elem = MX ? 1 : 2, boxK = 128 / elem;
     CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * elem, 128, boxK, elem));
-    CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * elem, BT, boxK, elem));
+    if (QUANT) p.a = (const __nv_bfloat16 *)a;
+    else CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * elem, BT, boxK, elem));
     p.C = c; p.M = M; p.N = N; p.K = K; p.split = split; p.outFp32 = outFp32; p.errorWord = GemmErrorWord();
     p.sfA = (const uint8_t *)sfa; p.sfB = (const uint8_t *)sfb; p.sfAtomsA = (M + 127) / 128; p.earlyB = earlyB;
     static std::atomic<bool> attrSet{false};
-    auto kern = GemmKernelSplitK<BT, MX>;
+    auto kern = GemmKernelSplitK<BT, MX, QUANT>;
     const size_t smem = S::kTotal + 1024;
     if (!attrSet) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return HCCL_E_RUNTIME;
@@ -67,6 +68,21 @@ HcclResult LaunchSplitK(SplitKChoice ch, const void *a, const void *sfa, const v
         case 64: return LaunchSplitKT<64, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
         case 128: return LaunchSplitKT<128, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
         case 256: return LaunchSplitKT<256, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        default: return HCCL_E_PARA;
+    }
+}
+
+// Block-scaled, A in bf16 and quantised by the kernel itself: up to 32 rows, one tile.
+inline HcclResult LaunchSplitKQuantized(SplitKChoice ch, const void *a, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32, cudaStream_t s)
+{
+    if (((uintptr_t)c | (uintptr_t)a | (uintptr_t)sfb) & 15u) {
+        HCCL_ERROR("split-K GEMM: activations %p, result %p and block scales %p must be 16-byte aligned", a, c, sfb);
+        return HCCL_E_PARA;
+    }
+    if (ch.split == 0 || ch.split > 8 || ch.split > K / kMxBK || M > ch.bt) return HCCL_E_PARA;
+    switch (ch.bt) {
+        case 16: return LaunchSplitKT<16, true, true>(a, nullptr, b, sfb, c, M, N, K, ch.split, outFp32, false, s);
+        case 32: return LaunchSplitKT<32, true, true>(a, nullptr, b, sfb, c, M, N, K, ch.split, outFp32, false, s);
         default: return HCCL_E_PARA;
     }
 }

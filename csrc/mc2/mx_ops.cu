@@ -18,6 +18,7 @@
 #include "gemm_sm100_mx.cuh"
 #include "gemm_sm100_mx_2cta.cuh"
 #include "gemm_splitk_launch.cuh"
+#include "mx_quantize.cuh"
 #include "hccl/hccl_mc2.h"
 
 namespace hccl {
@@ -29,7 +30,9 @@ namespace {
 __global__ void QuantizeMxfp8Kernel(const __nv_bfloat16 *__restrict__ in, uint8_t *__restrict__ payload, uint8_t *__restrict__ scales, uint32_t rows,
                                     uint32_t rowsPadded, uint32_t K)
 {
-    LetDependentsStart();                        // the product that reads this sets up meanwhile
+    // Starts while the kernel before it drains. The product that reads this may start when that kernel has ended, and not before: it reads B at once.
+    DependencyWait();
+    LetDependentsStart();
     const uint32_t kBlocks = K / 32;
     const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (uint64_t)rowsPadded * kBlocks) return;
@@ -40,35 +43,11 @@ __global__ void QuantizeMxfp8Kernel(const __nv_bfloat16 *__restrict__ in, uint8_
     uint4 raw[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) raw[i] = src[i];
-    float v[32];
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 *h = (const __nv_bfloat162 *)&raw[i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float2 f = __bfloat1622float2(h[j]);
-            v[i * 8 + 2 * j] = f.x; v[i * 8 + 2 * j + 1] = f.y;
-            amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-        }
-    }
-    // biased exponent of amax (finite inputs assumed; NaN / Inf saturate through the conversion below)
-    int e = (int)((__float_as_uint(amax) >> 23) & 0xff);         // floor(log2(amax)) + 127 for normal amax; 0 for zero / denormal
-    int se = e - 8;                                              // scale exponent, biased
-    if (se < 0) se = 0;
-    if (se > 254) se = 254;
-    *sf = (uint8_t)se;
-    const float inv = __uint_as_float((uint32_t)(254 - se) << 23);    // 2^(127 - se): exact reciprocal of the scale (se = 0 gives 2^127)
-    uint32_t packed[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[i * 4] * inv, v[i * 4 + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-        __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[i * 4 + 2] * inv, v[i * 4 + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-        packed[i] = (uint32_t)lo | ((uint32_t)hi << 16);
-    }
+    uint4 q[2];
+    *sf = QuantizeBlock(raw, q);
     uint4 *dst = (uint4 *)(payload + (uint64_t)r * K + (uint64_t)kb * 32);
-    dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-    dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+    dst[0] = q[0];
+    dst[1] = q[1];
 }
 
 template <int BN> HcclResult LaunchPlainMx(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32,
@@ -177,6 +156,49 @@ HcclResult GemmMxfp8(const void *a, const void *sfa, const void *b, const void *
     return LaunchPlainMx<128>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
 }
 
+// overlap: the launch may start while the kernel before it drains
+HcclResult Quantize(const void *in, void *payload, void *scales, uint64_t rows, uint64_t k, cudaStream_t stream, bool overlap)
+{
+    if (!in || !payload || !scales) return HCCL_E_PTR;
+    if (rows == 0 || k == 0 || k % 128 || rows > 0x7fffffff || k > 0x7fffffff) {
+        HCCL_ERROR("HcclQuantizeMxfp8: K (%llu) must be a non-zero multiple of 128", (unsigned long long)k);
+        return HCCL_E_PARA;
+    }
+    if (((uintptr_t)in & 15u) || ((uintptr_t)payload & 15u)) { HCCL_ERROR("HcclQuantizeMxfp8: buffers must be 16-byte aligned"); return HCCL_E_PARA; }
+    const uint64_t rowsPadded = (rows + 127) / 128 * 128;
+    const uint64_t threads = rowsPadded * (k / 32);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((uint32_t)((threads + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, QuantizeMxfp8Kernel, (const __nv_bfloat16 *)in, (uint8_t *)payload, (uint8_t *)scales, (uint32_t)rows, (uint32_t)rowsPadded,
+                                             (uint32_t)k);
+    CountLaunch();
+    if (e != cudaSuccess) { HCCL_ERROR("MXFP8 quantiser launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return HCCL_E_RUNTIME; }
+    return HCCL_SUCCESS;
+}
+
+// Split-K with the quantisation in the kernel, or no split where the quantiser comes first. Up to 16 rows always: us in a graph, quantiser and product / one kernel, 1 x 512 x 512
+// 5.05 / 3.37, 8 x 4096 x 4096 8.28 / 6.41, 16 x 14336 x 4096 15.4 / 14.4, 2 x 13328 x 5632 18.0 / 16.7. Up to 32 rows while a CTA has few k-blocks (17 x 4096 x 4096 8.64 / 8.38): four warps
+// quantise more slowly than the weights arrive (32 x 8192 x 14336 24.4 / 26.3).
+SplitKChoice ChooseQuantizing(uint64_t m, uint64_t n, uint64_t k)
+{
+    if (m == 0 || n == 0 || k == 0 || (k % 128) || (n % 8) || m > 32 || n > 0x7fffffff || k > 0x7fffffff || getenv("HCCL_MX_TILE_N")) return {};
+    const SplitKChoice sk = ChooseSplitK(m, n, k, true, false);
+    return sk.split && (sk.bt == 16 || (sk.bt == 32 && k / kMxBK <= 8 * (uint64_t)sk.split)) ? sk : SplitKChoice{};
+}
+
+bool Capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
 }  // namespace
 }  // namespace mc2
 }  // namespace hccl
@@ -190,19 +212,7 @@ uint64_t HcclMxfp8ScaleBytes(uint64_t rows, uint64_t k) { return ((rows + 127) /
 
 HcclResult HcclQuantizeMxfp8(const void *in, void *payload, void *scales, uint64_t rows, uint64_t k, cudaStream_t stream)
 {
-    if (!in || !payload || !scales) return HCCL_E_PTR;
-    if (rows == 0 || k == 0 || k % 128 || rows > 0x7fffffff || k > 0x7fffffff) {
-        HCCL_ERROR("HcclQuantizeMxfp8: K (%llu) must be a non-zero multiple of 128", (unsigned long long)k);
-        return HCCL_E_PARA;
-    }
-    if (((uintptr_t)in & 15u) || ((uintptr_t)payload & 15u)) { HCCL_ERROR("HcclQuantizeMxfp8: buffers must be 16-byte aligned"); return HCCL_E_PARA; }
-    const uint64_t rowsPadded = (rows + 127) / 128 * 128;
-    const uint64_t threads = rowsPadded * (k / 32);
-    QuantizeMxfp8Kernel<<<(uint32_t)((threads + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16 *)in, (uint8_t *)payload, (uint8_t *)scales, (uint32_t)rows,
-                                                                             (uint32_t)rowsPadded, (uint32_t)k);
-    CountLaunch();
-    if (cudaGetLastError() != cudaSuccess) return HCCL_E_RUNTIME;
-    return HCCL_SUCCESS;
+    return Quantize(in, payload, scales, rows, k, stream, true);
 }
 
 // C[M,N] = dequant(A)[M,K] * dequant(B)[N,K]^T; operands in the format above; bf16 or fp32 output. K % 128 == 0, N % 8 == 0.
@@ -212,12 +222,21 @@ HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const vo
     return GemmMxfp8(a, sfa, b, sfb, c, m, n, k, outFp32, stream, false);
 }
 
-// The same with A given in bf16: quantised into payload and scales first. The quantiser starts when everything before it is complete and lets
-// the product in at once, whose split-K form reads B meanwhile: 32 x 8192 x 14336 on one B200 26.8 us as two calls, 26.6 as one.
+int HcclQuantizeGemmMxfp8InOne(uint64_t m, uint64_t n, uint64_t k) { return ChooseQuantizing(m, n, k).split != 0; }
+
+// The same with A given in bf16: quantised into payload and scales first, or by the product itself. A quantiser ahead of a split-K product starts while the kernel before it drains
+// and lets the product in as soon as that kernel has ended, so that B is read meanwhile: 32 x 8192 x 14336 on one B200 27.1 -> 25.6 us a call. In a graph, whose
+// launches follow one another more closely, that order costs 0.4 us, and ahead of other products up to 1 (1000 x 6144 x 4096 25.1 / 26.1).
 HcclResult HcclQuantizeGemmMxfp8(const void *a, void *payload, void *scales, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
                                  cudaStream_t stream)
 {
-    CHK_RET(HcclQuantizeMxfp8(a, payload, scales, m, k, stream));
+    if (!payload && !scales) {
+        const SplitKChoice sk = ChooseQuantizing(m, n, k);
+        if (!a || !b || !sfb || !c || !sk.split) return HCCL_E_PTR;
+        return LaunchSplitKQuantized(sk, a, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    }
+    const bool few = m > 0 && n > 0 && !getenv("HCCL_MX_TILE_N") && ChooseSplitK(m, n, k, true, false).split;
+    CHK_RET(Quantize(a, payload, scales, m, k, stream, few && !Capturing(stream)));
     return GemmMxfp8(payload, scales, b, sfb, c, m, n, k, outFp32, stream, true);
 }
 

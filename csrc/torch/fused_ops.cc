@@ -77,10 +77,14 @@ std::pair<int, at::Tensor> MxMatmul(uint64_t comm, const at::Tensor &a, const at
     const int64_t m = a.size(0), k = a.size(1);
     at::Tensor o = out ? *out : at::empty({m, n}, a.options());
     cudaStream_t s = StreamOf(stream);
-    const at::Tensor act = at::empty({m * k + (int64_t)HcclMxfp8ScaleBytes(m, k)}, a.options().dtype(at::kByte));
-    uint8_t *q = act.numel() ? act.data_ptr<uint8_t>() : nullptr;
-    const HcclResult r = HcclQuantizeMatmulMxfp8(a.data_ptr(), q, q + m * k, payload.data_ptr(), scales.data_ptr(), o.data_ptr(), m, n, k, (HcclComm)(uintptr_t)comm, s);
-    if (stream) UsedOn(act, s);
+    at::Tensor act;
+    uint8_t *q = nullptr;
+    if (!HcclQuantizeGemmMxfp8InOne(m, n, k)) {
+        act = at::empty({m * k + (int64_t)HcclMxfp8ScaleBytes(m, k)}, a.options().dtype(at::kByte));
+        q = act.data_ptr<uint8_t>();
+    }
+    const HcclResult r = HcclQuantizeMatmulMxfp8(a.data_ptr(), q, q ? q + m * k : nullptr, payload.data_ptr(), scales.data_ptr(), o.data_ptr(), m, n, k, (HcclComm)(uintptr_t)comm, s);
+    if (stream && act.defined()) UsedOn(act, s);
     return {(int)r, std::move(o)};
 }
 

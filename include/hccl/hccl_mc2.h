@@ -87,7 +87,9 @@ HcclResult HcclQuantizeMxfp8(const void *in, void *payload, void *scales, uint64
 /* C[m,n] = A[m,k] * B[n,k]^T on one GPU, both operands block-scaled, bf16 (or fp32) result. */
 HcclResult HcclGemmMxfp8(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
                          cudaStream_t stream);
-/* The same with A in bf16: quantised into payload and scales first, the product may read B while that runs. */
+/* The same with A in bf16: quantised into payload and scales first, the product may read B while that runs. Where HcclQuantizeGemmMxfp8InOne(m, n, k) is not 0 both may be null: the
+ * product then quantises A itself, by the same rule. */
+int HcclQuantizeGemmMxfp8InOne(uint64_t m, uint64_t n, uint64_t k);
 HcclResult HcclQuantizeGemmMxfp8(const void *a, void *payload, void *scales, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32,
                                  cudaStream_t stream);
 /* tileN 128, 192 or 256 forces the tile width, 2192 / 2256 CTA pairs of that width, 100000 + 1000 * S + BT split-K (0 = automatic). */
@@ -101,7 +103,7 @@ HcclResult HcclMatmulReduceScatterMxfp8(const void *a, const void *sfa, const vo
                                         HcclComm comm, cudaStream_t stream);
 HcclResult HcclMatmulAllReduceMxfp8(const void *a, const void *sfa, const void *b, const void *sfb, void *out, uint64_t m, uint64_t n, uint64_t kLocal,
                                     HcclComm comm, cudaStream_t stream);
-/* Any of the three on a communicator of one rank, activations in bf16 (quantised into payload and scales in the same call). */
+/* Any of the three on a communicator of one rank, activations in bf16 (quantised into payload and scales in the same call; null as for HcclQuantizeGemmMxfp8). */
 HcclResult HcclQuantizeMatmulMxfp8(const void *a, void *payload, void *scales, const void *b, const void *sfb, void *out, uint64_t m, uint64_t n, uint64_t k, HcclComm comm,
                                    cudaStream_t stream);
 

@@ -198,3 +198,32 @@ def test_one_rank_calls_keep_their_activations_apart():
         assert all(torch.equal(a, b) for a, b in zip(got, want))
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 256), (1, 512, 512), (3, 136, 640), (8, 4096, 4096), (15, 1000, 1152), (16, 14336, 4096), (16, 264, 16384), (17, 4096, 4096), (25, 2056, 2048), (32, 4096, 4096),
+                                   (32, 1024, 14336), (33, 4096, 4096)])
+def test_products_that_quantise_their_activations(m, n, k):
+    """Few rows: the kernel that quantises for itself against the quantiser and the product, on both sides of the choice, rows and columns that do not fill a tile, blocks of zeros, of
+    the largest values, of subnormals and with a NaN. The same bits: one rule, one order of sums."""
+    from hccl_b200._lib import lib
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops import gemm as g, mxfp8 as mx
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        a, w = _wild((m, k), m + n), mx.quantize(_wild((n, k), n + k, 0.05))
+        a[0, :32] = 0
+        a[m // 2, 32:64] = 3.0e38
+        a[m - 1, 64:96] = 1.0e-39
+        for nan in (False, True):
+            if nan:
+                a[m // 3, 100] = float("nan")
+            got = mx.matmul_all_reduce(comm, a, w)
+            want = mx.gemm(mx.quantize(a), w)
+            torch.cuda.synchronize()
+            g.check_error()
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+        in_one = lib().HcclQuantizeGemmMxfp8InOne
+        in_one.argtypes = [__import__("ctypes").c_uint64] * 3
+        assert bool(in_one(m, n, k)) == (2 <= k // 128 and (m <= 16 and k >= 512 or 16 < m <= 32 and k >= 2048 and (m, n, k) != (32, 1024, 14336))), in_one(m, n, k)
+    finally:
+        comm.destroy()
