@@ -246,6 +246,8 @@ template <int D> __global__ void __launch_bounds__(kAttThreads * kGroups<D>) Att
     extern __shared__ __align__(16) __nv_bfloat16 sm[];
     __shared__ float sLse[kGroups<D>][kTile], sDot[kGroups<D>][kTile];
     static_assert((kGroups<D> - 1) * (D / 8) * 4 * kAttThreads * 4 <= kBwdBytes<D>, "the groups' parts fit");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // started while the kernel before drains: nothing touches memory before its end
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t grp = threadIdx.x / kAttThreads, tid = threadIdx.x % kAttThreads, warp = tid >> 5, lane = tid & 31;
     __nv_bfloat16 *own0 = sm, *own1 = sm + kTileElems<D>, *met0 = sm + (2 + 2 * grp) * kTileElems<D>, *met1 = met0 + kTileElems<D>;
     const uint32_t blocks = (A.seq + kTile - 1) / kTile, b = blockIdx.y, heads = A.hq / A.hk;
@@ -358,10 +360,19 @@ template <int D> HcclResult LaunchBwd(const AttArgs &A, uint32_t batch, cudaStre
         if (cudaFuncSetAttribute(AttentionBwdKernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBwdBytes<D>) != cudaSuccess) return HCCL_E_RUNTIME;
         allowed.fetch_or(bit);
     }
-    AttentionBwdKernel<D><<<dim3(blocks * (A.hq + A.hk), batch), kAttThreads * kGroups<D>, kBwdBytes<D>, stream>>>(A);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks * (A.hq + A.hk), batch);
+    cfg.blockDim = dim3(kAttThreads * kGroups<D>);
+    cfg.dynamicSmemBytes = kBwdBytes<D>;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, AttentionBwdKernel<D>, A);
     CountLaunch();
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) { HCCL_ERROR("attention backward launch failed: %s", cudaGetErrorString(e)); return HCCL_E_RUNTIME; }
+    if (e != cudaSuccess) { HCCL_ERROR("attention backward launch failed: %s", cudaGetErrorString(e)); (void)cudaGetLastError(); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
 
