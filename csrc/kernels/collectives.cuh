@@ -54,7 +54,7 @@ template <typename T, bool EMU> __device__ void AllReduceOneShotBody(KCtx &k, co
     Part p = PartOf(A.bytes, gridDim.x, blockIdx.x);
     BlockCopyToAll(n, [&](int d) { return k.Ccl((k.rank + d) % n) + (uint64_t)k.rank * slot + p.off; }, (const char *)A.in + p.off, p.len);
     if (!ChannelBarrier(k, 1)) return;
-    ReduceSlotsBy<T>(A.op, (T *)((char *)A.out + p.off), (T *)nullptr, k.Ccl(k.rank) + p.off, slot, n, p.len / sizeof(T));
+    ReduceSlotsBy<T, true>(A.op, (T *)((char *)A.out + p.off), (T *)nullptr, k.Ccl(k.rank) + p.off, slot, n, p.len / sizeof(T));
 }
 
 // ================================================================================================ AllReduce two-shot

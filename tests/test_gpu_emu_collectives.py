@@ -99,6 +99,24 @@ def test_allreduce_groups_of_copies(emu_mod, nranks, alg):
                 assert not o[count:].any()
 
 
+@pytest.mark.parametrize("alg,mult", [("SmAllReduceMesh1DOneShot", 2), ("SmAllReducePipelined", 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int8, torch.int64])
+def test_allreduce_of_two_ranks(emu_mod, dtype, alg, mult):
+    """Two slots are reduced several vectors of a thread at a time: counts below, at and above one turn of a CTA and of two, ends inside a vector, buffers that are
+    not 16-byte aligned, in place. One addition of two elements, rounded once: exact."""
+    turn = 512 * mult * 16 // dtype.itemsize
+    with emu_mod.EmuWorld(2, 8 << 20) as w:
+        for count, off, inplace in ((5, 0, False), (turn, 0, False), (turn + 1, 0, True), (4 * turn - 3, 0, False), (6 * turn + 77, 0, False), (2 * turn + 9, 1, False)):
+            bufs = [_rand(count + off, dtype, 17 * count + r)[off:] for r in range(2)]
+            acc = torch.float32 if dtype.is_floating_point else torch.int64
+            ref = (bufs[0].to(acc) + bufs[1].to(acc)).to(dtype)
+            outs = bufs if inplace else [torch.zeros(count + 2 * off + 8, dtype=dtype, device="cuda")[off:] for _ in range(2)]
+            assert w.run(CMD["ALLREDUCE"], alg, bufs, outs, count, dtype, max_ctas=2) == 0
+            for o in outs:
+                assert torch.equal(o[:count], ref)
+                assert not o[count:].any()
+
+
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.uint16, torch.uint32])
 def test_allreduce_unsigned(emu_mod, dtype):
     nranks, count = 4, 2051
