@@ -1,6 +1,7 @@
 // Kernel of a plain product. Host arithmetic alone, so that the choice can be tested without a GPU.
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 namespace hccl {
@@ -60,19 +61,38 @@ struct SplitKChoice { uint32_t bt = 0, split = 0; };
 // 967 products: with one cluster more than fit the product takes 1.4 times as long on average as with one CTA less along K.
 constexpr uint32_t kClustersAtOnce[9] = {0, 148, 71, 44, 33, 26, 22, 15, 15};
 
+// The same with two CTAs on an SM (16- to 64-row tiles), read off the step in time over 4900 products.
+constexpr uint32_t kClustersOfTwoAtOnce[9] = {0, 296, 147, 91, 71, 55, 45, 37, 33};
+
+// Time of a split-K product of one row tile, in us up to a constant, as far as it depends on the CTAs along K: a CTA's stream of B and A, at its own rate (a third of it where
+// rows start inside 32-byte sectors) and at the rate that all CTAs share, for each wave of clusters, and what a cluster and a further wave cost.
+inline double SplitKCost(uint64_t nt, uint32_t bt, uint64_t rowBytes, uint32_t s)
+{
+    const double kb = (double)(((rowBytes + 127) / 128 + s - 1) / s) * 0.128 * (128 + 0.7 * bt), rate = rowBytes % 32 ? 25 : 78;
+    auto wave = [&](uint64_t clusters) { return std::hypot(kb / rate, (double)(clusters * s) * kb / 9700); };
+    const uint64_t cap = kClustersOfTwoAtOnce[s], full = (nt - 1) / cap;
+    return (s > 1 ? 0.9 : 0.0) + 0.09 * s + (double)full * (wave(cap) + 2.4) + wave(nt - full * cap);
+}
+
 // Whether the split-K form is the better one for this product, and its shape. narrowWave: the best tiles are 64 wide on one CTA and take one wave of at
 // least 90 CTAs.
 // Measured on one B200 with weights that rotate through more than L2, us per product in a graph of many (tile kernels / split-K):
-//   rows <= 64, K >= 2048: split-K wins or ties. m x n x k = 4 x 4096 x 4096: 25.2 / 10.3; 16 x 4096 x 14336: 42.3 / 22.9; 1 x 512 x 16384:
-//     47.8 / 11.1; 8 x 28672 x 4096: 50.5 / 40.6; 64 x 128256 x 4096: 195.8 / 171; 64 x 28672 x 8192: 81.3 / 79.8. With K = 1024 it
-//     wins with up to 16 rows (16 x 8192 x 1024: 9.8 / 7.1) and not with 64 (64 x 4096 x 1024: 7.2 / 7.4).
+//   rows <= 64: split-K wins or ties from K = 768 on with up to 32 rows (20 x 5016 x 1960: 18.6 / 8.2; 512 where N >= 2000: 24 x 9376 x 616 10.0 / 6.0), from 1024 on with up to
+//     64 (44 x 584 x 1528 7.4 / 5.3, 55 x 5088 x 928 8.6 / 7.4; 39 x 2128 x 680 5.0 / 5.9), up to K = 2048 only where rows straddle sectors or N < 6000 (61 x 7224 x 1168 7.1 / 8.5);
+//     block-scaled from 512 on (30 x 18280 x 1536 13.7 / 8.0). Long K: m x n x k = 4 x 4096 x 4096: 25.2 / 10.3; 16 x 4096 x 14336: 42.3 / 22.9; 1 x 512 x 16384:
+//     47.8 / 11.1; 8 x 28672 x 4096: 50.5 / 40.6; 64 x 128256 x 4096: 195.8 / 171; 64 x 28672 x 8192: 81.3 / 79.8; 16 x 8192 x 1024: 9.8 / 7.1.
 //   more rows: where the tile kernels leave the GPU partly empty (200 x 1024 x 8192: 26.1 / 13.4; 512 x 1024 x 4096: 15.4 / 12.2), not
 //     where they have about as many CTAs as SMs (128 x 8192 x 1024: 8.1 / 10.3). One wave of 64-wide tiles is better up to K = 3700 (2400 where K straddles
 //     sectors, which costs tiles more), and for every K where 257 to 384 rows leave the second 256-row tile half empty and two CTAs along
 //     K: 193 x 4512 x 2624 11.0 / 12.7, 349 x 2216 x 2056 13.1 / 17.5, 365 x 3120 x 2880 11.7 / 16.6. Of 489 such products the choice takes 1.020 of the
 //     best kernel's time on average; split-K for all of them 1.30.
-//   CTAs in all: about one per SM while K is short (32 tiles, K 4096: split 4 10.3, 8 11.0; 64 tiles, K 1024: 2 7.1, 4 7.9), two per SM for a
-//     long K (64 tiles, K 8192: 2 27.6, 4 25.9) or several row tiles (100 x 4096 x 4096: 3 14.2, 4 13.5).
+//   more than 512 rows: where 256-row tiles with four or more CTAs along K run at once (683 x 624 x 16016: 49.4 / 21.8; 1191 x 528 x 3632: 13.7 / 13.1; 957 x 512 x 2176: 9.0 / 10.6),
+//     with three where K straddles sectors or is long (1722 x 672 x 15048: 90.7 / 52.8; 1629 x 520 x 4112: 15.4 / 16.5), with two where it straddles (1.00 at K = 4700, 0.87 at
+//     10000, aligned 1.02 at 9088). Over 276 products of 513 to 2048 rows with N up to 4096 and K from 2048 the best kernel is 1.15 times as fast as the tiles.
+//   CTAs in all, rows <= 64: about one per SM while K is short (32 tiles, K 4096: split 4 10.3, 8 11.0; 64 tiles, K 1024: 2 7.1, 4 7.9), two per SM for a
+//     long K (64 tiles, K 8192: 2 27.6, 4 25.9) or several row tiles (100 x 4096 x 4096: 3 14.2, 4 13.5). That rounds down: 92 tiles, K 3112 took one, 20.5, and with three 15.9. So
+//     with up to 64 rows another number is taken where SplitKCost gives it less than 0.88 of that (0.75 below K = 2048): over 2739 bf16 and 2173 block-scaled products (1 to 64 rows, N 512 to 28672, K 512
+//     to 16384, half of them held out of the fit) 1.016 and 1.010 of the best kernel's time on average, 1.058 and 1.044 before, these bounds on K included.
 //   65 to 512 rows, bf16, us with 64-row tiles / chosen (split x rows): one tile of 128 rows in two CTAs per SM 88 x 10120 x 7160 74 / 39 (3 x 128),
 //     122 x 10368 x 13952 91 / 56 (3 x 128), 69 x 4088 x 13504 30.7 / 24.3 (8 x 128); 256-row tiles, one CTA per SM, as many along K as run at once:
 //     336 x 3704 x 15208 143 / 76 (3 x 256 although two would run at once, 91: K straddles sectors). 64-row tiles stay where six CTAs share one
@@ -82,18 +102,31 @@ constexpr uint32_t kClustersAtOnce[9] = {0, 148, 71, 44, 33, 26, 22, 15, 15};
 inline SplitKChoice ChooseSplitK(uint64_t m, uint64_t n, uint64_t k, bool mx, bool narrowWave)
 {
     const uint64_t nt = (n + 127) / 128, tileCtas = (m + 127) / 128 * nt;       // tileCtas: CTAs that 128-wide tiles would use
-    if (m <= 64 ? (k < 2048 && (m > 16 || k < 512)) : (k < 2048 || m > 512 || tileCtas >= 90 || (narrowWave && k < (k % 16 ? 2400 : 3700)))) return {};
+    const bool straddle = !mx && k % 16 != 0;
     auto parts = [&](uint64_t s) { return (uint32_t)std::min<uint64_t>(8, std::min<uint64_t>(std::max<uint64_t>(1, s), k / 256)); };
+    auto atOnce = [&](uint64_t tiles) { uint64_t s = 8; while (s > 1 && tiles > kClustersAtOnce[s]) --s; return s; };
+    const uint64_t t256 = nt * ((m + 255) / 256);
+    if (m > 512) {
+        const uint64_t s = atOnce(t256), least = s >= 4 ? 3300 : s == 3 ? (straddle ? 3300 : 6000) : s == 2 && straddle ? 4600 : UINT64_MAX;
+        return mx || k < least ? SplitKChoice{} : SplitKChoice{256, parts(s)};
+    }
+    if (m > 64 && (k < 2048 || tileCtas >= 90 || (narrowWave && k < (straddle ? 2400 : 3700)))) return {};
+    if (m <= 64 && k < 512) return {};
+    if (m > 16 && m <= 64 && !mx && k < 2048 && (m <= 32 ? k < 768 && n < 2000 : k < 1024 || (!straddle && n >= 6000))) return {};
     const uint32_t bt = m <= 16 ? 16 : m <= 32 ? 32 : 64;
     const uint64_t tiles = nt * ((m + bt - 1) / bt), ctas = k > 6144 || m > 64 ? 256 : 148;
-    const SplitKChoice narrow{bt, parts(ctas / tiles)};
+    SplitKChoice narrow{bt, parts(ctas / tiles)};
+    if (m <= 64) {
+        const uint64_t rowBytes = mx ? k : 2 * k;
+        double cost = (k < 2048 ? 0.75 : 0.88) * SplitKCost(nt, bt, rowBytes, narrow.split);
+        for (uint32_t s = 1; s <= parts(8); ++s)
+            if (const double c = SplitKCost(nt, bt, rowBytes, s); c < cost) { narrow.split = s; cost = c; }
+    }
     if (m <= 64 || mx || narrow.split >= 6 || (k < 5000 && narrow.split >= 3)) return narrow;
     if (m <= 128) return k >= 4096 ? SplitKChoice{128, parts(256 / nt)} : SplitKChoice{};     // 72 x 7192 x 2576: 11.6, tiles 10.6
-    const uint64_t t256 = nt * ((m + 255) / 256);
-    uint64_t s = 8;
-    while (s > 1 && t256 > kClustersAtOnce[s]) --s;
+    const uint64_t s = atOnce(t256);
     if (s == 2 && narrowWave) return {};
-    return {256, parts(s == 2 && k % 16 ? 3 : s)};
+    return {256, parts(s == 2 && straddle ? 3 : s)};
 }
 
 // The kernel of C = A * B^T in bf16: split-K where `split` is not 0, else the tile.
@@ -110,12 +143,13 @@ inline PlainChoice ChoosePlain(uint64_t m, uint64_t n, uint64_t k, uint64_t sms,
 }
 
 // Pair tile width of the product with SwiGLU in its epilogue (forward: half of it gate, half up; backward: columns of the intermediate gradient), 0 = the product and the
-// element-wise kernel one after the other. Forward: wherever the plain product would not split K (few rows, bound by reading the weights); us separate / fused 60 x 2 x 512
+// element-wise kernel one after the other. Forward: wherever the plain product would not split K (few rows, bound by reading the weights; up to 64 rows only K from 2048, up to 16 from 512); us separate / fused 60 x 2 x 512
 // x 256 5.5 / 5.2, 200 x 2 x 14336 x 4096 61.2 / 60.9, 300 x 2 x 3584 x 1024 11.5 / 12.2. Backward: above 512 rows (777 x 14336 x 4096 135 / 126, 513 x 2056 x 1032 14.1 / 13.7); up to there
 // one-CTA tiles fill the GPU better: 300 x 7168 x 2048 22.8 / 24.2, 130 x 14336 x 4096 37.0 / 40.1, 256 x 512 x 256 6.3 / 8.5.
 inline uint32_t ChooseSwiGlu(uint64_t m, uint64_t ffn, uint64_t k, bool backward, uint64_t sms, bool pairsEnabled)
 {
-    if (!pairsEnabled || (backward ? m <= 512 : ChoosePlain(m, 2 * ffn, k, sms, true).splitK.split != 0)) return 0;
+    const bool few = m <= 16 ? k >= 512 : m <= 64 ? k >= 2048 : m <= 512;        // up to 64 rows split-K is worth a second kernel from there on only
+    if (!pairsEnabled || (backward ? m <= 512 : few && ChoosePlain(m, 2 * ffn, k, sms, true).splitK.split != 0)) return 0;
     const uint64_t pairs = sms / 2, rowPairs = (m + 255) / 256;
     const double k4 = (double)k / 4096;
     uint32_t best = 0;

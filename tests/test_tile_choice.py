@@ -45,6 +45,34 @@ FEW_ROWS = [
     ((343, 3032, 5328), {64: 19.2}),
 ]
 
+# the same for up to 64 rows and for more than 512: ((m, n, k, block-scaled), {1000 * S + BT: us, 0 = the tile kernels}), the kernels within 15 % of the best one
+SPLITS = [
+    ((25, 6400, 4400, 0), {4032: 13.1, 5032: 13.1, 3032: 13.7}),
+    ((32, 14928, 592, 0), {1032: 7.0, 2032: 7.5}),
+    ((2, 10688, 1320, 0), {3016: 9.2, 2016: 9.9, 1016: 10.4}),
+    ((1, 13696, 1592, 0), {2016: 11.1, 1016: 12.5}),
+    ((2, 26320, 8376, 0), {4016: 72.4, 5016: 73.4, 2016: 74.1, 6016: 77.0, 8016: 77.8, 3016: 78.2, 7016: 79.5, 1016: 83.1}),
+    ((28, 3816, 4920, 0), {7032: 11.1, 8032: 11.1, 6032: 11.8, 5032: 11.9}),
+    ((21, 7096, 568, 0), {2032: 6.1, 1032: 6.2}),
+    ((31, 1344, 1160, 0), {4032: 5.1, 3032: 5.6, 2032: 5.8}),
+    ((49, 1448, 1832, 0), {7064: 6.6, 4064: 6.8, 5064: 7.2, 6064: 7.4, 3064: 7.5}),
+    ((2, 9696, 3720, 0), {3016: 15.9, 2016: 16.4}),
+    ((24, 640, 864, 0), {3032: 4.2, 2032: 4.4}),
+    ((30, 3104, 1280, 1), {2032: 5.0, 5032: 5.1, 3032: 5.2, 4032: 5.2, 1032: 5.5}),
+    ((44, 14032, 1024, 1), {1064: 7.0, 2064: 7.5}),
+    ((56, 10664, 5120, 1), {3064: 13.8, 2064: 14.3}),
+    ((19, 3592, 1280, 1), {2032: 5.1, 3032: 5.1, 4032: 5.1, 5032: 5.1, 1032: 5.5}),
+    ((28, 16888, 1664, 1), {1032: 8.2, 2032: 9.1}),
+    ((41, 11000, 4224, 1), {3064: 12.1, 2064: 12.6}),
+    ((1172, 576, 7776, 0), {5256: 17.5, 4256: 18.9, 5128: 19.4}),
+    ((728, 1328, 7216, 0), {4256: 19.3}),
+    ((1177, 520, 10240, 0), {5256: 20.1, 5128: 21.9, 4256: 21.9}),
+    ((1322, 1120, 2408, 0), {0: 17.9, 2256: 19.9}),
+    ((922, 1976, 12360, 0), {2256: 69.0, 4256: 70.8}),
+    ((734, 1024, 14376, 0), {5256: 34.3}),
+    ((912, 536, 3512, 0), {6256: 14.2, 5256: 14.2, 4256: 15.6, 6128: 16.2}),
+]
+
 
 def _choose(tmp_path, products):
     src = tmp_path / "choose.cc"
@@ -67,3 +95,25 @@ def test_few_rows_take_a_kernel_near_the_best(tmp_path):
     for (shape, us), (split, pair, width) in zip(FEW_ROWS, _choose(tmp_path, [p for p, _ in FEW_ROWS])):
         kernel = split or ((2 if width == 256 else width) if pair else {64: 64, 128: 128, 256: 129}[width])
         assert us.get(kernel, 1e9) <= 1.08 * min(us.values()), (shape, kernel, us)
+
+
+def test_number_of_ctas_along_k(tmp_path):
+    """Up to 64 rows: as many CTAs along K as the waves of clusters make good, block-scaled too. More than 512: 256-row tiles where they pay. Every choice can be launched."""
+    src = tmp_path / "split.cc"
+    src.write_text('#include <cstdio>\n#include "mc2/tile_choice.h"\nusing namespace hccl::mc2;\nint main() { unsigned long long m, n, k; int mx; '
+                   'while (scanf("%llu %llu %llu %d", &m, &n, &k, &mx) == 4) { auto c = mx ? ChooseSplitK(m, n, k, true, false) : ChoosePlain(m, n, k, 148, true).splitK; '
+                   'printf("%u\\n", c.split ? c.split * 1000 + c.bt : 0); } }\n')
+    exe = tmp_path / "split"
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'csrc'}", str(src), "-o", str(exe)], check=True, timeout=120)
+
+    def choose(products):
+        out = subprocess.run([str(exe)], input="".join("%d %d %d %d\n" % p for p in products), capture_output=True, text=True, check=True, timeout=60)
+        return [int(v) for v in out.stdout.split()]
+
+    for (shape, us), kernel in zip(SPLITS, choose([p for p, _ in SPLITS])):
+        assert us.get(kernel, 1e9) <= 1.08 * min(us.values()), (shape, kernel, us)
+    every = [(m, n, k, mx) for m in (1, 16, 17, 32, 33, 64, 65, 512, 513, 4096, 100000) for n in (8, 120, 128, 4096, 128256) for k in (8, 128, 504, 512, 768, 2048, 3304, 16384)
+             for mx in (0, 1) if not mx or k % 128 == 0]
+    for (m, n, k, mx), kernel in zip(every, choose(every)):
+        s, bt = divmod(kernel, 1000)
+        assert not kernel or (1 <= s <= 8 and s * 256 <= max(k, 256) and bt in (16, 32, 64, 128, 256) and (not mx or bt <= 64 and (bt == 64 or m <= bt))), (m, n, k, mx, kernel)
