@@ -12,7 +12,7 @@
 // One B200, us per product before / with this kernel (weights rotating through more than L2): 4 x 4096 x 4096 25.2 / 9.3 (floor 5.1), 16 x 4096 x 14336
 // 42.3 / 21.8 (18.1), 64 x 128256 x 4096 196 / 171 (164); block-scaled 32 x 8192 x 14336 31.6 / 24.1 (18.8). What is left over the floor is start,
 // drain and the reduction, about 4 us.
-// The automatic choice takes BT = 128 and 256 for bf16 products only (ChooseSplitK).
+// The automatic choice takes BT = 128 for bf16 products only.
 // No TMA multicast. Rows of A past M and of B past N are zero-filled by the TMA loads and never stored.
 #pragma once
 #include "gemm_sm100_2cta.cuh"

@@ -117,6 +117,13 @@ template <int BN> HcclResult LaunchPlainMxPair(const void *a, const void *sfa, c
     return HCCL_SUCCESS;
 }
 
+// HCCL_MX_PAIR=0 keeps the one-CTA kernels
+MxChoice Choose(uint64_t m, uint64_t n, uint64_t k)
+{
+    const char *e = getenv("HCCL_MX_PAIR");
+    return ChooseMx(m, n, k, (uint64_t)SmCount(), !(e && e[0] == '0'));
+}
+
 // earlyB: see LaunchSplitK
 HcclResult GemmMxfp8(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint64_t m, uint64_t n, uint64_t k, int outFp32, cudaStream_t stream, bool earlyB)
 {
@@ -126,34 +133,22 @@ HcclResult GemmMxfp8(const void *a, const void *sfa, const void *b, const void *
                    (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    const char *tileEnv = getenv("HCCL_MX_TILE_N");
-    if (!tileEnv) {
-        const SplitKChoice sk = ChooseSplitK(m, n, k, true, false);
-        if (sk.split) return LaunchSplitK<true>(sk, a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream, earlyB);
-    }
-    // CTA pairs when the product about fills the GPU with pair tiles (HCCL_MX_PAIR=0 keeps the one-CTA kernels): 192-wide tiles with two
-    // accumulators or 256-wide ones with one, whose epilogue is exposed. Time of a wave of tiles, measured on one B200: 192 wide 11.2 us
-    // per 4096 of K, 256 wide 14 us per 4096 of K and 4.5 us. Us with 192- / 256-wide tiles: 2048 x 28672 x 4096 190 / 240, 1000 x 6144 x 4096
-    // 23.7 / 31.8, 600 x 6144 x 8192 56 / 44, 2048 x 4096 x 14336 110 / 104, 2048 x 4096 x 28672 230 / 205.
-    {
-        const char *e = getenv("HCCL_MX_PAIR");
-        const uint64_t pairs = (uint64_t)SmCount() / 2, rowPairs = (m + 255) / 256, t192 = rowPairs * ((n + 191) / 192), t256 = rowPairs * ((n + 255) / 256);
-        if (!(e && e[0] == '0') && !tileEnv && n >= 256 && (t192 >= pairs || t256 * 8 >= pairs * 7)) {
-            const double k4 = (double)k / 4096, c192 = (double)((t192 + pairs - 1) / pairs) * 11.2 * k4, c256 = (double)((t256 + pairs - 1) / pairs) * (14.0 * k4 + 4.5);
-            return c256 < c192 ? LaunchPlainMxPair<256>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream)
-                               : LaunchPlainMxPair<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
-        }
-    }
+    const uint32_t M = (uint32_t)m, N = (uint32_t)n, K = (uint32_t)k;
+    const bool fp32 = outFp32 != 0;
     // HCCL_MX_TILE_N = 192 | 256 picks the wide tile of large products (as for the fused operators)
-    if (tileEnv) {
+    if (const char *tileEnv = getenv("HCCL_MX_TILE_N")) {
         const int v = atoi(tileEnv);
-        const uint64_t tiles = ((m + 127) / 128) * ((n + (uint64_t)(v > 0 ? v : 256) - 1) / (uint64_t)(v > 0 ? v : 256));
-        if (v == 192 && tiles >= (uint64_t)SmCount()) return LaunchPlainMx<192>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+        const uint64_t rows = (m + 127) / 128, sms = (uint64_t)SmCount(), wide = (uint64_t)(v > 0 ? v : 256);
+        if (v == 192 && rows * ((n + wide - 1) / wide) >= sms) return LaunchPlainMx<192>(a, sfa, b, sfb, c, M, N, K, fp32, stream);
+        if (rows * ((n + 255) / 256) >= sms) return LaunchPlainMx<256>(a, sfa, b, sfb, c, M, N, K, fp32, stream);
+        return LaunchPlainMx<128>(a, sfa, b, sfb, c, M, N, K, fp32, stream);
     }
-    // 256-wide tiles (one accumulator) when they fill the GPU, 128-wide (two accumulators) otherwise
-    uint64_t tiles256 = ((m + 127) / 128) * ((n + 255) / 256);
-    if (tiles256 >= (uint64_t)SmCount()) return LaunchPlainMx<256>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
-    return LaunchPlainMx<128>(a, sfa, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
+    const auto [sk, t] = Choose(m, n, k);
+    if (sk.split) return LaunchSplitK<true>(sk, a, sfa, b, sfb, c, M, N, K, fp32, stream, earlyB);
+    if (t.pair) return t.bn == 256 ? LaunchPlainMxPair<256>(a, sfa, b, sfb, c, M, N, K, fp32, stream) : LaunchPlainMxPair<192>(a, sfa, b, sfb, c, M, N, K, fp32, stream);
+    if (t.bn == 256) return LaunchPlainMx<256>(a, sfa, b, sfb, c, M, N, K, fp32, stream);
+    if (t.bn == 192) return LaunchPlainMx<192>(a, sfa, b, sfb, c, M, N, K, fp32, stream);
+    return LaunchPlainMx<128>(a, sfa, b, sfb, c, M, N, K, fp32, stream);
 }
 
 // overlap: the launch may start while the kernel before it drains
@@ -235,7 +230,7 @@ HcclResult HcclQuantizeGemmMxfp8(const void *a, void *payload, void *scales, con
         if (!a || !b || !sfb || !c || !sk.split) return HCCL_E_PTR;
         return LaunchSplitKQuantized(sk, a, b, sfb, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     }
-    const bool few = m > 0 && n > 0 && !getenv("HCCL_MX_TILE_N") && ChooseSplitK(m, n, k, true, false).split;
+    const bool few = m > 0 && n > 0 && !getenv("HCCL_MX_TILE_N") && Choose(m, n, k).splitK.split;
     CHK_RET(Quantize(a, payload, scales, m, k, stream, few && !Capturing(stream)));
     return GemmMxfp8(payload, scales, b, sfb, c, m, n, k, outFp32, stream, true);
 }

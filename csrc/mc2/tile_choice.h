@@ -64,14 +64,15 @@ constexpr uint32_t kClustersAtOnce[9] = {0, 148, 71, 44, 33, 26, 22, 15, 15};
 // The same with two CTAs on an SM (16- to 64-row tiles), read off the step in time over 4900 products.
 constexpr uint32_t kClustersOfTwoAtOnce[9] = {0, 296, 147, 91, 71, 55, 45, 37, 33};
 
-// Time of a split-K product of one row tile, in us up to a constant, as far as it depends on the CTAs along K: a CTA's stream of B and A, at its own rate (a third of it where
-// rows start inside 32-byte sectors) and at the rate that all CTAs share, for each wave of clusters, and what a cluster and a further wave cost.
-inline double SplitKCost(uint64_t nt, uint32_t bt, uint64_t rowBytes, uint32_t s)
+// Time of a split-K product, in us up to `start`, as far as it depends on the tiles and the CTAs along K: a CTA's stream of B and A at its own rate (KB per us) and at the
+// rate that all CTAs share, for each wave of clusters, and what a cluster and a further wave cost.
+struct SplitKRates { double start, own, shared, cluster, wave; };
+inline double SplitKCost(uint64_t tiles, uint32_t bt, uint64_t rowBytes, uint32_t s, const SplitKRates &r)
 {
-    const double kb = (double)(((rowBytes + 127) / 128 + s - 1) / s) * 0.128 * (128 + 0.7 * bt), rate = rowBytes % 32 ? 25 : 78;
-    auto wave = [&](uint64_t clusters) { return std::hypot(kb / rate, (double)(clusters * s) * kb / 9700); };
-    const uint64_t cap = kClustersOfTwoAtOnce[s], full = (nt - 1) / cap;
-    return (s > 1 ? 0.9 : 0.0) + 0.09 * s + (double)full * (wave(cap) + 2.4) + wave(nt - full * cap);
+    const double kb = (double)(((rowBytes + 127) / 128 + s - 1) / s) * 0.128 * (128 + 0.7 * bt);
+    auto wave = [&](uint64_t clusters) { return std::hypot(kb / r.own, (double)(clusters * s) * kb / r.shared); };
+    const uint64_t cap = (bt <= 128 ? kClustersOfTwoAtOnce : kClustersAtOnce)[s], full = (tiles - 1) / cap;
+    return r.start + (s > 1 ? r.cluster : 0.0) + 0.09 * s + (double)full * (wave(cap) + r.wave) + wave(tiles - full * cap);
 }
 
 // Whether the split-K form is the better one for this product, and its shape. narrowWave: the best tiles are 64 wide on one CTA and take one wave of at
@@ -92,7 +93,7 @@ inline double SplitKCost(uint64_t nt, uint32_t bt, uint64_t rowBytes, uint32_t s
 //   CTAs in all, rows <= 64: about one per SM while K is short (32 tiles, K 4096: split 4 10.3, 8 11.0; 64 tiles, K 1024: 2 7.1, 4 7.9), two per SM for a
 //     long K (64 tiles, K 8192: 2 27.6, 4 25.9) or several row tiles (100 x 4096 x 4096: 3 14.2, 4 13.5). That rounds down: 92 tiles, K 3112 took one, 20.5, and with three 15.9. So
 //     with up to 64 rows another number is taken where SplitKCost gives it less than 0.88 of that (0.75 below K = 2048): over 2739 bf16 and 2173 block-scaled products (1 to 64 rows, N 512 to 28672, K 512
-//     to 16384, half of them held out of the fit) 1.016 and 1.010 of the best kernel's time on average, 1.058 and 1.044 before, these bounds on K included.
+//     to 16384, half of them held out of the fit) 1.014 and 1.010 of the best kernel's time on average, 1.058 and 1.044 before, these bounds on K included.
 //   65 to 512 rows, bf16, us with 64-row tiles / chosen (split x rows): one tile of 128 rows in two CTAs per SM 88 x 10120 x 7160 74 / 39 (3 x 128),
 //     122 x 10368 x 13952 91 / 56 (3 x 128), 69 x 4088 x 13504 30.7 / 24.3 (8 x 128); 256-row tiles, one CTA per SM, as many along K as run at once:
 //     336 x 3704 x 15208 143 / 76 (3 x 256 although two would run at once, 91: K straddles sectors). 64-row tiles stay where six CTAs share one
@@ -118,9 +119,10 @@ inline SplitKChoice ChooseSplitK(uint64_t m, uint64_t n, uint64_t k, bool mx, bo
     SplitKChoice narrow{bt, parts(ctas / tiles)};
     if (m <= 64) {
         const uint64_t rowBytes = mx ? k : 2 * k;
-        double cost = (k < 2048 ? 0.75 : 0.88) * SplitKCost(nt, bt, rowBytes, narrow.split);
+        const SplitKRates rates{0, rowBytes % 32 ? 25.0 : 78.0, 9700, 0.9, 2.4};          // a third where rows start inside 32-byte sectors
+        double cost = (k < 2048 ? 0.75 : 0.88) * SplitKCost(nt, bt, rowBytes, narrow.split, rates);
         for (uint32_t s = 1; s <= parts(8); ++s)
-            if (const double c = SplitKCost(nt, bt, rowBytes, s); c < cost) { narrow.split = s; cost = c; }
+            if (const double c = SplitKCost(nt, bt, rowBytes, s, rates); c < cost) { narrow.split = s; cost = c; }
     }
     if (m <= 64 || mx || narrow.split >= 6 || (k < 5000 && narrow.split >= 3)) return narrow;
     if (m <= 128) return k >= 4096 ? SplitKChoice{128, parts(256 / nt)} : SplitKChoice{};     // 72 x 7192 x 2576: 11.6, tiles 10.6
@@ -140,6 +142,55 @@ inline PlainChoice ChoosePlain(uint64_t m, uint64_t n, uint64_t k, uint64_t sms,
     const TileChoice t = ChooseTile(m, n, k, false, sms, pairsEnabled);
     const uint64_t narrow = !t.pair && t.bn == 64 ? (m + 127) / 128 * ((n + 63) / 64) : 0;
     return {m <= 64 ? SplitKChoice{} : ChooseSplitK(m, n, k, false, narrow >= 90 && narrow <= sms), t};
+}
+
+// The kernel of a block-scaled product: split-K where `split` is not 0, else tiles of CTA pairs (192 or 256 wide) or of one CTA (128, 192, 256).
+// Up to 64 rows see ChooseSplitK. More: the rule by which products were split up to 512 rows and K from 2048, pair tiles taken where they about fill the GPU and 256-wide
+// tiles where they do, kept most of the GPU idle just below each of its bounds. Another kernel is taken where its cost is below 0.92 of that rule's: a start, waves of
+// tiles (a quarter of them by the fraction of the GPU that the tiles fill) of a fixed part and a part along K, or SplitKCost. Fitted on one B200 to 829 products of 65 to 8192
+// rows, N 512 to 28672 and K 512 to 16384; over 828 others the choice takes 1.016 of the best kernel's time on average, the rule alone 1.080 and up to 1.72. us, rule / now:
+// 125 x 520 x 1792 7.2 / 4.9, 197 x 10544 x 15104 64.9 / 41.3, 252 x 5432 x 11392 31.9 / 21.2, 620 x 4160 x 5120 23.1 / 15.4, 739 x 1176 x 16256 32.0 / 19.8.
+struct MxChoice { SplitKChoice splitK; TileChoice tile; };
+inline MxChoice ChooseMx(uint64_t m, uint64_t n, uint64_t k, uint64_t sms, bool pairsEnabled)
+{
+    const uint64_t rows = (m + 127) / 128, pairRows = (m + 255) / 256, pairs = sms / 2, t192 = pairRows * ((n + 191) / 192), t256 = pairRows * ((n + 255) / 256);
+    const double k4 = (double)k / 4096;
+    const SplitKChoice sk = ChooseSplitK(m, n, k, true, false);
+    if (m <= 64 && sk.split) return {sk, {false, 128}};
+    const bool canPair = pairsEnabled && n >= 256;
+    auto tiles = [&](TileChoice t) {
+        constexpr double kStart[5] = {3.2, 2.9, 2.9, 2.5, 2.1}, kWave[5] = {0.46, 1.2, 2.45, 1.75, 3.85}, kAlongK[5] = {7.9, 9.4, 11.8, 8.3, 10.2};
+        const int i = t.pair ? (t.bn == 192 ? 3 : 4) : t.bn == 128 ? 0 : t.bn == 192 ? 1 : 2;
+        const uint64_t count = (t.pair ? pairRows : rows) * ((n + t.bn - 1) / t.bn), slots = t.pair ? pairs : sms;
+        const double waves = 0.75 * (double)((count + slots - 1) / slots) + 0.25 * std::max(1.0, (double)count / (double)slots);
+        return kStart[i] + waves * (kWave[i] + kAlongK[i] * k4);
+    };
+    auto split = [&](SplitKChoice c) {
+        const uint64_t count = (n + 127) / 128 * ((m + c.bt - 1) / c.bt);
+        return SplitKCost(count, c.bt, k, c.split, c.bt == 64 ? SplitKRates{2.9, 98, 16300, 1.06, 2.8} : SplitKRates{6.0, 141, 17800, 0.94, 2.45});
+    };
+    MxChoice best{sk, {false, 128}};
+    if (!sk.split) {
+        if (canPair && (t192 >= pairs || t256 * 8 >= pairs * 7)) {
+            const double c192 = (double)((t192 + pairs - 1) / pairs) * 11.2 * k4, c256 = (double)((t256 + pairs - 1) / pairs) * (14.0 * k4 + 4.5);
+            best.tile = {true, c256 < c192 ? 256u : 192u};
+        } else if (rows * ((n + 255) / 256) >= sms) best.tile = {false, 256};
+    }
+    if (m <= 64) return best;
+    double cost = 0.92 * (sk.split ? split(sk) : tiles(best.tile));
+    auto offer = [&](const MxChoice &c) {
+        const double t = c.splitK.split ? split(c.splitK) : tiles(c.tile);
+        if (t < cost) { best = c; cost = t; }
+    };
+    for (uint32_t bn : {128u, 192u, 256u}) {
+        offer({{}, {false, bn}});
+        if (canPair && bn > 128) offer({{}, {true, bn}});
+    }
+    for (uint32_t s = 1; s <= 8 && s * 256 <= k; ++s) {
+        if (m <= 512) offer({{64, s}, {false, 128}});
+        if (s > 1) offer({{256, s}, {false, 128}});
+    }
+    return best;
 }
 
 // Pair tile width of the product with SwiGLU in its epilogue (forward: half of it gate, half up; backward: columns of the intermediate gradient), 0 = the product and the

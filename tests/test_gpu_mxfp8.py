@@ -145,6 +145,20 @@ def test_block_scaled_split_k(m, n, k, bt, split):
     assert bool(((out.double() - ref).abs() <= mag * k * 2.0 ** -24 + 1e-30).all())
 
 
+@pytest.mark.parametrize("m,n,k", [(65, 520, 512), (129, 5432, 1024), (513, 640, 8192), (700, 264, 4096), (1030, 776, 2048), (620, 4160, 512), (334, 6840, 768), (300, 11616, 2048), (1024, 4736, 4096)])
+def test_chosen_kernel_of_many_rows(m, n, k):
+    """Each kind of kernel that products of more than 64 rows take, ragged: fp32 results within k roundings of the sum of magnitudes, a result in bf16 its rounding."""
+    from hccl_b200.ops import gemm as g, mxfp8 as mx
+    a, w = mx.quantize(_wild((m, k), 1 + m)), mx.quantize(_wild((n, k), 2 + n, 0.05))
+    da, dw = mx.dequantize(a).double(), mx.dequantize(w).double()
+    ref, mag = da @ dw.t(), da.abs() @ dw.abs().t()
+    out, half = mx.gemm(a, w, out_dtype=torch.float32), mx.gemm(a, w)
+    torch.cuda.synchronize()
+    g.check_error()
+    assert bool(((out.double() - ref).abs() <= mag * k * 2.0 ** -24 + 1e-30).all())
+    assert torch.equal(half, out.to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 512, 512), (32, 8192, 1024), (64, 264, 14336), (300, 1024, 2048), (2048, 512, 256)])
 def test_one_rank_operators_quantise_in_the_call(m, n, k):
     """bf16 activations on one rank: the bits of quantising first, also where the weights were written by the kernel right before the call

@@ -73,6 +73,35 @@ SPLITS = [
     ((912, 536, 3512, 0), {6256: 14.2, 5256: 14.2, 4256: 15.6, 6128: 16.2}),
 ]
 
+# block-scaled, more than 64 rows: -128, -192, -256 one-CTA tiles, -2192, -2256 pair tiles, else split-K as above
+BLOCK_SCALED = [
+    ((154, 3376, 640), {1064: 5.1, -128: 5.4, -2192: 5.7, 2064: 5.7}),
+    ((167, 7656, 1024), {-128: 6.9, 1064: 7.0, -2192: 7.8, -192: 7.9}),
+    ((2069, 1696, 896), {-256: 8.1, -128: 8.1, -2192: 8.4, -2256: 8.6, -192: 8.7}),
+    ((646, 15008, 9984), {-2192: 95.0, -2256: 96.5, -128: 106.2, -192: 108.5}),
+    ((123, 1304, 640), {1064: 4.3, 2064: 4.9}),
+    ((793, 17936, 9600), {-2256: 128.3, -192: 129.0, -2192: 132.5, -128: 140.4, -256: 142.5}),
+    ((3331, 960, 1664), {-192: 8.4, -2192: 8.4}),
+    ((72, 7624, 512), {1064: 5.4, -128: 5.6, 1128: 5.6, 1256: 5.6, -192: 6.1, -2192: 6.1, 2064: 6.2}),
+    ((5210, 12968, 7040), {-2192: 356.0, -192: 369.3, -2256: 381.1, -256: 384.0}),
+    ((471, 3320, 1152), {-128: 6.9, 1064: 6.9, -2192: 7.5, -192: 7.9}),
+    ((933, 4048, 2816), {-2256: 13.7, -256: 14.2, 1128: 14.5, 1256: 14.5, -128: 15.3, -2192: 15.6}),
+    ((223, 904, 10368), {8064: 10.1, 7064: 10.4, 6064: 10.7, 5064: 11.0, 4064: 11.1}),
+    ((98, 7352, 2432), {-128: 9.8, 2064: 9.8, 1064: 10.2, 2256: 10.2, -2192: 10.5, 4128: 10.7, -192: 11.2, 3128: 11.2}),
+    ((800, 12096, 896), {-192: 13.2, -128: 14.0}),
+    ((2087, 8240, 768), {-192: 18.0, -128: 18.8}),
+    ((767, 4808, 9472), {-2256: 31.2, -256: 34.6}),
+    ((101, 21704, 3328), {-192: 17.4, 1128: 18.8, -256: 19.6}),
+    ((424, 3016, 11008), {-128: 24.5, 2256: 24.6, 2128: 25.1, -2192: 26.1}),
+    ((233, 5632, 7936), {3256: 17.7, 3128: 18.2, -128: 19.5}),
+    ((1394, 632, 5248), {4256: 12.0, 3256: 13.0, -128: 13.7}),
+    ((748, 544, 10368), {4064: 12.2, 8256: 12.6, 7256: 13.0, 8128: 13.3, 3064: 13.6, 6256: 13.7, 7128: 13.7, 5256: 13.8}),
+    ((838, 1272, 6016), {2064: 13.3, 4128: 13.5, 3256: 13.8, 3128: 14.5, -128: 15.1}),
+    ((261, 22368, 11904), {-256: 93.2, -192: 101.9, -128: 104.7}),
+    ((252, 18048, 1536), {-128: 11.8, -2256: 11.8, -256: 12.0, 1128: 12.0, -2192: 12.3, 1256: 12.8}),
+    ((279, 10192, 2688), {-256: 14.3, -128: 15.1, 1128: 15.1, -2192: 16.1}),
+]
+
 
 def _choose(tmp_path, products):
     src = tmp_path / "choose.cc"
@@ -117,3 +146,27 @@ def test_number_of_ctas_along_k(tmp_path):
     for (m, n, k, mx), kernel in zip(every, choose(every)):
         s, bt = divmod(kernel, 1000)
         assert not kernel or (1 <= s <= 8 and s * 256 <= max(k, 256) and bt in (16, 32, 64, 128, 256) and (not mx or bt <= 64 and (bt == 64 or m <= bt))), (m, n, k, mx, kernel)
+
+
+def test_block_scaled_products_of_many_rows(tmp_path):
+    """A kernel near the best, and one that can be launched: pairs only where they are enabled and N has a tile of them, 64-row tiles from whole scale atoms on."""
+    src = tmp_path / "mx.cc"
+    src.write_text('#include <cstdio>\n#include "mc2/tile_choice.h"\nint main() { unsigned long long m, n, k; int pairs; while (scanf("%llu %llu %llu %d", &m, &n, &k, &pairs) == 4) { '
+                   'auto c = hccl::mc2::ChooseMx(m, n, k, 148, pairs); printf("%d\\n", c.splitK.split ? (int)(c.splitK.split * 1000 + c.splitK.bt) '
+                   ': c.tile.pair ? -(int)(2000 + c.tile.bn) : -(int)c.tile.bn); } }\n')
+    exe = tmp_path / "mx"
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'csrc'}", str(src), "-o", str(exe)], check=True, timeout=120)
+
+    def choose(products):
+        out = subprocess.run([str(exe)], input="".join("%d %d %d %d\n" % p for p in products), capture_output=True, text=True, check=True, timeout=60)
+        return [int(v) for v in out.stdout.split()]
+
+    for (shape, us), kernel in zip(BLOCK_SCALED, choose([p + (1,) for p, _ in BLOCK_SCALED])):
+        assert us.get(kernel, 1e9) <= 1.08 * min(us.values()), (shape, kernel, us)
+    every = [(m, n, k, pairs) for m in (1, 17, 33, 64, 65, 129, 513, 4096, 100000) for n in (8, 248, 256, 4096, 128256) for k in (128, 256, 768, 2048, 16384) for pairs in (0, 1)]
+    for (m, n, k, pairs), kernel in zip(every, choose(every)):
+        if kernel > 0:
+            s, bt = divmod(kernel, 1000)
+            assert 1 <= s <= 8 and s * 128 <= k and bt in (16, 32, 64, 256) and (m <= bt or bt >= 64)
+        else:
+            assert kernel in (-128, -192, -256) or (kernel in (-2192, -2256) and pairs and n >= 256), (m, n, k, pairs, kernel)
