@@ -49,6 +49,7 @@ struct MoeState {
     uint64_t wsOff = 0;
     uint32_t ctas = 0;
     bool solo = false;
+    bool rings = false;           // one rank: rows move through shared memory (moe_bulk.cuh)
     uint32_t bulkCtas = 0;        // one rank: CTAs of the kernels that fill an SM
     uint32_t lastTokens = 0;
 };
@@ -78,10 +79,14 @@ uint32_t SoloCtas(const MoeArgs &a, uint32_t segVecs, uint32_t ctas)
     return (uint32_t)std::min<uint64_t>(ctas, items);
 }
 
-// The shared memory of the one-rank kernels, on the current device.
+// Whether the current device grants the shared memory of the one-rank kernels.
 bool RingsAllowed()
 {
-    auto allow = [](const void *fn, uint32_t bytes) { return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess; };
+    auto allow = [](const void *fn, uint32_t bytes) {
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess) return true;
+        (void)cudaGetLastError();
+        return false;
+    };
     return allow((const void *)MoeDispatchBulkKernel<false>, kDispatchRing) && allow((const void *)MoeDispatchBulkKernel<true>, kDispatchRing) &&
            allow(CombineBulk(1), kCombineSmem) && allow(CombineBulk(4), kCombineSmem) && allow(CombineBulk(8), kCombineSmem) && allow(CombineBulk(16), kCombineSmem);
 }
@@ -112,7 +117,7 @@ template <bool EMU> HcclResult LaunchMoe(bool dispatch, const DevComm *comms, co
 {
     MoeArgs av = a;
     void *params[] = {(void *)&comms, (void *)&av, (void *)&emuArgs};
-    const void *fn = dispatch ? (const void *)MoeDispatchKernel<EMU>
+    const void *fn = dispatch ? (const void *)MoeDispatchKernel<EMU, false>
                               : a.K <= 8 ? (const void *)MoeCombineKernel<EMU, false, 8> : (const void *)MoeCombineKernel<EMU, false, 16>;
     const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(ctas, ranksY), dim3(kMoeThreads), params, 0, s);
     if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u x %u)", cudaGetErrorString(e), ctas, ranksY); return HCCL_E_RUNTIME; }
@@ -143,7 +148,9 @@ HcclResult HcclMoeCreate(HcclComm comm, const HcclMoeConfig *config, HcclMoeHand
     st->solo = c->nranks == 1;
     st->bulkCtas = (uint32_t)SmCountNow();
     if (const char *e = getenv("HCCL_MOE_CTAS")) { int v = atoi(e); if (v > 0 && v <= SmCountNow()) st->ctas = st->bulkCtas = (uint32_t)v; }
-    if (st->solo && !RingsAllowed()) { HCCL_ERROR("MoE: %u bytes of shared memory per CTA are not available", kCombineSmem); delete st; return HCCL_E_RUNTIME; }
+    // the register kernels where the rings' shared memory is not granted, or with HCCL_MOE_RINGS=0
+    const char *rings = getenv("HCCL_MOE_RINGS");
+    st->rings = st->solo && !(rings && rings[0] == '0') && RingsAllowed();
     st->L = MakeLayout(*config);
     HcclResult r = SymAlloc(c, st->L.total, &st->ws);
     if (r != HCCL_SUCCESS) { delete st; return r; }
@@ -173,7 +180,9 @@ HcclResult HcclMoeDispatch(HcclMoeHandle handle, const void *x, const int32_t *t
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.x = x;
     a.topkIdx = topkIdx;
-    if (st->solo) {
+    if (st->solo && !st->rings) {
+        CHK_RET(LaunchSolo((const void *)MoeDispatchKernel<false, true>, c->devCommPtr, a, SoloCtas(a, kSegVecs, st->bulkCtas), kMoeThreads, 0, stream));
+    } else if (st->solo) {
         const void *fn = a.mxfp8 ? (const void *)MoeDispatchBulkKernel<true> : (const void *)MoeDispatchBulkKernel<false>;
         CHK_RET(LaunchSolo(fn, c->devCommPtr, a, SoloCtas(a, kSegVecs, st->bulkCtas), kMoeThreads, kDispatchRing, stream));
     } else {
@@ -209,12 +218,13 @@ HcclResult HcclMoeCombine(HcclMoeHandle handle, const float *topkWeights, void *
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
     a.weights = topkWeights;
     a.out = out;
+    const bool few = (uint64_t)a.T * (a.H / 8) <= (uint64_t)st->bulkCtas * kMoeWarps * 2 * kSegVecsFew;
     if (!st->solo) {
         CHK_RET(LaunchMoe<false>(false, c->devCommPtr, a, nullptr, st->ctas, 1, stream));
-    } else if ((uint64_t)a.T * (a.H / 8) <= (uint64_t)st->bulkCtas * kMoeWarps * 2 * kSegVecsFew) {
+    } else if (few || !st->rings) {
         // Up to two pieces per warp: the kernel that loads into registers has no tables to fill first. Us with it / with the ring, top-8, 256 experts, hidden
         // 7168: 64 tokens 3.0 / 3.6, 128 4.0 / 4.4, 256 6.5 / 6.4, 512 14.6 / 12.9; 4000 x 1024 top-1 7.0 / 6.4.
-        a.segVecs = kSegVecsFew;
+        if (few) a.segVecs = kSegVecsFew;
         const void *fn = a.K <= 8 ? (const void *)MoeCombineKernel<false, true, 8> : (const void *)MoeCombineKernel<false, true, 16>;
         CHK_RET(LaunchSolo(fn, c->devCommPtr, a, SoloCtas(a, a.segVecs, st->bulkCtas), kMoeThreads, 0, stream));
     } else {

@@ -382,3 +382,10 @@ def test_one_rank_rings(T, E, K, H, mxfp8, ctas, monkeypatch):
         d.close()
     finally:
         comm.destroy()
+
+
+@pytest.mark.parametrize("T,E,K,H,mxfp8", [(1, 8, 2, 1024, False), (333, 256, 7, 4352, True), (2500, 60, 6, 1024, False), (700, 64, 16, 512, True)])
+def test_one_rank_without_rings(T, E, K, H, mxfp8, monkeypatch):
+    """The kernels that move rows through registers, for contexts without the rings' shared memory: the same rows, scales and sums."""
+    monkeypatch.setenv("HCCL_MOE_RINGS", "0")
+    test_one_rank_rings(T, E, K, H, mxfp8, "", monkeypatch)
