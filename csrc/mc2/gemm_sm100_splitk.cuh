@@ -12,7 +12,7 @@
 // One B200, us per product before / with this kernel (weights rotating through more than L2): 4 x 4096 x 4096 25.2 / 9.3 (floor 5.1), 16 x 4096 x 14336
 // 42.3 / 21.8 (18.1), 64 x 128256 x 4096 196 / 171 (164); block-scaled 32 x 8192 x 14336 31.6 / 24.1 (18.8). What is left over the floor is start,
 // drain and the reduction, about 4 us.
-// The automatic choice takes BT = 128 for bf16 products only.
+// The automatic choice takes BT = 128 and 192 for bf16 products only. 192 rows, one CTA per SM with five stages: 384 x 4096 x 14336 41.5 us, 128 x 128 tiles of one CTA 76.9, 256 rows 50.0.
 // No TMA multicast. Rows of A past M and of B past N are zero-filled by the TMA loads and never stored.
 #pragma once
 #include "gemm_sm100_2cta.cuh"
@@ -23,14 +23,14 @@ namespace hccl {
 namespace mc2 {
 
 template <int BT_, bool MX_> struct GemmSplitKSmem {
-    static_assert(BT_ == 16 || BT_ == 32 || BT_ == 64 || BT_ == 128 || BT_ == 256, "rows of A per tile");
+    static_assert(BT_ == 16 || BT_ == 32 || BT_ == 64 || BT_ == 128 || (BT_ == 192 && !MX_) || BT_ == 256, "rows of A per tile; block-scaled ones start on half a scale atom");
     static constexpr int BT = BT_;
     static constexpr int kStageK = MX_ ? kMxBK : kBK;                        // elements of K per stage: 128 bytes per row either way
     static constexpr int kBBytes = 128 * 128;                                // 128 rows of B
     static constexpr int kABytes = BT * 128;
     static constexpr int kAtomsA = (BT + 127) / 128;                         // scale atoms of A (block-scaled form)
     static constexpr int kSfBytes = MX_ ? (1 + kAtomsA) * kSfAtomBytes : 0;
-    static constexpr int kStages = BT <= 16 ? (MX_ ? 5 : 6) : BT <= 32 ? 5 : BT <= 64 ? 4 : BT <= 128 ? 3 : 4;   // BT <= 128: two CTAs per SM
+    static constexpr int kStages = BT <= 16 ? (MX_ ? 5 : 6) : BT <= 32 ? 5 : BT <= 64 ? 4 : BT <= 128 ? 3 : BT <= 192 ? 5 : 4;   // BT <= 128: two CTAs per SM
     static constexpr int kRing = kStages * (kBBytes + kABytes);
     static constexpr int kSfOff = kRing;
     static constexpr int kBarOff = kSfOff + kStages * kSfBytes;

@@ -67,6 +67,7 @@ HcclResult LaunchSplitK(SplitKChoice ch, const void *a, const void *sfa, const v
         case 32: return LaunchSplitKT<32, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
         case 64: return LaunchSplitKT<64, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
         case 128: return LaunchSplitKT<128, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 192: if constexpr (!MX) return LaunchSplitKT<192, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s); else return HCCL_E_PARA;
         case 256: return LaunchSplitKT<256, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
         default: return HCCL_E_PARA;
     }

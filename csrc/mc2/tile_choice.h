@@ -16,7 +16,7 @@ namespace mc2 {
 // and 1.108, 1.42 at most. With sectors and 128-byte lines taken for the same, K of 16s took 1.046 and up to 1.40: 5200 x 24872 x 864 274 us with 512
 // columns, 195 with 256. Where rows start on sectors a width above 256 has to win by 2 %: 998 x 9128 x 5104 76.4 us with 512 columns and 68.2 with 256,
 // 1358 x 12120 x 4480 129.5 and 113.9, 1000 x 6144 x 4096 42.1 with 352 columns and 43.0.
-struct TileChoice { bool pair; uint32_t bn; };
+struct TileChoice { bool pair; uint32_t bn; double cost = 0; };          // cost: about 0.1 us
 inline TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposedB, uint64_t sms, bool pairsEnabled)
 {
     const uint64_t pairs = sms / 2, rows = (m + 127) / 128, rowPairs = (rows + 1) / 2;
@@ -33,9 +33,9 @@ inline TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposed
         const double whole = straddle ? 0.5 : 0.7, start = bn <= 256 ? 0 : straddle ? 20 : 45;
         return 40 + (whole * waves(tiles, pairs) + (1 - whole) * filled(tiles, pairs)) * (start + k4 * (bn + (straddle ? 200 : 45)));
     };
-    TileChoice best{false, 64};
-    double cost = one(64);
-    auto offer = [&](bool isPair, uint32_t bn, double c) { if (c <= cost) { best = {isPair, bn}; cost = c; } };
+    TileChoice best{false, 64, one(64)};
+    double &cost = best.cost;
+    auto offer = [&](bool isPair, uint32_t bn, double c) { if (c <= cost) best = {isPair, bn, c}; };
     offer(false, 128, one(128));
     // 256-wide one-CTA tiles where N is made of them (another N was not measured)
     if (!transposedB && n % 256 == 0) offer(false, 256, one(256));
@@ -54,7 +54,7 @@ inline TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposed
     return best;
 }
 
-// bt rows of A per tile (16, 32, 64, 128, 256), split CTAs along K per tile (1 ... 8)
+// bt rows of A per tile (16, 32, 64, 128, 192, 256), split CTAs along K per tile (1 ... 8)
 struct SplitKChoice { uint32_t bt = 0, split = 0; };
 
 // Clusters of 1 ... 8 CTAs that run at once with one CTA on an SM: SMs come in groups that a cluster does not cross. Read off the step in time over
@@ -131,6 +131,35 @@ inline SplitKChoice ChooseSplitK(uint64_t m, uint64_t n, uint64_t k, bool mx, bo
     return {256, parts(s == 2 && straddle ? 3 : s)};
 }
 
+// The same for more than 64 rows, beside the tile that would be taken.
+inline SplitKChoice ChooseSplitK(uint64_t m, uint64_t n, uint64_t k, const TileChoice &t, uint64_t sms)
+{
+    const uint64_t narrow = !t.pair && t.bn == 64 ? (m + 127) / 128 * ((n + 63) / 64) : 0;
+    return ChooseSplitK(m, n, k, false, narrow >= 90 && narrow <= sms);
+}
+
+// Split-K with tiles of 192 or 256 rows, as many CTAs along K as run at once, where it beats the tiles (or ChooseSplitK's 256-row tiles) by its cost: 257 to 384 rows leave half of a second
+// 256-row tile empty and three 128-row tiles of one CTA each wait for their operands, 384 x 4096 x 14336 76.9 us, now 41.5. Measured on one B200, 60 to 300 tiles of 128 x
+// 128, us before / now: 367 x 3792 x 13504 55.0 / 40.5, 305 x 2528 x 14336 35.5 / 28.3, 671 x 2032 x 7920 38.0 / 30.1, 156 x 5736 x 15496 95.2 / 66.7. Over 426 products of 129 to 1100 rows and K from
+// 4500 0.960 of the time before on average; two are 3 to 5 % slower. With a shorter K it is mixed: K = 3840 up to 17 % faster and up to 13 % slower, 273 x 4280 x 2048 11.4 / 13.2.
+inline SplitKChoice ChooseWideSplit(uint64_t m, uint64_t n, uint64_t k, const TileChoice &t, SplitKChoice sk)
+{
+    if (m <= 128 || k < 4500 || (sk.split && sk.bt != 256)) return sk;
+    auto cost = [&](uint32_t bt, uint64_t s) {
+        const double part = (double)k / 4096 / (double)s;
+        if (bt == 192) return k % 16 ? 6.9 + 0.1 * (double)s + 32.2 * part : 4.5 + 1.2 * (double)s + 18.9 * part;
+        return k % 16 ? 7.7 + 37.6 * part : 6.1 + 0.7 * (double)s + 24.65 * part;
+    };
+    double least = sk.split ? 0.97 * cost(256, sk.split) : 0.9 * 0.084 * t.cost;
+    for (uint32_t bt : {192u, 256u}) {
+        const uint64_t tiles = (n + 127) / 128 * ((m + bt - 1) / bt);
+        uint64_t s = 8;
+        while (s > 1 && tiles > kClustersAtOnce[s]) --s;
+        if (s > 1 && cost(bt, s) < least) { sk = {bt, (uint32_t)s}; least = cost(bt, s); }
+    }
+    return sk;
+}
+
 // The kernel of C = A * B^T in bf16: split-K where `split` is not 0, else the tile.
 struct PlainChoice { SplitKChoice splitK; TileChoice tile; };
 inline PlainChoice ChoosePlain(uint64_t m, uint64_t n, uint64_t k, uint64_t sms, bool pairsEnabled)
@@ -140,8 +169,7 @@ inline PlainChoice ChoosePlain(uint64_t m, uint64_t n, uint64_t k, uint64_t sms,
         if (sk.split) return {sk, {false, 64}};
     }
     const TileChoice t = ChooseTile(m, n, k, false, sms, pairsEnabled);
-    const uint64_t narrow = !t.pair && t.bn == 64 ? (m + 127) / 128 * ((n + 63) / 64) : 0;
-    return {m <= 64 ? SplitKChoice{} : ChooseSplitK(m, n, k, false, narrow >= 90 && narrow <= sms), t};
+    return {m <= 64 ? SplitKChoice{} : ChooseWideSplit(m, n, k, t, ChooseSplitK(m, n, k, t, sms)), t};
 }
 
 // The kernel of a block-scaled product: split-K where `split` is not 0, else tiles of CTA pairs (192 or 256 wide) or of one CTA (128, 192, 256).
@@ -199,8 +227,12 @@ inline MxChoice ChooseMx(uint64_t m, uint64_t n, uint64_t k, uint64_t sms, bool 
 // one-CTA tiles fill the GPU better: 300 x 7168 x 2048 22.8 / 24.2, 130 x 14336 x 4096 37.0 / 40.1, 256 x 512 x 256 6.3 / 8.5.
 inline uint32_t ChooseSwiGlu(uint64_t m, uint64_t ffn, uint64_t k, bool backward, uint64_t sms, bool pairsEnabled)
 {
-    const bool few = m <= 16 ? k >= 512 : m <= 64 ? k >= 2048 : m <= 512;        // up to 64 rows split-K is worth a second kernel from there on only
-    if (!pairsEnabled || (backward ? m <= 512 : few && ChoosePlain(m, 2 * ffn, k, sms, true).splitK.split != 0)) return 0;
+    // not every product that splits K is worth a second kernel: up to 64 rows from these K on, more by ChooseSplitK's rule
+    auto splits = [&] {
+        if (m <= 64) return (m <= 16 ? k >= 512 : k >= 2048) && ChooseSplitK(m, 2 * ffn, k, false, false).split != 0;
+        return m <= 512 && ChooseSplitK(m, 2 * ffn, k, ChooseTile(m, 2 * ffn, k, false, sms, true), sms).split != 0;
+    };
+    if (!pairsEnabled || (backward ? m <= 512 : splits())) return 0;
     const uint64_t pairs = sms / 2, rowPairs = (m + 255) / 256;
     const double k4 = (double)k / 4096;
     uint32_t best = 0;

@@ -76,6 +76,13 @@ def test_gemm_split_k(shape, bt, split, out_dtype):
     assert bool((out[M] == 7.0).all())
 
 
+@pytest.mark.parametrize("shape,split", [((192, 128, 512), 1), ((193, 264, 520), 2), ((384, 136, 4104), 4), ((577, 520, 2048), 8), ((1, 8, 64), 1), ((384, 4096, 4608), 0), ((300, 2528, 4512), 0)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_split_k_of_192_rows(shape, split, out_dtype):
+    """192 rows of A per tile: whole tiles, one row more, one row, uneven K parts, and (0) where the choice takes it."""
+    test_gemm_split_k(shape, 192 if split else 0, split, out_dtype)
+
+
 @pytest.mark.parametrize("shape", [(65, 4088, 5128), (128, 8200, 5000), (129, 1744, 5240), (200, 520, 2048), (257, 3704, 5128), (512, 1448, 5128), (512, 2824, 2048), (300, 5408, 2056)])
 def test_gemm_split_k_of_65_to_512_rows(shape):
     """Products that the automatic choice sends to 64-, 128- and 256-row split-K tiles, and the first beyond its lines (bound as above)."""

@@ -71,6 +71,16 @@ SPLITS = [
     ((922, 1976, 12360, 0), {2256: 69.0, 4256: 70.8}),
     ((734, 1024, 14376, 0), {5256: 34.3}),
     ((912, 536, 3512, 0), {6256: 14.2, 5256: 14.2, 4256: 15.6, 6128: 16.2}),
+    ((158, 6040, 2720, 0), {2192: 14.2, 0: 14.3, 2064: 15.2, 2256: 15.7}),
+    ((480, 8376, 3136, 0), {0: 23.2, 1256: 26.1}),
+    ((305, 2528, 14336, 0), {3192: 28.3}),
+    ((180, 5376, 14912, 0), {3192: 36.5, 3256: 40.8}),
+    ((133, 7432, 5568, 0), {2192: 22.4, 2256: 25.1}),
+    ((150, 7024, 10368, 0), {2192: 34.6}),
+    ((205, 6528, 14656, 0), {2256: 55.0, 5256: 56.5, 4256: 62.1, 2128: 62.8}),
+    ((422, 3904, 14464, 0), {2256: 53.4, 2128: 59.4}),
+    ((448, 3336, 13504, 0), {2256: 48.3, 2128: 55.1}),
+    ((210, 6752, 10968, 0), {2256: 61.1, 4256: 62.1}),
 ]
 
 # block-scaled, more than 64 rows: -128, -192, -256 one-CTA tiles, -2192, -2256 pair tiles, else split-K as above
@@ -145,7 +155,7 @@ def test_number_of_ctas_along_k(tmp_path):
              for mx in (0, 1) if not mx or k % 128 == 0]
     for (m, n, k, mx), kernel in zip(every, choose(every)):
         s, bt = divmod(kernel, 1000)
-        assert not kernel or (1 <= s <= 8 and s * 256 <= max(k, 256) and bt in (16, 32, 64, 128, 256) and (not mx or bt <= 64 and (bt == 64 or m <= bt))), (m, n, k, mx, kernel)
+        assert not kernel or (1 <= s <= 8 and s * 256 <= max(k, 256) and bt in (16, 32, 64, 128, 192, 256) and (not mx or bt <= 64 and (bt == 64 or m <= bt))), (m, n, k, mx, kernel)
 
 
 def test_block_scaled_products_of_many_rows(tmp_path):
