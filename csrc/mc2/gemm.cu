@@ -283,7 +283,8 @@ HcclResult HcclGemmBf16Nn(const void *a, const void *b, void *c, uint64_t m, uin
         HCCL_ERROR("HcclGemmBf16Nn: unsupported shape %llux%llux%llu (K and N must be multiples of 8)", (unsigned long long)m, (unsigned long long)n, (unsigned long long)k);
         return HCCL_E_PARA;
     }
-    const TileChoice t = ChooseTile(m, n, k, true, SmCount(), Gemm2CtaEnabled());
+    const auto [sk, t] = ChooseNn(m, n, k, SmCount(), Gemm2CtaEnabled());
+    if (sk.split) return LaunchSplitK<false, true>(sk, a, nullptr, b, nullptr, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.pair && t.bn == 512) return LaunchWide<true>(512, a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, GroupMOverride(8), stream);
     if (t.pair) return LaunchPlain2CtaT<256, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);
     if (t.bn == 128) return LaunchPlain<128, true>(a, b, c, (uint32_t)m, (uint32_t)n, (uint32_t)k, outFp32 != 0, stream);

@@ -46,7 +46,7 @@ template <int BT_, bool MX_> struct GemmSplitKSmem {
 };
 
 struct SplitKParams {
-    CUtensorMap tmapB;            // [N, K], box 128 rows
+    CUtensorMap tmapB;            // [N, K], box 128 rows; BMN: [K, N], box 64 columns x 64 rows of K
     CUtensorMap tmapA;            // [M, K], box BT rows
     void *C;
     uint32_t M, N, K;
@@ -70,15 +70,17 @@ __device__ __forceinline__ void ClusterArrive() { asm volatile("barrier.cluster.
 __device__ __forceinline__ void ClusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 }  // namespace splitk
 
+// BMN: B is [K, N] row-major, read MN-major (see GemmKernel).
 // QUANT (block-scaled, up to 32 rows per tile): A is given in bf16. The four epilogue warps, which have nothing to do before the accumulator is complete, turn this CTA's part of it into
 // e4m3 values and scales, straight into the ring, in place of the TMA loads.
-template <int BT_, bool MX, bool QUANT = false>
+template <int BT_, bool MX, bool QUANT = false, bool BMN = false>
 __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasPerSm)) GemmKernelSplitK(const __grid_constant__ SplitKParams p)
 {
     using S = GemmSplitKSmem<BT_, MX>;
     constexpr int BT = S::BT, STAGES = S::kStages;
     static_assert(!QUANT || (MX && BT <= 32 && STAGES >= 4), "rows that an epilogue warp quantises, stages for four of them");
-    constexpr uint32_t kIdesc = MakeInstrDesc(FMT_BF16, FMT_BF16, 128, BT);
+    static_assert(!BMN || !MX, "MN-major operands are bf16");
+    constexpr uint32_t kIdesc = MakeInstrDesc(FMT_BF16, FMT_BF16, 128, BT) | (BMN ? kInstrAMajorMN : 0u);
     extern __shared__ uint8_t smemRaw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
     uint8_t *sB = smem;
@@ -115,7 +117,12 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
     const uint8_t *sfB = MX ? p.sfB + (uint64_t)(n0 / 128) * kTotal * kSfAtomBytes : nullptr;
     auto loadB = [&](uint32_t kb, uint32_t stage) {
         MbarExpectTx(&full[stage], QUANT ? S::kBBytes + kSfAtomBytes : S::kBBytes + S::kABytes + S::kSfBytes);
-        TmaLoad2D(sB + stage * S::kBBytes, &p.tmapB, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)n0);
+        if (BMN) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) TmaLoad2D(sB + stage * S::kBBytes + j * kMnBoxBytes, &p.tmapB, &full[stage], (int32_t)(n0 + j * 64), (int32_t)(kb * S::kStageK));
+        } else {
+            TmaLoad2D(sB + stage * S::kBBytes, &p.tmapB, &full[stage], (int32_t)(kb * S::kStageK), (int32_t)n0);
+        }
         if (MX) BulkLoadG2S(sSF + stage * S::kSfBytes, sfB + (uint64_t)kb * kSfAtomBytes, kSfAtomBytes, &full[stage]);
     };
     const uint32_t early = !p.earlyB ? 0 : kHi - kLo < (uint32_t)STAGES ? kHi - kLo : (uint32_t)STAGES;
@@ -156,7 +163,7 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
                 ok = MbarWait(&full[stage], phase, abortWord);
                 if (!ok) break;
                 TcFenceAfter();
-                const uint64_t bDesc = MakeSmemDescSw128(SmemAddr(sB + stage * S::kBBytes));
+                const uint64_t bDesc = BMN ? MakeSmemDescMnSw128(SmemAddr(sB + stage * S::kBBytes)) : MakeSmemDescSw128(SmemAddr(sB + stage * S::kBBytes));
                 const uint64_t aDesc = MakeSmemDescSw128(SmemAddr(sA + stage * S::kABytes));
                 if (MX) {
                     const uint32_t sfCol = tmemBase + S::kSfColBase + stage * S::kSfCols, sfSmem = SmemAddr(sSF + stage * S::kSfBytes);
@@ -171,7 +178,7 @@ __global__ void __launch_bounds__(kGemmThreads, (GemmSplitKSmem<BT_, MX>::kCtasP
                 } else {
 #pragma unroll
                     for (uint32_t k = 0; k < kBK / 16; ++k)
-                        UmmaF16(tmemBase, AdvanceDescK(bDesc, k * 32), AdvanceDescK(aDesc, k * 32), kIdesc, kb != kLo || k != 0 ? 1u : 0u);
+                        UmmaF16(tmemBase, AdvanceDescK(bDesc, k * (BMN ? 2048 : 32)), AdvanceDescK(aDesc, k * 32), kIdesc, kb != kLo || k != 0 ? 1u : 0u);
                 }
                 UmmaCommit(&empty[stage]);
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }

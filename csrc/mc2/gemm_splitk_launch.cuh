@@ -11,20 +11,21 @@
 namespace hccl {
 namespace mc2 {
 
-template <int BT, bool MX, bool QUANT = false>
+template <int BT, bool MX, bool QUANT = false, bool BMN = false>
 HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, uint32_t split, bool outFp32,
                          bool earlyB, cudaStream_t s)
 {
     using S = GemmSplitKSmem<BT, MX>;
     SplitKParams p{};
     const uint32_t elem = MX ? 1 : 2, boxK = 128 / elem;
-    CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * elem, 128, boxK, elem));
+    if (BMN) CHK_RET(EncodeTmap2D(&p.tmapB, b, K, N, (uint64_t)N * 2, kBK, 64, 2));
+    else CHK_RET(EncodeTmap2D(&p.tmapB, b, N, K, (uint64_t)K * elem, 128, boxK, elem));
     if (QUANT) p.a = (const __nv_bfloat16 *)a;
     else CHK_RET(EncodeTmap2D(&p.tmapA, a, M, K, (uint64_t)K * elem, BT, boxK, elem));
     p.C = c; p.M = M; p.N = N; p.K = K; p.split = split; p.outFp32 = outFp32; p.errorWord = GemmErrorWord();
     p.sfA = (const uint8_t *)sfa; p.sfB = (const uint8_t *)sfb; p.sfAtomsA = (M + 127) / 128; p.earlyB = earlyB;
     static std::atomic<bool> attrSet{false};
-    auto kern = GemmKernelSplitK<BT, MX, QUANT>;
+    auto kern = GemmKernelSplitK<BT, MX, QUANT, BMN>;
     const size_t smem = S::kTotal + 1024;
     if (!attrSet) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return HCCL_E_RUNTIME;
@@ -50,7 +51,7 @@ HcclResult LaunchSplitKT(const void *a, const void *sfa, const void *b, const vo
 }
 
 // earlyB: the kernel before this one in the stream wrote nothing but A, and itself waited for all before it
-template <bool MX>
+template <bool MX, bool BMN = false>
 HcclResult LaunchSplitK(SplitKChoice ch, const void *a, const void *sfa, const void *b, const void *sfb, void *c, uint32_t M, uint32_t N, uint32_t K, bool outFp32,
                         cudaStream_t s, bool earlyB = false)
 {
@@ -63,12 +64,12 @@ HcclResult LaunchSplitK(SplitKChoice ch, const void *a, const void *sfa, const v
     // block-scaled tiles have to start on a scale atom
     if (ch.split == 0 || ch.split > 8 || ch.split > kBlocks || (MX && ch.bt < 64 && M > ch.bt)) return HCCL_E_PARA;
     switch (ch.bt) {
-        case 16: return LaunchSplitKT<16, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
-        case 32: return LaunchSplitKT<32, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
-        case 64: return LaunchSplitKT<64, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
-        case 128: return LaunchSplitKT<128, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
-        case 192: if constexpr (!MX) return LaunchSplitKT<192, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s); else return HCCL_E_PARA;
-        case 256: return LaunchSplitKT<256, MX>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 16: return LaunchSplitKT<16, MX, false, BMN>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 32: return LaunchSplitKT<32, MX, false, BMN>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 64: return LaunchSplitKT<64, MX, false, BMN>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 128: return LaunchSplitKT<128, MX, false, BMN>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
+        case 192: if constexpr (!MX) return LaunchSplitKT<192, MX, false, BMN>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s); else return HCCL_E_PARA;
+        case 256: return LaunchSplitKT<256, MX, false, BMN>(a, sfa, b, sfb, c, M, N, K, ch.split, outFp32, earlyB, s);
         default: return HCCL_E_PARA;
     }
 }

@@ -252,7 +252,7 @@ __device__ __forceinline__ uint64_t MakeSmemDescSw128(uint32_t smemAddr)
 // Leading byte offset = from one box to the next, stride byte offset = from one group of 8 rows of K to the next; 16 rows of K
 // (one instruction) are 2048 bytes.
 constexpr uint32_t kMnBoxBytes = 64 * 128;
-constexpr uint32_t kInstrBMajorMN = 1u << 16;
+constexpr uint32_t kInstrAMajorMN = 1u << 15, kInstrBMajorMN = 1u << 16;
 __device__ __forceinline__ uint64_t MakeSmemDescMnSw128(uint32_t smemAddr)
 {
     uint64_t d = 0;

@@ -172,6 +172,34 @@ inline PlainChoice ChoosePlain(uint64_t m, uint64_t n, uint64_t k, uint64_t sms,
     return {m <= 64 ? SplitKChoice{} : ChooseWideSplit(m, n, k, t, ChooseSplitK(m, n, k, t, sms)), t};
 }
 
+// The kernel of C = A * B with B stored [K, N] (the input gradient of a linear layer). It had no split-K form: few tiles each walked all of K. Measured on
+// one B200, us tiles / split-K: 12 x 512 x 26784 74.5 / 13.8, 19 x 4456 x 2448 16.1 / 8.6, 94 x 312 x 21624 95.4 / 17.8, 109 x 9136 x 15336 76.5 / 60.3, 548 x 2528 x 12352 45.2 / 35.5.
+// Up to 64 rows split-K from K = 512 on, 0.51 of the tiles' time on average over 384 products (1.015 of the best number of CTAs). More rows: the tile height whose one wave of
+// clusters costs least, where that is below 0.85 of the tiles' cost: 0.70 on average over 570 products of 65 to 1100 rows, N 256 to 14336 and K 512 to 28672; 7 of them are more than 3 % slower.
+inline PlainChoice ChooseNn(uint64_t m, uint64_t n, uint64_t k, uint64_t sms, bool pairsEnabled)
+{
+    PlainChoice best{{}, ChooseTile(m, n, k, true, sms, pairsEnabled)};
+    if (k < 512) return best;
+    const uint64_t nt = (n + 127) / 128;
+    if (m <= 64) {
+        const uint32_t bt = m <= 16 ? 16 : m <= 32 ? 32 : 64;
+        double least = HUGE_VAL;
+        for (uint32_t s = 1; s <= 8 && s * 256 <= k; ++s)
+            if (const double c = SplitKCost(nt, bt, 2 * k, s, {0, 60, 9700, 0.9, 2.4}); c < least) { best.splitK = {bt, s}; least = c; }
+        return best;
+    }
+    struct Rows { uint32_t bt; double start, perCta, along, straddling; };              // us, along 4096 of K in a CTA (rows of B inside 32-byte sectors)
+    double least = 0.85 * 0.0917 * best.tile.cost;
+    for (const Rows &r : {Rows{64, 4.5, 0.23, 23.8, 33.7}, Rows{128, 6.3, 0.27, 32.5, 41.4}, Rows{192, 6.0, 0.1, 22, 26.4}, Rows{256, 6.9, 0.05, 26.5, 30.6}}) {
+        const uint64_t tiles = nt * ((m + r.bt - 1) / r.bt);
+        uint64_t s = std::min<uint64_t>(8, k / 256);
+        while (s > 1 && tiles > (r.bt <= 128 ? kClustersOfTwoAtOnce : kClustersAtOnce)[s]) --s;
+        const double c = r.start + r.perCta * (double)s + (n % 16 ? r.straddling : r.along) * (double)k / 4096 / (double)s;
+        if (s > 1 && c < least) { best.splitK = {r.bt, (uint32_t)s}; least = c; }
+    }
+    return best;
+}
+
 // The kernel of a block-scaled product: split-K where `split` is not 0, else tiles of CTA pairs (192 or 256 wide) or of one CTA (128, 192, 256).
 // Up to 64 rows see ChooseSplitK. More: the rule by which products were split up to 512 rows and K from 2048, pair tiles taken where they about fill the GPU and 256-wide
 // tiles where they do, kept most of the GPU idle just below each of its bounds. Another kernel is taken where its cost is below 0.92 of that rule's: a start, waves of

@@ -297,3 +297,22 @@ def test_products_as_the_first_call_of_a_thread(M):
         torch.cuda.synchronize()
         assert not failed, failed
         assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 512), (4, 4096, 1032), (16, 264, 16384), (20, 136, 2056), (64, 1000, 520), (94, 312, 4104), (200, 520, 4104), (300, 392, 8192), (384, 4096, 4608), (548, 2528, 4096)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_nn_split_k(shape, out_dtype):
+    """B stored [K, N] read by clusters that share K: every tile height, ragged rows, columns and K. Bound as in test_gemm_split_k."""
+    from hccl_b200.ops import gemm
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N * 3 + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(K, N, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M + 1, N), 7.0, device="cuda", dtype=out_dtype)
+    gemm.gemm_bf16_nn(a, w, out[:M])
+    torch.cuda.synchronize()
+    gemm.check_error()
+    ref, mag = a.double() @ w.double(), a.double().abs() @ w.double().abs()
+    bound = mag * K * 2.0 ** -24 + (ref.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0)
+    assert bool(((out[:M].double() - ref).abs() <= bound + 1e-30).all())
+    assert bool((out[M] == 7.0).all())
