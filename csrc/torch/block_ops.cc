@@ -570,13 +570,22 @@ struct MlpNode : OpNode {
     SavedVariable x, w, gu, h, wd;
     std::vector<int64_t> shape;
     at::TensorOptions options;
+    bool copied = false;                       // x is the node's own copy, its second output: a gradient of the gradient finds its way to the caller's x through it
     std::string name() const override { return "_SwiGluMlpBackward"; }
-    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(shape); }
-    std::vector<Saved> Keeps() override { return {{&x, false}, {&w, false}, {&gu, false}, {&h, false}, {&wd, false}}; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(shape); args.collect(copied); }
+    std::vector<Saved> Keeps() override { return {{&x, copied}, {&w, false}, {&gu, false}, {&h, false}, {&wd, false}}; }
     variable_list Backward(variable_list &&g) override
     {
+        if (!copied) return Gradients(g[0]);
+        if (!g[0].defined() && g[1].defined()) return {g[1], at::Tensor(), at::Tensor()};
+        variable_list out = Gradients(g[0]);
+        if (g[1].defined()) out[0] = out[0].defined() ? out[0] + g[1] : g[1];
+        return out;
+    }
+    variable_list Gradients(const at::Tensor &incoming)
+    {
         const auto [xv, wv, guv, hv, wdv] = Unpack(x, w, gu, h, wd);
-        at::Tensor dy = ZerosWhereUndefined(g[0], shape, options);
+        at::Tensor dy = ZerosWhereUndefined(incoming, shape, options);
         bool direct = !traced && !at::GradMode::is_enabled() && g_nativeGemm && !g_nativeWgrad;
         {
             py::gil_scoped_acquire gil;
@@ -625,14 +634,15 @@ py::object Mlp(py::handle xh, py::handle wh, py::handle wdh, py::object comm, ui
             Check(HcclMatmulReduceScatter(h.data_ptr(), wd.data_ptr(), y.data_ptr(), m, n, f, HCCL_DATA_TYPE_BFP16, (HcclComm)(uintptr_t)handle, Stream(x)), "HcclMatmulReduceScatter");
         }
         if (wanted) {
-            node->x = SavedVariable(kept, false);
+            node->copied = !own;
+            node->shape = y.sizes().vec();
+            node->options = y.options();
+            torch::autograd::set_history(own ? variable_list{y} : variable_list{y, kept}, node);
+            node->x = SavedVariable(kept, !own);
             node->w = SavedVariable(w, false);
             node->gu = SavedVariable(gu, false);
             node->h = SavedVariable(h, false);
             node->wd = SavedVariable(wd, false);
-            node->shape = y.sizes().vec();
-            node->options = y.options();
-            torch::autograd::set_history({y}, node);
         }
     }
     return py::cast(y);

@@ -185,7 +185,7 @@ def _one_rank_linear(x: torch.Tensor, w: torch.Tensor, comm, column: bool, own: 
 
 def _mlp_backward(comm, x, w, gu, h, wd, dy):
     """The SwiGLU layer's gradients by its parts; by single operations where something has to see them. What was kept for the kernels alone has no history: a gradient of
-    the gradient starts from the input again."""
+    the gradient starts from the input again, or from its copy, which is an output of the node."""
     if torch.is_grad_enabled() or not all([_block._plain_tensor(t) for t in (x, w, gu, h, wd, dy)]):
         return _block._plain_backward(_plain_mlp, [t if t.requires_grad else t.detach().requires_grad_() for t in (x, w, wd)], dy)
     dh, dwd = _row_backward(comm, h, wd, dy)

@@ -641,6 +641,29 @@ def test_swiglu_layer_keeps_the_engine_s_rules():
         comm.destroy()
 
 
+@pytest.mark.parametrize("given", ["leaf", "tensor", "away"])
+def test_swiglu_layer_second_derivatives_reach_the_input(given):
+    """The gradient of every first gradient by every input of the layer: a leaf, a tensor with a history, and one that the caller gives away (kept without a copy). Bounds as above: 16 roundings to bf16
+    on the way of both sides."""
+    from hccl_b200.parallel import tensor_parallel as tp
+    _native_nodes()
+    comm, mlp, leaf, up = _swiglu_layer(640, 64, 128)
+    try:
+        ins = [leaf, *mlp.parameters()]
+        layer = {"leaf": lambda: mlp(leaf), "tensor": lambda: mlp(leaf * 1), "away": lambda: tp.mlp_of_own(mlp, leaf * 1)}[given]
+        got, plain = (torch.autograd.grad(f(), ins, up, create_graph=True) for f in (layer, lambda: tp._plain_mlp(*ins)))
+        square = lambda t: t.float().square().sum()
+        for i, (a, b) in enumerate(zip(got, plain)):
+            seconds = [torch.autograd.grad(square(t), ins, retain_graph=True, allow_unused=True) for t in (a, b)]
+            for c, d in zip(*seconds):
+                assert (c is None) == (d is None), i
+                assert c is None or (c.double() - d.double()).norm() <= 16 * 2.0 ** -8 * d.double().norm(), i
+        square(got[2]).backward()
+        assert leaf.grad is not None and (leaf.grad.double() - seconds[1][0].double()).norm() <= 16 * 2.0 ** -8 * seconds[1][0].double().norm()
+    finally:
+        comm.destroy()
+
+
 def _attention_case(batch, seq, heads, kv_heads, hd, seed=2):
     import functools
     from hccl_b200.models.llama import _plain_attention, _rope_tables
