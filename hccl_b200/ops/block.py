@@ -15,6 +15,7 @@ import ctypes
 from typing import Callable, Optional
 
 import torch
+from torch.utils._device import DeviceContext
 
 from .._ext import ops as _extension
 from .._lib import check, lib
@@ -59,6 +60,15 @@ _any_global_hook = torch.nn.modules.module._has_any_global_hook
 def _watched() -> bool:
     """Whether something has to see the single operations: a function transform, dispatch mode, forward-mode level, compiler or tracer."""
     return _transforms() is not None or _modes() > 0 or _forward_ad._current_level >= 0 or torch.compiler.is_compiling() or torch.jit.is_tracing()
+
+
+_function_modes, _function_mode, _sdpa = torch._C._len_torch_function_stack, torch._C._get_function_stack_at, torch._C._nn.scaled_dot_product_attention
+
+
+def _functions_watched() -> bool:
+    """Whether a function mode has to see the operations that a caller writes as such (the attention, a residual addition, an index). The mode behind a default device
+    changes where tensors are made and nothing else."""
+    return any(type(_function_mode(i)) is not DeviceContext for i in range(_function_modes()))
 
 
 def _plain_tensor(t) -> bool:
@@ -239,7 +249,7 @@ def rms_norm_kept(x: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable)
 def rms_norm_add(x: torch.Tensor, d: torch.Tensor, w: torch.Tensor, eps: float, plain: Callable):
     """(norm of x + d, x + d), the bits of the two operations one after the other. None without the native nodes."""
     n = native_nodes(x)
-    return None if n is None else n.rms_norm_add(x, d, w, eps, plain)
+    return None if n is None or _functions_watched() else n.rms_norm_add(x, d, w, eps, plain)
 
 
 def bare(module: torch.nn.Module, cls: type, forward: Callable) -> bool:
@@ -321,11 +331,14 @@ def _default_attention() -> bool:
 
 def attention(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, batch: int, heads: int, kv_heads: int, head_dim: int, plain: Callable) -> Optional[torch.Tensor]:
     """Causal attention from the packed projection, [batch * seq, heads * head_dim], for sequences short enough that the backward kernel is the better choice, where a gradient may be asked for and
-    the library's attention would run anyway; the tables as `rope_qkv`. The projection is kept as it is, so nobody else may change it. `plain(qkv)` is the same in PyTorch."""
+    the library's attention would run anyway (no function mode, and nothing in the place of `scaled_dot_product_attention`); the tables as `rope_qkv`. The projection is kept as it is, so nobody else
+    may change it. `plain(qkv)` is the same in PyTorch."""
     n = native_nodes(qkv)
+    if (n is None and not _usable(qkv)) or _functions_watched() or torch.nn.functional.scaled_dot_product_attention is not _sdpa:
+        return None
     if n is not None:
         return n.attention(qkv, cos, sin, batch, heads, kv_heads, head_dim, plain)
-    if not _usable(qkv) or not _floats_ok(qkv.get_device(), cos, sin) or not _default_attention() or not (torch.is_grad_enabled() and qkv.requires_grad):
+    if not _floats_ok(qkv.get_device(), cos, sin) or not _default_attention() or not (torch.is_grad_enabled() and qkv.requires_grad):
         return None
     seq = cos.shape[0] if cos.dim() else 0
     if qkv.shape != (batch * seq, (heads + 2 * kv_heads) * head_dim) or cos.shape != (seq, head_dim // 2) or sin.shape != cos.shape:
@@ -465,9 +478,11 @@ class _Embedding(torch.autograd.Function):
 def embedding(w: torch.Tensor, ids: torch.Tensor) -> Optional[torch.Tensor]:
     """w[ids] for a vector of few ids, whose gradient then takes one kernel."""
     n = native_nodes(w)
+    if (n is None and not _usable(w)) or _functions_watched():
+        return None
     if n is not None:
         return n.embedding(w, ids)
-    if not _usable(w) or not (torch.is_grad_enabled() and w.requires_grad) or w.dim() != 2 or w.shape[1] % 8 or not _plain_tensor(ids):
+    if not (torch.is_grad_enabled() and w.requires_grad) or w.dim() != 2 or w.shape[1] % 8 or not _plain_tensor(ids):
         return None
     if ids.dtype is not torch.int64 or ids.device != w.device or not ids.is_contiguous() or ids.dim() != 1 or not 0 < ids.numel() <= _decl().HcclEmbeddingGradTokens():
         return None

@@ -762,6 +762,46 @@ def test_attention_keeps_the_engine_s_rules():
         assert f(qkv) is None and nodes is block.nodes()
 
 
+def test_function_modes_and_a_replaced_attention_see_the_model(monkeypatch):
+    """A function mode around the model and another function in the place of the library's attention meet the operations that the model is written with: attention, residual additions, the
+    embedding's index. A default device is a mode as well and changes nothing."""
+    import torch.nn.functional as F
+    from torch.overrides import TorchFunctionMode
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.models.llama import Llama, LlamaConfig
+    from hccl_b200.ops import block
+    _native_nodes()
+    torch.zeros(1, device="cuda")
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        cfg = LlamaConfig.tiny(vocab=512, hidden=256, layers=2, heads=8, kv_heads=4, ffn=512)
+        model = Llama(cfg, comm, dtype=torch.bfloat16, device="cuda", seed=3)
+        tokens = torch.randint(0, 512, (2, 64), device="cuda")
+        seen, calls = [], []
+
+        class See(TorchFunctionMode):
+            def __torch_function__(self, func, types, args=(), kwargs=None):
+                seen.append(getattr(func, "__name__", ""))
+                return func(*args, **(kwargs or {}))
+
+        close = lambda a, b: (a.double() - b.double()).norm() <= 2.0 ** -6 * b.double().norm()
+        ref = model(tokens)
+        with See():
+            assert close(model(tokens), ref)
+        assert seen.count("scaled_dot_product_attention") == 2 and "__getitem__" in seen
+        assert sum(name in ("add", "__add__") for name in seen) >= 4
+        library = F.scaled_dot_product_attention
+        monkeypatch.setattr(F, "scaled_dot_product_attention", lambda *a, **k: (calls.append(1), library(*a, **k))[1])
+        assert close(model(tokens), ref) and len(calls) == 2
+        monkeypatch.undo()
+        f, _, qkv, *_ = _attention_case(2, 100, 4, 2, 32)
+        with torch.device("cuda"):
+            assert f(qkv).grad_fn.name() == "_AttentionBackward"
+            assert block.embedding(model.embed, tokens.reshape(-1)).grad_fn.name() == "_EmbeddingBackward"
+    finally:
+        comm.destroy()
+
+
 @pytest.mark.parametrize("native", [True, False])
 @pytest.mark.parametrize("tokens,hidden,vocab", [(1, 8, 1), (33, 264, 7), (255, 2056, 300), (257, 256, 512), (2048, 64, 50), (2049, 64, 50)])
 def test_embedding_gradient_of_few_tokens(tokens, hidden, vocab, native, monkeypatch):
