@@ -1,6 +1,7 @@
 // Native face of the matmul, block-scaled and MoE operators for PyTorch: argument checks, result allocation, the current stream and the C call in one
 // step. A decode-sized product takes under ten microseconds on the device; the same steps in Python and ctypes took
 // longer than that, so the GPU waited for the host between such calls.
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime.h>
 #include <torch/extension.h>
@@ -61,15 +62,13 @@ std::pair<int, at::Tensor> Fused(uint64_t comm, int kind, int64_t ranks, const a
     return {(int)r, std::move(o)};
 }
 
-// Memory of a call's own that it uses on a stream other than the one it was allocated for.
-void UsedOn(const at::Tensor &t, cudaStream_t s)
+c10::cuda::CUDAStream OfTorch(cudaStream_t s, c10::DeviceIndex device)
 {
-    const auto current = c10::cuda::getCurrentCUDAStream(t.device().index());
-    if (s != current.stream()) t.record_stream(c10::cuda::getStreamFromExternal(s, t.device().index()).unwrap());
+    return s == cudaStreamLegacy ? c10::cuda::getDefaultCUDAStream(device) : c10::cuda::getStreamFromExternal(s, device);
 }
 
-// The quantised activations live for the call alone, in the order of its stream: nothing is shared between threads or kept between calls, and a captured
-// graph has them in its own pool.
+// The quantised activations live for the call alone and are allocated for the stream that uses them: a block that has just become free on another stream may still be read there.
+// Nothing is shared between threads or kept between calls, and a captured graph has them in its own pool.
 std::pair<int, at::Tensor> MxMatmul(uint64_t comm, const at::Tensor &a, const at::Tensor &payload, const at::Tensor &scales, int64_t n, const std::optional<at::Tensor> &out,
                                     std::optional<uint64_t> stream)
 {
@@ -80,11 +79,12 @@ std::pair<int, at::Tensor> MxMatmul(uint64_t comm, const at::Tensor &a, const at
     at::Tensor act;
     uint8_t *q = nullptr;
     if (!HcclQuantizeGemmMxfp8InOne(m, n, k)) {
+        c10::cuda::OptionalCUDAStreamGuard on;
+        if (stream) on.reset_stream(OfTorch(s, a.device().index()));
         act = at::empty({m * k + (int64_t)HcclMxfp8ScaleBytes(m, k)}, a.options().dtype(at::kByte));
         q = act.data_ptr<uint8_t>();
     }
     const HcclResult r = HcclQuantizeMatmulMxfp8(a.data_ptr(), q, q ? q + m * k : nullptr, payload.data_ptr(), scales.data_ptr(), o.data_ptr(), m, n, k, (HcclComm)(uintptr_t)comm, s);
-    if (stream && act.defined()) UsedOn(act, s);
     return {(int)r, std::move(o)};
 }
 

@@ -214,6 +214,30 @@ def test_one_rank_calls_keep_their_activations_apart():
         comm.destroy()
 
 
+def test_activations_of_a_call_on_an_explicit_stream_belong_to_that_stream():
+    """Memory that has just become free on the current stream, where a copy that is still to run will read it, is not taken for a call on another stream."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops import mxfp8
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        m, n, k = 256, 512, 4096
+        w, a = mxfp8.quantize(torch.randn(n, k, device="cuda").to(torch.bfloat16)), torch.randn(m, k, device="cuda").to(torch.bfloat16)
+        want, out, s = mxfp8.gemm(mxfp8.quantize(a), w), torch.empty(m, n, dtype=torch.bfloat16, device="cuda"), torch.cuda.Stream()
+        size = m * k + mxfp8.scale_bytes(m, k)
+        for stream in (s, torch.cuda.ExternalStream(s.cuda_stream)):
+            src, dst = torch.full((size,), 7, dtype=torch.uint8, device="cuda"), torch.empty(size, dtype=torch.uint8, device="cuda")
+            out.zero_()
+            torch.cuda.synchronize()
+            torch.cuda._sleep(20_000_000)                      # about 10 ms: the copy is queued, its source is free
+            dst.copy_(src)
+            del src
+            assert mxfp8.matmul_all_reduce(comm, a, w, out=out, stream=stream) is out
+            torch.cuda.synchronize()
+            assert bool((dst == 7).all()) and torch.equal(out, want)
+    finally:
+        comm.destroy()
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 8, 256), (1, 512, 512), (3, 136, 640), (8, 4096, 4096), (15, 1000, 1152), (16, 14336, 4096), (16, 264, 16384), (17, 4096, 4096), (25, 2056, 2048), (32, 4096, 4096),
                                    (32, 1024, 14336), (33, 4096, 4096)])
 def test_products_that_quantise_their_activations(m, n, k):
