@@ -250,17 +250,15 @@ inline MxChoice ChooseMx(uint64_t m, uint64_t n, uint64_t k, uint64_t sms, bool 
 }
 
 // Pair tile width of the product with SwiGLU in its epilogue (forward: half of it gate, half up; backward: columns of the intermediate gradient), 0 = the product and the
-// element-wise kernel one after the other. Forward: wherever the plain product would not split K (few rows, bound by reading the weights; up to 64 rows only K from 2048, up to 16 from 512); us separate / fused 60 x 2 x 512
-// x 256 5.5 / 5.2, 200 x 2 x 14336 x 4096 61.2 / 60.9, 300 x 2 x 3584 x 1024 11.5 / 12.2. Backward: above 512 rows (777 x 14336 x 4096 135 / 126, 513 x 2056 x 1032 14.1 / 13.7); up to there
+// element-wise kernel one after the other. Not where the product by itself splits K: the fused kernel has no such form, its tiles each walk all of K, and its sums would have another order. Us
+// separate / fused there, one B200: forward 52 x 2 x 13152 x 1384 23.1 / 23.8, 35 x 2 x 3072 x 1144 9.3 / 11.7, 168 x 2 x 2952 x 8616 39.0 / 47.4, 781 x 2 x 184 x 16352 20.6 / 55.5; backward 1098 x 1400 x 10784
+// 44.6 / 48.0, 620 x 128 x 13320 17.7 / 53.6. Of 340 such products fused would be faster for 26, by 17 % at most (two CTAs along K: 832 x 2 x 1040 x 5064 35.2 / 29.3), and takes 1.4 times as long on average. Elsewhere
+// forward always: 60 x 2 x 512 x 256 5.5 / 5.2, 200 x 2 x 14336 x 4096 61.2 / 60.9, 300 x 2 x 3584 x 1024 11.5 / 12.2. Backward: above 512 rows (777 x 14336 x 4096 135 / 126, 513 x 2056 x 1032 14.1 / 13.7); up to there
 // one-CTA tiles fill the GPU better: 300 x 7168 x 2048 22.8 / 24.2, 130 x 14336 x 4096 37.0 / 40.1, 256 x 512 x 256 6.3 / 8.5.
 inline uint32_t ChooseSwiGlu(uint64_t m, uint64_t ffn, uint64_t k, bool backward, uint64_t sms, bool pairsEnabled)
 {
-    // not every product that splits K is worth a second kernel: up to 64 rows from these K on, more by ChooseSplitK's rule
-    auto splits = [&] {
-        if (m <= 64) return (m <= 16 ? k >= 512 : k >= 2048) && ChooseSplitK(m, 2 * ffn, k, false, false).split != 0;
-        return m <= 512 && ChooseSplitK(m, 2 * ffn, k, ChooseTile(m, 2 * ffn, k, false, sms, true), sms).split != 0;
-    };
-    if (!pairsEnabled || (backward ? m <= 512 : splits())) return 0;
+    if (!pairsEnabled || (backward && m <= 512)) return 0;
+    if ((backward ? ChooseNn(m, ffn, k, sms, pairsEnabled) : ChoosePlain(m, 2 * ffn, k, sms, pairsEnabled)).splitK.split) return 0;
     const uint64_t pairs = sms / 2, rowPairs = (m + 255) / 256;
     const double k4 = (double)k / 4096;
     uint32_t best = 0;

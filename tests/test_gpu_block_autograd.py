@@ -579,6 +579,12 @@ def test_swiglu_layer_gives_the_bits_of_its_parts(rows, hidden, ffn):
         comm.destroy()
 
 
+@pytest.mark.parametrize("rows,hidden,ffn", [(20, 2016, 64), (40, 1024, 504), (200, 8192, 3584), (300, 16384, 256), (512, 4096, 512), (520, 16384, 512), (700, 4096, 512), (1344, 4184, 1408)])
+def test_swiglu_layer_gives_the_bits_of_its_parts_where_they_split_k(rows, hidden, ffn):
+    """Long K and few columns on both sides of 512 rows: the products split K, forward or backward or both, which the fused kernels cannot."""
+    test_swiglu_layer_gives_the_bits_of_its_parts(rows, hidden, ffn)
+
+
 def test_swiglu_layer_keeps_the_engine_s_rules():
     """Input that changes after the pass, a gradient's gradient, compiled autograd, batched gradients, saved tensors of another size or on the CPU, a weight that changes in
     place, the switch of the weight gradients."""

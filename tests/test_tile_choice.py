@@ -112,6 +112,42 @@ BLOCK_SCALED = [
     ((279, 10192, 2688), {-256: 14.3, -128: 15.1, 1128: 15.1, -2192: 16.1}),
 ]
 
+# B stored [K, N] (input gradients), drawn from the products that the choice was measured on (384 of up to 64 rows and 570 of 65 to 1100; within 8 % of the best one for 358 and 474): as SPLITS
+INPUT_GRADIENTS = [
+    ((59, 2360, 18168), {8064: 26.8, 7064: 28.7, 6064: 28.7}),
+    ((42, 2448, 13984), {8064: 18.1, 7064: 18.1, 6064: 18.4, 5064: 20.1}),
+    ((11, 320, 1544), {6016: 3.8, 5016: 3.8, 4016: 4.1}),
+    ((8, 3360, 2472), {5016: 6.6, 4016: 6.6, 7016: 6.9, 8016: 6.9, 3016: 7.1, 6016: 7.2, 2016: 7.6}),
+    ((36, 1376, 1656), {6064: 5.6, 5064: 5.8, 4064: 6.1}),
+    ((2, 3448, 21040), {8016: 29.0, 7016: 30.0, 5016: 30.4, 6016: 32.4}),
+    ((467, 6736, 7192), {0: 46.4}),
+    ((134, 1344, 14424), {8192: 16.4, 7192: 17.4, 8256: 17.9, 6192: 18.3}),
+    ((883, 1696, 4360), {2192: 21.8, 0: 24.8}),
+    ((289, 6208, 11728), {0: 51.0, 2128: 55.1, 1192: 58.4}),
+    ((546, 560, 4168), {8192: 10.8, 6192: 11.2, 7192: 11.3, 6064: 11.5, 5064: 11.9, 5192: 12.3}),
+    ((222, 4592, 11208), {3256: 37.4}),
+    ((546, 480, 1480), {4064: 7.3, 5064: 7.6, 3064: 7.9, 2064: 8.0}),
+    ((796, 344, 576), {0: 4.6}),
+    ((69, 2248, 7216), {6192: 12.3, 5192: 13.2, 6256: 13.2}),
+    ((477, 432, 9536), {8192: 12.2, 7192: 12.7, 6192: 13.1, 8064: 13.4, 7064: 13.8}),
+]
+
+# (m, ffn, k, backward) of a product with SwiGLU and whether the fused kernel is the faster one: us separate / fused
+FUSED_SWIGLU = [
+    ((60, 512, 256, 0), True),               # 5.5 / 5.2
+    ((2048, 14336, 4096, 0), True),          # 369 / 356
+    ((1000, 3584, 1024, 0), True),           # 20.0 / 19.3
+    ((35, 3072, 1144, 0), False),            # 9.3 / 11.7
+    ((168, 2952, 8616, 0), False),           # 39.0 / 47.4
+    ((650, 136, 4528, 0), False),            # 12.9 / 18.4
+    ((781, 184, 16352, 0), False),           # 20.6 / 55.5
+    ((2048, 14336, 4096, 1), True),          # 253 / 214
+    ((777, 14336, 4096, 1), True),           # 135 / 126
+    ((300, 7168, 2048, 1), False),           # 22.8 / 24.2
+    ((602, 1688, 14560, 1), False),          # 46.2 / 64.3
+    ((620, 128, 13320, 1), False),           # 17.7 / 53.6
+]
+
 
 def _choose(tmp_path, products):
     src = tmp_path / "choose.cc"
@@ -180,3 +216,30 @@ def test_block_scaled_products_of_many_rows(tmp_path):
             assert 1 <= s <= 8 and s * 128 <= k and bt in (16, 32, 64, 256) and (m <= bt or bt >= 64)
         else:
             assert kernel in (-128, -192, -256) or (kernel in (-2192, -2256) and pairs and n >= 256), (m, n, k, pairs, kernel)
+
+
+def test_input_gradients_take_a_kernel_near_the_best(tmp_path):
+    """B stored [K, N]: split-K where it pays, and a choice that can be launched. Where the SwiGLU layer's products are fused with it: never where the product by itself splits K, which the
+    fused kernel cannot."""
+    src = tmp_path / "nn.cc"
+    src.write_text('#include <cstdio>\n#include "mc2/tile_choice.h"\nusing namespace hccl::mc2;\nint main() { unsigned long long m, n, k; while (scanf("%llu %llu %llu", &m, &n, &k) == 3) { '
+                   'auto c = ChooseNn(m, n, k, 148, true), f = ChoosePlain(m, 2 * n, k, 148, true); printf("%u %d %u %u %u %u %u\\n", c.splitK.split * 1000 + c.splitK.bt, (int)c.tile.pair, c.tile.bn, '
+                   'f.splitK.split, ChooseSwiGlu(m, n, k, false, 148, true), ChooseSwiGlu(m, n, k, true, 148, true), ChooseSwiGlu(m, n, k, true, 148, false) + ChooseSwiGlu(m, n, k, false, 148, false)); } }\n')
+    exe = tmp_path / "nn"
+    subprocess.run(["g++", "-std=c++17", "-O1", f"-I{ROOT / 'csrc'}", str(src), "-o", str(exe)], check=True, timeout=120)
+
+    def choose(products):
+        out = subprocess.run([str(exe)], input="".join("%d %d %d\n" % p for p in products), capture_output=True, text=True, check=True, timeout=60)
+        return [tuple(int(v) for v in line.split()) for line in out.stdout.splitlines()]
+
+    for (shape, us), (kernel, *_) in zip(INPUT_GRADIENTS, choose([p for p, _ in INPUT_GRADIENTS])):
+        assert us.get(kernel if kernel >= 1000 else 0, 1e9) <= 1.08 * min(us.values()), (shape, kernel, us)
+    for ((m, n, k, backward), fused), c in zip(FUSED_SWIGLU, choose([p[:3] for p, _ in FUSED_SWIGLU])):
+        assert bool(c[5 if backward else 4]) == fused, (m, n, k, backward, c)
+    every = [(m, n, k) for m in (1, 16, 17, 40, 64, 65, 200, 512, 513, 700, 1100, 4096, 100000) for n in (8, 64, 120, 512, 3584, 14336) for k in (8, 256, 504, 512, 1024, 2048, 4096, 16384)]
+    for (m, n, k), (kernel, pair, bn, splits, forward, backward, off) in zip(every, choose(every)):
+        s, bt = divmod(kernel, 1000)
+        assert not s or (s <= 8 and s * 256 <= k and bt in (16, 32, 64, 128, 192, 256)), (m, n, k, kernel)
+        assert (pair and bn in (256, 512)) or (not pair and bn in (64, 128)), (m, n, k, pair, bn)
+        assert forward in (0, 128, 192, 224, 256) and backward in (0, 128, 256) and not off
+        assert not (forward and splits) and not (backward and s) and bool(forward) == (not splits) and bool(backward) == (m > 512 and not s), (m, n, k)
