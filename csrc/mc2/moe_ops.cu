@@ -108,7 +108,7 @@ HcclResult LaunchSolo(const void *fn, const DevComm *comms, const MoeArgs &a, ui
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, params);
-    if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u)", cudaGetErrorString(e), ctas); return HCCL_E_RUNTIME; }
+    if (e != cudaSuccess) { HCCL_ERROR("MoE kernel launch failed: %s (grid %u)", cudaGetErrorString(e), ctas); (void)cudaGetLastError(); return HCCL_E_RUNTIME; }
     return HCCL_SUCCESS;
 }
 
@@ -175,6 +175,8 @@ HcclResult HcclMoeDispatch(HcclMoeHandle handle, const void *x, const int32_t *t
     auto *st = (MoeState *)handle;
     if (!st || !x || !topkIdx) return HCCL_E_PTR;
     if (numTokens == 0 || numTokens > st->cfg.maxTokens) { HCCL_ERROR("MoE dispatch: %u tokens, configured maximum %u", numTokens, st->cfg.maxTokens); return HCCL_E_PARA; }
+    // rows move in 16-byte pieces
+    if (((uintptr_t)x & 15u) || ((uintptr_t)topkIdx & 3u)) { HCCL_ERROR("MoE dispatch: tokens must be 16-byte aligned, expert indices by their elements"); return HCCL_E_PARA; }
     Comm *c = st->comm;
     CHK_RET(CommCheckReady(c));
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);
@@ -212,7 +214,8 @@ HcclResult HcclMoeCombine(HcclMoeHandle handle, const float *topkWeights, void *
 {
     auto *st = (MoeState *)handle;
     if (!st || !topkWeights || !out) return HCCL_E_PTR;
-    if (numTokens != st->lastTokens) { HCCL_ERROR("MoE combine: %u tokens but the last dispatch routed %u", numTokens, st->lastTokens); return HCCL_E_PARA; }
+    if (numTokens == 0 || numTokens != st->lastTokens) { HCCL_ERROR("MoE combine: %u tokens but the last dispatch routed %u", numTokens, st->lastTokens); return HCCL_E_PARA; }
+    if (((uintptr_t)out & 15u) || ((uintptr_t)topkWeights & 3u)) { HCCL_ERROR("MoE combine: the result must be 16-byte aligned, weights by their elements"); return HCCL_E_PARA; }
     Comm *c = st->comm;
     CHK_RET(CommCheckReady(c));
     MoeArgs a = MakeArgs(st->cfg, st->L, st->wsOff, numTokens);

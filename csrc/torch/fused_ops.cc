@@ -27,6 +27,17 @@ void CheckResult(const std::optional<at::Tensor> &t, int64_t elems, bool fp32Too
     if (!t->is_cuda()) throw py::value_error(std::string(what) + " must be a CUDA tensor");
 }
 
+// A kernel reads or writes `bytes` at the tensor's address.
+void CheckMemory(const at::Tensor &t, uint64_t bytes, const char *what)
+{
+    if (!t.is_contiguous() || t.nbytes() < bytes) throw py::value_error(std::string(what) + " must be a contiguous tensor of at least " + std::to_string(bytes) + " bytes");
+}
+void CheckOnGpu(std::initializer_list<const at::Tensor *> ts)
+{
+    for (const at::Tensor *t : ts)
+        if (!t->is_cuda()) throw py::value_error("a CUDA tensor is needed, not one on " + t->device().str());
+}
+
 // Both return (HcclResult, out).
 std::pair<int, at::Tensor> Gemm(const at::Tensor &a, const at::Tensor &w, const std::optional<at::Tensor> &out, bool fp32, bool transposedB, int variant,
                                 std::optional<uint64_t> stream)
@@ -72,8 +83,13 @@ c10::cuda::CUDAStream OfTorch(cudaStream_t s, c10::DeviceIndex device)
 std::pair<int, at::Tensor> MxMatmul(uint64_t comm, const at::Tensor &a, const at::Tensor &payload, const at::Tensor &scales, int64_t n, const std::optional<at::Tensor> &out,
                                     std::optional<uint64_t> stream)
 {
-    py::gil_scoped_release nogil;
+    if (a.dim() != 2 || n < 0 || a.scalar_type() != at::kBFloat16 || !a.is_contiguous()) throw py::value_error("the product takes contiguous bf16 activations [m, k]");
     const int64_t m = a.size(0), k = a.size(1);
+    CheckResult(out, m * n, false, "out");
+    CheckMemory(payload, (uint64_t)n * k, "the weight's payload");
+    CheckMemory(scales, HcclMxfp8ScaleBytes(n, k), "the weight's scales");
+    CheckOnGpu({&a, &payload, &scales});
+    py::gil_scoped_release nogil;
     at::Tensor o = out ? *out : at::empty({m, n}, a.options());
     cudaStream_t s = StreamOf(stream);
     at::Tensor act;
@@ -91,8 +107,12 @@ std::pair<int, at::Tensor> MxMatmul(uint64_t comm, const at::Tensor &a, const at
 std::tuple<int, at::Tensor, at::Tensor> MxQuantize(const at::Tensor &x, const std::optional<at::Tensor> &payload, const std::optional<at::Tensor> &scales,
                                                    std::optional<uint64_t> stream)
 {
-    py::gil_scoped_release nogil;
+    if (x.dim() != 2 || x.scalar_type() != at::kBFloat16 || !x.is_contiguous()) throw py::value_error("quantize takes a contiguous bf16 tensor [rows, k]");
     const int64_t rows = x.size(0), k = x.size(1);
+    if (payload) CheckMemory(*payload, (uint64_t)rows * k, "the payload");
+    if (scales) CheckMemory(*scales, HcclMxfp8ScaleBytes(rows, k), "the scales");
+    CheckOnGpu({&x, payload ? &*payload : &x, scales ? &*scales : &x});
+    py::gil_scoped_release nogil;
     at::Tensor p = payload ? *payload : at::empty({rows, k}, x.options().dtype(at::kByte));
     at::Tensor f = scales ? *scales : at::empty({(int64_t)HcclMxfp8ScaleBytes(rows, k)}, x.options().dtype(at::kByte));
     const HcclResult r = HcclQuantizeMxfp8(x.data_ptr(), p.data_ptr(), f.data_ptr(), rows, k, StreamOf(stream));
@@ -101,8 +121,12 @@ std::tuple<int, at::Tensor, at::Tensor> MxQuantize(const at::Tensor &x, const st
 
 // `kept` holds the tensors over the receive buffers that the caller made for the addresses `at`. -> (HcclResult, addresses, new tensors over the same memory with a
 // version count of their own, or None where the addresses are others)
-py::tuple MoeDispatch(uint64_t handle, const at::Tensor &x, const at::Tensor &idx, std::optional<uint64_t> stream, const py::object &at, const py::tuple &kept)
+py::tuple MoeDispatch(uint64_t handle, int64_t topK, int64_t hidden, const at::Tensor &x, const at::Tensor &idx, std::optional<uint64_t> stream, const py::object &at, const py::tuple &kept)
 {
+    if (x.dim() == 0) throw py::value_error("x must be [tokens, hidden]");
+    CheckMemory(x, (uint64_t)x.size(0) * hidden * 2, "x");
+    CheckMemory(idx, (uint64_t)x.size(0) * topK * 4, "topk_idx");
+    CheckOnGpu({&x, &idx});
     void *rx = nullptr, *rs = nullptr;
     int32_t *rc = nullptr, *src = nullptr;
     HcclResult r;
@@ -117,9 +141,12 @@ py::tuple MoeDispatch(uint64_t handle, const at::Tensor &x, const at::Tensor &id
     return py::make_tuple((int)r, now, out);
 }
 
-std::pair<int, at::Tensor> MoeCombine(uint64_t handle, const at::Tensor &weights, int64_t tokens, int64_t hidden, const std::optional<at::Tensor> &out,
+std::pair<int, at::Tensor> MoeCombine(uint64_t handle, int64_t topK, const at::Tensor &weights, int64_t tokens, int64_t hidden, const std::optional<at::Tensor> &out,
                                       std::optional<uint64_t> stream)
 {
+    CheckMemory(weights, (uint64_t)tokens * topK * 4, "topk_weights");
+    CheckResult(out, tokens * hidden, false, "out");
+    CheckOnGpu({&weights});
     py::gil_scoped_release nogil;
     at::Tensor o = out ? *out : at::empty({tokens, hidden}, weights.options().dtype(at::kBFloat16));
     const HcclResult r = HcclMoeCombine((HcclMoeHandle)(uintptr_t)handle, weights.data_ptr<float>(), o.data_ptr(), (uint32_t)tokens, StreamOf(stream));

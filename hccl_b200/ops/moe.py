@@ -8,6 +8,7 @@ import torch
 
 from .._ext import ops as _native
 from .._lib import check, lib
+from .gemm import check_result
 
 
 class HcclMoeConfig(ctypes.Structure):
@@ -44,6 +45,11 @@ def _view(ptr: int, shape, dtype, device) -> torch.Tensor:
     return torch.as_tensor(_Holder(), device=device).view(dtype).view(*shape)
 
 
+def _need(t: torch.Tensor, elems: int, what: str) -> None:
+    if t.numel() < elems or not t.is_cuda:
+        raise ValueError(f"{what} must be a CUDA tensor of at least {elems} elements")
+
+
 class MoeDispatcher:
     """Keeps the symmetric buffers of one MoE layer configuration.
 
@@ -65,7 +71,7 @@ class MoeDispatcher:
         self.expert_out = _view(y.value, (self.cap, hidden), torch.bfloat16, dev)
         self.local_experts = num_experts // comm.size
         self.mxfp8 = mxfp8
-        self.hidden = hidden
+        self.hidden, self.top_k = hidden, top_k
         self._tokens = 0
         self._recv = None      # receive buffers as tensors, and the addresses they were made for
 
@@ -73,13 +79,16 @@ class MoeDispatcher:
         assert x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and topk_idx.dtype == torch.int32 and topk_idx.is_contiguous()
         n = _native()
         if n is not None:
-            rc, at, recv = n.moe_dispatch(self._h.value if self._h else 0, x, topk_idx, None if stream is None else stream.cuda_stream, *(((), ()) if self._recv is None else self._recv))
+            rc, at, recv = n.moe_dispatch(self._h.value if self._h else 0, self.top_k, self.hidden, x, topk_idx, None if stream is None else stream.cuda_stream,
+                                          *(((), ()) if self._recv is None else self._recv))
             if rc:
                 check(rc, "HcclMoeDispatch")
             self._tokens = x.shape[0]
             if recv is not None:
                 return recv
         else:
+            _need(x, x.shape[0] * self.hidden, "x")
+            _need(topk_idx, x.shape[0] * self.top_k, "topk_idx")
             s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) if stream is None else stream.cuda_stream
             rx, rs, rc, rsrc = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
             check(_decl().HcclMoeDispatch(self._h, x.data_ptr(), topk_idx.data_ptr(), x.shape[0], ctypes.byref(rx), ctypes.byref(rs), ctypes.byref(rc),
@@ -105,11 +114,14 @@ class MoeDispatcher:
         assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
         n = _native()
         if n is not None:
-            rc, out = n.moe_combine(self._h.value if self._h else 0, topk_weights, self._tokens, self.hidden, out, None if stream is None else stream.cuda_stream)
+            rc, out = n.moe_combine(self._h.value if self._h else 0, self.top_k, topk_weights, self._tokens, self.hidden, out, None if stream is None else stream.cuda_stream)
             if rc:
                 check(rc, "HcclMoeCombine")
             return out
-        if out is None:
+        _need(topk_weights, self._tokens * self.top_k, "topk_weights")
+        if out is not None:
+            check_result(out, self._tokens * self.hidden, (torch.bfloat16,))
+        else:
             out = torch.empty((self._tokens, self.hidden), dtype=torch.bfloat16, device=topk_weights.device)
         s = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()) if stream is None else stream.cuda_stream
         check(_decl().HcclMoeCombine(self._h, topk_weights.data_ptr(), out.data_ptr(), self._tokens, s), "HcclMoeCombine")

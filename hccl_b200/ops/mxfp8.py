@@ -15,6 +15,7 @@ import torch
 
 from .._ext import ops as _native
 from .._lib import check, lib
+from .gemm import check_result
 
 
 @dataclass
@@ -60,6 +61,12 @@ def _check_quantizable(x: torch.Tensor) -> None:
         raise ValueError("quantize takes a contiguous 2-D bf16 CUDA tensor")
 
 
+def _need(t: MxTensor, rows: int, k: int) -> None:
+    for part, size, what in ((t.payload, rows * k, "payload"), (t.scales, scale_bytes(rows, k), "scales")):
+        if not (part.is_cuda and part.is_contiguous() and part.nbytes >= size):
+            raise ValueError(f"the {what} must be a contiguous CUDA tensor of at least {size} bytes")
+
+
 def quantize(x: torch.Tensor, out: Optional[MxTensor] = None, stream=None) -> MxTensor:
     """bf16 [rows, K] (K % 128 == 0) -> MxTensor, on the GPU."""
     _check_quantizable(x)
@@ -72,6 +79,8 @@ def quantize(x: torch.Tensor, out: Optional[MxTensor] = None, stream=None) -> Mx
         return MxTensor(payload, scales, rows, k) if out is None else out
     if out is None:
         out = empty_like_quantized(rows, k, x.device)
+    else:
+        _need(out, rows, k)
     check(_decl().HcclQuantizeMxfp8(x.data_ptr(), out.payload.data_ptr(), out.scales.data_ptr(), rows, k, _stream(stream)), "HcclQuantizeMxfp8")
     return out
 
@@ -141,15 +150,20 @@ def _one_rank(comm, a: torch.Tensor, w, out: Optional[torch.Tensor], stream) -> 
     """The three operators on one rank with activations in bf16: the product alone, quantisation in the same call."""
     _check_quantizable(a)
     w = _as_mx_fresh(w, stream)
+    if w.k != a.shape[1]:
+        raise ValueError(f"activations of {a.shape[1]} columns and a weight of {w.k}")
     n = _native()
     if n is not None:
         rc, out = n.mx_matmul(comm.handle, a, w.payload, w.scales, w.rows, out, None if stream is None else stream.cuda_stream)
         if rc:
             check(rc, "HcclQuantizeMatmulMxfp8")
         return out
-    buf = _act_buffer(a, stream)
     m, k = a.shape
-    if out is None:
+    _need(w, w.rows, k)
+    buf = _act_buffer(a, stream)
+    if out is not None:
+        check_result(out, m * w.rows, (torch.bfloat16,))
+    else:
         out = torch.empty((m, w.rows), dtype=torch.bfloat16, device=a.device)
     check(_decl().HcclQuantizeMatmulMxfp8(a.data_ptr(), buf.payload.data_ptr(), buf.scales.data_ptr(), w.payload.data_ptr(), w.scales.data_ptr(), out.data_ptr(), m, w.rows, k,
                                           comm.handle, _stream(stream)), "HcclQuantizeMatmulMxfp8")

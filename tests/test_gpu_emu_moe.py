@@ -240,6 +240,34 @@ def test_receive_views_belong_to_their_call():
         comm.destroy()
 
 
+def test_calls_that_the_host_refuses_leave_the_dispatcher_usable():
+    """Rows and results that are not 16-byte aligned (they move in such pieces) and a combine before the first dispatch are refused on the host, and the next call is right."""
+    from hccl_b200._lib import HcclError
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.ops.moe import MoeDispatcher
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        d = MoeDispatcher(comm, 8, 2, 256, 16, max_recv_rows=32)
+        x = torch.randn(16, 256, device="cuda").to(torch.bfloat16)
+        idx = torch.randint(0, 8, (16, 2), device="cuda", dtype=torch.int32)
+        weights = torch.rand(16, 2, device="cuda")
+        off = torch.empty(16 * 256 + 8, dtype=torch.bfloat16, device="cuda")[1:16 * 256 + 1].view(16, 256)
+        with pytest.raises(HcclError):
+            d.combine(weights)
+        with pytest.raises(HcclError):
+            d.dispatch(off.copy_(x), idx)
+        recv, _, counts, src = d.dispatch(x, idx)
+        assert torch.equal(recv[:32], x[src.long()]) and torch.equal(counts.long(), torch.bincount(idx.flatten().long(), minlength=8))
+        d.expert_out.copy_(recv)
+        with pytest.raises(HcclError):
+            d.combine(weights, out=off)
+        want = (x.double()[:, None] * weights.double()[..., None]).sum(1)
+        assert bool(((d.combine(weights).double() - want).abs() <= want.abs() * 2.0 ** -8 + x.double().abs() * 2.0 ** -21).all())
+        d.close()
+    finally:
+        comm.destroy()
+
+
 @pytest.mark.parametrize("T,E,K", [(1, 8, 1), (37, 16, 3), (700, 256, 8)])
 def test_one_rank_routing_table_that_is_not_16_byte_aligned(T, E, K):
     """The histogram reads four entries at a time where it can, one at a time from an address that does not allow it."""

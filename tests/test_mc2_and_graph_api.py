@@ -277,3 +277,40 @@ def test_fused_operators_check_shapes_and_results_on_the_host(native, monkeypatc
     else:
         with pytest.raises(ValueError, match="bf16 or fp32"):
             gemm.check_result(e(8, 23), 8 * 24, (torch.bfloat16, torch.float32))
+
+
+def test_block_scaled_and_moe_calls_check_their_memory_on_the_host():
+    """What the kernels read or write at an address has to be there: sizes, types and devices are errors before anything is launched (CPU tensors, as above)."""
+    from hccl_b200.ops import mxfp8
+
+    ext = mxfp8._native()
+    if ext is None:
+        pytest.skip("the extension is not built")
+    e = lambda *s, dt=torch.bfloat16: torch.empty(*s, dtype=dt)
+    byte = lambda *s: e(*s, dt=torch.uint8)
+    rows, n, k = 5, 24, 256
+    x, payload, scales = e(rows, k), byte(n, k), byte(mxfp8.scale_bytes(n, k))
+    for bad, match in (((e(rows, k, 1), payload, scales), "activations"), ((e(k, rows).t(), payload, scales), "activations"), ((e(rows, k, dt=torch.float16), payload, scales), "activations"),
+                       ((x, byte(n, k - 1), scales), "payload"), ((x, byte(k, n).t(), scales), "payload"), ((x, payload, scales[:-1]), "scales"),
+                       ((e(rows, 2 * k), payload, scales), "payload")):
+        with pytest.raises(ValueError, match=match):
+            ext.mx_matmul(0, *bad, n, None, None)
+    for out in (e(rows, n - 1), e(rows, n, dt=torch.float32), e(n, rows).t()):
+        with pytest.raises(ValueError, match="out must be a contiguous"):
+            ext.mx_matmul(0, x, payload, scales, n, out, None)
+    with pytest.raises(ValueError, match="CUDA"):
+        ext.mx_matmul(0, x, payload, scales, n, None, None)
+    good = byte(rows, k), byte(mxfp8.scale_bytes(rows, k))
+    for bad, match in (((byte(rows, k - 1), good[1]), "payload"), ((good[0], good[1][:-1]), "scales"), ((byte(k, rows).t(), good[1]), "payload"), (good, "CUDA")):
+        with pytest.raises(ValueError, match=match):
+            ext.mx_quantize(x, *bad, None)
+        with pytest.raises(ValueError):
+            mxfp8._need(mxfp8.MxTensor(*bad, rows, k), rows, k)
+    tokens, hidden, top_k = 6, 256, 2
+    xs, idx, weights = e(tokens, hidden), e(tokens, top_k, dt=torch.int32), e(tokens, top_k, dt=torch.float32)
+    for bad, match in (((e(tokens, hidden - 1), idx), "x must"), ((xs, idx[:, :1].contiguous()), "topk_idx"), ((xs, idx[:-1]), "topk_idx"), ((xs, idx), "CUDA")):
+        with pytest.raises(ValueError, match=match):
+            ext.moe_dispatch(0, top_k, hidden, *bad, None, (), ())
+    for bad, match in (((weights[:-1], None), "topk_weights"), ((weights, e(tokens, hidden - 1)), "out"), ((weights, e(tokens, hidden, dt=torch.float32)), "out"), ((weights, None), "CUDA")):
+        with pytest.raises(ValueError, match=match):
+            ext.moe_combine(0, top_k, bad[0], tokens, hidden, bad[1], None)
