@@ -57,6 +57,7 @@ inline TileChoice ChooseTile(uint64_t m, uint64_t n, uint64_t k, bool transposed
 // bt rows of A per tile (16, 32, 64, 128, 192, 256), split CTAs along K per tile (1 ... 8)
 struct SplitKChoice { uint32_t bt = 0, split = 0; };
 
+// The split-K rules below, their tables and their numbers of CTAs hold for the 148 SMs of a B200, whatever `sms` the tile rules are given: with fewer a choice is slower, not wrong.
 // Clusters of 1 ... 8 CTAs that run at once with one CTA on an SM: SMs come in groups that a cluster does not cross. Read off the step in time over
 // 967 products: with one cluster more than fit the product takes 1.4 times as long on average as with one CTA less along K.
 constexpr uint32_t kClustersAtOnce[9] = {0, 148, 71, 44, 33, 26, 22, 15, 15};

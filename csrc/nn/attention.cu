@@ -2,7 +2,8 @@
 // five products in one kernel. A small decoder is bound by launches and by what the host does around them: the library's backward pass, the transposed
 // rotary embedding and the views between them are six kernels and 130 us of host time per layer, this is one launch.
 //
-// Tiles of 64 queries and 64 keys, products by mma.sync (m16n8k16, bf16, 32-bit sums): at these sizes latency counts, not the tensor cores' rate. Scores,
+// Tiles of 64 queries and 64 keys, products by mma.sync (m16n8k16, bf16, 32-bit sums): at these sizes latency counts, not the tensor cores' rate (2 x 128 tokens of 8 heads: 48 CTAs, the tensor pipe 10 %
+// of the time on their SMs). Scores,
 // probabilities, their gradients' sums and all results stay in 32 bits; what an MMA reads is rounded to bf16 first, the rotated queries and keys as the rotary kernel
 // rounds them. No CTA waits for another and nothing is added by atomics: the gradient of a block of queries and that of a block of keys are found by
 // different CTAs of the launch, each of which computes its probabilities again from the forward pass's log-sums.

@@ -473,7 +473,8 @@ __global__ void __launch_bounds__(1024) MeanKernel(const float *__restrict__ row
 }
 
 // Gradient of an embedding by its few tokens: the block of a token that is the first of its id adds up the rows of all tokens with that id, in their order and in 32 bits.
-// Every block looks at all ids (16 KB at most), where the general way sorts them in some ten launches.
+// Every block looks at all ids (16 KB at most), where the general way sorts them in some ten launches. A common id is one block's walk over its rows, a load at a time: us a backward pass among others on
+// one B200, general / this, 2048 tokens of hidden 256 random 92 / 47, half of them one id 658 / 220, all 1288 / 438; hidden 4096 118 / 69, 1288 / 563, 2469 / 1063.
 constexpr uint32_t kEmbedTokens = 2048;
 __global__ void __launch_bounds__(kThreads) EmbeddingGradKernel(const int64_t *__restrict__ ids, const __nv_bfloat16 *__restrict__ dy, __nv_bfloat16 *__restrict__ grad, uint32_t T,
                                                                uint32_t H, int64_t V)

@@ -849,6 +849,22 @@ def test_embedding_gradient_of_few_tokens(tokens, hidden, vocab, native, monkeyp
         torch.autograd.grad(y, w, dy)
 
 
+@pytest.mark.parametrize("tokens,hidden,vocab,common", [(2, 8, 3, 2), (300, 264, 40, 280), (2048, 256, 512, 2048), (2048, 4096, 1000, 1500)])
+def test_embedding_gradient_of_a_common_id(tokens, hidden, vocab, common):
+    """A batch that is mostly one padding id, at its end: one block adds up its rows, in 32 bits and rounded once; rows of other ids and ids without a token as before."""
+    from hccl_b200.ops import block
+    _native_nodes()
+    g = torch.Generator(device="cuda").manual_seed(tokens + common)
+    w = torch.randn(vocab, hidden, generator=g, device="cuda").to(torch.bfloat16).requires_grad_()
+    ids = torch.randint(0, vocab, (tokens,), generator=g, device="cuda")
+    ids[tokens - common:] = vocab - 1
+    dy = torch.randn(tokens, hidden, generator=g, device="cuda").to(torch.bfloat16)
+    got, = torch.autograd.grad(block.embedding(w, ids), w, dy)
+    ref, mag = (torch.zeros(vocab, hidden, dtype=torch.float64, device="cuda").index_put((ids,), t, accumulate=True) for t in (dy.double(), dy.double().abs()))
+    _close(got, ref, mag, tokens)
+    assert not got[torch.bincount(ids, minlength=vocab) == 0].any()
+
+
 @pytest.mark.parametrize("rows,vocab", [(1, 1), (6, 24), (300, 1000), (1025, 515), (64, 128256)])
 def test_cross_entropy_of_one_rank(rows, vocab):
     """The loss against 64 bits, by the native node and the Python function alike: 32-bit sums over a row and over the rows."""
