@@ -494,20 +494,34 @@ py::object SwiGlu(py::handle guh, py::object plain)
     return py::cast(h);
 }
 
+// Gradients of a node that may keep a copy of its first input. The copy is then its second output: a gradient of the gradient finds its way to the caller's
+// tensor through it, and comes back here by itself.
+template <class F> variable_list WithCopy(bool copied, const variable_list &g, size_t inputs, F gradients)
+{
+    if (!copied || !g[1].defined()) return gradients();
+    variable_list out = g[0].defined() ? gradients() : variable_list(inputs);
+    out[0] = out[0].defined() ? out[0] + g[1] : g[1];
+    return out;
+}
+
 // ---- linear layers of one rank -------------------------------------------------------------------------------------------
 // y = x @ w^T. The column-parallel layer keeps the gathered activations, on one rank a copy of x unless the caller gives x away; the row-parallel one keeps x.
 struct LinearNode : OpNode {
     SavedVariable x, w;
     std::vector<int64_t> shape;
     at::TensorOptions options;
-    bool column = false;
+    bool column = false, copied = false;       // copied: x is the node's own copy, see WithCopy
     std::string name() const override { return column ? "_ColumnSeqParallelBackward" : "_RowSeqParallelBackward"; }
-    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(shape); }
-    std::vector<Saved> Keeps() override { return {{&x, false}, {&w, false}}; }
+    void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(shape); args.collect(copied); }
+    std::vector<Saved> Keeps() override { return {{&x, copied}, {&w, false}}; }
     variable_list Backward(variable_list &&g) override
     {
+        return WithCopy(copied, g, 2, [&] { return Gradients(g[0]); });
+    }
+    variable_list Gradients(const at::Tensor &incoming)
+    {
         const auto [xv, wv] = Unpack(x, w);
-        at::Tensor dy = ZerosWhereUndefined(g[0], shape, options);
+        at::Tensor dy = ZerosWhereUndefined(incoming, shape, options);
         bool direct = !traced && !at::GradMode::is_enabled() && g_nativeGemm && !g_nativeWgrad;
         {
             py::gil_scoped_acquire gil;
@@ -553,11 +567,12 @@ py::object Linear(py::handle xh, py::handle wh, py::object comm, uint64_t handle
         }
         if (wanted) {
             node->column = column;
-            node->x = SavedVariable(gathered.defined() ? gathered : x, false);
-            node->w = SavedVariable(w, false);
+            node->copied = gathered.defined();
             node->shape = y.sizes().vec();
             node->options = y.options();
-            torch::autograd::set_history({y}, node);
+            torch::autograd::set_history(node->copied ? variable_list{y, gathered} : variable_list{y}, node);
+            node->x = SavedVariable(node->copied ? gathered : x, node->copied);
+            node->w = SavedVariable(w, false);
         }
     }
     return py::cast(y);
@@ -570,17 +585,13 @@ struct MlpNode : OpNode {
     SavedVariable x, w, gu, h, wd;
     std::vector<int64_t> shape;
     at::TensorOptions options;
-    bool copied = false;                       // x is the node's own copy, its second output: a gradient of the gradient finds its way to the caller's x through it
+    bool copied = false;                       // x is the node's own copy, see WithCopy
     std::string name() const override { return "_SwiGluMlpBackward"; }
     void Constants(torch::dynamo::autograd::CompiledNodeArgs &args) const override { args.collect(shape); args.collect(copied); }
     std::vector<Saved> Keeps() override { return {{&x, copied}, {&w, false}, {&gu, false}, {&h, false}, {&wd, false}}; }
     variable_list Backward(variable_list &&g) override
     {
-        if (!copied) return Gradients(g[0]);
-        if (!g[0].defined() && g[1].defined()) return {g[1], at::Tensor(), at::Tensor()};
-        variable_list out = Gradients(g[0]);
-        if (g[1].defined()) out[0] = out[0].defined() ? out[0] + g[1] : g[1];
-        return out;
+        return WithCopy(copied, g, 3, [&] { return Gradients(g[0]); });
     }
     variable_list Gradients(const at::Tensor &incoming)
     {

@@ -166,8 +166,9 @@ def _row_backward(comm, x, w, dy_local):
 
 
 def _one_rank_backward(backward):
-    """The products by single operations where a tensor is a stand-in (a traced or batched one has no memory for the kernels)."""
-    return lambda comm, x, w, dy: backward(comm, x, w, dy) if all([_block._plain_tensor(t) for t in (x, w, dy)]) else (dy @ w, dy.t() @ x)
+    """The products by single operations where the gradient is itself differentiated, or a tensor is a stand-in (a traced or batched one has no memory for the kernels)."""
+    return lambda comm, x, w, dy: (backward(comm, x, w, dy) if not torch.is_grad_enabled() and all([_block._plain_tensor(t) for t in (x, w, dy)])
+                                   else (dy @ w, dy.t() @ x))
 
 
 _block.PYTHON_BACKWARD["column"] = _one_rank_backward(_column_backward)

@@ -670,6 +670,31 @@ def test_swiglu_layer_second_derivatives_reach_the_input(given):
         comm.destroy()
 
 
+@pytest.mark.parametrize("given", ["leaf", "tensor", "away"])
+@pytest.mark.parametrize("column", [True, False])
+def test_linear_layer_second_derivatives(column, given):
+    """The gradient of every first gradient of a one-rank linear layer by its input and weight, as of the SwiGLU layer: a product each way, four roundings to bf16 on both sides."""
+    from hccl_b200.comm import Communicator, get_root_info
+    from hccl_b200.parallel import tensor_parallel as tp
+    _native_nodes()
+    torch.zeros(1, device="cuda")
+    comm = Communicator.from_root_info(1, get_root_info(), 0)
+    try:
+        g = torch.Generator(device="cuda").manual_seed(3)
+        ins = [torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16).requires_grad_() for s in ((130, 64), (192, 64))]
+        up = torch.randn(130, 192, generator=g, device="cuda").to(torch.bfloat16)
+        x = ins[0] if given == "leaf" else ins[0] * 1
+        y = tp._one_rank_linear(x, ins[1], comm, column, given == "away")
+        got, plain = (torch.autograd.grad(t, ins, up, create_graph=True) for t in (y, ins[0] @ ins[1].t()))
+        for i, pair in enumerate(zip(got, plain)):
+            seconds = [torch.autograd.grad(t.float().square().sum(), ins, retain_graph=True, allow_unused=True) for t in pair]
+            for c, d in zip(*seconds):
+                assert (c is None) == (d is None), i
+                assert c is None or (c.double() - d.double()).norm() <= 4 * 2.0 ** -8 * d.double().norm(), i
+    finally:
+        comm.destroy()
+
+
 def _attention_case(batch, seq, heads, kv_heads, hd, seed=2):
     import functools
     from hccl_b200.models.llama import _plain_attention, _rope_tables
