@@ -68,7 +68,7 @@ _function_modes, _function_mode, _sdpa = torch._C._len_torch_function_stack, tor
 def _functions_watched() -> bool:
     """Whether a function mode has to see the operations that a caller writes as such (the attention, a residual addition, an index). The mode behind a default device
     changes where tensors are made and nothing else."""
-    return any(type(_function_mode(i)) is not DeviceContext for i in range(_function_modes()))
+    return _function_modes() > 0 and any(type(_function_mode(i)) is not DeviceContext for i in range(_function_modes()))
 
 
 def _plain_tensor(t) -> bool:
